@@ -367,6 +367,75 @@ template <int DIR> struct Dft<11, DIR> : DftOdd<11, DIR> {};
 template <int DIR> struct Dft<13, DIR> : DftOdd<13, DIR> {};
 template <int DIR> struct Dft<17, DIR> : DftOdd<17, DIR> {};
 
+// 9 = 3 x 3: 3-point DFTs over n2 of x[n1 + 3 n2], twiddles W9^(n1 k2),
+// 3-point DFTs over n1 -> X[k2 + 3 k1].
+template <int DIR>
+struct Dft<9, DIR> {
+  template <class E>
+  __device__ __forceinline__ static void run(E* v) {
+    const float sg = DIR < 0 ? -1.f : 1.f;
+    E y[3][3];
+#pragma unroll
+    for (int n1 = 0; n1 < 3; n1++) {
+      E t[3] = {v[n1], v[n1 + 3], v[n1 + 6]};
+      Dft<3, DIR>::run(t);
+#pragma unroll
+      for (int k2 = 0; k2 < 3; k2++) y[n1][k2] = t[k2];
+    }
+    // cos and sin of 2 pi m / 9, m = n1 k2 in {1, 2, 4}
+    y[1][1] = crot(y[1][1], 0.76604444311897803520f, sg, 0.64278760968653932632f);
+    y[1][2] = crot(y[1][2], 0.17364817766693034885f, sg, 0.98480775301220805937f);
+    y[2][1] = crot(y[2][1], 0.17364817766693034885f, sg, 0.98480775301220805937f);
+    y[2][2] = crot(y[2][2], -0.93969262078590838405f, sg, 0.34202014332566873304f);
+#pragma unroll
+    for (int k2 = 0; k2 < 3; k2++) {
+      E t[3] = {y[0][k2], y[1][k2], y[2][k2]};
+      Dft<3, DIR>::run(t);
+#pragma unroll
+      for (int k1 = 0; k1 < 3; k1++) v[k2 + 3 * k1] = t[k1];
+    }
+  }
+};
+
+// A x B points, A and B coprime (the prime factor algorithm): with the inputs
+// taken as n = (B n1 + A n2) mod AB the kernel exp(2 pi i n k / AB) splits into
+// exp(2 pi i n1 k / A) exp(2 pi i n2 k / B), so X[k] is the A x B 2-D DFT at
+// (k mod A, k mod B): no twiddles between the two stages.
+template <int A, int B, int DIR>
+struct DftCoprime {
+  // the index with residues (1, 0) resp. (0, 1): residues (k1, k2) are k1 e(1, 0) + k2 e(0, 1)
+  static constexpr int e(int k1, int k2) {
+    for (int k = 0; k < A * B; k++)
+      if (k % A == k1 && k % B == k2) return k;
+    return 0;
+  }
+  static constexpr int E1 = e(1, 0), E2 = e(0, 1);
+  template <class E>
+  __device__ __forceinline__ static void run(E* v) {
+    E y[A][B];
+#pragma unroll
+    for (int n2 = 0; n2 < B; n2++) {
+      E t[A];
+#pragma unroll
+      for (int n1 = 0; n1 < A; n1++) t[n1] = v[(B * n1 + A * n2) % (A * B)];
+      Dft<A, DIR>::run(t);
+#pragma unroll
+      for (int k1 = 0; k1 < A; k1++) y[k1][n2] = t[k1];
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < A; k1++) {
+      Dft<B, DIR>::run(y[k1]);
+#pragma unroll
+      for (int k2 = 0; k2 < B; k2++) v[(k1 * E1 + k2 * E2) % (A * B)] = y[k1][k2];
+    }
+  }
+};
+template <int DIR> struct Dft<6, DIR> : DftCoprime<2, 3, DIR> {};
+template <int DIR> struct Dft<10, DIR> : DftCoprime<2, 5, DIR> {};
+template <int DIR> struct Dft<12, DIR> : DftCoprime<4, 3, DIR> {};
+template <int DIR> struct Dft<14, DIR> : DftCoprime<2, 7, DIR> {};
+template <int DIR> struct Dft<18, DIR> : DftCoprime<2, 9, DIR> {};
+
 // ---------------------------------------------------------------------------
 // Radix plans per length (product of radices == N).
 // ---------------------------------------------------------------------------
@@ -375,17 +444,10 @@ struct RadixList {};
 
 template <int N>
 struct FftPlan;
-template <> struct FftPlan<16> { using type = RadixList<16>; };
-template <> struct FftPlan<24> { using type = RadixList<3, 8>; };
-template <> struct FftPlan<32> { using type = RadixList<4, 8>; };
-template <> struct FftPlan<48> { using type = RadixList<3, 16>; };
 template <> struct FftPlan<64> { using type = RadixList<8, 8>; };
-template <> struct FftPlan<72> { using type = RadixList<3, 3, 8>; };
-template <> struct FftPlan<144> { using type = RadixList<3, 3, 16>; };
 template <> struct FftPlan<96> { using type = RadixList<3, 4, 8>; };
 template <> struct FftPlan<128> { using type = RadixList<16, 8>; };
 template <> struct FftPlan<192> { using type = RadixList<3, 8, 8>; };
-template <> struct FftPlan<216> { using type = RadixList<3, 3, 3, 8>; };
 template <> struct FftPlan<256> { using type = RadixList<16, 16>; };
 template <> struct FftPlan<384> { using type = RadixList<3, 16, 8>; };
 template <> struct FftPlan<512> { using type = RadixList<8, 8, 8>; };

@@ -250,60 +250,74 @@ struct PyrWin {  // separable pyramid window of one level (device arrays v0..v2)
   const float* v1;
   const float* v2;
 };
-// One pass of a batched 3-D FFT with a fused prologue / epilogue
-// (k_vol3d_pass.cu).  Ranges along the two non-transformed axes select the
-// CTA's sequences: axis 2 (z rows): a = x, b = y; axis 1: a = x, b = z;
-// axis 0: a = y, b = z (b_n need not be a multiple of the 8-sequence group).
-enum { V3_LD_CPLX = 0, V3_LD_REAL = 1, V3_LD_PAIR = 2, V3_LD_MASKED = 3 };
-enum { V3_ST_CPLX = 0, V3_ST_REAL = 1, V3_ST_THRESH = 2, V3_ST_SPEC = 3, V3_ST_PAIR = 4 };
-struct V3Pass {
-  int axis = 2;
-  int D1 = 0, D2 = 0;             // work buffer dims 1, 2
-  int a_lo = 0, a_n = 0, b_lo = 0, b_n = 0;
-  int in_lo = 0, in_n = 0;        // loaded range along the axis (zero elsewhere)
-  int out_lo = 0, out_n = 0;      // stored range along the axis
-  size_t item_stride = 0;         // float2 per item of the work buffers
-  const float2* spec = nullptr;   // LD_PAIR / ST_SPEC: filter-pair spectrum (shared by the items)
-  const float* rsrc = nullptr;    // LD_REAL / LD_MASKED: real volume of a box
-  float* rdst = nullptr;          // ST_REAL / ST_THRESH / ST_PAIR: real volume of a box
-  float* rdst2 = nullptr;         // ST_PAIR: second band
-  size_t r_stride = 0;            // floats per item of rsrc / rdst
-  int r1 = 0, r2 = 0;             // box dims 1, 2
-  int o0 = 0, o1 = 0, o2 = 0;     // box origin in work-buffer coordinates
-  const uint8_t* mka = nullptr;   // LD_MASKED keep bits (linear bit order over the box)
-  const uint8_t* mkb = nullptr;
-  uint8_t* mwa = nullptr;         // ST_THRESH keep bits written
-  uint8_t* mwb = nullptr;
-  size_t m_stride = 0;            // mask bytes per item
-  const float* th = nullptr;      // ST_THRESH thresholds [item][nb_item]
-  int ia = 0, ib = -1, nb_item = 0;
-  float scale = 1.f;
-  int first = 0;                  // ST_SPEC: assign instead of accumulate
-  int m_r2 = 0;                   // keep-bit row pitch along dim 2 (0: r2), a multiple of 8 when r2 is not
+// Passes of the 3-D FFTs (vol3d_fft.cuh).  Complex volumes are item-strided
+// arrays whose axis 2 is contiguous; "lines" run along the transformed axis.
+enum { V3_LD_CPLX = 0, V3_LD_HP = 1, V3_LD_SYM = 2, V3_LD_MASKED = 3 };
+enum { V3_ST_CPLX = 0, V3_ST_REC = 1, V3_ST_THRESH = 2, V3_ST_PAIR = 3 };
+// One pass along axis 1 or 0: lines (a, z), a < an the other strided axis,
+// z < zn.  Element i of a line is at in + item in_item + pair in_pair +
+// a in_a + (i - in_lo) in_i + z for i in [in_lo, in_lo + in_n) and zero
+// elsewhere; outputs likewise.
+struct V3Cols {
+  const float2* in = nullptr;
+  float2* out = nullptr;
+  int items = 1, an = 0, zn = 0;
+  size_t in_item = 0, out_item = 0, in_pair = 0, out_pair = 0;
+  int in_a = 0, out_a = 0, in_i = 0, out_i = 0;
+  int in_lo = 0, in_n = 0, out_lo = 0, out_n = 0;
+  int sym_a = 0, sym_z = 0;        // LD_SYM: dims of axes a and 2 of the full spectrum
+  PyrWin win{};                    // LD_HP / ST_REC (axis 0)
+  const float2* lp = nullptr;      // ST_REC: the next level's half spectrum [s0][s1][s2p], item stride in_item
+  int s0 = 0, s1 = 0, s2p = 0;
+  float scale = 1.f;               // ST_REC: D^(N/2); ST_THRESH / ST_PAIR: the inverse's 1/N
+  // real box [.][r1][r2] of LD_MASKED (rsrc), ST_THRESH and ST_PAIR (rdst), axis 0
+  const float* rsrc = nullptr;
+  float* rdst = nullptr;
+  size_t r_stride = 0, band_stride = 0;
+  int r1 = 0, r2 = 0;
+  int pairs = 1, nbands = 0;       // launches that loop over the pairs of a chunk
+  uint8_t* mask = nullptr;         // keep bits of the chunk's first band (linear bit order, rows of m_r2 bits)
+  size_t m_stride = 0, m_band = 0; // bytes per item, per band
+  int m_r2 = 0;
+  const float* th = nullptr;       // thresholds of the chunk's first band, nb_item per item
+  int nb_item = 0;
+  int first = 1;                   // ST_THRESH: assign instead of add
 };
-bool v3_pass_len_supported(int n);
-// the lengths with the factors 11 and 17 (k_vol3d_pass_odd.cu)
-bool v3_pass_len_supported_odd(int n);
-cudaError_t prepare_v3_pass_odd(int n);
-cudaError_t launch_v3_pass_odd(int N, int dir, int ld, int st, float2* out, const float2* in, const V3Pass& P,
-                               const float2* tw, int nitems, cudaStream_t stream);
-cudaError_t prepare_v3_pass(int n);
-cudaError_t launch_v3_pass(int N, int dir, int ld, int st, float2* out, const float2* in, const V3Pass& P,
-                           const float2* tw, int nitems, cudaStream_t stream);
-cudaError_t launch_pad_real(const float* in, size_t in_stride, float2* out, size_t out_stride, int n, int m0, int m1,
-                            int m2, int L0, int L1, int L2, cudaStream_t st);
-cudaError_t launch_pad_edge(const float* in, size_t in_stride, float2* out, size_t out_stride, int n, int n0, int n1,
-                            int n2, int d0, int d1, int d2, cudaStream_t st);
-cudaError_t launch_crop_real(const float2* in, size_t in_stride, float* out, size_t out_stride, int n, int m0, int m1,
-                             int m2, int L1, int L2, int o0, int o1, int o2, float scale, cudaStream_t st);
-cudaError_t launch_half(const float2* in, size_t in_stride, float2* out, size_t out_stride, int n, int d0, int d1,
-                        int d2, cudaStream_t st);
-cudaError_t launch_conj_extend(const float2* in, size_t in_stride, float2* out, size_t out_stride, int n, int d0,
-                               int d1, int d2, cudaStream_t st);
-cudaError_t launch_pyr_dec(float2* Xh, size_t stride, float2* Lp, size_t lp_stride, int n, int d0, int d1, int d2,
-                           int s0, int s1, int s2, const PyrWin& w, float invDN, cudaStream_t st);
-cudaError_t launch_pyr_rec(float2* Hh, size_t stride, const float2* Lp, size_t lp_stride, int n, int d0, int d1,
-                           int d2, int s0, int s1, int s2, const PyrWin& w, float DN, cudaStream_t st);
+// Real rows <-> half spectra along axis 2: rows0 x rows1 rows; spectrum row
+// (x, y) at spec + item spec_stride + (x s1 + y) pitch.
+struct V3Real {
+  const float* src = nullptr;      // forward: n0 x n1 x n2, zero (or, edge: its last sample) beyond
+  float* dst = nullptr;            // inverse: rows0 x rows1 x n2, the first n2 samples of each line
+  float2* spec = nullptr;
+  size_t r_stride = 0, spec_stride = 0;
+  int rows0 = 0, rows1 = 0, n0 = 0, n1 = 0, n2 = 0, s1 = 0, pitch = 0, line = 0, edge = 0;
+  float scale = 1.f;
+};
+// The directional product along axis 2 (see k_v3_pair_inv / k_v3_pair_fwd).
+struct V3Pair {
+  const float2* Y = nullptr;       // half spectrum, rows of `pitch`
+  const float2* spec = nullptr;    // F_a + i F_b of the chunk's first pair, N0 N1 N2 per pair
+  float2* W = nullptr;             // [pair][item][N0][N1][wpitch], the box's z
+  float2* S = nullptr;             // full spectrum sum (adjoint)
+  size_t y_item = 0, w_item = 0, w_pair = 0, s_item = 0;
+  int N0 = 0, N1 = 0, pitch = 0, wpitch = 0, z_lo = 0, z_n = 0, pairs = 0, items = 1, first = 1;
+};
+// Launchers of one transform length; `pyr`: usable by the pyramid, `conv`: by
+// the directional stage.  cols returns cudaErrorInvalidValue for a
+// combination that the length does not have.
+struct V3Ops {
+  cudaError_t (*real)(int dir, const V3Real&, const float2* tw, int items, cudaStream_t);
+  cudaError_t (*cols)(int dir, int ld, int st, const V3Cols&, const float2* tw, int npairs, cudaStream_t);
+  cudaError_t (*pair)(int dir, const V3Pair&, const float2* tw, int shares, cudaStream_t);
+  bool pyr, conv;
+};
+const V3Ops* v3_ops(int n);  // nullptr: length not compiled
+const V3Ops* v3_ops_mid(int n);
+const V3Ops* v3_ops_large(int n);
+const V3Ops* v3_ops_grid(int n);
+inline int v3_pitch(int n) { return (n + 3) / 4 * 4; }  // rows of whole 32-byte sectors
+cudaError_t launch_pyr_dec_lp(const float2* Xh, float2* Lp, size_t stride, int n, int d1, int pitch, int s0, int s1,
+                              int s2, const PyrWin& w, float invDN, cudaStream_t st);
 cudaError_t launch_fold_edge(const float* g, size_t g_stride, float* out, size_t o_stride, float* scratch,
                              size_t s_stride, int n, int n0, int n1, int n2, int d0, int d1, int d2, cudaStream_t st);
 std::vector<double> meyer_filters_3d(int cube, int nlevels, const int* num_dirs);

@@ -10,10 +10,12 @@
 // caller's stream over all volumes of the batch at once.
 //
 // Pipeline of one level of the directional stage (convnfft.m:79-201, 'same'):
-//   Y = FFT3(zero-pad(BP_l, Lc))            once per level
+//   Y = FFT3(zero-pad(BP_l, Lc))            once per level, half spectrum
 //   W = F_a .* Y + i F_b .* Y               two real filters per complex IFFT
 //   IFFT3(W); real part -> band a, imaginary part -> band b, cropped at
 //   offset ceil((24-1)/2) = 12; hard threshold and band sum (ShRec.m:11-24).
+// All band pairs of a level go through each of the inverse's three passes in
+// one launch (in chunks, where the plan's work buffer does not hold them all).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -32,6 +34,10 @@ namespace {
 constexpr int kCube = 24;          // Meyer filter support (GetMeyerBasedFilter.m:18)
 constexpr int kSameOff = 12;       // convnfft 'same' offset: ceil((24 - 1) / 2)
 constexpr int kMaxGrid = 192;      // largest padded grid per dimension
+constexpr int kSmCount = 152;
+constexpr int kCtasPerSm = 8;      // CTAs per SM that keep the z product pass's loads in flight
+// Band pairs in flight per level: the work buffer holds as many as fit here (at least one).
+constexpr size_t kPairBytes = (size_t)1 << 30;
 const int kFftLens[] = {16, 24, 32, 48, 64, 72, 96, 128, 144, 192, 216, 256};
 
 bool is_fft_len(int n) {
@@ -159,6 +165,7 @@ int host_threads3() {
 }
 
 size_t align_up3(size_t v, size_t a) { return (v + a - 1) / a * a; }
+size_t mask_band_bytes(const int* m) { return align_up3((size_t)m[0] * m[1] * mask_pitch(m[2]) / 8, 256); }
 
 }  // namespace
 
@@ -179,16 +186,20 @@ struct nsst3_plan {
     int K[3] = {0, 0, 0};   // window support of the decomposition step (levels < L)
     size_t win_off[3] = {0, 0, 0};
     size_t vol() const { return (size_t)m[0] * m[1] * m[2]; }
-    size_t half() const { return (size_t)m[0] * m[1] * (m[2] / 2 + 1); }
+    size_t half() const { return (size_t)m[0] * m[1] * v3_pitch(m[2] / 2 + 1); }
     size_t conv() const { return (size_t)lc[0] * lc[1] * lc[2]; }
+    // one band pair's partly inverted spectrum: the box's z kept
+    size_t pair() const { return (size_t)lc[0] * lc[1] * v3_pitch(m[2]); }
+    int npairs() const { return (nb + 1) / 2; }
   };
   std::vector<Level> lev;  // L + 1 entries
   std::vector<int> band_level, band_cone, band_l2, band_l1;
 
   size_t bp_floats = 0;    // sub-band layout per volume
-  size_t vol_elems = 0;    // complex scratch volume per item (grid)
+  size_t vol_elems = 0;    // voxels of the grid
   size_t xh_elems = 0;     // half spectra of every level per item
-  size_t conv_elems = 0;   // largest convolution volume
+  size_t conv_elems = 0;   // largest convolution spectrum
+  size_t wk_elems = 0;     // band-pair work buffer (all items)
   size_t in_elems = 0;     // n0 n1 n2
 
   char* arena = nullptr;
@@ -197,7 +208,6 @@ struct nsst3_plan {
   float* win = nullptr;
   float2* tw = nullptr;
   std::map<int, size_t> tw_off;  // transform length -> offset (float2) in tw
-  float2* vol = nullptr;
   float2* xh = nullptr;
   float2* Y = nullptr;
   float2* Wk = nullptr;
@@ -221,78 +231,80 @@ struct nsst3_plan {
 
 namespace {
 
-// Pass descriptors.  A pass transforms `axis`; (a, b) select the sequences
-// (axis 2: x, y; axis 1: x, z; axis 0: y, z), `in` the loaded index range and
-// `out` the stored one.
+// Strides of a line pass along `axis` (1 or 0) in an array d0 x d1 x pitch.
+void set_axis(V3Cols& P, int axis, int d1, int pitch) {
+  P.in_a = P.out_a = axis == 1 ? d1 * pitch : pitch;
+  P.in_i = P.out_i = axis == 1 ? pitch : d1 * pitch;
+}
+// A pass along `axis` of n items in place on v (d0 x d1 x pitch, item stride
+// `stride`): lines (a < an, z < zn), elements [in] loaded, [out] stored, both
+// ranges kept at the start of the line.
 struct Range {
   int lo, n;
 };
-V3Pass make_pass(int axis, const int* D, size_t stride, Range a, Range b, Range in, Range out) {
-  V3Pass P;
-  P.axis = axis;
-  P.D1 = D[1];
-  P.D2 = D[2];
-  P.a_lo = a.lo, P.a_n = a.n, P.b_lo = b.lo, P.b_n = b.n;
+V3Cols line_pass(int axis, float2* v, size_t stride, int d1, int pitch, int n, int an, int zn, Range in, Range out) {
+  V3Cols P;
+  P.in = v;
+  P.out = v;
+  P.items = n, P.an = an, P.zn = zn;
+  P.in_item = P.out_item = stride;
+  set_axis(P, axis, d1, pitch);
   P.in_lo = in.lo, P.in_n = in.n, P.out_lo = out.lo, P.out_n = out.n;
-  P.item_stride = stride;
   return P;
 }
-void set_box(V3Pass& P, const int* m, int o) {
-  P.r1 = m[1];
-  P.r2 = m[2];
-  P.o0 = P.o1 = P.o2 = o;
-}
-
-nsst_status run_pass(nsst3_plan* p, const V3Pass& P, int dir, int ld, int st_mode, float2* out, const float2* in,
-                     int D_axis, int n, cudaStream_t st) {
-  V3_CUDA(launch_v3_pass(D_axis, dir, ld, st_mode, out, in, P, p->twid(D_axis), n, st));
+nsst_status run_cols(nsst3_plan* p, int len, int dir, int ld, int st_mode, const V3Cols& P, int npairs,
+                     cudaStream_t st) {
+  V3_CUDA(v3_ops(len)->cols(dir, ld, st_mode, P, p->twid(len), npairs, st));
   return NSST_OK;
 }
 
-// Batched full 3-D FFT of n complex volumes d0 x d1 x d2 (item stride
-// `stride`), in place: axis 2, then 1, then 0; unnormalised.
-nsst_status fft3(nsst3_plan* p, float2* v, size_t stride, int n, const int* d, int dir, cudaStream_t st) {
-  V3_TRY(run_pass(p, make_pass(2, d, stride, {0, d[0]}, {0, d[1]}, {0, d[2]}, {0, d[2]}), dir, V3_LD_CPLX, V3_ST_CPLX,
-                  v, v, d[2], n, st));
-  V3_TRY(run_pass(p, make_pass(1, d, stride, {0, d[0]}, {0, d[2]}, {0, d[1]}, {0, d[1]}), dir, V3_LD_CPLX, V3_ST_CPLX,
-                  v, v, d[1], n, st));
-  V3_TRY(run_pass(p, make_pass(0, d, stride, {0, d[1]}, {0, d[2]}, {0, d[0]}, {0, d[0]}), dir, V3_LD_CPLX, V3_ST_CPLX,
-                  v, v, d[0], n, st));
-  return NSST_OK;
+// Forward FFT of n real volumes m (item stride rstride floats, dims src[3];
+// beyond them zero or, edge, the last sample repeated) on a grid d: half
+// spectra d0 x d1 x pitch(d2/2 + 1) in h.  rec: the axis-0 pass merges the next
+// level's half spectrum (ST_REC fields set by the caller in *rec).
+nsst_status fft3_real(nsst3_plan* p, const float* x, size_t rstride, const int* src, bool edge, const int* m,
+                      float2* h, size_t stride, const int* d, int n, cudaStream_t st, const V3Cols* rec = nullptr) {
+  const int H = d[2] / 2 + 1, pitch = v3_pitch(H);
+  V3Real R;
+  R.src = x;
+  R.spec = h;
+  R.r_stride = rstride, R.spec_stride = stride;
+  R.rows0 = m[0], R.rows1 = m[1];
+  R.n0 = src[0], R.n1 = src[1], R.n2 = src[2];
+  R.s1 = d[1], R.pitch = pitch, R.line = d[2], R.edge = edge;
+  V3_CUDA(v3_ops(d[2])->real(-1, R, p->twid(d[2]), n, st));
+  V3_TRY(run_cols(p, d[1], -1, V3_LD_CPLX, V3_ST_CPLX,
+                  line_pass(1, h, stride, d[1], pitch, n, m[0], H, {0, m[1]}, {0, d[1]}), 1, st));
+  V3Cols P = line_pass(0, h, stride, d[1], pitch, n, d[1], H, {0, m[0]}, {0, d[0]});
+  if (rec) {
+    P.win = rec->win;
+    P.lp = rec->lp;
+    P.s0 = rec->s0, P.s1 = rec->s1, P.s2p = rec->s2p;
+    P.scale = rec->scale;
+  }
+  return run_cols(p, d[0], -1, V3_LD_CPLX, rec ? V3_ST_REC : V3_ST_CPLX, P, 1, st);
 }
 
-// Forward FFT of real volumes of dims m (item stride rstride floats) zero
-// padded at the origin to the complex buffer v of dims d: the passes read
-// only the non-zero part.
-nsst_status fft3_real(nsst3_plan* p, const float* x, size_t rstride, const int* m, float2* v, size_t stride,
-                      const int* d, int n, cudaStream_t st) {
-  V3Pass P = make_pass(2, d, stride, {0, m[0]}, {0, m[1]}, {0, m[2]}, {0, d[2]});
-  P.rsrc = x;
-  P.r_stride = rstride;
-  set_box(P, m, 0);
-  V3_TRY(run_pass(p, P, -1, V3_LD_REAL, V3_ST_CPLX, v, v, d[2], n, st));
-  V3_TRY(run_pass(p, make_pass(1, d, stride, {0, m[0]}, {0, d[2]}, {0, m[1]}, {0, d[1]}), -1, V3_LD_CPLX, V3_ST_CPLX,
-                  v, v, d[1], n, st));
-  V3_TRY(run_pass(p, make_pass(0, d, stride, {0, d[1]}, {0, d[2]}, {0, m[0]}, {0, d[0]}), -1, V3_LD_CPLX, V3_ST_CPLX,
-                  v, v, d[0], n, st));
+// Inverse FFT of half spectra in h (grid d, destroyed) whose first out[k]
+// samples per axis, times scale, go to the real volumes x.  hp: the axis-0
+// pass first applies the level's high-pass window.
+nsst_status ifft3_real(nsst3_plan* p, float2* h, size_t stride, const int* d, float* x, size_t rstride,
+                       const int* out, float scale, int n, cudaStream_t st, const PyrWin* hp = nullptr) {
+  const int H = d[2] / 2 + 1, pitch = v3_pitch(H);
+  V3Cols P = line_pass(0, h, stride, d[1], pitch, n, d[1], H, {0, d[0]}, {0, out[0]});
+  if (hp) P.win = *hp;
+  V3_TRY(run_cols(p, d[0], +1, hp ? V3_LD_HP : V3_LD_CPLX, V3_ST_CPLX, P, 1, st));
+  V3_TRY(run_cols(p, d[1], +1, V3_LD_CPLX, V3_ST_CPLX,
+                  line_pass(1, h, stride, d[1], pitch, n, out[0], H, {0, d[1]}, {0, out[1]}), 1, st));
+  V3Real R;
+  R.dst = x;
+  R.spec = h;
+  R.r_stride = rstride, R.spec_stride = stride;
+  R.rows0 = out[0], R.rows1 = out[1], R.n2 = out[2];
+  R.s1 = d[1], R.pitch = pitch, R.line = d[2];
+  R.scale = scale;
+  V3_CUDA(v3_ops(d[2])->real(+1, R, p->twid(d[2]), n, st));
   return NSST_OK;
-}
-
-// Inverse FFT of the complex buffer v (dims d) whose real part, times scale,
-// is wanted only in the box [o, o + m) of each axis: later passes skip the
-// sequences outside the box, the last one writes the real box to x.
-nsst_status ifft3_real_box(nsst3_plan* p, float2* v, size_t stride, const int* d, const int* m, int o, float* x,
-                           size_t rstride, float scale, int n, cudaStream_t st) {
-  V3_TRY(run_pass(p, make_pass(2, d, stride, {0, d[0]}, {0, d[1]}, {0, d[2]}, {o, m[2]}), +1, V3_LD_CPLX, V3_ST_CPLX,
-                  v, v, d[2], n, st));
-  V3_TRY(run_pass(p, make_pass(1, d, stride, {0, d[0]}, {o, m[2]}, {0, d[1]}, {o, m[1]}), +1, V3_LD_CPLX, V3_ST_CPLX,
-                  v, v, d[1], n, st));
-  V3Pass P = make_pass(0, d, stride, {o, m[1]}, {o, m[2]}, {0, d[0]}, {o, m[0]});
-  P.rdst = x;
-  P.r_stride = rstride;
-  P.scale = scale;
-  set_box(P, m, o);
-  return run_pass(p, P, +1, V3_LD_CPLX, V3_ST_REAL, v, v, d[0], n, st);
 }
 
 PyrWin level_window(const nsst3_plan* p, int l) {
@@ -314,25 +326,20 @@ PyrWin level_window(const nsst3_plan* p, int l) {
 nsst_status run_pyr_dec(nsst3_plan* p, const float* x, const int* in, float* bp, int n, cudaStream_t st,
                         bool zero_pad = false) {
   const size_t xs = (size_t)in[0] * in[1] * in[2];
-  const nsst3_plan::Level& l0 = p->lev[0];
-  if (zero_pad)
-    V3_CUDA(launch_pad_real(x, xs, p->vol, p->vol_elems, n, in[0], in[1], in[2], p->g[0], p->g[1], p->g[2], st));
-  else
-    V3_CUDA(launch_pad_edge(x, xs, p->vol, p->vol_elems, n, in[0], in[1], in[2], p->g[0], p->g[1], p->g[2], st));
-  V3_TRY(fft3(p, p->vol, p->vol_elems, n, p->g, -1, st));
-  V3_CUDA(launch_half(p->vol, p->vol_elems, p->xh + l0.xh_off, p->xh_elems, n, p->g[0], p->g[1], p->g[2], st));
+  V3_TRY(fft3_real(p, x, xs, in, !zero_pad, p->g, p->xh + p->lev[0].xh_off, p->xh_elems, p->g, n, st));
   for (int l = 0; l <= p->L; l++) {
     const nsst3_plan::Level& a = p->lev[l];
+    PyrWin win;
     if (l < p->L) {
+      // PrySDdec_onestep.m:82-125: Lp into the next level's block; Hp in the inverse's first pass
       const nsst3_plan::Level& b = p->lev[l + 1];
-      // PrySDdec_onestep.m:82-125: Lp into the next level's block, Hp in place
-      V3_CUDA(launch_pyr_dec(p->xh + a.xh_off, p->xh_elems, p->xh + b.xh_off, p->xh_elems, n, a.m[0], a.m[1], a.m[2],
-                             b.m[0], b.m[1], b.m[2], level_window(p, l), (float)(1.0 / std::pow(p->D[l], 1.5)), st));
+      win = level_window(p, l);
+      V3_CUDA(launch_pyr_dec_lp(p->xh + a.xh_off, p->xh + b.xh_off, p->xh_elems, n, a.m[1], v3_pitch(a.m[2] / 2 + 1),
+                                b.m[0], b.m[1], b.m[2], win, (float)(1.0 / std::pow(p->D[l], 1.5)), st));
     }
     // subs{l} = real(ifftn(ccsym(Hp, 3, 'e')))   (lowpass: the last Lp)
-    V3_CUDA(launch_conj_extend(p->xh + a.xh_off, p->xh_elems, p->vol, p->vol_elems, n, a.m[0], a.m[1], a.m[2], st));
-    V3_TRY(ifft3_real_box(p, p->vol, p->vol_elems, a.m, a.m, 0, bp + a.bp_off, p->bp_floats,
-                          (float)(1.0 / (double)a.vol()), n, st));
+    V3_TRY(ifft3_real(p, p->xh + a.xh_off, p->xh_elems, a.m, bp + a.bp_off, p->bp_floats, a.m,
+                      (float)(1.0 / (double)a.vol()), n, st, l < p->L ? &win : nullptr));
   }
   return NSST_OK;
 }
@@ -341,22 +348,52 @@ nsst_status run_pyr_dec(nsst3_plan* p, const float* x, const int* in, float* bp,
 nsst_status run_pyr_rec(nsst3_plan* p, const float* bp, float* x, const int* out, int n, cudaStream_t st) {
   for (int l = p->L; l >= 0; l--) {
     const nsst3_plan::Level& a = p->lev[l];
-    // ccsym(fftn(subs{l}), 3, 'c')
-    V3_TRY(fft3_real(p, bp + a.bp_off, p->bp_floats, a.m, p->vol, p->vol_elems, a.m, n, st));
-    V3_CUDA(launch_half(p->vol, p->vol_elems, p->xh + a.xh_off, p->xh_elems, n, a.m[0], a.m[1], a.m[2], st));
-    if (l < p->L) {
+    V3Cols rec;
+    if (l < p->L) {  // PrySDrec_onestep.m:96-119
       const nsst3_plan::Level& b = p->lev[l + 1];
-      // PrySDrec_onestep.m:96-119, in place over Hp
-      V3_CUDA(launch_pyr_rec(p->xh + a.xh_off, p->xh_elems, p->xh + b.xh_off, p->xh_elems, n, a.m[0], a.m[1], a.m[2],
-                             b.m[0], b.m[1], b.m[2], level_window(p, l), (float)std::pow(p->D[l], 1.5), st));
+      rec.win = level_window(p, l);
+      rec.lp = p->xh + b.xh_off;
+      rec.s0 = b.m[0], rec.s1 = b.m[1], rec.s2p = v3_pitch(b.m[2] / 2 + 1);
+      rec.scale = (float)std::pow(p->D[l], 1.5);
     }
+    // ccsym(fftn(subs{l}), 3, 'c')
+    V3_TRY(fft3_real(p, bp + a.bp_off, p->bp_floats, a.m, false, a.m, p->xh + a.xh_off, p->xh_elems, a.m, n, st,
+                     l < p->L ? &rec : nullptr));
   }
   const nsst3_plan::Level& l0 = p->lev[0];
-  V3_CUDA(launch_conj_extend(p->xh + l0.xh_off, p->xh_elems, p->vol, p->vol_elems, n, p->g[0], p->g[1], p->g[2], st));
-  V3_TRY(fft3(p, p->vol, p->vol_elems, n, p->g, +1, st));
-  V3_CUDA(launch_crop_real(p->vol, p->vol_elems, x, (size_t)out[0] * out[1] * out[2], n, out[0], out[1], out[2],
-                           p->g[1], p->g[2], 0, 0, 0, (float)(1.0 / (double)l0.vol()), st));
-  return NSST_OK;
+  return ifft3_real(p, p->xh + l0.xh_off, p->xh_elems, p->g, x, (size_t)out[0] * out[1] * out[2], out,
+                    (float)(1.0 / (double)l0.vol()), n, st);
+}
+
+// Pairs of a level that one pass over the work buffer takes for n items.
+int pair_chunk(const nsst3_plan* p, const nsst3_plan::Level& a, int n) {
+  return (int)std::max<size_t>(1, std::min<size_t>(a.npairs(), p->wk_elems / (a.pair() * n)));
+}
+// Keep bits of the level's bands from band k on.
+void set_masks(const nsst3_plan* p, V3Cols& P, int l, int k) {
+  const nsst3_plan::Level& a = p->lev[l];
+  P.m_r2 = mask_pitch(a.m[2]);
+  P.m_band = mask_band_bytes(a.m);
+  P.m_stride = p->mask_bytes;
+  P.mask = p->mask + p->mask_off[a.first_band] + (size_t)k * P.m_band;
+}
+V3Pair pair_pass(const nsst3_plan* p, const nsst3_plan::Level& a, int k0, int pairs, int n) {
+  V3Pair P;
+  P.spec = p->spec + a.spec_off + (size_t)k0 * a.conv();
+  P.W = p->Wk;
+  P.w_item = a.pair();
+  P.w_pair = a.pair() * n;
+  P.N0 = a.lc[0], P.N1 = a.lc[1];
+  P.wpitch = v3_pitch(a.m[2]);
+  P.z_lo = kSameOff, P.z_n = a.m[2];
+  P.pairs = pairs, P.items = n;
+  return P;
+}
+// The chunk's pass along axis 1 in the work buffer, in place.
+V3Cols pair_cols(const nsst3_plan* p, const nsst3_plan::Level& a, int n, Range in, Range out) {
+  V3Cols P = line_pass(1, p->Wk, a.pair(), a.lc[1], v3_pitch(a.m[2]), n, a.lc[0], a.m[2], in, out);
+  P.in_pair = P.out_pair = a.pair() * n;
+  return P;
 }
 
 // Directional stage of one level.  Y = FFT3(zero-pad(bp_l)) once; per band
@@ -370,42 +407,40 @@ nsst_status run_sh_level(nsst3_plan* p, const float* bp, int l, float* acc, cons
   const nsst3_plan::Level& a = p->lev[l];
   const int* N = a.lc;
   const int* m = a.m;
-  const int o = kSameOff;
-  const size_t cs = p->conv_elems;
-  V3_TRY(fft3_real(p, bp + a.bp_off, p->bp_floats, m, p->Y, cs, N, n, st));
-  const float scale = (float)(1.0 / (double)a.conv());
-  for (int k = 0; k < a.nb; k += 2) {
-    const int ba = a.first_band + k;
-    const int bb = k + 1 < a.nb ? ba + 1 : -1;
-    const float2* C = p->spec + a.spec_off + (size_t)(k / 2) * a.conv();
+  const int wp = v3_pitch(m[2]);
+  V3_TRY(fft3_real(p, bp + a.bp_off, p->bp_floats, m, false, m, p->Y, p->conv_elems, N, n, st));
+  const int chunk = pair_chunk(p, a, n);
+  for (int k0 = 0; k0 < a.npairs(); k0 += chunk) {
+    const int pairs = std::min(chunk, a.npairs() - k0);
     // z rows: the product, stored only where the box needs it
-    V3Pass P1 = make_pass(2, N, cs, {0, N[0]}, {0, N[1]}, {0, N[2]}, {o, m[2]});
-    P1.spec = C;
-    V3_TRY(run_pass(p, P1, +1, V3_LD_PAIR, V3_ST_CPLX, p->Wk, p->Y, N[2], n, st));
-    V3_TRY(run_pass(p, make_pass(1, N, cs, {0, N[0]}, {o, m[2]}, {0, N[1]}, {o, m[1]}), +1, V3_LD_CPLX, V3_ST_CPLX,
-                    p->Wk, p->Wk, N[1], n, st));
-    V3Pass P3 = make_pass(0, N, cs, {o, m[1]}, {o, m[2]}, {0, N[0]}, {o, m[0]});
-    set_box(P3, m, o);
-    P3.r_stride = p->bp_floats;
-    P3.scale = scale;
+    V3Pair P1 = pair_pass(p, a, k0, pairs, n);
+    P1.Y = p->Y;
+    P1.y_item = p->conv_elems;
+    P1.pitch = v3_pitch(N[2] / 2 + 1);
+    // the CTAs loop over the pairs, so that Y is read once, as far as the grid still fills the GPU
+    const int ctas = (N[0] * N[1] + 7) / 8 * n;
+    const int shares = std::min(pairs, std::max(1, (kSmCount * kCtasPerSm + ctas - 1) / ctas));
+    V3_CUDA(v3_ops(N[2])->pair(+1, P1, p->twid(N[2]), shares, st));
+    V3_TRY(run_cols(p, N[1], +1, V3_LD_CPLX, V3_ST_CPLX, pair_cols(p, a, n, {0, N[1]}, {kSameOff, m[1]}), pairs, st));
+    V3Cols P3 = line_pass(0, p->Wk, a.pair(), N[1], wp, n, m[1], m[2], {0, N[0]}, {kSameOff, m[0]});
+    P3.in_pair = a.pair() * n;
+    P3.pairs = pairs;
+    P3.nbands = a.nb - 2 * k0;
+    P3.scale = (float)(1.0 / (double)a.conv());
+    P3.r1 = m[1], P3.r2 = m[2];
     if (acc) {
       P3.rdst = acc + a.bp_off;
-      P3.th = th;
-      P3.ia = ba;
-      P3.ib = bb;
+      P3.r_stride = p->bp_floats;
+      P3.th = th ? th + a.first_band + 2 * k0 : nullptr;
       P3.nb_item = p->nbands;
-      if (record_masks) {
-        P3.m_r2 = mask_pitch(m[2]);
-        P3.mwa = p->mask + p->mask_off[ba];
-        P3.mwb = bb >= 0 ? p->mask + p->mask_off[bb] : nullptr;
-        P3.m_stride = p->mask_bytes;
-      }
-      V3_TRY(run_pass(p, P3, +1, V3_LD_CPLX, V3_ST_THRESH, p->Wk, p->Wk, N[0], n, st));
+      P3.first = k0 == 0;
+      if (record_masks) set_masks(p, P3, l, 2 * k0);
+      V3_TRY(run_cols(p, N[0], +1, V3_LD_CPLX, V3_ST_THRESH, P3, 1, st));
     } else {
-      P3.rdst = coeffs + (size_t)k * a.vol();
-      P3.rdst2 = bb >= 0 ? P3.rdst + a.vol() : nullptr;
+      P3.rdst = coeffs + (size_t)(2 * k0) * a.vol();
       P3.r_stride = (size_t)a.nb * a.vol();
-      V3_TRY(run_pass(p, P3, +1, V3_LD_CPLX, V3_ST_PAIR, p->Wk, p->Wk, N[0], n, st));
+      P3.band_stride = a.vol();
+      V3_TRY(run_cols(p, N[0], +1, V3_LD_CPLX, V3_ST_PAIR, P3, 1, st));
     }
   }
   return NSST_OK;
@@ -432,8 +467,13 @@ nsst_status upload_th(nsst3_plan* p, int n, const double* sigma, const double* T
 // bands; lowpass copied from bp.
 nsst_status run_dec_thresh_rec(nsst3_plan* p, const float* bp, float* rec, int n, const float* th, cudaStream_t st,
                                bool record_masks = false) {
-  V3_CUDA(cudaMemsetAsync(rec, 0, (size_t)n * p->bp_floats * sizeof(float), st));
   for (int l = 0; l < p->L; l++) V3_TRY(run_sh_level(p, bp, l, rec, th, nullptr, n, st, record_masks));
+  // the layout's alignment gaps read as zero
+  for (const nsst3_plan::Level& a : p->lev) {
+    const size_t gap = align_up3(a.vol(), 64) - a.vol();
+    if (gap)
+      V3_CUDA(cudaMemset2DAsync(rec + a.bp_off + a.vol(), p->bp_floats * sizeof(float), 0, gap * sizeof(float), n, st));
+  }
   const nsst3_plan::Level& lp = p->lev[p->L];
   V3_CUDA(cudaMemcpy2DAsync(rec + lp.bp_off, p->bp_floats * sizeof(float), bp + lp.bp_off,
                             p->bp_floats * sizeof(float), lp.vol() * sizeof(float), n, cudaMemcpyDeviceToDevice, st));
@@ -536,6 +576,14 @@ nsst_status nsst3_plan_create(const nsst3_config* cfg, int n0, int n1, int n2, i
     spec_off += (size_t)((a.nb + 1) / 2) * a.conv();  // one spectrum F_a + i F_b per band pair
     p->conv_elems = std::max(p->conv_elems, a.conv());
   }
+  for (int l = 0; l < p->L; l++) {
+    const nsst3_plan::Level& a = p->lev[l];
+    const size_t one = a.pair() * batch;
+    const size_t fit = std::max<size_t>(1, kPairBytes / (one * sizeof(float2)));
+    p->wk_elems = std::max(p->wk_elems, one * std::min<size_t>(a.npairs(), fit));
+    // the backward's half spectra of S and its fold scratch live there too
+    p->wk_elems = std::max(p->wk_elems, (size_t)a.m[0] * a.lc[1] * v3_pitch(a.lc[2] / 2 + 1) * batch);
+  }
   p->bp_floats = bp_off;
   p->xh_elems = xh_off;
   p->vol_elems = (size_t)p->g[0] * p->g[1] * p->g[2];
@@ -569,12 +617,10 @@ nsst_status nsst3_plan_create(const nsst3_config* cfg, int n0, int n1, int n2, i
     for (int k = 0; k < 3; k++) {
       add_tw(p->lev[l].m[k]);
       if (l < p->L) add_tw(p->lev[l].lc[k]);
+      const V3Ops *om = v3_ops(p->lev[l].m[k]), *oc = l < p->L ? v3_ops(p->lev[l].lc[k]) : nullptr;
+      if (!om || !om->pyr || (l < p->L && (!oc || !oc->conv)))
+        return fail3(NSST_ERR_UNSUPPORTED_SIZE, "volume transform length not compiled");
     }
-  for (auto& kv : p->tw_off) {
-    cudaError_t e = prepare_v3_pass(kv.first);
-    if (e != cudaSuccess) return cuda_fail3(e, "prepare_v3_pass");
-  }
-
   // one device arena
   const size_t B = (size_t)batch;
   size_t off = 0;
@@ -586,10 +632,9 @@ nsst_status nsst3_plan_create(const nsst3_config* cfg, int n0, int n1, int n2, i
   const size_t o_spec = take(spec_off * sizeof(float2));
   const size_t o_win = take(win_host.size() * sizeof(float));
   const size_t o_tw = take(tw_host.size() * sizeof(float2));
-  const size_t o_vol = take(B * p->vol_elems * sizeof(float2));
   const size_t o_xh = take(B * p->xh_elems * sizeof(float2));
   const size_t o_y = take(B * p->conv_elems * sizeof(float2));
-  const size_t o_w = take(B * p->conv_elems * sizeof(float2));
+  const size_t o_w = take(p->wk_elems * sizeof(float2));
   const size_t o_bp = take(B * p->bp_floats * sizeof(float));
   const size_t o_rbp = take(B * p->bp_floats * sizeof(float));
   const size_t o_th = take(B * p->nbands * sizeof(float));
@@ -601,7 +646,6 @@ nsst_status nsst3_plan_create(const nsst3_config* cfg, int n0, int n1, int n2, i
   p->spec = (float2*)(p->arena + o_spec);
   p->win = (float*)(p->arena + o_win);
   p->tw = (float2*)(p->arena + o_tw);
-  p->vol = (float2*)(p->arena + o_vol);
   p->xh = (float2*)(p->arena + o_xh);
   p->Y = (float2*)(p->arena + o_y);
   p->Wk = (float2*)(p->arena + o_w);
@@ -848,7 +892,7 @@ nsst_status nsst3_plan_enable_grad(nsst3_plan* p) {
   for (int b = 0; b < p->nbands; b++) {
     p->mask_off[b] = bytes;
     const nsst3_plan::Level& lv = p->lev[p->band_level[b]];
-    bytes += align_up3((size_t)lv.m[0] * lv.m[1] * mask_pitch(lv.m[2]) / 8, 256);
+    bytes += mask_band_bytes(lv.m);
   }
   p->mask_bytes = bytes;
   void* m = nullptr;
@@ -876,29 +920,46 @@ nsst_status nsst3_denoise_backward(nsst3_plan* p, const float* gy, float* gx, in
     const nsst3_plan::Level& a = p->lev[l];
     const int* N = a.lc;
     const int* m = a.m;
-    const int o = kSameOff;
+    const int wp = v3_pitch(m[2]);
     const size_t cs = p->conv_elems;
-    for (int k = 0; k < a.nb; k += 2) {
-      const int ba = a.first_band + k;
-      const int bb = k + 1 < a.nb ? ba + 1 : -1;
-      V3Pass P1 = make_pass(0, N, cs, {o, m[1]}, {o, m[2]}, {o, m[0]}, {0, N[0]});
-      set_box(P1, m, o);
+    const int chunk = pair_chunk(p, a, n);
+    for (int k0 = 0; k0 < a.npairs(); k0 += chunk) {
+      const int pairs = std::min(chunk, a.npairs() - k0);
+      V3Cols P1 = line_pass(0, p->Wk, a.pair(), N[1], wp, n, m[1], m[2], {kSameOff, m[0]}, {0, N[0]});
+      P1.out_pair = a.pair() * n;
+      P1.pairs = pairs;
+      P1.nbands = a.nb - 2 * k0;
+      P1.r1 = m[1], P1.r2 = m[2];
       P1.rsrc = p->rbp + a.bp_off;
       P1.r_stride = p->bp_floats;
-      P1.m_r2 = mask_pitch(m[2]);
-      P1.mka = p->mask + p->mask_off[ba];
-      P1.mkb = bb >= 0 ? p->mask + p->mask_off[bb] : nullptr;
-      P1.m_stride = p->mask_bytes;
-      V3_TRY(run_pass(p, P1, -1, V3_LD_MASKED, V3_ST_CPLX, p->Wk, p->Wk, N[0], n, st));
-      V3_TRY(run_pass(p, make_pass(1, N, cs, {0, N[0]}, {o, m[2]}, {o, m[1]}, {0, N[1]}), -1, V3_LD_CPLX, V3_ST_CPLX,
-                      p->Wk, p->Wk, N[1], n, st));
-      V3Pass P3 = make_pass(2, N, cs, {0, N[0]}, {0, N[1]}, {o, m[2]}, {0, N[2]});
-      P3.spec = p->spec + a.spec_off + (size_t)(k / 2) * a.conv();
-      P3.first = k == 0;
-      V3_TRY(run_pass(p, P3, -1, V3_LD_CPLX, V3_ST_SPEC, p->Y, p->Wk, N[2], n, st));
+      set_masks(p, P1, l, 2 * k0);
+      V3_TRY(run_cols(p, N[0], -1, V3_LD_MASKED, V3_ST_CPLX, P1, 1, st));
+      V3_TRY(run_cols(p, N[1], -1, V3_LD_CPLX, V3_ST_CPLX, pair_cols(p, a, n, {kSameOff, m[1]}, {0, N[1]}), pairs, st));
+      V3Pair P3 = pair_pass(p, a, k0, pairs, n);
+      P3.S = p->Y;
+      P3.s_item = cs;
+      P3.first = k0 == 0;
+      V3_CUDA(v3_ops(N[2])->pair(-1, P3, p->twid(N[2]), 1, st));
     }
-    V3_TRY(ifft3_real_box(p, p->Y, cs, N, m, 0, p->bp + a.bp_off, p->bp_floats, (float)(1.0 / (double)a.conv()), n,
-                          st));
+    // the real part of S's inverse: that of its Hermitian part, on half spectra in the work buffer
+    const int H = N[2] / 2 + 1, hp = v3_pitch(H);
+    const size_t hs = (size_t)m[0] * N[1] * hp;
+    V3Cols P = line_pass(0, p->Wk, hs, N[1], hp, n, N[1], H, {0, N[0]}, {0, m[0]});
+    P.in = p->Y;
+    P.in_item = cs;
+    P.in_a = N[2], P.in_i = N[1] * N[2];
+    P.sym_a = N[1], P.sym_z = N[2];
+    V3_TRY(run_cols(p, N[0], +1, V3_LD_SYM, V3_ST_CPLX, P, 1, st));
+    V3_TRY(run_cols(p, N[1], +1, V3_LD_CPLX, V3_ST_CPLX,
+                    line_pass(1, p->Wk, hs, N[1], hp, n, m[0], H, {0, N[1]}, {0, m[1]}), 1, st));
+    V3Real R;
+    R.dst = p->bp + a.bp_off;
+    R.spec = p->Wk;
+    R.r_stride = p->bp_floats, R.spec_stride = hs;
+    R.rows0 = m[0], R.rows1 = m[1], R.n2 = m[2];
+    R.s1 = N[1], R.pitch = hp, R.line = N[2];
+    R.scale = (float)(1.0 / (double)a.conv());
+    V3_CUDA(v3_ops(N[2])->real(+1, R, p->twid(N[2]), n, st));
   }
   // the lowpass passes through unchanged
   const nsst3_plan::Level& lp = p->lev[p->L];
@@ -906,7 +967,7 @@ nsst_status nsst3_denoise_backward(nsst3_plan* p, const float* gy, float* gx, in
                             p->bp_floats * sizeof(float), lp.vol() * sizeof(float), n, cudaMemcpyDeviceToDevice, st));
   // pyr_rec (the adjoint of pyr_dec) to the full grid, then fold the edge padding
   V3_TRY(run_pyr_rec(p, p->bp, p->rbp, p->g, n, st));
-  V3_CUDA(launch_fold_edge(p->rbp, p->vol_elems, gx, p->in_elems, (float*)p->vol, 2 * p->vol_elems, n, p->n[0],
+  V3_CUDA(launch_fold_edge(p->rbp, p->vol_elems, gx, p->in_elems, (float*)p->Wk, 2 * p->vol_elems, n, p->n[0],
                            p->n[1], p->n[2], p->g[0], p->g[1], p->g[2], st));
   return NSST_OK;
 }
