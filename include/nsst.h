@@ -519,7 +519,9 @@ int nsst3_num_bands(const nsst3_plan* plan);           /* directional bands over
 size_t nsst3_subband_floats(const nsst3_plan* plan);   /* floats per volume of the sub-band layout */
 size_t nsst3_plan_device_bytes(const nsst3_plan* plan);
 /* level -1: dims[0..2] = the padded grid; level l in [0, nlevels]: dims of band-pass l
- * (l = nlevels: lowpass) and conv[0..2] = its convolution FFT lengths. */
+ * (l = nlevels: lowpass) and conv[0..2] = its convolution lengths: the smallest
+ * 2^a 3^b length >= dims + 12 per axis, which holds the 'same' part without
+ * wrap-around (the transforms may run at a shorter one that does too). */
 nsst_status nsst3_level_dims(const nsst3_plan* plan, int level, int* dims, int* conv);
 /* level, cone, l2, l1 of directional band b. */
 nsst_status nsst3_band_info(const nsst3_plan* plan, int band, int* info4);

@@ -14,7 +14,7 @@ const V3Ops* v3_ops_grid(int n) {
       return &ops;
     }
     case 44: {
-      static const V3Ops ops = V3Launch<44, true, false>::ops();
+      static const V3Ops ops = V3Launch<44, true, true>::ops();
       return &ops;
     }
     case 68: {
@@ -22,7 +22,7 @@ const V3Ops* v3_ops_grid(int n) {
       return &ops;
     }
     case 88: {
-      static const V3Ops ops = V3Launch<88, true, false>::ops();
+      static const V3Ops ops = V3Launch<88, true, true>::ops();
       return &ops;
     }
     case 132: {
@@ -31,10 +31,6 @@ const V3Ops* v3_ops_grid(int n) {
     }
     case 136: {
       static const V3Ops ops = V3Launch<136, true, false>::ops();
-      return &ops;
-    }
-    case 204: {
-      static const V3Ops ops = V3Launch<204, true, false>::ops();
       return &ops;
     }
     default:

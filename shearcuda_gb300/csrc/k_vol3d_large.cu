@@ -1,4 +1,4 @@
-// Volume FFT passes (vol3d_fft.cuh): 192 and 216 points.
+// Volume FFT passes (vol3d_fft.cuh): 192 points and more.
 #include "vol3d_fft.cuh"
 
 namespace nsst {
@@ -6,7 +6,11 @@ namespace nsst {
 const V3Ops* v3_ops_large(int n) {
   switch (n) {
     case 192: {
-      static const V3Ops ops = V3Launch<192, true, true>::ops();
+      static const V3Ops ops = V3Launch<192, true, false>::ops();
+      return &ops;
+    }
+    case 204: {
+      static const V3Ops ops = V3Launch<204, true, true>::ops();
       return &ops;
     }
     case 216: {

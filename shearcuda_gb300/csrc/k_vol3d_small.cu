@@ -1,4 +1,4 @@
-// Volume FFT passes (vol3d_fft.cuh): the 2^a 3^b lengths up to 96.
+// Volume FFT passes (vol3d_fft.cuh): lengths up to 96.
 #include "vol3d_fft.cuh"
 
 namespace nsst {
@@ -21,6 +21,10 @@ const V3Ops* v3_ops(int n) {
       static const V3Ops ops = V3Launch<48, true, true>::ops();
       return &ops;
     }
+    case 56: {
+      static const V3Ops ops = V3Launch<56, false, true>::ops();
+      return &ops;
+    }
     case 64: {
       static const V3Ops ops = V3Launch<64, true, true>::ops();
       return &ops;
@@ -29,8 +33,12 @@ const V3Ops* v3_ops(int n) {
       static const V3Ops ops = V3Launch<72, true, true>::ops();
       return &ops;
     }
+    case 80: {
+      static const V3Ops ops = V3Launch<80, false, true>::ops();
+      return &ops;
+    }
     case 96: {
-      static const V3Ops ops = V3Launch<96, true, true>::ops();
+      static const V3Ops ops = V3Launch<96, true, false>::ops();
       return &ops;
     }
     default:

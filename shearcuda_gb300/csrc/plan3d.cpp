@@ -35,7 +35,7 @@ constexpr int kCube = 24;          // Meyer filter support (GetMeyerBasedFilter.
 constexpr int kSameOff = 12;       // convnfft 'same' offset: ceil((24 - 1) / 2)
 constexpr int kMaxGrid = 192;      // largest padded grid per dimension
 constexpr int kSmCount = 152;
-constexpr int kCtasPerSm = 8;      // CTAs per SM that keep the z product pass's loads in flight
+constexpr int kCtasPerSm = 8;      // CTAs per SM that keep a pass's loads in flight
 // Band pairs in flight per level: the work buffer holds as many as fit here (at least one).
 constexpr size_t kPairBytes = (size_t)1 << 30;
 const int kFftLens[] = {16, 24, 32, 48, 64, 72, 96, 128, 144, 192, 216, 256};
@@ -51,6 +51,16 @@ bool is_fft_len(int n) {
 // the kept range), so the full m + 23 is not needed.
 int conv_len(int m) {
   for (int v : kFftLens)
+    if (v >= m + kSameOff) return v;
+  return -1;
+}
+// The length the transforms run at: the shortest compiled one, with factors 5
+// and 7 beside 2 and 3 (and 11 and 17 where the padded grids have them anyway).
+// A level costs its convolution volume, so 156 -> 160 instead of 192, 108
+// instead of 128 and 76 -> 80 instead of 96 are 0.58, 0.60 and 0.58 of it.
+const int kConvLens[] = {32, 44, 48, 56, 64, 72, 80, 88, 100, 108, 140, 144, 160, 204, 216};
+int run_len(int m) {
+  for (int v : kConvLens)
     if (v >= m + kSameOff) return v;
   return -1;
 }
@@ -178,7 +188,7 @@ struct nsst3_plan {
 
   struct Level {
     int m[3] = {0, 0, 0};   // band-pass dims (level L: lowpass)
-    int lc[3] = {0, 0, 0};  // convolution FFT lengths (levels < L)
+    int lc[3] = {0, 0, 0};  // convolution transform lengths (levels < L)
     int nd = 0, nb = 0, first_band = 0;
     size_t bp_off = 0;      // floats, in the sub-band layout
     size_t xh_off = 0;      // float2, in one volume's half-spectrum block
@@ -369,6 +379,11 @@ nsst_status run_pyr_rec(nsst3_plan* p, const float* bp, float* x, const int* out
 int pair_chunk(const nsst3_plan* p, const nsst3_plan::Level& a, int n) {
   return (int)std::max<size_t>(1, std::min<size_t>(a.npairs(), p->wk_elems / (a.pair() * n)));
 }
+// The passes whose CTAs loop over the chunk's pairs (what the pairs share is
+// then read once) split them over the grid until it fills the GPU.
+int pair_shares(int ctas, int pairs) {
+  return std::min(pairs, std::max(1, (kSmCount * kCtasPerSm + ctas - 1) / ctas));
+}
 // Keep bits of the level's bands from band k on.
 void set_masks(const nsst3_plan* p, V3Cols& P, int l, int k) {
   const nsst3_plan::Level& a = p->lev[l];
@@ -417,10 +432,7 @@ nsst_status run_sh_level(nsst3_plan* p, const float* bp, int l, float* acc, cons
     P1.Y = p->Y;
     P1.y_item = p->conv_elems;
     P1.pitch = v3_pitch(N[2] / 2 + 1);
-    // the CTAs loop over the pairs, so that Y is read once, as far as the grid still fills the GPU
-    const int ctas = (N[0] * N[1] + 7) / 8 * n;
-    const int shares = std::min(pairs, std::max(1, (kSmCount * kCtasPerSm + ctas - 1) / ctas));
-    V3_CUDA(v3_ops(N[2])->pair(+1, P1, p->twid(N[2]), shares, st));
+    V3_CUDA(v3_ops(N[2])->pair(+1, P1, p->twid(N[2]), pair_shares((N[0] * N[1] + 7) / 8 * n, pairs), st));
     V3_TRY(run_cols(p, N[1], +1, V3_LD_CPLX, V3_ST_CPLX, pair_cols(p, a, n, {0, N[1]}, {kSameOff, m[1]}), pairs, st));
     V3Cols P3 = line_pass(0, p->Wk, a.pair(), N[1], wp, n, m[1], m[2], {0, N[0]}, {kSameOff, m[0]});
     P3.in_pair = a.pair() * n;
@@ -440,7 +452,7 @@ nsst_status run_sh_level(nsst3_plan* p, const float* bp, int l, float* acc, cons
       P3.rdst = coeffs + (size_t)(2 * k0) * a.vol();
       P3.r_stride = (size_t)a.nb * a.vol();
       P3.band_stride = a.vol();
-      V3_TRY(run_cols(p, N[0], +1, V3_LD_CPLX, V3_ST_PAIR, P3, 1, st));
+      V3_TRY(run_cols(p, N[0], +1, V3_LD_CPLX, V3_ST_PAIR, P3, pair_shares(m[1] * ((m[2] + 7) / 8) * n, pairs), st));
     }
   }
   return NSST_OK;
@@ -559,7 +571,9 @@ nsst_status nsst3_plan_create(const nsst3_config* cfg, int n0, int n1, int n2, i
     a.xh_off = xh_off;
     xh_off += align_up3(a.half(), 32);
     if (l == p->L) break;
-    for (int k = 0; k < 3; k++) a.lc[k] = conv_len(a.m[k]);
+    for (int k = 0; k < 3; k++)
+      if ((a.lc[k] = run_len(a.m[k])) < 0)
+        return fail3(NSST_ERR_UNSUPPORTED_SIZE, "volume level too large for the compiled convolution lengths");
     a.nd = cfg->num_dirs[l];
     a.nb = 3 * a.nd * a.nd;
     a.first_band = p->nbands;
@@ -733,7 +747,7 @@ nsst_status nsst3_level_dims(const nsst3_plan* p, int level, int* dims, int* con
   if (level < -1 || level > p->L) return fail3(NSST_ERR_INVALID_ARG, "level out of range");
   for (int k = 0; k < 3; k++) {
     if (dims) dims[k] = level < 0 ? p->g[k] : p->lev[level].m[k];
-    if (conv) conv[k] = (level < 0 || level == p->L) ? 0 : p->lev[level].lc[k];
+    if (conv) conv[k] = (level < 0 || level == p->L) ? 0 : conv_len(p->lev[level].m[k]);
   }
   return NSST_OK;
 }
@@ -933,7 +947,7 @@ nsst_status nsst3_denoise_backward(nsst3_plan* p, const float* gy, float* gx, in
       P1.rsrc = p->rbp + a.bp_off;
       P1.r_stride = p->bp_floats;
       set_masks(p, P1, l, 2 * k0);
-      V3_TRY(run_cols(p, N[0], -1, V3_LD_MASKED, V3_ST_CPLX, P1, 1, st));
+      V3_TRY(run_cols(p, N[0], -1, V3_LD_MASKED, V3_ST_CPLX, P1, pair_shares(m[1] * ((m[2] + 7) / 8) * n, pairs), st));
       V3_TRY(run_cols(p, N[1], -1, V3_LD_CPLX, V3_ST_CPLX, pair_cols(p, a, n, {kSameOff, m[1]}, {0, N[1]}), pairs, st));
       V3Pair P3 = pair_pass(p, a, k0, pairs, n);
       P3.S = p->Y;

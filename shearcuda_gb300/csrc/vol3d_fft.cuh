@@ -82,6 +82,11 @@ struct V3Cfg {
   static constexpr int EXZ = SZ * kLines;
 };
 
+// Launch bound for at most `regs` registers a thread.
+constexpr int v3_min_ctas(int threads, int regs) { return 65536 / (threads * regs); }
+// Column passes that loop over the band pairs in the CTA.
+constexpr bool v3_loops(int ld, int st) { return ld == V3_LD_MASKED || st == V3_ST_THRESH || st == V3_ST_PAIR; }
+
 // First stage: load, R1-point DFTs, twiddles, exchange write at ex[row(k1, j)].
 template <int N, int DIR, class Ld, class Row>
 __device__ __forceinline__ void v3_stage1(float2* ex, const float2* __restrict__ tw, int j, const Ld& ld, const Row& row) {
@@ -114,20 +119,23 @@ __device__ __forceinline__ float v3_win(const float* __restrict__ v, int K, int 
 // ---------------------------------------------------------------------------
 // Axes 1 and 0: 8 lines adjacent along z.
 // ---------------------------------------------------------------------------
-// CTA x: line group (a, 8 z) and item, item fastest; y: band pair (loads and
-// stores that loop over the pairs: 1).
-template <int N, int DIR, int LD, int ST>
-__global__ void __launch_bounds__(V3Cfg<N>::T) k_v3_cols(const V3Cols P, const float2* __restrict__ tw) {
+// CTA x: line group (a, 8 z) and item, item fastest; y: band pair, or, for the
+// loads and stores that loop over the pairs, the share of them.  G: thread
+// groups of a CTA that take every G-th pair of a band sum.
+template <int N, int DIR, int LD, int ST, int G = 1>
+__global__ void __launch_bounds__(V3Cfg<N>::T * G, v3_loops(LD, ST) ? v3_min_ctas(V3Cfg<N>::T * G, 96) : 1)
+    k_v3_cols(const V3Cols P, const float2* __restrict__ tw) {
   using C = V3Cfg<N>;
   constexpr int R1 = C::R1, R2 = C::R2;
-  constexpr bool kLoop = LD == V3_LD_MASKED || ST == V3_ST_THRESH || ST == V3_ST_PAIR;
-  __shared__ float2 ex[kLoop ? 2 : 1][C::EX];
+  constexpr bool kLoop = v3_loops(LD, ST);
+  __shared__ float2 ex[kLoop && G == 1 ? 2 : G][C::EX];
+  const int grp = G > 1 ? threadIdx.x / C::T : 0, tid = threadIdx.x - grp * C::T;
   const int item = blockIdx.x % P.items, g = blockIdx.x / P.items;
   const int zg = (P.zn + kLines - 1) / kLines;
-  const int a = g / zg, z = (g % zg) * kLines + (threadIdx.x & (kLines - 1));
-  const int j = threadIdx.x / kLines;
+  const int a = g / zg, z = (g % zg) * kLines + (tid & (kLines - 1));
+  const int j = tid / kLines;
   const bool zin = z < P.zn;
-  auto row = [&](int k1, int q) { return (k1 * C::P2 + q) * kLines + (int)(threadIdx.x & (kLines - 1)); };
+  auto row = [&](int k1, int q) { return (k1 * C::P2 + q) * kLines + (tid & (kLines - 1)); };
   const size_t ibase = (size_t)item * P.in_item + (size_t)a * P.in_a + z;
   const size_t obase = (size_t)item * P.out_item + (size_t)a * P.out_a + z;
 
@@ -217,7 +225,8 @@ __global__ void __launch_bounds__(V3Cfg<N>::T) k_v3_cols(const V3Cols P, const f
         u0[r] = zin && n >= 0 && n < P.in_n ? P.rsrc[rbase + (size_t)n * r_i] : 0.f;
       }
     }
-    for (int k = 0; k < P.pairs; k++) {
+    int it = 0;
+    for (int k = blockIdx.y; k < P.pairs; k += gridDim.y, it ^= 1) {
       const uint8_t* ma = P.mask + item * P.m_stride + (size_t)(2 * k) * P.m_band;
       const uint8_t* mb = 2 * k + 1 < P.nbands ? ma + P.m_band : nullptr;
       const unsigned bit = 1u << (z & 7);
@@ -232,12 +241,12 @@ __global__ void __launch_bounds__(V3Cfg<N>::T) k_v3_cols(const V3Cols P, const f
           }
           return v;
         };
-        v3_stage1<N, DIR>(ex[k & 1], tw, j, ld, row);
+        v3_stage1<N, DIR>(ex[it], tw, j, ld, row);
       }
       __syncthreads();
       if (j < R1) {
         float2 u[R2];
-        v3_stage2<N, DIR>(ex[k & 1], j, u, row);
+        v3_stage2<N, DIR>(ex[it], j, u, row);
         float2* out = P.out + obase + (size_t)k * P.out_pair;
         if (zin) {
 #pragma unroll
@@ -250,21 +259,33 @@ __global__ void __launch_bounds__(V3Cfg<N>::T) k_v3_cols(const V3Cols P, const f
     }
   } else {
     const unsigned members = __ballot_sync(0xffffffffu, j < R1);
+    // The band sum adds the pairs in their order whatever the chunks and groups
+    // are, so that a batch and its volumes one by one give the same bits.
     float acc[R2];
 #pragma unroll
-    for (int k2 = 0; k2 < R2; k2++) acc[k2] = 0.f;
-    for (int k = 0; k < P.pairs; k++) {
+    for (int k2 = 0; k2 < R2; k2++) {
+      const int n = j + R1 * k2 - P.out_lo;
+      acc[k2] = ST == V3_ST_THRESH && !P.first && grp == 0 && j < R1 && zin && n >= 0 && n < P.out_n
+                    ? P.rdst[rbase + (size_t)n * r_i]
+                    : 0.f;
+    }
+    float* part = reinterpret_cast<float*>(ex[grp]);  // G > 1: the group's summands of this round
+    int it = 0;
+    for (int k0 = blockIdx.y * G; k0 < P.pairs; k0 += gridDim.y * G) {
+      const int k = k0 + grp;
+      const bool live = G == 1 || k < P.pairs;
+      float2* x = ex[G == 1 ? it : grp];
       const float2* in = P.in + ibase + (size_t)k * P.in_pair;
-      if (j < R2) {
+      if (live && j < R2) {
         auto ld = [&](int, int n) -> float2 {
           return zin && n >= P.in_lo && n < P.in_lo + P.in_n ? in[(n - P.in_lo) * P.in_i] : make_float2(0.f, 0.f);
         };
-        v3_stage1<N, DIR>(ex[k & 1], tw, j, ld, row);
+        v3_stage1<N, DIR>(x, tw, j, ld, row);
       }
       __syncthreads();
-      if (j < R1) {
-        float2 u[R2];
-        v3_stage2<N, DIR>(ex[k & 1], j, u, row);
+      float2 u[R2];
+      if (live && j < R1) {
+        v3_stage2<N, DIR>(x, j, u, row);
         const bool has_b = 2 * k + 1 < P.nbands;
         float ta = -1.f, tb = -1.f;
         if constexpr (ST == V3_ST_THRESH)
@@ -280,14 +301,15 @@ __global__ void __launch_bounds__(V3Cfg<N>::T) k_v3_cols(const V3Cols P, const f
           if constexpr (ST == V3_ST_THRESH) {
             // ThresholdShCoeff.m:7 zeroes |c| <= t
             const bool ka = st && !(fabsf(ca) <= ta), kb = st && has_b && !(fabsf(cb) <= tb);
-            acc[k2] += (ka ? ca : 0.f) + (kb ? cb : 0.f);
+            u[k2].x = (ka ? ca : 0.f) + (kb ? cb : 0.f);
+            if (grp == 0) acc[k2] += u[k2].x;
             if (P.mask) {  // uniform across the grid; the eight lanes of a line group give one byte
               const unsigned ba = __ballot_sync(members, ka), bb = __ballot_sync(members, kb);
-              if (n >= 0 && n < P.out_n && (threadIdx.x & 7) == 0) {
+              if (n >= 0 && n < P.out_n && (tid & 7) == 0) {
                 uint8_t* b = P.mask + item * P.m_stride + (size_t)(2 * k) * P.m_band +
                              ((((size_t)n * P.r1 + a) * P.m_r2 + z) >> 3);
-                *b = (uint8_t)(ba >> (threadIdx.x & 24));
-                if (has_b) b[P.m_band] = (uint8_t)(bb >> (threadIdx.x & 24));
+                *b = (uint8_t)(ba >> (tid & 24));
+                if (has_b) b[P.m_band] = (uint8_t)(bb >> (tid & 24));
               }
             }
           } else if (st) {
@@ -297,17 +319,35 @@ __global__ void __launch_bounds__(V3Cfg<N>::T) k_v3_cols(const V3Cols P, const f
           }
         }
       }
+      if constexpr (G > 1) {
+        __syncthreads();  // every thread has read its group's exchange
+        if (grp > 0 && live && j < R1) {
+#pragma unroll
+          for (int k2 = 0; k2 < R2; k2++) part[k2 * (R1 * kLines) + tid] = u[k2].x;
+        }
+        __syncthreads();
+        if (grp == 0 && j < R1) {
+          for (int q = 1; q < G && k0 + q < P.pairs; q++) {
+            const float* pq = reinterpret_cast<const float*>(ex[q]);
+#pragma unroll
+            for (int k2 = 0; k2 < R2; k2++) acc[k2] += pq[k2 * (R1 * kLines) + tid];
+          }
+        }
+        __syncthreads();
+      }
+      it ^= 1;
     }
-    if constexpr (ST == V3_ST_THRESH)
-      if (j < R1 && zin) {
+    if constexpr (ST == V3_ST_THRESH) {
+      if (grp == 0 && j < R1 && zin) {
 #pragma unroll
         for (int k2 = 0; k2 < R2; k2++) {
           const int n = j + R1 * k2 - P.out_lo;
           if (n < 0 || n >= P.out_n) continue;
           float* d = P.rdst + rbase + (size_t)n * r_i;
-          *d = P.first ? acc[k2] : *d + acc[k2];
+          *d = acc[k2];
         }
       }
+    }
   }
 }
 
@@ -424,7 +464,7 @@ __global__ void __launch_bounds__(V3Cfg<N>::T) k_v3_real_inv(const V3Real P, con
 // is the conjugate mirror of the stored half).  CTA x: 8 rows and item, item
 // fastest, so the items share each filter row through L2; y: share of the pairs.
 template <int N>
-__global__ void __launch_bounds__(V3Cfg<N>::T) k_v3_pair_inv(const V3Pair P, const float2* __restrict__ tw) {
+__global__ void __launch_bounds__(V3Cfg<N>::T, v3_min_ctas(V3Cfg<N>::T, 112)) k_v3_pair_inv(const V3Pair P, const float2* __restrict__ tw) {
   using C = V3Cfg<N>;
   constexpr int R1 = C::R1, R2 = C::R2;
   __shared__ float2 ex[2][C::EXZ];
@@ -449,12 +489,19 @@ __global__ void __launch_bounds__(V3Cfg<N>::T) k_v3_pair_inv(const V3Pair P, con
     }
     spec = P.spec + (size_t)r * N + j;
   }
+  // the next pair's filter row is loaded while this pair's second stage runs
+  float2 c[R1];
+  auto fetch = [&](int k) {
+    if (l1 && k < P.pairs) {
+#pragma unroll
+      for (int q = 0; q < R1; q++) c[q] = __ldg(spec + (size_t)k * rows * N + R2 * q);
+    }
+  };
+  fetch(blockIdx.y);
   int it = 0;
   for (int k = blockIdx.y; k < P.pairs; k += gridDim.y, it ^= 1) {
-    if (l1) {
-      const float2* c = spec + (size_t)k * rows * N;
-      v3_stage1<N, +1>(ex[it], tw, j, [&](int q, int) { return cmul(y[q], __ldg(c + R2 * q)); }, at(s1));
-    }
+    if (l1) v3_stage1<N, +1>(ex[it], tw, j, [&](int q, int) { return cmul(y[q], c[q]); }, at(s1));
+    fetch(k + gridDim.y);
     __syncthreads();
     if (l2) {
       float2 u[R2];
@@ -472,7 +519,7 @@ __global__ void __launch_bounds__(V3Cfg<N>::T) k_v3_pair_inv(const V3Pair P, con
 // Its adjoint: per band pair of the chunk the box's z, forward transform,
 // S (+)= conj(C) .* Z summed over the pairs in registers.
 template <int N>
-__global__ void __launch_bounds__(V3Cfg<N>::T) k_v3_pair_fwd(const V3Pair P, const float2* __restrict__ tw) {
+__global__ void __launch_bounds__(V3Cfg<N>::T, v3_min_ctas(V3Cfg<N>::T, 128)) k_v3_pair_fwd(const V3Pair P, const float2* __restrict__ tw) {
   using C = V3Cfg<N>;
   constexpr int R1 = C::R1, R2 = C::R2;
   __shared__ float2 ex[2][C::EXZ];
@@ -485,16 +532,24 @@ __global__ void __launch_bounds__(V3Cfg<N>::T) k_v3_pair_fwd(const V3Pair P, con
   const bool l2 = s2 < kLines && row0 + s2 < rows;
   float2 acc[R2];
 #pragma unroll
-  for (int k2 = 0; k2 < R2; k2++) acc[k2] = make_float2(0.f, 0.f);
-  for (int k = 0; k < P.pairs; k++) {
-    if (l1) {
+  for (int k2 = 0; k2 < R2; k2++)
+    acc[k2] = l2 && !P.first ? P.S[(size_t)item * P.s_item + (size_t)(row0 + s2) * N + k1 + R1 * k2] : make_float2(0.f, 0.f);
+  // the next pair's row is loaded while this pair's second stage runs
+  float2 v[R1];
+  auto fetch = [&](int k) {
+    if (l1 && k < P.pairs) {
       const float2* w = P.W + (size_t)k * P.w_pair + (size_t)item * P.w_item + (size_t)(row0 + s1) * P.wpitch;
-      auto ld = [&](int, int nn) -> float2 {
-        const int n = nn - P.z_lo;
-        return n >= 0 && n < P.z_n ? w[n] : make_float2(0.f, 0.f);
-      };
-      v3_stage1<N, -1>(ex[k & 1], tw, j, ld, at(s1));
+#pragma unroll
+      for (int q = 0; q < R1; q++) {
+        const int n = j + R2 * q - P.z_lo;
+        v[q] = n >= 0 && n < P.z_n ? w[n] : make_float2(0.f, 0.f);
+      }
     }
+  };
+  fetch(0);
+  for (int k = 0; k < P.pairs; k++) {
+    if (l1) v3_stage1<N, -1>(ex[k & 1], tw, j, [&](int q, int) { return v[q]; }, at(s1));
+    fetch(k + 1);
     __syncthreads();
     if (l2) {
       float2 u[R2];
@@ -507,7 +562,7 @@ __global__ void __launch_bounds__(V3Cfg<N>::T) k_v3_pair_fwd(const V3Pair P, con
   if (!l2) return;
   float2* S = P.S + (size_t)item * P.s_item + (size_t)(row0 + s2) * N + k1;
 #pragma unroll
-  for (int k2 = 0; k2 < R2; k2++) S[R1 * k2] = P.first ? acc[k2] : cadd(S[R1 * k2], acc[k2]);
+  for (int k2 = 0; k2 < R2; k2++) S[R1 * k2] = acc[k2];
 }
 
 // ---------------------------------------------------------------------------
@@ -528,6 +583,13 @@ struct V3Launch {
   static cudaError_t cols(int dir, int ld, int st_mode, const V3Cols& P, const float2* tw, int npairs, cudaStream_t st) {
     const dim3 grid((unsigned)(P.an * ((P.zn + kLines - 1) / kLines) * P.items), (unsigned)npairs);
     count_launch();
+    // A band sum over few lines: its CTAs' chain of pairs is the time, so four
+    // groups of threads share it; with more CTAs the groups only wait for one another.
+    if constexpr (CONV && N <= 108)
+      if (st_mode == V3_ST_THRESH && P.pairs >= 4 && grid.x <= 2 * 152) {
+        k_v3_cols<N, 1, V3_LD_CPLX, V3_ST_THRESH, 4><<<grid, 4 * T, 0, st>>>(P, tw);
+        return cudaGetLastError();
+      }
 #define V3_COLS(cond, d, l, s)                          \
   if constexpr (cond)                                   \
     if (dir == d && ld == l && st_mode == s) {          \
