@@ -1106,6 +1106,27 @@ nsst_status enqueue_band_analysis(nsst_plan* p, int n, bool grad, cudaStream_t s
   return NSST_OK;
 }
 
+// The band synthesis of n items (p->band -> p->sum) as choice c runs it.
+// sums_dct2: see enqueue_directional.
+nsst_status enqueue_band_synthesis(nsst_plan* p, int n, const DirChoice& c, cudaStream_t st, bool* sums_dct2) {
+  char* A = p->arena;
+  const bool tma = c.cols_tma && p->cols_tma_ok;
+  const bool dct2 = sums_dct2 && tma && c.syn_regs && !c.cols_packed && p->wdH && dct_syn_fusion_pays(p);
+  const ColOp syn = c.cols_packed          ? ColOp::SynthesisPairs
+                    : (tma && c.syn_regs) ? (dct2 ? ColOp::SynthesisRegsDct2 : ColOp::SynthesisRegs)
+                                          : ColOp::Synthesis;
+  const float2* twc = c.cols_packed ? (const float2*)p->twH4 : p->twH;
+  if (tma)
+    NSST_CUDA(launch_cols_tma(syn, p->cols_tmap, p->j_synthesis, p->B * p->nlev, n, p->H, p->W, (float2*)A, p->spec,
+                              p->spec_row0, (size_t)p->H * p->WH, twc, p->dev_err, st, p->wdH, p->B));
+  else
+    NSST_CUDA(launch_cols(syn, p->j_synthesis, p->B * p->nlev, n, p->H, p->W, (float2*)A, (float2*)A, p->spec,
+                          (size_t)p->H * p->WH, twc, st));
+  timer_mark(p, "band_synthesis_cols", st);
+  if (dct2) *sums_dct2 = true;
+  return NSST_OK;
+}
+
 // The directional stage of the fused denoise (level spectra in p->lev, band
 // sums out in p->sum): one cluster kernel, or the split analysis / row /
 // synthesis kernels with the bands in p->band.
@@ -1129,20 +1150,7 @@ nsst_status enqueue_directional(nsst_plan* p, int n, int mode, const float* TH, 
   NSST_CUDA(launch_rows_thresh(p->j_rows_bands, p->B * p->ndir_total, n, p->H, p->W, A, A, p->twWh, p->twW, TH, mode,
                                c.row_tile, st, c.packed, p->twWh4, p->twW4));
   timer_mark(p, "band_rows_threshold", st);
-  const bool dct2 = sums_dct2 && tma && c.syn_regs && !c.cols_packed && p->wdH && dct_syn_fusion_pays(p);
-  const ColOp syn = c.cols_packed          ? ColOp::SynthesisPairs
-                    : (tma && c.syn_regs) ? (dct2 ? ColOp::SynthesisRegsDct2 : ColOp::SynthesisRegs)
-                                          : ColOp::Synthesis;
-  const float2* twc = c.cols_packed ? (const float2*)p->twH4 : p->twH;
-  if (tma)
-    NSST_CUDA(launch_cols_tma(syn, p->cols_tmap, p->j_synthesis, p->B * p->nlev, n, p->H, p->W, (float2*)A, p->spec,
-                              p->spec_row0, (size_t)p->H * p->WH, twc, p->dev_err, st, p->wdH, p->B));
-  else
-    NSST_CUDA(launch_cols(syn, p->j_synthesis, p->B * p->nlev, n, p->H, p->W, (float2*)A, (float2*)A, p->spec,
-                          (size_t)p->H * p->WH, twc, st));
-  timer_mark(p, "band_synthesis_cols", st);
-  if (dct2) *sums_dct2 = true;
-  return NSST_OK;
+  return enqueue_band_synthesis(p, n, c, st, sums_dct2);
 }
 
 // Whether a fused pipeline call can take the DCT-domain pyramid: symmetric
@@ -1187,9 +1195,10 @@ nsst_status enqueue_dct_cols_out(nsst_plan* p, int n, const float* const* src, f
 // Spectral analysis front of n items: X = DCT2(x) in pyr plane 0 (through
 // plane 1), then every level's spectrum (p->lev) from X .* R_l.
 // skip_cols_levels: the directional stage's level analysis finishes the
-// level spectra's columns (analysis_takes_dct).
+// level spectra's columns (analysis_takes_dct).  resp: the level responses,
+// R_l, or, for the adjoint of the synthesis, Q_l.
 nsst_status enqueue_dct_analysis(nsst_plan* p, int n, const float* const* x, cudaStream_t st,
-                                 bool skip_cols_levels = false) {
+                                 bool skip_cols_levels = false, const float* resp = nullptr) {
   char* A = p->arena;
   const int B = p->B, H = p->H, W = p->W;
   const size_t HW = (size_t)H * W;
@@ -1199,8 +1208,8 @@ nsst_status enqueue_dct_analysis(nsst_plan* p, int n, const float* const* x, cud
   timer_mark(p, "dct_rows_image", st);
   NSST_CUDA(launch_dct_cols(kDct2, p->j_dct_x, B, n, H, W, A, A, p->twH, p->wdH, st));
   timer_mark(p, "dct_cols_image", st);
-  NSST_CUDA(launch_dct_rows_ana(p->j_dct_ana, B * p->nlev, n, H, W, A, A, p->dct_ra, HW, p->twWh, p->twW, p->twDW,
-                                false, st));
+  NSST_CUDA(launch_dct_rows_ana(p->j_dct_ana, B * p->nlev, n, H, W, A, A, resp ? resp : p->dct_ra, HW, p->twWh,
+                                p->twW, p->twDW, false, st));
   timer_mark(p, "dct_rows_levels", st);
   if (!skip_cols_levels) {
     NSST_CUDA(launch_dct_cols(kDctAna, p->j_cols_lev, B * p->nlev, n, H, W, A, A, p->twH, p->wdH, st));
@@ -1210,11 +1219,13 @@ nsst_status enqueue_dct_analysis(nsst_plan* p, int n, const float* const* x, cud
 }
 
 // The lowpass band y0 = IDCT2(X .* R_low) of n items as rows DCT-III'd into
-// tmp plane 0 (its columns still in the DCT domain).
-nsst_status enqueue_dct_lowpass_rows(nsst_plan* p, int n, cudaStream_t st) {
+// tmp plane 0 (its columns still in the DCT domain).  synthesis: G_low in
+// R_low's place, the plane after it.
+nsst_status enqueue_dct_lowpass_rows(nsst_plan* p, int n, cudaStream_t st, bool synthesis = false) {
   char* A = p->arena;
-  NSST_CUDA(launch_dct_rows_ana(p->j_dct_low, p->B, n, p->H, p->W, A, A, p->dct_ra, (size_t)p->H * p->W, p->twWh,
-                                p->twW, p->twDW, true, st));
+  const size_t HW = (size_t)p->H * p->W;
+  NSST_CUDA(launch_dct_rows_ana(p->j_dct_low, p->B, n, p->H, p->W, A, A, p->dct_ra + (synthesis ? HW : 0), HW,
+                                p->twWh, p->twW, p->twDW, true, st));
   return NSST_OK;
 }
 
@@ -1223,8 +1234,10 @@ nsst_status enqueue_dct_lowpass_rows(nsst_plan* p, int n, cudaStream_t st) {
 // .* Q_l summed over the levels with low .* lowtab (low: a DCT-domain plane
 // per item at lowbase + i * lowstride), DCT-III (pyr plane 1), and DCT-III down
 // the columns into out[i].
+// resp: the level responses, Q_l, or, for the adjoint of the analysis, R_l.
 nsst_status enqueue_dct_synthesis(nsst_plan* p, int n, const float* lowbase, size_t lowstride, const float* lowtab,
-                                  float* const* out, cudaStream_t st, bool sums_dct2 = false) {
+                                  float* const* out, cudaStream_t st, bool sums_dct2 = false,
+                                  const float* resp = nullptr) {
   char* A = p->arena;
   const int B = p->B, H = p->H, W = p->W;
   const size_t HW = (size_t)H * W;
@@ -1233,7 +1246,7 @@ nsst_status enqueue_dct_synthesis(nsst_plan* p, int n, const float* lowbase, siz
     timer_mark(p, "dct_cols_sums", st);
   }
   NSST_CUDA(launch_dct_rows_syn(p->j_dct_syn, B, n, p->nlev, (size_t)H * p->WH, H, W, A, A, lowbase, lowstride,
-                                p->dct_rs, HW, lowtab, p->twWh, p->twW, p->twDW, st));
+                                resp ? resp : p->dct_rs, HW, lowtab, p->twWh, p->twW, p->twDW, st));
   timer_mark(p, "dct_rows_synthesis", st);
   std::vector<const float*> p1(n);
   for (int i = 0; i < n; i++) p1[i] = p->pyr + (size_t)i * p->s_pyr + HW;
@@ -1369,16 +1382,29 @@ nsst_status enqueue_band_maxima(nsst_plan* p, int n, const float* const* x, unsi
   return NSST_OK;
 }
 
+// The split choice of a one-image call whose band planes the caller keeps.
+DirChoice split_choice(const nsst_plan* p) {
+  DirChoice c = dir_choice(p, 1);
+  c.fused = false;
+  return c;
+}
+
 // shear_trans of one image into nbands caller planes; the plan must be locked.
-nsst_status enqueue_shear_trans(nsst_plan* p, const float* x, float* coeffs, cudaStream_t st) {
+// adjoint: with the synthesis pyramid's responses, which is the adjoint of
+// inverse_shear (spectral pyramid only: tau_backward_dct has the reason).
+nsst_status enqueue_shear_trans(nsst_plan* p, const float* x, float* coeffs, cudaStream_t st, bool adjoint = false) {
   char* A = p->arena;
   float2* A2 = (float2*)A;
   float* yb = p->pyr;
+  const DirChoice c = split_choice(p);
+  const bool tma = c.cols_tma && p->cols_tma_ok;
+  bool ana_dct = false;
   if (p->dct_on && aligned16(x)) {
     // spectral pyramid: the level spectra from X = DCT2(x); the lowpass
     // IDCT2(X .* R_low) straight to coefficient plane 0
-    NSST_TRY(enqueue_dct_analysis(p, 1, &x, st));
-    NSST_TRY(enqueue_dct_lowpass_rows(p, 1, st));
+    ana_dct = analysis_takes_dct(p, 1);
+    NSST_TRY(enqueue_dct_analysis(p, 1, &x, st, ana_dct, adjoint ? p->dct_rs : p->dct_ra));
+    NSST_TRY(enqueue_dct_lowpass_rows(p, 1, st, adjoint));
     const float* t0 = p->tmp;
     NSST_TRY(enqueue_dct_cols_out(p, 1, &t0, &coeffs, st));
     timer_mark(p, "dct_lowpass", st);
@@ -1390,13 +1416,40 @@ nsst_status enqueue_shear_trans(nsst_plan* p, const float* x, float* coeffs, cud
     NSST_CUDA(launch_cols(ColOp::Fwd, p->j_cols_lev, p->nlev, 1, p->H, p->W, A2, A2, nullptr, 0, p->twH, st));
   }
   // the job list covers every item; n_active = 1 skips the others
-  NSST_CUDA(launch_cols(ColOp::Analysis, p->j_analysis, p->B * p->ndir_total, 1, p->H, p->W, A2, A2, p->spec, 0,
-                        p->twH, st));
+  NSST_TRY(enqueue_band_analysis(p, 1, false, st, c.ana, c.cols_packed, tma, ana_dct));
   timer_mark(p, "band_analysis_cols", st);
   NSST_CUDA(launch_rows(RowOp::Inv, p->j_band_to_coeff, p->ndir_total, 1, p->H, p->W, A, coeffs, p->twWh, p->twW,
                         nullptr, 0, st));
   timer_mark(p, "band_rows_inv", st);
   return NSST_OK;
+}
+
+// inverse_shear of nbands caller planes; the plan must be locked.  adjoint:
+// with the analysis pyramid's responses, the adjoint of shear_trans (spectral
+// pyramid only).
+nsst_status enqueue_inverse_shear(nsst_plan* p, const float* coeffs, float* x, cudaStream_t st, bool adjoint = false) {
+  char* A = p->arena;
+  NSST_CUDA(launch_rows(RowOp::Fwd, p->j_coeff_fwd, p->ndir_total, 1, p->H, p->W, coeffs, A, p->twWh, p->twW,
+                        nullptr, 0, st));
+  timer_mark(p, "band_rows_fwd", st);
+  const bool spectral = p->dct_on && aligned16(x);
+  bool sums_dct2 = false;
+  NSST_TRY(enqueue_band_synthesis(p, 1, split_choice(p), st, spectral ? &sums_dct2 : nullptr));
+  if (spectral) {
+    // spectral pyramid: the lowpass coefficients DCT2'd into tmp plane 0,
+    // then the band sums and that plane through the synthesis back end
+    float* t0 = p->tmp;
+    NSST_TRY(enqueue_dct_rows_io(p, 1, &coeffs, &t0, st));
+    NSST_CUDA(launch_dct_cols(kDct2, p->j_dct_lowc, p->B, 1, p->H, p->W, A, A, p->twH, p->wdH, st));
+    timer_mark(p, "dct_lowpass", st);
+    const float* low = adjoint ? p->dct_ra + (size_t)p->dct_rl_plane * p->H * p->W : p->dct_gl;
+    return enqueue_dct_synthesis(p, 1, p->tmp, p->s_tmp, low, &x, st, sums_dct2, adjoint ? p->dct_ra : p->dct_rs);
+  }
+  NSST_CUDA(launch_rows(RowOp::Inv, p->j_rows_lev_inv, p->nlev, 1, p->H, p->W, A, A, p->twWh, p->twW, nullptr, 0,
+                        st));
+  timer_mark(p, "fft_rows_inv", st);
+  const float* yr = p->rec;
+  return run_atrousrec(p, 1, &yr, &coeffs, &x, st);
 }
 
 }  // namespace
@@ -1595,28 +1648,7 @@ nsst_status nsst_inverse_shear(nsst_plan* p, const float* coeffs, float* x, void
   p->saved_n = 0;  // the arena no longer holds the last differentiable forward
   cudaStream_t st = (cudaStream_t)stream;
   timer_begin(p, st);
-  char* A = p->arena;
-  float2* A2 = (float2*)A;
-  NSST_CUDA(launch_rows(RowOp::Fwd, p->j_coeff_fwd, p->ndir_total, 1, p->H, p->W, coeffs, A, p->twWh, p->twW,
-                        nullptr, 0, st));
-  timer_mark(p, "band_rows_fwd", st);
-  NSST_CUDA(launch_cols(ColOp::Synthesis, p->j_synthesis, p->B * p->nlev, 1, p->H, p->W, A2, A2, p->spec,
-                        (size_t)p->H * p->WH, p->twH, st));
-  timer_mark(p, "band_synthesis_cols", st);
-  if (p->dct_on && aligned16(x)) {
-    // spectral pyramid: the lowpass coefficients DCT2'd into tmp plane 0,
-    // then the band sums and that plane through the synthesis back end
-    float* t0 = p->tmp;
-    NSST_TRY(enqueue_dct_rows_io(p, 1, &coeffs, &t0, st));
-    NSST_CUDA(launch_dct_cols(kDct2, p->j_dct_lowc, p->B, 1, p->H, p->W, A, A, p->twH, p->wdH, st));
-    timer_mark(p, "dct_lowpass", st);
-    return enqueue_dct_synthesis(p, 1, p->tmp, p->s_tmp, p->dct_gl, &x, st);
-  }
-  NSST_CUDA(launch_rows(RowOp::Inv, p->j_rows_lev_inv, p->nlev, 1, p->H, p->W, A, A, p->twWh, p->twW, nullptr, 0,
-                        st));
-  timer_mark(p, "fft_rows_inv", st);
-  const float* yr = p->rec;
-  return run_atrousrec(p, 1, &yr, &coeffs, &x, st);
+  return enqueue_inverse_shear(p, coeffs, x, st);
 }
 
 nsst_status nsst_denoise_batch(nsst_plan* p, const float* const* x, float* const* out, int n, const double* sigma,
@@ -2362,11 +2394,15 @@ nsst_status nsst_plan_enable_grad(nsst_plan* p) {
 // spectra, then the transpose of the analysis pyramid).
 nsst_status nsst_shear_trans_adjoint(nsst_plan* p, const float* coeffs, float* x, void* stream) {
   if (!p || !coeffs || !x) return fail(NSST_ERR_INVALID_ARG, "NULL argument");
+  if (!aligned16(coeffs)) return fail(NSST_ERR_INVALID_ARG, "coeffs must be 16-byte aligned");
   NSST_TRY(need_grad(p));
   std::lock_guard<std::mutex> lk(p->mu);
   p->saved_n = 0;  // the arena no longer holds the last differentiable forward
   cudaStream_t st = (cudaStream_t)stream;
   timer_begin(p, st);
+  // spectral pyramid: every pyramid operator is symmetric, so the adjoint of
+  // the analysis is the synthesis with the analysis responses
+  if (p->dct_on && aligned16(x)) return enqueue_inverse_shear(p, coeffs, x, st, true);
   char* G = p->garena;
   float2* G2 = (float2*)G;
   const size_t HW = (size_t)p->H * p->W;
@@ -2391,6 +2427,7 @@ nsst_status nsst_inverse_shear_adjoint(nsst_plan* p, const float* x, float* coef
   p->saved_n = 0;  // the arena no longer holds the last differentiable forward
   cudaStream_t st = (cudaStream_t)stream;
   timer_begin(p, st);
+  if (p->dct_on && aligned16(x)) return enqueue_shear_trans(p, x, coeffs, st, true);
   char* G = p->garena;
   float2* G2 = (float2*)G;
   const size_t HW = (size_t)p->H * p->W;
