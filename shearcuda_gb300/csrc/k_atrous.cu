@@ -24,6 +24,7 @@
 #include <mutex>
 
 #include "internal.h"
+#include "tiles.cuh"
 
 namespace nsst {
 
@@ -314,32 +315,46 @@ bool atrous_pair_supported(int FA, int FB) {
   return false;
 }
 
-// Elementwise threshold of a band (used for the lowpass band and the
-// standalone thresh entry point).  One launch covers nbands bands of n
-// values each; band b uses thr[b].
-__global__ void k_thresh_bands(float* __restrict__ data, size_t n, int nbands, const float* __restrict__ thr,
-                               int mode) {
-  size_t total = n * (size_t)nbands;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-    float th = thr[i / n];
-    float v = data[i];
-    float r;
-    if (mode == THRESH_HARD) {
-      r = fabsf(v) > th ? v : 0.0f;
-    } else {
-      float a = fabsf(v) - th;
-      r = a > 0.0f ? copysignf(a, v) : 0.0f;
-    }
-    data[i] = r;
+// Elementwise threshold of nbands bands of n values each (the standalone
+// thresh entry point); band b uses thr[b].  One read and one write of every
+// coefficient: bound by HBM, so each thread has four 16-byte loads in flight
+// and the band comes from the grid, not from a division per value (49 bands
+// of 2048 x 2048: 479 -> 247 us, of 1024 x 1024 131 -> 74 us).
+constexpr int kThreshVec = 4;  // 16-byte loads per thread
+template <bool VEC>
+__global__ void __launch_bounds__(256) k_thresh_bands(float* __restrict__ data, size_t n, const float* __restrict__ thr,
+                                                      int mode) {
+  const float th = thr[blockIdx.y];
+  float* band = data + blockIdx.y * n;
+  if (VEC) {
+    float4* v4 = reinterpret_cast<float4*>(band);
+    const size_t m = n / 4, base = (size_t)blockIdx.x * (256 * kThreshVec) + threadIdx.x;
+    float4 v[kThreshVec];
+#pragma unroll
+    for (int k = 0; k < kThreshVec; k++)
+      if (base + k * 256 < m) v[k] = v4[base + k * 256];
+#pragma unroll
+    for (int k = 0; k < kThreshVec; k++)
+      if (base + k * 256 < m)
+        v4[base + k * 256] = make_float4(apply_thresh(v[k].x, th, mode), apply_thresh(v[k].y, th, mode),
+                                         apply_thresh(v[k].z, th, mode), apply_thresh(v[k].w, th, mode));
+  } else {
+    for (size_t i = blockIdx.x * (size_t)256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256)
+      band[i] = apply_thresh(band[i], th, mode);
   }
 }
 
+// The vector form needs whole 16-byte groups per band from an aligned start
+// (every image size has them; the caller's buffer may not).
 cudaError_t launch_thresh_bands(float* data, size_t n, int nbands, const float* thr, int mode, cudaStream_t st) {
-  size_t total = n * (size_t)nbands;
-  if (total == 0) return cudaSuccess;
-  int blocks = (int)std::min<size_t>((total + 255) / 256, 152 * 16);
+  if (n == 0 || nbands == 0) return cudaSuccess;
   count_launch();
-  k_thresh_bands<<<blocks, 256, 0, st>>>(data, n, nbands, thr, mode);
+  const size_t per = 256 * 4 * kThreshVec;
+  const dim3 grid((unsigned)((n + per - 1) / per), (unsigned)nbands);
+  if (n % 4 == 0 && ((uintptr_t)data & 15) == 0)
+    k_thresh_bands<true><<<grid, 256, 0, st>>>(data, n, thr, mode);
+  else
+    k_thresh_bands<false><<<grid, 256, 0, st>>>(data, n, thr, mode);
   return cudaGetLastError();
 }
 
