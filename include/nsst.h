@@ -425,7 +425,8 @@ nsst_status nsst_mrdwt(const float* x, int n, int H, int W, const double* h, int
 
 /* Inverse of nsst_mrdwt: mirdwt / mirdwt_cuda (src/mirdwt_r.h:115-219,
  * src_cuda/mirdwt_cuda.cpp).  yl, yh are left unchanged; x may equal yl.
- * Takes two planes of stream-ordered scratch per image. */
+ * Takes up to two planes of stream-ordered scratch per image, as does
+ * nsst_mrdwt. */
 nsst_status nsst_mirdwt(const float* yl, const float* yh, int n, int H, int W, const double* h, int lh, int L,
                         float* x, void* stream);
 

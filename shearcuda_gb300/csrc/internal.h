@@ -398,16 +398,13 @@ struct WvPlanes {   // one level of n items (item strides in floats)
   float* yl; size_t s_yl;           // lowpass output
   float* yh; size_t s_yh;           // this level's three planes [LH, HL, HH]
 };
-// mrdwt, one level: columns into yh planes 1 (lowpass) and 0 (highpass), then
-// rows in place: LL -> yl, HL -> 1, LH -> 0, HH -> 2.  thr (n floats, or
-// NULL) hard-thresholds the three highpass planes: c * (|c| > thr[item]).
+// mrdwt, one level: cur -> LL in yl, the planes LH, HL, HH in yh; thr (n floats,
+// or NULL) hard-thresholds the three.  cur, yl and yh must not overlap.
 cudaError_t launch_rdwt_level(const WvPlanes& P, int n, int H, int W, int sf, const WvTaps& t, const float* thr,
                               cudaStream_t st);
-// mirdwt, one level: rows (LL, HL) -> tl, (LH, HH) -> th; columns (tl, th) -> x.
-// tl / th may be the level's HL / LH planes (the coefficients are then consumed).
-cudaError_t launch_irdwt_level(const float* ll, size_t s_ll, const float* yh, size_t s_yh, float* tl, float* th,
-                               size_t s_t, float* x, size_t s_x, int n, int H, int W, int sf, const WvTaps& t,
-                               cudaStream_t st);
+// mirdwt, one level: (ll, yh) -> x.  x must not overlap ll or yh.
+cudaError_t launch_irdwt_level(const float* ll, size_t s_ll, const float* yh, size_t s_yh, float* x, size_t s_x, int n,
+                               int H, int W, int sf, const WvTaps& t, cudaStream_t st);
 bool rdwt_width_supported(int W);
 // TVCorrection (separate.m:268-276): Haar mrdwt of one level, soft threshold
 // gamma on the three highpass planes, mirdwt -- fused into one 3 x 3 stencil.

@@ -4,22 +4,23 @@
 // mrdwt (shearcuda/src/mrdwt_r.h:104-209) filters each level's lowpass along
 // rows and then columns with the level's dilation sf = 2^(l-1), periodically;
 // mirdwt (mirdwt_r.h:115-219) undoes it columns first.  The filters are
-// separable, so a level here runs in the other order -- columns, then rows --
-// which lets the row pass (one CTA per image row, the whole row staged in
-// shared memory) write its outputs over its inputs: an analysis level needs no
-// scratch beyond its own output planes.  Per level:
-//   analysis   columns: cur -> (C_lo, C_hi) in yh planes 1 and 0
-//              rows:    C_lo -> LL (yl), HL (plane 1); C_hi -> LH (plane 0), HH (plane 2)
-//   synthesis  rows:    (LL, HL) -> tl, (LH, HH) -> th
-//              columns: (tl, th) -> x
-// The column passes read their taps straight from global memory (each warp a
-// 128-byte row segment, re-reads served by L1/L2); the row passes from shared
-// memory.  All passes are HBM- or L2-bound stencils of at most 32 taps.
+// separable, so a level here runs columns first in both directions, and as one
+// kernel: a CTA owns TH rows of one row phase (rows p + sf i of a level only
+// meet rows of their own phase) at the full width, filters them down the
+// columns from global memory with the taps sliding over registers, keeps the
+// two results in shared memory and filters those along the rows.  So a level
+// moves each plane once (analysis 1 read, 4 writes; synthesis 4 reads, 1
+// write) where separate column and row kernels moved two more, and a column
+// step reads (TH + lh - 1) / TH rows per output row instead of lh.
+//   analysis   (C_lo, C_hi) = columns of cur; LL, HL = rows of C_lo; LH, HH = rows of C_hi
+//   synthesis  x1 = columns of (LL, LH), xh = columns of (HL, HH); x = rows of (x1, xh)
+// A level reads its input while other CTAs write its output, so the lowpass
+// alternates between two buffers.
 #include "internal.h"
 
 namespace nsst {
 
-constexpr int kWvRowThreads = 256;
+constexpr int kWvThreads = 256;
 constexpr int kWvMaxW = 8192;
 
 __device__ __forceinline__ float hard_keep(float v, float t) { return fabsf(v) > t ? v : 0.0f; }
@@ -28,128 +29,157 @@ __device__ __forceinline__ float soft(float v, float t) {
   return r > 0.0f ? copysignf(r, v) : 0.0f;
 }
 
-// ---------------------------------------------------------------- analysis
-// C_lo[r][c] = sum_j a[j] cur[(r + j sf) mod H][c] -> yh plane 1; C_hi with b -> plane 0
-__global__ void __launch_bounds__(256) k_rdwt_cols_fwd(const float* __restrict__ cur, size_t s_cur,
-                                                       float* __restrict__ yh, size_t s_yh, int H, int W, int sf,
-                                                       WvTaps t) {
-  const int c = blockIdx.x * 32 + threadIdx.x, r = blockIdx.y * 8 + threadIdx.y, item = blockIdx.z;
-  if (c >= W || r >= H) return;
-  const float* x = cur + item * s_cur + c;
-  float lo = 0.0f, hi = 0.0f;
-  int rr = r;
-  for (int j = 0; j < t.lh; j++) {
-    const float v = __ldg(x + (size_t)rr * W);
-    lo = fmaf(t.a[j], v, lo);
-    hi = fmaf(t.b[j], v, hi);
-    rr += sf;
-    if (rr >= H) rr -= H;
-  }
-  const size_t HW = (size_t)H * W;
-  float* out = yh + item * s_yh + (size_t)r * W + c;
-  out[HW] = lo;
-  out[0] = hi;
-}
+// LH: the filter length (0: t.lh, taps re-read per output row); TH: rows per CTA.
+// Grid: x = row phase (fastest) and group of TH rows of the phase, y = item.
+// Taps are applied in ascending order whatever the form.  Two results that take
+// the same taps or the same sample share packed FP32 FMAs, which round as two
+// single ones.  Bound by latency and issue (40 % of it at 32 images of 256 x 256,
+// 6 to 15 % of HBM: the planes stay in L2): 64 registers, so that four CTAs share
+// an SM, took the four Symmlet-4 levels there from 93 to 66 us (analysis) and 105
+// to 78 us (synthesis); six CTAs (spills) 87 and 84.  Separate column and row
+// kernels measured 133 and 150 us.
+__device__ __forceinline__ float2 twice(float v) { return make_float2(v, v); }
 
-// one CTA per (row, item): LL = rows_a(C_lo), HL = rows_b(C_lo), LH = rows_a(C_hi), HH = rows_b(C_hi)
-__global__ void __launch_bounds__(kWvRowThreads) k_rdwt_rows_fwd(float* yl, size_t s_yl, float* yh, size_t s_yh,
-                                                                 int H, int W, int sf, WvTaps t,
-                                                                 const float* __restrict__ thr) {
-  extern __shared__ float sm[];
-  float* slo = sm;
-  float* shi = sm + W;
-  const int r = blockIdx.x, item = blockIdx.y;
-  const size_t HW = (size_t)H * W;
-  float* p0 = yh + item * s_yh + (size_t)r * W;  // C_hi in, LH out
-  float* p1 = p0 + HW;                           // C_lo in, HL out
-  float* p2 = p1 + HW;                           // HH out
-  for (int c = threadIdx.x; c < W; c += kWvRowThreads) {
-    slo[c] = p1[c];
-    shi[c] = p0[c];
+template <int LH, int TH>
+__global__ void __launch_bounds__(kWvThreads, 4)
+    k_rdwt_fwd(const float* __restrict__ cur, size_t s_cur, float* __restrict__ yl, size_t s_yl,
+               float* __restrict__ yh, size_t s_yh, int H, int W, int sf, const __grid_constant__ WvTaps t,
+               const float* __restrict__ thr) {
+  extern __shared__ float2 sm[];  // [row][column] (C_lo, C_hi)
+  const int ph = blockIdx.x % sf, i0 = blockIdx.x / sf * TH, item = blockIdx.y, Hp = H / sf;
+  const size_t HW = (size_t)H * W, rs = (size_t)sf * W;
+  const float* x = cur + item * s_cur + (size_t)ph * W;
+  for (int c = threadIdx.x; c < W; c += kWvThreads) {
+    float2 lh[TH];  // (lo, hi)
+#pragma unroll
+    for (int k = 0; k < TH; k++) lh[k] = twice(0.0f);
+    if constexpr (LH > 0) {
+      int i = i0;
+#pragma unroll
+      for (int m = 0; m < TH + LH - 1; m++) {
+        const float2 v = twice(__ldg(x + i * rs + c));
+        if (++i == Hp) i = 0;
+#pragma unroll
+        for (int k = 0; k < TH; k++)
+          if (m - k >= 0 && m - k < LH) lh[k] = __ffma2_rn(make_float2(t.a[m - k], t.b[m - k]), v, lh[k]);
+      }
+    } else {
+      for (int k = 0; k < TH; k++) {
+        int i = (i0 + k) % Hp;
+        for (int j = 0; j < t.lh; j++) {
+          lh[k] = __ffma2_rn(make_float2(t.a[j], t.b[j]), twice(__ldg(x + i * rs + c)), lh[k]);
+          if (++i == Hp) i = 0;
+        }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < TH; k++) sm[k * W + c] = lh[k];
   }
   __syncthreads();
   const float th = thr ? thr[item] : -1.0f;
-  float* ylr = yl + item * s_yl + (size_t)r * W;
-  for (int c = threadIdx.x; c < W; c += kWvRowThreads) {
-    float ll = 0.0f, hl = 0.0f, lh = 0.0f, hh = 0.0f;
+  const int lh_n = LH > 0 ? LH : t.lh;
+  for (int c = threadIdx.x; c < W; c += kWvThreads) {
+    float2 lo[TH], hi[TH];  // (LL, LH), (HL, HH)
+#pragma unroll
+    for (int k = 0; k < TH; k++) lo[k] = hi[k] = twice(0.0f);
     int cc = c;
-    for (int j = 0; j < t.lh; j++) {
-      const float vl = slo[cc], vh = shi[cc];
-      ll = fmaf(t.a[j], vl, ll);
-      hl = fmaf(t.b[j], vl, hl);
-      lh = fmaf(t.a[j], vh, lh);
-      hh = fmaf(t.b[j], vh, hh);
+#pragma unroll
+    for (int j = 0; j < lh_n; j++) {
+      const float2 a = twice(t.a[j]), b = twice(t.b[j]);
+#pragma unroll
+      for (int k = 0; k < TH; k++) {
+        const float2 v = sm[k * W + cc];
+        lo[k] = __ffma2_rn(a, v, lo[k]);
+        hi[k] = __ffma2_rn(b, v, hi[k]);
+      }
       cc += sf;
       if (cc >= W) cc -= W;
     }
-    if (th >= 0.0f) {
-      hl = hard_keep(hl, th);
-      lh = hard_keep(lh, th);
-      hh = hard_keep(hh, th);
+#pragma unroll
+    for (int k = 0; k < TH; k++) {
+      if (i0 + k >= Hp) break;
+      const size_t o = (size_t)(ph + (i0 + k) * sf) * W + c;
+      float lv = lo[k].y, hl = hi[k].x, hh = hi[k].y;
+      if (th >= 0.0f) {
+        hl = hard_keep(hl, th);
+        lv = hard_keep(lv, th);
+        hh = hard_keep(hh, th);
+      }
+      yl[item * s_yl + o] = lo[k].x;
+      float* d = yh + item * s_yh + o;
+      d[0] = lv;
+      d[HW] = hl;
+      d[2 * HW] = hh;
     }
-    ylr[c] = ll;
-    p0[c] = lh;
-    p1[c] = hl;
-    p2[c] = hh;
   }
 }
 
-// --------------------------------------------------------------- synthesis
-// one CTA per (row, item): tl = a * LL + b * HL, th = a * LH + b * HH along the row (taps at c - t sf)
-__global__ void __launch_bounds__(kWvRowThreads) k_rdwt_rows_inv(const float* ll, size_t s_ll, const float* yh,
-                                                                 size_t s_yh, float* tl, float* th, size_t s_t,
-                                                                 int H, int W, int sf, WvTaps t) {
-  extern __shared__ float sm[];
-  float* sll = sm;
-  float* shl = sm + W;
-  float* slh = sm + 2 * W;
-  float* shh = sm + 3 * W;
-  const int r = blockIdx.x, item = blockIdx.y;
-  const size_t HW = (size_t)H * W;
-  const float* q0 = yh + item * s_yh + (size_t)r * W;
-  const float* q = ll + item * s_ll + (size_t)r * W;
-  for (int c = threadIdx.x; c < W; c += kWvRowThreads) {
-    sll[c] = q[c];
-    slh[c] = q0[c];
-    shl[c] = q0[HW + c];
-    shh[c] = q0[2 * HW + c];
+template <int LH, int TH>
+__global__ void __launch_bounds__(kWvThreads, 4)
+    k_rdwt_inv(const float* __restrict__ ll, size_t s_ll, const float* __restrict__ yh, size_t s_yh,
+               float* __restrict__ out, size_t s_out, int H, int W, int sf, const __grid_constant__ WvTaps t) {
+  extern __shared__ float2 sm[];
+  float2 *s1 = sm, *sh = sm + TH / 2 * W;  // [row pair][column]: x1, xh of rows 2 q and 2 q + 1
+  const int ph = blockIdx.x % sf, i0 = blockIdx.x / sf * TH, item = blockIdx.y, Hp = H / sf;
+  const size_t HW = (size_t)H * W, rs = (size_t)sf * W;
+  const float* p = ll + item * s_ll + (size_t)ph * W;
+  const float* q = yh + item * s_yh + (size_t)ph * W;
+  for (int c = threadIdx.x; c < W; c += kWvThreads) {
+    float2 x[TH];  // (x1, xh)
+#pragma unroll
+    for (int k = 0; k < TH; k++) x[k] = twice(0.0f);
+    if constexpr (LH > 0) {
+      int i = (i0 + TH - 1) % Hp;  // input row of output row i0 + k at tap t: i0 + k - t
+#pragma unroll
+      for (int m = 0; m < TH + LH - 1; m++) {
+        const size_t o = i * rs + c;
+        const float2 v = make_float2(__ldg(p + o), __ldg(q + HW + o));           // LL, HL
+        const float2 w = make_float2(__ldg(q + o), __ldg(q + 2 * HW + o));       // LH, HH
+        if (--i < 0) i = Hp - 1;
+#pragma unroll
+        for (int k = 0; k < TH; k++) {
+          const int tt = m - (TH - 1) + k;
+          if (tt >= 0 && tt < LH) x[k] = __ffma2_rn(twice(t.b[tt]), w, __ffma2_rn(twice(t.a[tt]), v, x[k]));
+        }
+      }
+    } else {
+      for (int k = 0; k < TH; k++) {
+        int i = (i0 + k) % Hp;
+        for (int tt = 0; tt < t.lh; tt++) {
+          const size_t o = i * rs + c;
+          const float2 v = make_float2(__ldg(p + o), __ldg(q + HW + o));
+          const float2 w = make_float2(__ldg(q + o), __ldg(q + 2 * HW + o));
+          x[k] = __ffma2_rn(twice(t.b[tt]), w, __ffma2_rn(twice(t.a[tt]), v, x[k]));
+          if (--i < 0) i = Hp - 1;
+        }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < TH; k += 2) {
+      s1[k / 2 * W + c] = make_float2(x[k].x, x[k + 1].x);
+      sh[k / 2 * W + c] = make_float2(x[k].y, x[k + 1].y);
+    }
   }
   __syncthreads();
-  float* outl = tl + item * s_t + (size_t)r * W;
-  float* outh = th + item * s_t + (size_t)r * W;
-  for (int c = threadIdx.x; c < W; c += kWvRowThreads) {
-    float a = 0.0f, b = 0.0f;
+  const int lh_n = LH > 0 ? LH : t.lh;
+  for (int c = threadIdx.x; c < W; c += kWvThreads) {
+    float2 acc[TH / 2];
+#pragma unroll
+    for (int k = 0; k < TH / 2; k++) acc[k] = twice(0.0f);
     int cc = c;
-    for (int k = 0; k < t.lh; k++) {
-      a = fmaf(t.a[k], sll[cc], a);
-      a = fmaf(t.b[k], shl[cc], a);
-      b = fmaf(t.a[k], slh[cc], b);
-      b = fmaf(t.b[k], shh[cc], b);
+#pragma unroll
+    for (int j = 0; j < lh_n; j++) {
+      const float2 a = twice(t.a[j]), b = twice(t.b[j]);
+#pragma unroll
+      for (int k = 0; k < TH / 2; k++) acc[k] = __ffma2_rn(b, sh[k * W + cc], __ffma2_rn(a, s1[k * W + cc], acc[k]));
       cc -= sf;
       if (cc < 0) cc += W;
     }
-    outl[c] = a;
-    outh[c] = b;
+#pragma unroll
+    for (int k = 0; k < TH; k++)
+      if (i0 + k < Hp)
+        out[item * s_out + (size_t)(ph + (i0 + k) * sf) * W + c] = k & 1 ? acc[k / 2].y : acc[k / 2].x;
   }
-}
-
-// x[r][c] = sum_t a[t] tl[(r - t sf) mod H][c] + b[t] th[(r - t sf) mod H][c]
-__global__ void __launch_bounds__(256) k_rdwt_cols_inv(const float* __restrict__ tl, const float* __restrict__ th,
-                                                       size_t s_t, float* __restrict__ x, size_t s_x, int H, int W,
-                                                       int sf, WvTaps t) {
-  const int c = blockIdx.x * 32 + threadIdx.x, r = blockIdx.y * 8 + threadIdx.y, item = blockIdx.z;
-  if (c >= W || r >= H) return;
-  const float* pl = tl + item * s_t + c;
-  const float* ph = th + item * s_t + c;
-  float acc = 0.0f;
-  int rr = r;
-  for (int k = 0; k < t.lh; k++) {
-    acc = fmaf(t.a[k], __ldg(pl + (size_t)rr * W), acc);
-    acc = fmaf(t.b[k], __ldg(ph + (size_t)rr * W), acc);
-    rr -= sf;
-    if (rr < 0) rr += H;
-  }
-  x[item * s_x + (size_t)r * W + c] = acc;
 }
 
 // ----------------------------------------------------- TV correction (Haar)
@@ -157,48 +187,54 @@ __global__ void __launch_bounds__(256) k_rdwt_cols_inv(const float* __restrict__
 // the Haar pair (analysis lo = a x[c] + a x[c+1], hi = a x[c] - a x[c+1];
 // synthesis x = a/2 (lo[c] + lo[c-1]) + a/2 (hi[c] - hi[c-1]), a = 1/sqrt 2):
 // an output pixel reads the 3 x 3 neighbourhood x[r-1..r+1][c-1..c+1].
-constexpr int kTvTx = 32, kTvTy = 8;
-__global__ void __launch_bounds__(kTvTx* kTvTy) k_tv_haar(const float* __restrict__ x, float* __restrict__ y,
-                                                          size_t stride, int H, int W, WvTaps ta, WvTaps ts,
-                                                          float gamma) {
-  __shared__ float tile[kTvTy + 2][kTvTx + 2];  // rows r0-1 .. r0+8, cols c0-1 .. c0+32
-  const int c0 = blockIdx.x * kTvTx, r0 = blockIdx.y * kTvTy, item = blockIdx.z;
+//
+// A warp walks kTvRows rows of 31 output columns (lane 0 holds the column to
+// their left): each lane computes its column's coefficients once per row, the
+// row above's stay in registers and the left column's column synthesis comes
+// from the next lane.  With one output per thread the four coefficient sets of
+// every output, their soft thresholds and the tile's periodic indices were the
+// time (instruction issue; 32 x 256^2: 26 -> 11 us).
+constexpr int kTvRows = 8, kTvWarps = 8, kTvCols = 31;
+__global__ void __launch_bounds__(32 * kTvWarps)
+    k_tv_haar(const float* __restrict__ x, float* __restrict__ y, size_t stride, int H, int W, WvTaps ta, WvTaps ts,
+              float gamma) {
+  const int lane = threadIdx.x, c0 = blockIdx.x * kTvCols, item = blockIdx.z;
+  const int r0 = (blockIdx.y * kTvWarps + threadIdx.y) * kTvRows;
+  if (r0 >= H) return;  // whole warps
+  const int c = (c0 + lane - 1 + W) % W, c1 = c + 1 == W ? 0 : c + 1;  // periodic
   const float* xi = x + item * stride;
-  for (int e = threadIdx.y * kTvTx + threadIdx.x; e < (kTvTy + 2) * (kTvTx + 2); e += kTvTx * kTvTy) {
-    const int i = e / (kTvTx + 2), j = e % (kTvTx + 2);
-    const int rr = ((r0 - 1 + i) % H + H) % H, cc = ((c0 - 1 + j) % W + W) % W;  // periodic, any H, W >= 1
-    tile[i][j] = __ldg(xi + (size_t)rr * W + cc);
-  }
-  __syncthreads();
-  const int r = r0 + threadIdx.y, c = c0 + threadIdx.x;
-  if (r >= H || c >= W) return;
-  // coefficients at (r - dr, c - dc), dr, dc in {0, 1}; tile index of x[r'][c'] is [r' - r0 + 1][c' - c0 + 1]
-  float LL[2][2], LH[2][2], HL[2][2], HH[2][2];
+  auto row = [&](int r, float& l, float& h) {  // rows first (mrdwt_r.h:157-177)
+    const float u = __ldg(xi + (size_t)r * W + c), v = __ldg(xi + (size_t)r * W + c1);
+    l = ta.a[0] * u + ta.a[1] * v;
+    h = ta.b[0] * u + ta.b[1] * v;
+  };
+  int r = r0 ? r0 - 1 : H - 1;
+  float l0, h0;
+  row(r, l0, h0);
+  float LLp = 0.f, LHp = 0.f, HLp = 0.f, HHp = 0.f;  // the row above's coefficients
 #pragma unroll
-  for (int dr = 0; dr < 2; dr++) {
-#pragma unroll
-    for (int dc = 0; dc < 2; dc++) {
-      const int ti = threadIdx.y + 1 - dr, tj = threadIdx.x + 1 - dc;
-      // rows first (mrdwt_r.h:157-177), then columns (:180-206)
-      const float lr0 = ta.a[0] * tile[ti][tj] + ta.a[1] * tile[ti][tj + 1];
-      const float hr0 = ta.b[0] * tile[ti][tj] + ta.b[1] * tile[ti][tj + 1];
-      const float lr1 = ta.a[0] * tile[ti + 1][tj] + ta.a[1] * tile[ti + 1][tj + 1];
-      const float hr1 = ta.b[0] * tile[ti + 1][tj] + ta.b[1] * tile[ti + 1][tj + 1];
-      LL[dr][dc] = ta.a[0] * lr0 + ta.a[1] * lr1;
-      LH[dr][dc] = soft(ta.b[0] * lr0 + ta.b[1] * lr1, gamma);
-      HL[dr][dc] = soft(ta.a[0] * hr0 + ta.a[1] * hr1, gamma);
-      HH[dr][dc] = soft(ta.b[0] * hr0 + ta.b[1] * hr1, gamma);
+  for (int k = -1; k < kTvRows; k++) {
+    if (r0 + k >= H) break;
+    r = r + 1 == H ? 0 : r + 1;
+    float l1, h1;
+    row(r, l1, h1);
+    // then columns (:180-206)
+    const float LL = ta.a[0] * l0 + ta.a[1] * l1;
+    const float LH = soft(ta.b[0] * l0 + ta.b[1] * l1, gamma);
+    const float HL = soft(ta.a[0] * h0 + ta.a[1] * h1, gamma);
+    const float HH = soft(ta.b[0] * h0 + ta.b[1] * h1, gamma);
+    if (k >= 0) {
+      // columns (mirdwt_r.h:163-189): x1 = a LL + b LH, xh = a HL + b HH over rows r, r-1
+      const float x1 = ts.a[0] * LL + ts.b[0] * LH + ts.a[1] * LLp + ts.b[1] * LHp;
+      const float xh = ts.a[0] * HL + ts.b[0] * HH + ts.a[1] * HLp + ts.b[1] * HHp;
+      // rows (:192-213) over columns c, c-1
+      const float x1l = __shfl_up_sync(0xffffffffu, x1, 1), xhl = __shfl_up_sync(0xffffffffu, xh, 1);
+      if (lane > 0 && c0 + lane - 1 < W)
+        y[item * stride + (size_t)(r0 + k) * W + c] = ts.a[0] * x1 + ts.b[0] * xh + ts.a[1] * x1l + ts.b[1] * xhl;
     }
+    l0 = l1, h0 = h1;
+    LLp = LL, LHp = LH, HLp = HL, HHp = HH;
   }
-  // columns (mirdwt_r.h:163-189): x1 = a LL + b LH, xh = a HL + b HH over rows r, r-1
-  float x1[2], xh[2];
-#pragma unroll
-  for (int dc = 0; dc < 2; dc++) {
-    x1[dc] = ts.a[0] * LL[0][dc] + ts.b[0] * LH[0][dc] + ts.a[1] * LL[1][dc] + ts.b[1] * LH[1][dc];
-    xh[dc] = ts.a[0] * HL[0][dc] + ts.b[0] * HH[0][dc] + ts.a[1] * HL[1][dc] + ts.b[1] * HH[1][dc];
-  }
-  // rows (:192-213) over columns c, c-1
-  y[item * stride + (size_t)r * W + c] = ts.a[0] * x1[0] + ts.b[0] * xh[0] + ts.a[1] * x1[1] + ts.b[1] * xh[1];
 }
 
 // ---------------------------------------------------- decimated HH (FP64)
@@ -243,43 +279,69 @@ __global__ void k_sep_residual(const float* __restrict__ img, const float* __res
 // ----------------------------------------------------------------- launchers
 bool rdwt_width_supported(int W) { return W >= 2 && W <= kWvMaxW; }
 
-static cudaError_t set_row_smem() {
-  static cudaError_t once = [] {
-    cudaError_t e = cudaFuncSetAttribute(k_rdwt_rows_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         2 * kWvMaxW * (int)sizeof(float));
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_rdwt_rows_inv, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               4 * kWvMaxW * (int)sizeof(float));
-    return e;
-  }();
-  return once;
+// Rows per CTA: as many as share the taps' rows (8, 4 or 2) while two CTAs fit
+// an SM and the grid fills the GPU; 2 where the width or the grid is small.
+static int rdwt_rows(int n, int H, int W, int sf) {
+  for (int th : {8, 4})
+    if ((size_t)2 * th * W * sizeof(float) <= 110 * 1024 && (long)n * sf * ((H / sf + th - 1) / th) >= 2 * 152)
+      return th;
+  return 2;
 }
+
+template <class K, class... Args>
+static cudaError_t launch_rdwt(K kernel, int th, int n, int H, int W, int sf, cudaStream_t st, Args... args) {
+  const size_t sm = (size_t)2 * th * W * sizeof(float);
+  if (sm > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return e;
+  }
+  count_launch();
+  kernel<<<dim3((unsigned)(sf * ((H / sf + th - 1) / th)), (unsigned)n), kWvThreads, sm, st>>>(args...);
+  return cudaGetLastError();
+}
+
+// the lengths of the Haar, Daubechies, Symmlet, Coiflet-1..3 and Beylkin filters
+#define NSST_RDWT_LENS(X) X(2) X(4) X(6) X(8) X(10) X(12) X(14) X(16) X(18) X(20)
 
 cudaError_t launch_rdwt_level(const WvPlanes& P, int n, int H, int W, int sf, const WvTaps& t, const float* thr,
                               cudaStream_t st) {
   if (!rdwt_width_supported(W) || t.lh < 1 || t.lh > kMaxQmf || n < 1 || n > 65535) return cudaErrorInvalidValue;
-  const cudaError_t e = set_row_smem();
-  if (e != cudaSuccess) return e;
-  const dim3 cb(32, 8), cg((W + 31) / 32, (H + 7) / 8, n);
-  count_launch(2);
-  k_rdwt_cols_fwd<<<cg, cb, 0, st>>>(P.cur, P.s_cur, P.yh, P.s_yh, H, W, sf, t);
-  k_rdwt_rows_fwd<<<dim3(H, n), kWvRowThreads, 2 * W * sizeof(float), st>>>(P.yl, P.s_yl, P.yh, P.s_yh, H, W, sf,
-                                                                             t, thr);
-  return cudaGetLastError();
+#define GO(l, h)                                                                                                   \
+  launch_rdwt(k_rdwt_fwd<l, h>, h, n, H, W, sf, st, P.cur, P.s_cur, P.yl, P.s_yl, P.yh, P.s_yh, H, W, sf, t, thr)
+#define CASE(l)                                         \
+  case l:                                               \
+    switch (rdwt_rows(n, H, W, sf)) {             \
+      case 8: return GO(l, 8);                          \
+      case 4: return GO(l, 4);                          \
+      default: return GO(l, 2);                         \
+    }
+  switch (t.lh) {
+    NSST_RDWT_LENS(CASE)
+    default:
+      return GO(0, 2);
+  }
+#undef CASE
+#undef GO
 }
 
-cudaError_t launch_irdwt_level(const float* ll, size_t s_ll, const float* yh, size_t s_yh, float* tl, float* th,
-                               size_t s_t, float* x, size_t s_x, int n, int H, int W, int sf, const WvTaps& t,
-                               cudaStream_t st) {
+cudaError_t launch_irdwt_level(const float* ll, size_t s_ll, const float* yh, size_t s_yh, float* x, size_t s_x, int n,
+                               int H, int W, int sf, const WvTaps& t, cudaStream_t st) {
   if (!rdwt_width_supported(W) || t.lh < 1 || t.lh > kMaxQmf || n < 1 || n > 65535) return cudaErrorInvalidValue;
-  const cudaError_t e = set_row_smem();
-  if (e != cudaSuccess) return e;
-  count_launch(2);
-  k_rdwt_rows_inv<<<dim3(H, n), kWvRowThreads, 4 * W * sizeof(float), st>>>(ll, s_ll, yh, s_yh, tl, th, s_t, H, W,
-                                                                             sf, t);
-  const dim3 cb(32, 8), cg((W + 31) / 32, (H + 7) / 8, n);
-  k_rdwt_cols_inv<<<cg, cb, 0, st>>>(tl, th, s_t, x, s_x, H, W, sf, t);
-  return cudaGetLastError();
+#define GO(l, h) launch_rdwt(k_rdwt_inv<l, h>, h, n, H, W, sf, st, ll, s_ll, yh, s_yh, x, s_x, H, W, sf, t)
+#define CASE(l)                                         \
+  case l:                                               \
+    switch (rdwt_rows(n, H, W, sf)) {             \
+      case 8: return GO(l, 8);                          \
+      case 4: return GO(l, 4);                          \
+      default: return GO(l, 2);                         \
+    }
+  switch (t.lh) {
+    NSST_RDWT_LENS(CASE)
+    default:
+      return GO(0, 2);
+  }
+#undef CASE
+#undef GO
 }
 
 cudaError_t launch_tv_haar(const float* x, float* y, size_t stride, int n, int H, int W, float a, float gamma,
@@ -288,7 +350,8 @@ cudaError_t launch_tv_haar(const float* x, float* y, size_t stride, int n, int H
   const std::vector<double> haar = {(double)a, (double)a};
   const WvTaps ta = analysis_taps(haar), ts = synthesis_taps(haar);
   count_launch();
-  k_tv_haar<<<dim3((W + kTvTx - 1) / kTvTx, (H + kTvTy - 1) / kTvTy, n), dim3(kTvTx, kTvTy), 0, st>>>(
+  const int rows = kTvRows * kTvWarps;
+  k_tv_haar<<<dim3((W + kTvCols - 1) / kTvCols, (H + rows - 1) / rows, n), dim3(32, kTvWarps), 0, st>>>(
       x, y, stride, H, W, ta, ts, gamma);
   return cudaGetLastError();
 }

@@ -2819,32 +2819,42 @@ nsst_status check_rdwt(int n, int H, int W, int lh, int L) {
   return NSST_OK;
 }
 
-// mrdwt_r.h:135-208 for n images (x item stride s_x; yl item stride HW; yh
-// item stride 3 L HW); thr (device, n floats) hard-thresholds every highpass
-// plane as it is written (thresh.m:44 with option 1), or NULL.
-nsst_status enqueue_mrdwt(const float* x, size_t s_x, int n, int H, int W, const WvTaps& t, int L, float* yl,
-                          float* yh, const float* thr, cudaStream_t st) {
+bool overlap(const float* a, const float* b, size_t n) { return a < b + n && b < a + n; }
+
+// mrdwt_r.h:135-208 for n images (item strides: x, yl HW; yh 3 L HW); thr
+// (device, n floats) hard-thresholds every highpass plane as it is written
+// (thresh.m:44 with option 1), or NULL.  A level's lowpass goes to yl and to
+// s0 (n images) in turn, the last one to yl; where that makes the first level
+// write the images it reads (x overlaps yl), to s1 instead (n images; may be
+// NULL if x does not overlap yl).
+nsst_status enqueue_mrdwt(const float* x, int n, int H, int W, const WvTaps& t, int L, float* yl, float* yh,
+                          const float* thr, float* s0, float* s1, cudaStream_t st) {
   const size_t HW = (size_t)H * W;
+  const float* cur = x;
   for (int l = 1; l <= L; l++) {
-    const WvPlanes P{l == 1 ? x : yl, l == 1 ? s_x : HW, yl, HW, yh + (size_t)3 * (l - 1) * HW, (size_t)3 * L * HW};
+    float* dst = (L - l) % 2 == 0 ? yl : s0;
+    if (l == 1 && dst == yl && overlap(x, yl, n * HW)) dst = s1;
+    const WvPlanes P{cur, HW, dst, HW, yh + (size_t)3 * (l - 1) * HW, (size_t)3 * L * HW};
     NSST_CUDA(launch_rdwt_level(P, n, H, W, 1 << (l - 1), t, thr, st));
+    cur = dst;
   }
+  if (cur != yl) NSST_CUDA(cudaMemcpyAsync(yl, cur, n * HW * sizeof(float), cudaMemcpyDeviceToDevice, st));
   return NSST_OK;
 }
 
-// mirdwt_r.h:148-218 for n images.  scratch == NULL: each level's HL / LH
-// planes take the row pass's outputs (yh is consumed); otherwise scratch holds
-// two planes per image.
-nsst_status enqueue_mirdwt(const float* yl, float* yh, float* scratch, int n, int H, int W, const WvTaps& t, int L,
-                           float* x, cudaStream_t st) {
+// mirdwt_r.h:148-218 for n images; s0 and s1 as above, with x in yl's place and
+// the last level's yl in x's.
+nsst_status enqueue_mirdwt(const float* yl, const float* yh, int n, int H, int W, const WvTaps& t, int L, float* x,
+                           float* s0, float* s1, cudaStream_t st) {
   const size_t HW = (size_t)H * W, s_yh = (size_t)3 * L * HW;
+  const float* cur = yl;
   for (int l = L; l >= 1; l--) {
-    float* lev = yh + (size_t)3 * (l - 1) * HW;
-    float* tl = scratch ? scratch : lev + HW;
-    float* th = scratch ? scratch + HW : lev;
-    const size_t s_t = scratch ? 2 * HW : s_yh;
-    NSST_CUDA(launch_irdwt_level(l == L ? yl : x, HW, lev, s_yh, tl, th, s_t, x, HW, n, H, W, 1 << (l - 1), t, st));
+    float* dst = (l - 1) % 2 == 0 ? x : s0;
+    if (l == L && dst == x && overlap(yl, x, n * HW)) dst = s1;
+    NSST_CUDA(launch_irdwt_level(cur, HW, yh + (size_t)3 * (l - 1) * HW, s_yh, dst, HW, n, H, W, 1 << (l - 1), t, st));
+    cur = dst;
   }
+  if (cur != x) NSST_CUDA(cudaMemcpyAsync(x, cur, n * HW * sizeof(float), cudaMemcpyDeviceToDevice, st));
   return NSST_OK;
 }
 
@@ -2904,7 +2914,14 @@ nsst_status nsst_mrdwt(const float* x, int n, int H, int W, const double* h, int
   if (!x || !h || !yl || !yh) return fail(NSST_ERR_INVALID_ARG, "NULL argument");
   NSST_TRY(check_rdwt(n, H, W, lh, L));
   const WvTaps t = analysis_taps(std::vector<double>(h, h + lh));
-  return enqueue_mrdwt(x, (size_t)H * W, n, H, W, t, L, yl, yh, nullptr, (cudaStream_t)stream);
+  cudaStream_t st = (cudaStream_t)stream;
+  const size_t nHW = (size_t)n * H * W;
+  const bool over = overlap(x, yl, nHW);
+  AsyncScratch s;
+  s.st = st;
+  if (L > 1 || over) NSST_CUDA(cudaMallocAsync(&s.ptr, sizeof(float) * (over ? 2 : 1) * nHW, st));
+  float* s0 = (float*)s.ptr;
+  return enqueue_mrdwt(x, n, H, W, t, L, yl, yh, nullptr, s0, over ? s0 + nHW : nullptr, st);
 }
 
 nsst_status nsst_mirdwt(const float* yl, const float* yh, int n, int H, int W, const double* h, int lh, int L,
@@ -2913,11 +2930,13 @@ nsst_status nsst_mirdwt(const float* yl, const float* yh, int n, int H, int W, c
   NSST_TRY(check_rdwt(n, H, W, lh, L));
   const WvTaps t = synthesis_taps(std::vector<double>(h, h + lh));
   cudaStream_t st = (cudaStream_t)stream;
+  const size_t nHW = (size_t)n * H * W;
+  const bool over = overlap(yl, x, nHW);
   AsyncScratch s;
   s.st = st;
-  NSST_CUDA(cudaMallocAsync(&s.ptr, sizeof(float) * 2 * (size_t)n * H * W, st));
-  // the scratch variant only reads yh
-  return enqueue_mirdwt(yl, const_cast<float*>(yh), (float*)s.ptr, n, H, W, t, L, x, st);
+  if (L > 1 || over) NSST_CUDA(cudaMallocAsync(&s.ptr, sizeof(float) * (over ? 2 : 1) * nHW, st));
+  float* s0 = (float*)s.ptr;
+  return enqueue_mirdwt(yl, yh, n, H, W, t, L, x, s0, over ? s0 + nHW : nullptr, st);
 }
 
 nsst_status nsst_tv_correction(const float* x, int n, int H, int W, double gamma, float* y, void* stream) {
@@ -2978,7 +2997,7 @@ nsst_status nsst_separate(nsst_plan* p, const float* img, int n, int level2, int
                b_hh = seg(sizeof(double) * n * (HW / 4));
   AsyncScratch ws;
   ws.st = st;
-  NSST_CUDA(cudaMallocAsync(&ws.ptr, 5 * b_plane + b_yh + b_ths + b_thw + b_bits + b_hh, st));
+  NSST_CUDA(cudaMallocAsync(&ws.ptr, 6 * b_plane + b_yh + b_ths + b_thw + b_bits + b_hh, st));
   char* q = (char*)ws.ptr;
   auto take = [&q](size_t b) {
     char* r = q;
@@ -2990,6 +3009,7 @@ nsst_status nsst_separate(nsst_plan* p, const float* img, int n, int level2, int
   float* ra2 = (float*)take(b_plane);
   float* S = (float*)take(b_plane);
   float* yl = (float*)take(b_plane);
+  float* wlow = (float*)take(b_plane);  // the wavelet levels' other lowpass buffer
   float* yh = (float*)take(b_yh);
   float* thS = (float*)take(b_ths);
   float* thW = (float*)take(b_thw);
@@ -3041,7 +3061,7 @@ nsst_status nsst_separate(nsst_plan* p, const float* img, int n, int level2, int
   NSST_TRY(enqueue_band_maxima(p, n, xw.data(), bits, st));
   // separate.m:119-126: buff(2) = max |yh| of the Symmlet-4 mrdwt, per image
   NSST_CUDA(cudaMemsetAsync(bits + (size_t)n * nb, 0, sizeof(unsigned) * n * 3 * L, st));
-  NSST_TRY(enqueue_mrdwt(imgw, HW, n, H, W, ta, L, yl, yh, nullptr, st));
+  NSST_TRY(enqueue_mrdwt(imgw, n, H, W, ta, L, yl, yh, nullptr, wlow, nullptr, st));
   NSST_CUDA(launch_plane_maxabs(yh, HW, n * 3 * L, bits + (size_t)n * nb, kRedBlocks, st));
   NSST_CUDA(cudaMemcpyAsync(hb, bits, sizeof(unsigned) * nbits, cudaMemcpyDeviceToHost, st));
   // the noise estimates on the host cores while the maxima are computed
@@ -3105,8 +3125,8 @@ nsst_status nsst_separate(nsst_plan* p, const float* img, int n, int level2, int
     NSST_CUDA(cudaEventRecord(p->fork_ev, st));
     NSST_CUDA(cudaStreamWaitEvent(sd, p->fork_ev, 0));
     // points: wavelet hard threshold (second stream)
-    NSST_TRY(enqueue_mrdwt(ra2, HW, n, H, W, ta, L, yl, yh, thW + (size_t)k * n, sd));
-    NSST_TRY(enqueue_mirdwt(yl, yh, nullptr, n, H, W, ts, L, P, sd));
+    NSST_TRY(enqueue_mrdwt(ra2, n, H, W, ta, L, yl, yh, thW + (size_t)k * n, wlow, nullptr, sd));
+    NSST_TRY(enqueue_mirdwt(yl, yh, n, H, W, ts, L, P, wlow, nullptr, sd));
     NSST_CUDA(cudaEventRecord(p->join_ev, sd));
     // curves: shearlet hard threshold, then TV correction
     NSST_TRY(enqueue_denoise(p, n, xs.data(), os.data(), NSST_THRESH_HARD, true, st, false,
