@@ -59,10 +59,10 @@ typedef struct nsst_config {
                                    allow it.  nsst_shear_trans,
                                    nsst_inverse_shear, nsst_atrousdec,
                                    nsst_atrousrec, the differentiable denoise
-                                   (forward and backward), the separation and
-                                   the operator adjoints follow the same
-                                   mode; calls that pass images not 16-byte
-                                   aligned and nsst_re_weight_band use the
+                                   (forward and backward), the separation,
+                                   nsst_re_weight_band and the operator
+                                   adjoints follow the same mode; calls that
+                                   pass images not 16-byte aligned use the
                                    direct pyramid. */
 } nsst_config;
 

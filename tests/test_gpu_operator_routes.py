@@ -38,3 +38,24 @@ def test_adjoints_on_the_spectral_pyramid_match_the_direct_one(sc, H, W, lpfilt,
     Ax = sc.shear_trans_cuda(x, lpfilt, plans[0])
     lhs, rhs = float((Ax.double() * c.double()).sum()), float((x.double() * a.double()).sum())
     assert abs(lhs - rhs) <= 1e-6 * float(Ax.double().norm() * c.double().norm())
+
+
+@pytest.mark.parametrize('H,W,lpfilt', [(192, 256, 'maxflat'), (384, 192, '9-7'), (512, 384, 'pyr'),
+                                        (256, 1024, 'pyrexc')])
+@pytest.mark.parametrize('levels', [1, 2, 4])
+def test_band_weights_on_the_spectral_pyramid_match_the_direct_one(sc, H, W, lpfilt, levels):
+    import torch
+    plans = [sc.prepare_shearing_filters_cuda([3, 3, 4, 4], [32, 32, 16, 16], H, W, lpfilt=lpfilt, pyramid=m)
+             for m in (sc.PYRAMID_AUTO, sc.PYRAMID_DIRECT)]
+    g = torch.Generator(device='cuda').manual_seed(H + levels)
+    x = 100 + 20 * torch.randn((H, W), device='cuda', generator=g)
+    w = [0.1, 1.5, 0.0, 2.0, -1.0][:levels + 1]
+    a, d = (sc.re_weight_band(x, w, p) for p in plans)
+    assert _rel(a, d) <= 1e-5
+    # in place, and from an image that is not 16-byte aligned (the direct pyramid)
+    y = x.clone()
+    assert torch.equal(sc.re_weight_band(y, w, plans[0], out=y), a)
+    buf = torch.empty(H * W + 1, device='cuda')
+    xm = buf[1:].view(H, W)
+    xm.copy_(x)
+    assert torch.equal(sc.re_weight_band(xm, w, plans[0], out=torch.empty_like(x)), d)
