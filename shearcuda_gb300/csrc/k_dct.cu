@@ -43,6 +43,7 @@
 // (c2r / r2c pre- and post-processing) of the directional kernels.
 #include "internal.h"
 #include "tiles.cuh"
+#include "tma.cuh"
 
 namespace nsst {
 
@@ -317,6 +318,81 @@ __global__ void __launch_bounds__(RowCfg<WH>::T, DctMinB<RowCfg<WH>::T>::value)
   }
 }
 
+// The same for few row tiles: a cluster of four CTAs per tile, CTA q
+// transforming level q (up to four levels), then owning a quarter of the
+// tile's rows: their sums over the levels come through distributed shared
+// memory, in the levels' order and with the FMAs of k_dct_rows_syn, so both
+// give the same bits.  A tile's chain is one level's transforms instead of
+// four: what bounds one or a few images, whose tiles do not fill the GPU (one
+// denoise of 512 x 512 198 -> 160 us, of 2048 x 2048 1.87 -> 1.82 ms).
+constexpr int kSynRanks = 4;
+template <int WH>
+__global__ void __cluster_dims__(1, 1, kSynRanks) __launch_bounds__(RowCfg<WH>::T, DctMinB<RowCfg<WH>::T>::value)
+    k_dct_rows_syn_split(const RowJob* __restrict__ jobs, int n_active, int nlev, size_t lev_stride,
+                         const float2* src_base, float2* dst_base, const float* __restrict__ xbase, size_t xstride,
+                         const float* __restrict__ resp, size_t resp_stride, const float* __restrict__ tlow,
+                         const float2* __restrict__ twWh, const float2* __restrict__ twW,
+                         const float4* __restrict__ tw) {
+  using C = RowCfg<WH>;
+  constexpr int W = 2 * WH, LD = WH + 2, RR = C::RS / kSynRanks;  // rows a CTA finishes
+  extern __shared__ float2 smem[];
+  float2* A = smem;               // transform tile
+  float2* S = smem + C::RS * LD;  // the level's DCT-II coefficients
+  const RowJob job = jobs[blockIdx.y];
+  if (job.item >= n_active) return;  // the whole cluster
+  const int rank = blockIdx.z;
+  const size_t off = (size_t)blockIdx.x * C::RS * WH;
+  if (rank < nlev) {
+    fetch_rows_rm<WH, C::RS, C::T>(A, src_base + job.src + (size_t)rank * lev_stride + off);
+    cp_async_wait_all();
+    __syncthreads();
+    block_fft_hook_ip<WH, C::RS, C::T, +1>(A, twWh, C2RPreLdRM<WH>{A, twW}, DctShufStRM<WH>{A});
+    block_fft_hook_ip<WH, C::RS, C::T, -1>(A, twWh, SmemLdRM<WH>{A}, SmemStRM<WH>{A});
+    for (int e = threadIdx.x; e < WH * C::RS; e += C::T) {
+      const int k = e % WH, s = e / WH;
+      float ck, cm;
+      dct2_row_pair<WH>(A + s * LD, k, tw, ck, cm);
+      float* c = reinterpret_cast<float*>(S + s * LD);
+      c[k] = ck;
+      c[k == 0 ? WH : W - k] = cm;
+    }
+  }
+  cluster_barrier();
+  // sums of rows rank RR .. + RR - 1, in A behind the rows of the transform below
+  const size_t orow = off + (size_t)rank * RR * WH;
+  {
+    const float4* X = reinterpret_cast<const float4*>(xbase + (size_t)job.item * xstride + 2 * orow);
+    const float4* T = reinterpret_cast<const float4*>(tlow + 2 * orow);
+    const float4* Q = reinterpret_cast<const float4*>(resp + 2 * orow);
+    for (int e = threadIdx.x; e < RR * (WH / 2); e += C::T) {
+      const int s = e / (WH / 2), c = e - s * (WH / 2);
+      const float4 x = X[e], t = __ldg(&T[e]);
+      float4 a = make_float4(x.x * t.x, x.y * t.y, x.z * t.z, x.w * t.w);
+      const uint32_t local = smem_u32(S + (rank * RR + s) * LD + 2 * c);
+      for (int l = 0; l < nlev; l++) {
+        const float4 y = ld_cluster4(mapa(local, l)), q = __ldg(&Q[(size_t)l * (resp_stride / 4) + e]);
+        a = make_float4(fmaf(y.x, q.x, a.x), fmaf(y.y, q.y, a.y), fmaf(y.z, q.z, a.z), fmaf(y.w, q.w, a.w));
+      }
+      *reinterpret_cast<float4*>(A + (RR + s) * LD + 2 * c) = a;
+    }
+  }
+  cluster_barrier();  // the sums are in place, and no peer reads S any more
+  constexpr int NP = WH / 2 + 1;
+  for (int e = threadIdx.x; e < RR * NP; e += C::T) {
+    const int s = e / NP, k = e - s * NP;
+    const float* sr = rowf<WH>(A, RR + s);
+    dct3_pre_pair<WH>([&](int j) { return sr[j]; }, k, tw, A + s * LD);
+  }
+  __syncthreads();
+  block_fft_hook_ip<WH, RR, C::T, +1>(A, twWh, SmemLdRM<WH>{A}, SmemStRM<WH>{A});
+  float2* dst = dst_base + job.dst + orow;
+  for (int e = threadIdx.x; e < WH * RR; e += C::T) {
+    const int m = e % WH, s = e / WH;
+    const float* v = rowf<WH>(A, s);
+    dst[(size_t)s * WH + m] = make_float2(v[m], v[W - 1 - m]);
+  }
+}
+
 // ---------------------------------------------------------------------------
 // Column kernels, grid = (WH / CS, jobs): CS columns of a packed H x WH array.
 // ---------------------------------------------------------------------------
@@ -460,6 +536,7 @@ cudaError_t prepare_dct_kernels(int H, int WH) {
     if (e == cudaSuccess) e = dct_opt_in(k_dct_rows_ana<n, true>, RowCfg<n>::smem_rm()); \
     if (e == cudaSuccess) e = dct_opt_in(k_dct_rows_syn<n, false>, 2 * RowCfg<n>::smem_rm()); \
     if (e == cudaSuccess) e = dct_opt_in(k_dct_rows_syn<n, true>, 2 * RowCfg<n>::smem_rm()); \
+    if (e == cudaSuccess) e = dct_opt_in(k_dct_rows_syn_split<n>, 2 * RowCfg<n>::smem_rm()); \
     break;
     NSST_DCT_ROW_SIZES(CASE)
 #undef CASE
@@ -531,6 +608,12 @@ cudaError_t launch_dct_rows_ana(const RowJob* jobs, int njobs, int n_active, int
   }
 }
 
+// Row tiles up to which the synthesis rows run as clusters: eight per SM.
+// Measured (one denoise, us, serial / cluster): 1024 tiles (16 x 512^2) 1203 /
+// 1182, 1536 (12 x 1024^2) 4010 / 3985, 2048 (64 x 256^2) 1226 / 1274, 4096
+// (64 x 512^2) 4329 / 4355.
+static bool syn_splits(long tiles) { return tiles <= 8 * 152; }
+
 cudaError_t launch_dct_rows_syn(const RowJob* jobs, int njobs, int n_active, int nlev, size_t lev_stride, int H,
                                 int W, const void* src_base, void* dst_base, const float* xbase, size_t xstride,
                                 const float* resp, size_t resp_stride, const float* tlow, const float2* twWh,
@@ -544,7 +627,10 @@ cudaError_t launch_dct_rows_syn(const RowJob* jobs, int njobs, int n_active, int
   case n_: {                                                                                                  \
     const dim3 grid(H / RowCfg<n_>::RS, njobs);                                                               \
     constexpr size_t sm = 2 * RowCfg<n_>::smem_rm();                                                          \
-    if (real_in)                                                                                              \
+    if (!real_in && nlev <= kSynRanks && syn_splits((long)grid.x * std::min(n_active, njobs)))                \
+      k_dct_rows_syn_split<n_><<<dim3(grid.x, njobs, kSynRanks), RowCfg<n_>::T, sm, st>>>(                    \
+          jobs, n_active, nlev, lev_stride, sb, db, xbase, xstride, resp, resp_stride, tlow, twWh, twW, twD); \
+    else if (real_in)                                                                                         \
       k_dct_rows_syn<n_, true><<<grid, RowCfg<n_>::T, sm, st>>>(jobs, n_active, nlev, lev_stride, sb, db, xbase, \
                                                                xstride, resp, resp_stride, tlow, twWh, twW, twD); \
     else                                                                                                      \
