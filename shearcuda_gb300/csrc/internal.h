@@ -312,6 +312,7 @@ struct V3Ops {
   cudaError_t (*real)(int dir, const V3Real&, const float2* tw, int items, cudaStream_t);
   cudaError_t (*cols)(int dir, int ld, int st, const V3Cols&, const float2* tw, int npairs, cudaStream_t);
   cudaError_t (*pair)(int dir, const V3Pair&, const float2* tw, int shares, cudaStream_t);
+  cudaError_t (*prepare)();  // once per device, before the first launch
   bool pyr, conv;
 };
 const V3Ops* v3_ops(int n);  // nullptr: length not compiled

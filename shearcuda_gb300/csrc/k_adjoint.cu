@@ -10,11 +10,13 @@
 // * threshold: the subgradient mask 1[|c| > t]; for the soft rule the
 //   threshold's own gradient is -sum sign(c) g 1[|c| > t] (per band).
 #include "internal.h"
+#include "launch.cuh"
 
 namespace nsst {
 
 // out[i][j] (+)= fold(Z1, E1) + fold(Z2, E2), each Z of size (H+2E) x (W+2E).
 __global__ void k_fold(const __grid_constant__ FoldJobs jobs, int H, int W, int E1, int E2, int accumulate) {
+  pdl_sync();
   const FoldJob& job = jobs.j[blockIdx.y];
   const int W1 = W + 2 * E1, W2 = W + 2 * E2;
   const size_t total = (size_t)H * W;
@@ -52,7 +54,7 @@ cudaError_t launch_fold(const FoldJobs& jobs, int njobs, int H, int W, int E1, i
   const size_t total = (size_t)H * W;
   int bx = (int)std::min<size_t>((total + 255) / 256, 1024);
   count_launch();
-  k_fold<<<dim3(bx, njobs), 256, 0, st>>>(jobs, H, W, E1, E2, accumulate ? 1 : 0);
+  launch_pdl(k_fold, dim3(bx, njobs), 256, 0, st, jobs, H, W, E1, E2, accumulate ? 1 : 0);
   return cudaGetLastError();
 }
 
@@ -60,6 +62,7 @@ cudaError_t launch_fold(const FoldJobs& jobs, int njobs, int H, int W, int E1, i
 // threshold gradient -sum g sign(c) 1[|c| > t] into partials[slot0 + item*nblk + blk].
 __global__ void k_lowpass_backward(const __grid_constant__ FoldJobs jobs, size_t n, const float* __restrict__ tau,
                                    int mode, float* __restrict__ partials, int slot0) {
+  pdl_sync();
   const FoldJob& job = jobs.j[blockIdx.y];  // z1 = c, z2 = g, out = g_c
   const float t = tau[0];
   float part = 0.0f;
@@ -84,7 +87,7 @@ cudaError_t launch_lowpass_backward(const FoldJobs& jobs, int njobs, size_t n, c
                                     float* partials, int slot0, int nblk, cudaStream_t st) {
   if (njobs == 0) return cudaSuccess;
   count_launch();
-  k_lowpass_backward<<<dim3(nblk, njobs), 256, 0, st>>>(jobs, n, tau, mode, partials, slot0);
+  launch_pdl(k_lowpass_backward, dim3(nblk, njobs), 256, 0, st, jobs, n, tau, mode, partials, slot0);
   return cudaGetLastError();
 }
 
@@ -92,6 +95,7 @@ cudaError_t launch_lowpass_backward(const FoldJobs& jobs, int njobs, size_t n, c
 // fixed summation order (deterministic).
 __global__ void k_reduce_tau(const float* __restrict__ partials, int cnt, size_t stride, float* __restrict__ grad_tau,
                              int accumulate) {
+  pdl_sync();
   const int b = blockIdx.x;
   double part = 0.0;
   for (int i = threadIdx.x; i < cnt; i += blockDim.x) part += partials[(size_t)b * stride + i];
@@ -108,19 +112,20 @@ __global__ void k_reduce_tau(const float* __restrict__ partials, int cnt, size_t
 cudaError_t launch_reduce_tau(const float* partials, int count, size_t stride, int nbands, float* grad_tau,
                               bool accumulate, cudaStream_t st) {
   count_launch();
-  k_reduce_tau<<<nbands, 256, 0, st>>>(partials, count, stride, grad_tau, accumulate ? 1 : 0);
+  launch_pdl(k_reduce_tau, nbands, 256, 0, st, partials, count, stride, grad_tau, accumulate ? 1 : 0);
   return cudaGetLastError();
 }
 
 // Copy the shared per-band thresholds into every item's threshold row.
 __global__ void k_broadcast_tau(const float* __restrict__ tau, float* __restrict__ th, int nbands, int n) {
+  pdl_sync();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nbands * n; i += gridDim.x * blockDim.x)
     th[i] = tau[i % nbands];
 }
 
 cudaError_t launch_broadcast_tau(const float* tau, float* th, int nbands, int n, cudaStream_t st) {
   count_launch();
-  k_broadcast_tau<<<std::max(1, std::min(64, (nbands * n + 255) / 256)), 256, 0, st>>>(tau, th, nbands, n);
+  launch_pdl(k_broadcast_tau, std::max(1, std::min(64, (nbands * n + 255) / 256)), 256, 0, st, tau, th, nbands, n);
   return cudaGetLastError();
 }
 

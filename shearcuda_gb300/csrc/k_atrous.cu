@@ -24,6 +24,7 @@
 #include <mutex>
 
 #include "internal.h"
+#include "launch.cuh"
 #include "tiles.cuh"
 
 namespace nsst {
@@ -120,6 +121,7 @@ template <int FA, int FB, bool ZERO = false, int P = kAtP, bool ZR = false>
 __global__ void __launch_bounds__(kAtThreads, (FA <= 13 && FB == 0) ? 4 : 3) k_atrous(const __grid_constant__ AtrousJobs jobs, int M,
                                                         const __grid_constant__ AtrousTaps<FA> ta,
                                                         const __grid_constant__ AtrousTaps<FB> tb) {
+  pdl_sync();
   extern __shared__ float at_smem[];
   __shared__ float s_taps[(FA > FB ? FA * FA : FB * FB)];
   __shared__ int s_cols[(FA > FB ? FA : FB)];
@@ -242,14 +244,14 @@ static cudaError_t launch_atrous_t(const AtrousJobs& jobs, int njobs, int maxH, 
   if ((size_t)grid.x * grid.y * grid.z < (size_t)2 * sm_count()) {  // half-height tiles: twice the CTAs
     grid.y = M * ((nprow_max + kAtPSmall * kAtTY - 1) / (kAtPSmall * kAtTY));
     if (zr)
-      k_atrous<FA, FB, false, kAtPSmall, true><<<grid, kAtThreads, sm, st>>>(jobs, M, ta, tb);
+      launch_pdl(k_atrous<FA, FB, false, kAtPSmall, true>, grid, kAtThreads, sm, st, jobs, M, ta, tb);
     else
-      k_atrous<FA, FB, false, kAtPSmall><<<grid, kAtThreads, sm, st>>>(jobs, M, ta, tb);
+      launch_pdl(k_atrous<FA, FB, false, kAtPSmall>, grid, kAtThreads, sm, st, jobs, M, ta, tb);
   } else {
     if (zr)
-      k_atrous<FA, FB, false, kAtP, true><<<grid, kAtThreads, sm, st>>>(jobs, M, ta, tb);
+      launch_pdl(k_atrous<FA, FB, false, kAtP, true>, grid, kAtThreads, sm, st, jobs, M, ta, tb);
     else
-      k_atrous<FA, FB, false><<<grid, kAtThreads, sm, st>>>(jobs, M, ta, tb);
+      launch_pdl(k_atrous<FA, FB, false>, grid, kAtThreads, sm, st, jobs, M, ta, tb);
   }
   return cudaGetLastError();
 }
@@ -266,9 +268,9 @@ static cudaError_t launch_atrous_full_t(const AtrousJobs& jobs, int njobs, int m
   dim3 grid((maxWo + kAtTX - 1) / kAtTX, M * ((nprow_max + kAtRows - 1) / kAtRows), njobs);
   count_launch();
   if (zero_rows_1(h, F))  // the same filter structure as the forward steps
-    k_atrous<F, 0, true, kAtP, true><<<grid, kAtThreads, sm, st>>>(jobs, M, ta, tb);
+    launch_pdl(k_atrous<F, 0, true, kAtP, true>, grid, kAtThreads, sm, st, jobs, M, ta, tb);
   else
-    k_atrous<F, 0, true><<<grid, kAtThreads, sm, st>>>(jobs, M, ta, tb);
+    launch_pdl(k_atrous<F, 0, true>, grid, kAtThreads, sm, st, jobs, M, ta, tb);
   return cudaGetLastError();
 }
 
@@ -324,6 +326,7 @@ constexpr int kThreshVec = 4;  // 16-byte loads per thread
 template <bool VEC>
 __global__ void __launch_bounds__(256) k_thresh_bands(float* __restrict__ data, size_t n, const float* __restrict__ thr,
                                                       int mode) {
+  pdl_sync();
   const float th = thr[blockIdx.y];
   float* band = data + blockIdx.y * n;
   if (VEC) {
@@ -352,9 +355,9 @@ cudaError_t launch_thresh_bands(float* data, size_t n, int nbands, const float* 
   const size_t per = 256 * 4 * kThreshVec;
   const dim3 grid((unsigned)((n + per - 1) / per), (unsigned)nbands);
   if (n % 4 == 0 && ((uintptr_t)data & 15) == 0)
-    k_thresh_bands<true><<<grid, 256, 0, st>>>(data, n, thr, mode);
+    launch_pdl(k_thresh_bands<true>, grid, 256, 0, st, data, n, thr, mode);
   else
-    k_thresh_bands<false><<<grid, 256, 0, st>>>(data, n, thr, mode);
+    launch_pdl(k_thresh_bands<false>, grid, 256, 0, st, data, n, thr, mode);
   return cudaGetLastError();
 }
 

@@ -20,6 +20,7 @@
 // the staging buffer (the after-read hook), so the copy overlaps the rest of
 // band k's transform, as the cp.async form does.
 #include "internal.h"
+#include "launch.cuh"
 #include "tiles.cuh"
 #include "tma.cuh"
 
@@ -111,6 +112,7 @@ __global__ void __launch_bounds__(AnaCfg<H>::T, AnaCfg<H>::MINB)
                            int WH, float2* dst_base, const float2* __restrict__ spec_base, int spec_row0,
                            size_t band_stride, const float2* __restrict__ twH, const float2* __restrict__ wd,
                            int* err, int per_level) {
+  pdl_sync();
   using C = AnaCfg<H>;
   constexpr int CS = C::CS;
   extern __shared__ __align__(1024) float2 tsm[];
@@ -179,6 +181,7 @@ __global__ void __launch_bounds__(AnaCfg<H>::T, AnaCfg<H>::MINB)
                              int n_active, int WH, float2* dst_base, const float2* __restrict__ spec_base,
                              int spec_row0, size_t band_stride, const float2* __restrict__ twH4, int* err,
                              int per_level) {
+  pdl_sync();
   using C = AnaCfg<H>;
   constexpr int CS = C::CS, NP = CS / 2;
   extern __shared__ __align__(1024) float2 tsm[];
@@ -232,6 +235,7 @@ __global__ void __launch_bounds__(SynCfg<H>::T, SynCfg<H>::MINB)
     k_band_synthesis_tma(const __grid_constant__ CUtensorMap amap, const ColJob* __restrict__ jobs, int n_active,
                          int WH, float2* dst_base, const float2* __restrict__ spec_base, size_t band_stride,
                          const float2* __restrict__ twH, int* err, int per_level) {
+  pdl_sync();
   using C = SynCfg<H>;
   constexpr int CS = C::CS;
   static_assert(C::LD == CS, "dense column groups");
@@ -285,6 +289,7 @@ __global__ void __launch_bounds__(SynCfg<H>::T, SynCfg<H>::MINB)
     k_band_synthesis_p_tma(const __grid_constant__ CUtensorMap amap, const ColJob* __restrict__ jobs, int n_active,
                            int WH, float2* dst_base, const float2* __restrict__ spec_base, size_t band_stride,
                            const float2* __restrict__ twH4, int* err, int per_level) {
+  pdl_sync();
   using C = SynCfg<H>;
   constexpr int CS = C::CS, NP = CS / 2;
   extern __shared__ __align__(1024) float2 tsm[];
@@ -373,6 +378,7 @@ __global__ void __launch_bounds__(RaccCfg<H>::T, RaccCfg<H>::MINB)
                           int WH, float2* dst_base, const float2* __restrict__ spec_base, int spec_row0,
                           size_t band_stride, const float2* __restrict__ twH, const float2* __restrict__ wd,
                           int* err, int per_level) {
+  pdl_sync();
   using C = RaccCfg<H>;
   constexpr int CS = C::CS, T = C::T, RL = C::RL, IPT = C::IPT;
   extern __shared__ __align__(1024) float2 tsm[];
@@ -516,25 +522,25 @@ cudaError_t launch_cols_tma(ColOp op, const void* amap, const ColJob* jobs, int 
     dim3 grid(WH / ColCfg<n>::CS, njobs);                                                                           \
     constexpr size_t sa = AnaCfg<n>::smem() + kBarBytes, ss = SynCfg<n>::smem() + kBarBytes;                        \
     if (op == ColOp::AnalysisLevel)                                                                                 \
-      k_band_analysis_ml_tma<n, false><<<grid, AnaCfg<n>::T, sa, st>>>(m, jobs, n_active, WH, dst_base, spec_base,  \
+      launch_pdl(k_band_analysis_ml_tma<n, false>, grid, AnaCfg<n>::T, sa, st, m, jobs, n_active, WH, dst_base, spec_base,  \
                                                                        sr, band_stride, twH, wd, err, per_level);   \
     else if (op == ColOp::AnalysisLevelDct)                                                                         \
-      k_band_analysis_ml_tma<n, true><<<grid, AnaCfg<n>::T, sa, st>>>(m, jobs, n_active, WH, dst_base, spec_base,   \
+      launch_pdl(k_band_analysis_ml_tma<n, true>, grid, AnaCfg<n>::T, sa, st, m, jobs, n_active, WH, dst_base, spec_base,   \
                                                                       sr, band_stride, twH, wd, err, per_level);    \
     else if (op == ColOp::AnalysisLevelPairs)                                                                       \
-      k_band_analysis_ml_p_tma<n><<<grid, AnaCfg<n>::T, sa, st>>>(m, jobs, n_active, WH, dst_base, spec_base, sr,   \
+      launch_pdl(k_band_analysis_ml_p_tma<n>, grid, AnaCfg<n>::T, sa, st, m, jobs, n_active, WH, dst_base, spec_base, sr,   \
                                                                   band_stride, twH, err, per_level);                \
     else if (op == ColOp::Synthesis)                                                                                \
-      k_band_synthesis_tma<n><<<grid, SynCfg<n>::T, ss, st>>>(m, jobs, n_active, WH, dst_base, spec_base,           \
+      launch_pdl(k_band_synthesis_tma<n>, grid, SynCfg<n>::T, ss, st, m, jobs, n_active, WH, dst_base, spec_base,           \
                                                               band_stride, twH, err, per_level);                    \
     else if (op == ColOp::SynthesisRegs)                                                                            \
-      k_band_synthesis_racc<n, false><<<grid, RaccCfg<n>::T, RaccCfg<n>::smem(), st>>>(                             \
+      launch_pdl(k_band_synthesis_racc<n, false>, grid, RaccCfg<n>::T, RaccCfg<n>::smem(), st,                              \
           m, jobs, n_active, WH, dst_base, spec_base, sr, band_stride, twH, wd, err, per_level);                    \
     else if (op == ColOp::SynthesisRegsDct2)                                                                        \
-      k_band_synthesis_racc<n, true><<<grid, RaccCfg<n>::T, RaccCfg<n>::smem(), st>>>(                              \
+      launch_pdl(k_band_synthesis_racc<n, true>, grid, RaccCfg<n>::T, RaccCfg<n>::smem(), st,                               \
           m, jobs, n_active, WH, dst_base, spec_base, sr, band_stride, twH, wd, err, per_level);                    \
     else                                                                                                            \
-      k_band_synthesis_p_tma<n><<<grid, SynCfg<n>::T, ss, st>>>(m, jobs, n_active, WH, dst_base, spec_base,         \
+      launch_pdl(k_band_synthesis_p_tma<n>, grid, SynCfg<n>::T, ss, st, m, jobs, n_active, WH, dst_base, spec_base,         \
                                                                 band_stride, twH, err, per_level);                  \
     return cudaGetLastError();                                                                                      \
   }

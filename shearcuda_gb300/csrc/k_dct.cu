@@ -42,6 +42,7 @@
 // complex data.  Rows are real: they use the W/2-point packed real FFT
 // (c2r / r2c pre- and post-processing) of the directional kernels.
 #include "internal.h"
+#include "launch.cuh"
 #include "tiles.cuh"
 #include "tma.cuh"
 
@@ -173,6 +174,7 @@ struct DctMinB {
 template <int WH, bool LEVEL>
 __global__ void __launch_bounds__(RowCfg<WH>::T, DctMinB<RowCfg<WH>::T>::value)
     k_dct_rows_fwd(const __grid_constant__ DctIo io, const float2* __restrict__ twWh, const float4* __restrict__ tw) {
+  pdl_sync();
   using C = RowCfg<WH>;
   extern __shared__ float2 smem[];
   float2* A = smem;
@@ -207,6 +209,7 @@ __global__ void __launch_bounds__(RowCfg<WH>::T, DctMinB<RowCfg<WH>::T>::value)
     k_dct_rows_ana(const RowJob* __restrict__ jobs, int n_active, const float2* src_base, float2* dst_base,
                    const float* __restrict__ resp, size_t resp_stride, const float2* __restrict__ twWh,
                    const float2* __restrict__ twW, const float4* __restrict__ tw) {
+  pdl_sync();
   using C = RowCfg<WH>;
   extern __shared__ float2 smem[];
   float2* A = smem;
@@ -249,6 +252,7 @@ __global__ void __launch_bounds__(RowCfg<WH>::T, DctMinB<RowCfg<WH>::T>::value)
                    const float2* src_base, float2* dst_base, const float* __restrict__ xbase, size_t xstride,
                    const float* __restrict__ resp, size_t resp_stride, const float* __restrict__ tlow,
                    const float2* __restrict__ twWh, const float2* __restrict__ twW, const float4* __restrict__ tw) {
+  pdl_sync();
   using C = RowCfg<WH>;
   constexpr int CH = WH / 2;
   constexpr int W = 2 * WH;
@@ -333,6 +337,7 @@ __global__ void __cluster_dims__(1, 1, kSynRanks) __launch_bounds__(RowCfg<WH>::
                          const float* __restrict__ resp, size_t resp_stride, const float* __restrict__ tlow,
                          const float2* __restrict__ twWh, const float2* __restrict__ twW,
                          const float4* __restrict__ tw) {
+  pdl_sync();
   using C = RowCfg<WH>;
   constexpr int W = 2 * WH, LD = WH + 2, RR = C::RS / kSynRanks;  // rows a CTA finishes
   extern __shared__ float2 smem[];
@@ -468,6 +473,7 @@ __global__ void __launch_bounds__(ColCfg<H>::T, DctMinB<ColCfg<H>::T>::value)
     k_dct_cols(const ColJob* __restrict__ jobs, int n_active, int WH, const float2* src_base, float2* dst_base,
                const float2* __restrict__ twH, const float2* __restrict__ wd, const float* __restrict__ thr,
                int th_stride, int tmode) {
+  pdl_sync();
   extern __shared__ float2 smem[];
   const ColJob job = jobs[blockIdx.y];
   if (job.item >= n_active) return;
@@ -481,6 +487,7 @@ template <int H>
 __global__ void __launch_bounds__(ColCfg<H>::T, DctMinB<ColCfg<H>::T>::value)
     k_dct_cols_out(const __grid_constant__ DctIo io, int WH, const float2* __restrict__ twH,
                    const float2* __restrict__ wd, const float2* add, float add_w) {
+  pdl_sync();
   extern __shared__ float2 smem[];
   const int col0 = blockIdx.x * ColCfg<H>::CS;
   dct_cols_body<H, kDct3>(reinterpret_cast<const float2*>(io.src[blockIdx.y]) + col0,
@@ -493,6 +500,7 @@ __global__ void __launch_bounds__(ColCfg<H>::T, DctMinB<ColCfg<H>::T>::value)
 __global__ void __launch_bounds__(256)
     k_dct_weights(const float4* __restrict__ ra, const float4* __restrict__ rs, const float4* __restrict__ tl, size_t n4,
                   int nlev, const __grid_constant__ PlaneWeights w, float scale, float base, float4* __restrict__ V) {
+  pdl_sync();
   const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= n4) return;
   const float4 t = __ldg(tl + i);
@@ -512,7 +520,7 @@ cudaError_t launch_dct_weights(const float* ra, const float* rs, const float* tl
                                const PlaneWeights& w, float base, float* V, cudaStream_t st) {
   if (nlev + 1 > kMaxPlaneWeights || n % 4) return cudaErrorInvalidValue;
   count_launch();
-  k_dct_weights<<<(unsigned)((n / 4 + 255) / 256), 256, 0, st>>>(
+  launch_pdl(k_dct_weights, (unsigned)((n / 4 + 255) / 256), 256, 0, st, 
       reinterpret_cast<const float4*>(ra), reinterpret_cast<const float4*>(rs), reinterpret_cast<const float4*>(tl),
       n / 4, nlev, w, (float)n, (float)(base / (double)n), reinterpret_cast<float4*>(V));
   return cudaGetLastError();
@@ -570,9 +578,9 @@ cudaError_t launch_dct_rows_fwd(const DctIo& io, int n, int H, int W, const floa
   case n_: {                                                                                        \
     const dim3 grid(H / RowCfg<n_>::RS, n);                                                         \
     if (level)                                                                                      \
-      k_dct_rows_fwd<n_, true><<<grid, RowCfg<n_>::T, RowCfg<n_>::smem_rm(), st>>>(io, twWh, twD);  \
+      launch_pdl(k_dct_rows_fwd<n_, true>, grid, RowCfg<n_>::T, RowCfg<n_>::smem_rm(), st, io, twWh, twD);  \
     else                                                                                            \
-      k_dct_rows_fwd<n_, false><<<grid, RowCfg<n_>::T, RowCfg<n_>::smem_rm(), st>>>(io, twWh, twD); \
+      launch_pdl(k_dct_rows_fwd<n_, false>, grid, RowCfg<n_>::T, RowCfg<n_>::smem_rm(), st, io, twWh, twD); \
     return cudaGetLastError();                                                                      \
   }
     NSST_DCT_ROW_SIZES(CASE)
@@ -594,10 +602,10 @@ cudaError_t launch_dct_rows_ana(const RowJob* jobs, int njobs, int n_active, int
   case n_: {                                                                                                \
     const dim3 grid(H / RowCfg<n_>::RS, njobs);                                                             \
     if (real_out)                                                                                           \
-      k_dct_rows_ana<n_, true><<<grid, RowCfg<n_>::T, RowCfg<n_>::smem_rm(), st>>>(                          \
+      launch_pdl(k_dct_rows_ana<n_, true>, grid, RowCfg<n_>::T, RowCfg<n_>::smem_rm(), st,                           \
           jobs, n_active, sb, db, resp, resp_stride, twWh, twW, twD);                                       \
     else                                                                                                    \
-      k_dct_rows_ana<n_, false><<<grid, RowCfg<n_>::T, RowCfg<n_>::smem_rm(), st>>>(                         \
+      launch_pdl(k_dct_rows_ana<n_, false>, grid, RowCfg<n_>::T, RowCfg<n_>::smem_rm(), st,                          \
           jobs, n_active, sb, db, resp, resp_stride, twWh, twW, twD);                                       \
     return cudaGetLastError();                                                                              \
   }
@@ -628,13 +636,13 @@ cudaError_t launch_dct_rows_syn(const RowJob* jobs, int njobs, int n_active, int
     const dim3 grid(H / RowCfg<n_>::RS, njobs);                                                               \
     constexpr size_t sm = 2 * RowCfg<n_>::smem_rm();                                                          \
     if (!real_in && nlev <= kSynRanks && syn_splits((long)grid.x * std::min(n_active, njobs)))                \
-      k_dct_rows_syn_split<n_><<<dim3(grid.x, njobs, kSynRanks), RowCfg<n_>::T, sm, st>>>(                    \
+      launch_pdl(k_dct_rows_syn_split<n_>, dim3(grid.x, njobs, kSynRanks), RowCfg<n_>::T, sm, st,                     \
           jobs, n_active, nlev, lev_stride, sb, db, xbase, xstride, resp, resp_stride, tlow, twWh, twW, twD); \
     else if (real_in)                                                                                         \
-      k_dct_rows_syn<n_, true><<<grid, RowCfg<n_>::T, sm, st>>>(jobs, n_active, nlev, lev_stride, sb, db, xbase, \
+      launch_pdl(k_dct_rows_syn<n_, true>, grid, RowCfg<n_>::T, sm, st, jobs, n_active, nlev, lev_stride, sb, db, xbase, \
                                                                xstride, resp, resp_stride, tlow, twWh, twW, twD); \
     else                                                                                                      \
-      k_dct_rows_syn<n_, false><<<grid, RowCfg<n_>::T, sm, st>>>(jobs, n_active, nlev, lev_stride, sb, db, xbase, \
+      launch_pdl(k_dct_rows_syn<n_, false>, grid, RowCfg<n_>::T, sm, st, jobs, n_active, nlev, lev_stride, sb, db, xbase, \
                                                                 xstride, resp, resp_stride, tlow, twWh, twW, twD); \
     return cudaGetLastError();                                                                                \
   }
@@ -661,13 +669,13 @@ cudaError_t launch_dct_cols(int mode, const ColJob* jobs, int njobs, int n_activ
     const dim3 grid(WH / ColCfg<n_>::CS, njobs);                                                   \
     constexpr size_t sm = ColCfg<n_>::smem() / 2;                                                  \
     if (mode == kDct2)                                                                             \
-      k_dct_cols<n_, kDct2><<<grid, ColCfg<n_>::T, sm, st>>>(jobs, n_active, WH, sb, db, twH, wdH,     \
+      launch_pdl(k_dct_cols<n_, kDct2>, grid, ColCfg<n_>::T, sm, st, jobs, n_active, WH, sb, db, twH, wdH,     \
                                                              thr, th_stride, th_mode);                 \
     else if (mode == kDctAna)                                                                      \
-      k_dct_cols<n_, kDctAna><<<grid, ColCfg<n_>::T, sm, st>>>(jobs, n_active, WH, sb, db, twH, wdH,   \
+      launch_pdl(k_dct_cols<n_, kDctAna>, grid, ColCfg<n_>::T, sm, st, jobs, n_active, WH, sb, db, twH, wdH,   \
                                                                thr, th_stride, th_mode);               \
     else                                                                                           \
-      k_dct_cols<n_, kDctThresh><<<grid, ColCfg<n_>::T, sm, st>>>(jobs, n_active, WH, sb, db, twH,     \
+      launch_pdl(k_dct_cols<n_, kDctThresh>, grid, ColCfg<n_>::T, sm, st, jobs, n_active, WH, sb, db, twH,     \
                                                                   wdH, thr, th_stride, th_mode);       \
     return cudaGetLastError();                                                                     \
   }
@@ -686,7 +694,7 @@ cudaError_t launch_dct_cols_out(const DctIo& io, int n, int H, int W, const floa
   switch (H) {
 #define CASE(n_)                                                                                                   \
   case n_:                                                                                                         \
-    k_dct_cols_out<n_><<<dim3(WH / ColCfg<n_>::CS, n), ColCfg<n_>::T, ColCfg<n_>::smem() / 2, st>>>(          \
+    launch_pdl(k_dct_cols_out<n_>, dim3(WH / ColCfg<n_>::CS, n), ColCfg<n_>::T, ColCfg<n_>::smem() / 2, st,           \
         io, WH, twH, wdH, reinterpret_cast<const float2*>(add), add_w);                                            \
     return cudaGetLastError();
     NSST_DCT_COL_SIZES(CASE)

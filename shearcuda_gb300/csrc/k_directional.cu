@@ -23,6 +23,7 @@
 // memory plus a tile index, so one launch covers a whole batch of images of
 // one size.
 #include "internal.h"
+#include "launch.cuh"
 #include "tiles.cuh"
 
 namespace nsst {
@@ -40,6 +41,7 @@ __global__ void __launch_bounds__(RowCfg<WH>::T, RowCfg<WH>::MINB) k_rows_fwd(co
                                                              const float2* src_base, float2* dst_base,
                                                              const float2* __restrict__ twWh,
                                                              const float2* __restrict__ twW) {
+  pdl_sync();
   using C = RowCfg<WH>;
   extern __shared__ float2 smem[];
   float2 *A = smem, *B = smem + (size_t)WH * C::LD;
@@ -60,6 +62,7 @@ __global__ void __launch_bounds__(RowCfg<WH>::T, RowCfg<WH>::MINB) k_rows_inv(co
                                                              const float2* src_base, float2* dst_base,
                                                              const float2* __restrict__ twWh,
                                                              const float2* __restrict__ twW) {
+  pdl_sync();
   using C = RowCfg<WH>;
   extern __shared__ float2 smem[];
   float2 *A = smem, *B = smem + (size_t)WH * C::LD;
@@ -89,6 +92,7 @@ __global__ void __launch_bounds__(RowTile<WH, RS>::T, RowTile<WH, RS>::MINB)
     k_rows_thresh(const RowJob* __restrict__ jobs, int n_active, const float2* src_base, float2* dst_base,
                   const float2* __restrict__ twWh, const float2* __restrict__ twW, const float* __restrict__ thr,
                   int mode) {
+  pdl_sync();
   constexpr int T = RowTile<WH, RS>::T;
   extern __shared__ float2 smem[];
   float2* A = smem;
@@ -161,6 +165,7 @@ __global__ void __launch_bounds__(RowTileP<WH, RS>::T, RowTileP<WH, RS>::MINB)
     k_rows_thresh_p(const RowJob* __restrict__ jobs, int n_active, const float2* src_base, float2* dst_base,
                     const float2* __restrict__ twWh4, const float4* __restrict__ twW4, const float* __restrict__ thr,
                     int mode) {
+  pdl_sync();
   constexpr int NP = RowTileP<WH, RS>::NP, T = RowTileP<WH, RS>::T, RP = WH + 2;
   extern __shared__ float2 smem[];
   float2* A = smem;                         // row-major rows, pitch WH + 2
@@ -239,6 +244,7 @@ __global__ void __launch_bounds__(RowCfg<WH>::T, RowCfg<WH>::MINB) k_rows_max(co
                                                              const float2* __restrict__ twWh,
                                                              const float2* __restrict__ twW,
                                                              unsigned* __restrict__ bits) {
+  pdl_sync();
   using C = RowCfg<WH>;
   extern __shared__ float2 smem[];
   float2* A = smem;
@@ -270,6 +276,7 @@ __global__ void __launch_bounds__(RowCfg<WH>::T) k_rows_backward(const RowJob* _
                                                                   const float2* __restrict__ twW,
                                                                   const float* __restrict__ tau, int mode,
                                                                   float* __restrict__ partials, size_t pstride) {
+  pdl_sync();
   using C = RowCfg<WH>;
   extern __shared__ float2 smem[];
   // three buffers of the padded row-major size (the dense layouts fit in them)
@@ -361,6 +368,7 @@ template <int H, int DIR>
 __global__ void __launch_bounds__(ColCfg<H>::T, ColCfg<H>::MINB) k_cols(const ColJob* __restrict__ jobs, int n_active, int WH,
                                                         const float2* src_base, float2* dst_base,
                                                         const float2* __restrict__ twH) {
+  pdl_sync();
   using C = ColCfg<H>;
   extern __shared__ float2 smem[];
   float2 *A = smem, *B = smem + (size_t)H * C::LD;
@@ -378,6 +386,7 @@ __global__ void __launch_bounds__(ColCfg<H>::T, ColCfg<H>::MINB) k_band_analysis
                                                                  int WH, const float2* src_base, float2* dst_base,
                                                                  const float2* __restrict__ spec_base,
                                                                  const float2* __restrict__ twH) {
+  pdl_sync();
   using C = ColCfg<H>;
   extern __shared__ float2 smem[];
   float2 *A = smem, *B = smem + (size_t)H * C::LD;
@@ -402,6 +411,7 @@ __global__ void __launch_bounds__(AnaCfg<H>::T, AnaCfg<H>::MINB) k_band_analysis
                                                                   const float2* __restrict__ spec_base,
                                                                   size_t band_stride,
                                                                   const float2* __restrict__ twH) {
+  pdl_sync();
   using C = AnaCfg<H>;
   constexpr int CS = C::CS, CH = CS / 2;  // 16-byte chunks per row of the column group
   extern __shared__ float2 smem[];
@@ -456,6 +466,7 @@ __global__ void __launch_bounds__(SynCfg<H>::T, SynCfg<H>::MINB) k_band_synthesi
                                                                   const float2* __restrict__ spec_base,
                                                                   size_t band_stride,
                                                                   const float2* __restrict__ twH) {
+  pdl_sync();
   using C = SynCfg<H>;
   extern __shared__ float2 smem[];
   float2 *A = smem, *S = smem + (size_t)H * C::LD, *D = smem + 2 * (size_t)H * C::LD;
@@ -517,6 +528,7 @@ __global__ void __launch_bounds__(AnaCfg<H>::T, AnaCfg<H>::MINB)
     k_band_analysis_ml_p(const ColJob* __restrict__ jobs, int n_active, int WH, const float2* src_base,
                          float2* dst_base, const float2* __restrict__ spec_base, size_t band_stride,
                          const float2* __restrict__ twH4) {
+  pdl_sync();
   using C = AnaCfg<H>;
   constexpr int CS = C::CS, CH = CS / 2, NP = CS / 2;
   extern __shared__ float2 smem[];
@@ -567,6 +579,7 @@ __global__ void __launch_bounds__(SynCfg<H>::T, SynCfg<H>::MINB)
     k_band_synthesis_p(const ColJob* __restrict__ jobs, int n_active, int WH, const float2* src_base,
                        float2* dst_base, const float2* __restrict__ spec_base, size_t band_stride,
                        const float2* __restrict__ twH4) {
+  pdl_sync();
   using C = SynCfg<H>;
   constexpr int CS = C::CS, NP = CS / 2;
   extern __shared__ float2 smem[];
@@ -718,11 +731,11 @@ cudaError_t launch_rows(RowOp op, const RowJob* jobs, int njobs, int n_active, i
     constexpr size_t smr = RowCfg<n>::smem_rm();                                       \
     (void)sm;                                                                          \
     if (op == RowOp::Fwd)                                                              \
-      k_rows_fwd<n><<<grid, RowCfg<n>::T, smr, st>>>(jobs, n_active, sb, db, twWh, twW);             \
+      launch_pdl(k_rows_fwd<n>, grid, RowCfg<n>::T, smr, st, jobs, n_active, sb, db, twWh, twW);             \
     else if (op == RowOp::Inv)                                                         \
-      k_rows_inv<n><<<grid, RowCfg<n>::T, smr, st>>>(jobs, n_active, sb, db, twWh, twW);             \
+      launch_pdl(k_rows_inv<n>, grid, RowCfg<n>::T, smr, st, jobs, n_active, sb, db, twWh, twW);             \
     else                                                                               \
-      k_rows_thresh<n><<<grid, RowCfg<n>::T, smr, st>>>(jobs, n_active, sb, db, twWh, twW, thr, mode); \
+      launch_pdl(k_rows_thresh<n>, grid, RowCfg<n>::T, smr, st, jobs, n_active, sb, db, twWh, twW, thr, mode); \
     return cudaGetLastError();                                                         \
   }
     NSST_ROW_SIZES(CASE)
@@ -752,13 +765,13 @@ cudaError_t launch_rows_thresh(const RowJob* jobs, int njobs, int n_active, int 
     if (tile_mult == 1) {                                                                                  \
       using Tl = RowTileP<n, R1>;                                                                          \
       count_launch();                                                                                      \
-      k_rows_thresh_p<n, R1><<<dim3(H / R1, njobs), Tl::T, Tl::smem(), st>>>(                              \
+      launch_pdl(k_rows_thresh_p<n, R1>, dim3(H / R1, njobs), Tl::T, Tl::smem(), st,                               \
           jobs, n_active, sb, db, reinterpret_cast<const float2*>(twWh4), twW4, thr, mode);                \
     } else {                                                                                               \
       if (H % R2 != 0) return cudaErrorInvalidValue;                                                       \
       using Tl = RowTileP<n, R2>;                                                                          \
       count_launch();                                                                                      \
-      k_rows_thresh_p<n, R2><<<dim3(H / R2, njobs), Tl::T, Tl::smem(), st>>>(                              \
+      launch_pdl(k_rows_thresh_p<n, R2>, dim3(H / R2, njobs), Tl::T, Tl::smem(), st,                               \
           jobs, n_active, sb, db, reinterpret_cast<const float2*>(twWh4), twW4, thr, mode);                \
     }                                                                                                      \
     return cudaGetLastError();                                                                             \
@@ -776,7 +789,7 @@ cudaError_t launch_rows_thresh(const RowJob* jobs, int njobs, int n_active, int 
     constexpr int RS2 = 2 * RowCfg<n>::RS;                                                              \
     using Tl = RowTile<n, RS2>;                                                                         \
     if (H % RS2 != 0) return cudaErrorInvalidValue;                                                     \
-    k_rows_thresh<n, RS2><<<dim3(H / RS2, njobs), Tl::T, Tl::smem(), st>>>(jobs, n_active, sb, db, twWh, twW, \
+    launch_pdl(k_rows_thresh<n, RS2>, dim3(H / RS2, njobs), Tl::T, Tl::smem(), st, jobs, n_active, sb, db, twWh, twW, \
                                                                          thr, mode);                    \
     return cudaGetLastError();                                                                          \
   }
@@ -797,7 +810,7 @@ cudaError_t launch_rows_max(const RowJob* jobs, int njobs, int n_active, int H, 
 #define CASE(n)                                                                                   \
   case n: {                                                                                       \
     constexpr size_t sm = RowCfg<n>::smem_rm();                                                   \
-    k_rows_max<n><<<dim3(H / RowCfg<n>::RS, njobs), RowCfg<n>::T, sm, st>>>(jobs, n_active, sb, twWh, twW, bits); \
+    launch_pdl(k_rows_max<n>, dim3(H / RowCfg<n>::RS, njobs), RowCfg<n>::T, sm, st, jobs, n_active, sb, twWh, twW, bits); \
     return cudaGetLastError();                                                                    \
   }
     NSST_ROW_SIZES(CASE)
@@ -820,7 +833,7 @@ cudaError_t launch_rows_backward(const RowJob* jobs, int njobs, int n_active, in
   case n: {                                                                                          \
     constexpr size_t sm = 3 * RowCfg<n>::smem_rm();                                                  \
     dim3 grid(H / RowCfg<n>::RS, njobs);                                                             \
-    k_rows_backward<n><<<grid, RowCfg<n>::T, sm, st>>>(jobs, n_active, sb, db, twWh, twW, tau, mode, \
+    launch_pdl(k_rows_backward<n>, grid, RowCfg<n>::T, sm, st, jobs, n_active, sb, db, twWh, twW, tau, mode, \
                                                       partials, pstride);                           \
     return cudaGetLastError();                                                                       \
   }
@@ -843,23 +856,23 @@ cudaError_t launch_cols(ColOp op, const ColJob* jobs, int njobs, int n_active, i
     constexpr size_t sm = ColCfg<n>::smem();                                                          \
     dim3 grid(WH / ColCfg<n>::CS, njobs);                                                             \
     if (op == ColOp::Fwd)  /* in-place transforms: one buffer */                                     \
-      k_cols<n, -1><<<grid, ColCfg<n>::T, sm / 2, st>>>(jobs, n_active, WH, src_base, dst_base, twH);               \
+      launch_pdl(k_cols<n, -1>, grid, ColCfg<n>::T, sm / 2, st, jobs, n_active, WH, src_base, dst_base, twH);               \
     else if (op == ColOp::Inv)                                                                        \
-      k_cols<n, 1><<<grid, ColCfg<n>::T, sm / 2, st>>>(jobs, n_active, WH, src_base, dst_base, twH);                \
+      launch_pdl(k_cols<n, 1>, grid, ColCfg<n>::T, sm / 2, st, jobs, n_active, WH, src_base, dst_base, twH);                \
     else if (op == ColOp::Analysis)                                                                   \
-      k_band_analysis<n><<<grid, ColCfg<n>::T, sm / 2, st>>>(jobs, n_active, WH, src_base, dst_base, spec_base,     \
+      launch_pdl(k_band_analysis<n>, grid, ColCfg<n>::T, sm / 2, st, jobs, n_active, WH, src_base, dst_base, spec_base,     \
                                                          twH);                                        \
     else if (op == ColOp::AnalysisLevelPairs)                                                         \
-      k_band_analysis_ml_p<n><<<grid, AnaCfg<n>::T, AnaCfg<n>::smem(), st>>>(jobs, n_active, WH, src_base,          \
+      launch_pdl(k_band_analysis_ml_p<n>, grid, AnaCfg<n>::T, AnaCfg<n>::smem(), st, jobs, n_active, WH, src_base,          \
                                                                           dst_base, spec_base, band_stride, twH); \
     else if (op == ColOp::SynthesisPairs)                                                             \
-      k_band_synthesis_p<n><<<grid, SynCfg<n>::T, SynCfg<n>::smem(), st>>>(jobs, n_active, WH, src_base, dst_base, \
+      launch_pdl(k_band_synthesis_p<n>, grid, SynCfg<n>::T, SynCfg<n>::smem(), st, jobs, n_active, WH, src_base, dst_base, \
                                                                         spec_base, band_stride, twH); \
     else if (op == ColOp::AnalysisLevel)                                                              \
-      k_band_analysis_ml<n><<<grid, AnaCfg<n>::T, AnaCfg<n>::smem(), st>>>(jobs, n_active, WH, src_base, dst_base, \
+      launch_pdl(k_band_analysis_ml<n>, grid, AnaCfg<n>::T, AnaCfg<n>::smem(), st, jobs, n_active, WH, src_base, dst_base, \
                                                                         spec_base, band_stride, twH); \
     else                                                                                              \
-      k_band_synthesis<n><<<grid, SynCfg<n>::T, SynCfg<n>::smem(), st>>>(jobs, n_active, WH, src_base, dst_base,   \
+      launch_pdl(k_band_synthesis<n>, grid, SynCfg<n>::T, SynCfg<n>::smem(), st, jobs, n_active, WH, src_base, dst_base,   \
                                                                        spec_base,                     \
                                                       band_stride, twH);                              \
     return cudaGetLastError();                                                                        \

@@ -4,6 +4,7 @@
 // Both are deterministic: fixed-order partials reduced on the host, and a
 // maximum of non-negative floats through their bit patterns.
 #include "internal.h"
+#include "launch.cuh"
 
 namespace nsst {
 
@@ -12,6 +13,7 @@ constexpr int kRedThreads = 256;
 // partial[plane * gridDim.x + block] = sum of x^2 over the block's share of the plane
 __global__ void __launch_bounds__(kRedThreads) k_plane_sumsq(const float* __restrict__ data, size_t n,
                                                             double* __restrict__ partial) {
+  pdl_sync();
   __shared__ double red[kRedThreads / 32];
   const float* x = data + (size_t)blockIdx.y * n;
   double s = 0.0;
@@ -33,6 +35,7 @@ __global__ void __launch_bounds__(kRedThreads) k_plane_sumsq(const float* __rest
 // non-negative floats); maxbits must start at 0
 __global__ void __launch_bounds__(kRedThreads) k_plane_maxabs(const float* __restrict__ data, size_t n,
                                                              unsigned* __restrict__ maxbits) {
+  pdl_sync();
   const float* x = data + (size_t)blockIdx.y * n;
   float m = 0.0f;
   for (size_t i = (size_t)blockIdx.x * kRedThreads + threadIdx.x; i < n; i += (size_t)gridDim.x * kRedThreads)
@@ -43,6 +46,7 @@ __global__ void __launch_bounds__(kRedThreads) k_plane_maxabs(const float* __res
 
 // data[plane][i] *= w[plane]
 __global__ void k_scale_planes(float* __restrict__ data, size_t n, PlaneWeights w) {
+  pdl_sync();
   float* x = data + (size_t)blockIdx.y * n;
   const float s = w.w[blockIdx.y];
   for (size_t i = (size_t)blockIdx.x * kRedThreads + threadIdx.x; i < n; i += (size_t)gridDim.x * kRedThreads)
@@ -52,21 +56,21 @@ __global__ void k_scale_planes(float* __restrict__ data, size_t n, PlaneWeights 
 cudaError_t launch_scale_planes(float* data, size_t n, int nplanes, const PlaneWeights& w, cudaStream_t st) {
   if (nplanes > kMaxPlaneWeights) return cudaErrorInvalidValue;
   count_launch();
-  k_scale_planes<<<dim3(64, nplanes), kRedThreads, 0, st>>>(data, n, w);
+  launch_pdl(k_scale_planes, dim3(64, nplanes), kRedThreads, 0, st, data, n, w);
   return cudaGetLastError();
 }
 
 cudaError_t launch_plane_sumsq(const float* data, size_t n, int nplanes, double* partial, int blocks,
                                cudaStream_t st) {
   count_launch();
-  k_plane_sumsq<<<dim3(blocks, nplanes), kRedThreads, 0, st>>>(data, n, partial);
+  launch_pdl(k_plane_sumsq, dim3(blocks, nplanes), kRedThreads, 0, st, data, n, partial);
   return cudaGetLastError();
 }
 
 cudaError_t launch_plane_maxabs(const float* data, size_t n, int nplanes, unsigned* maxbits, int blocks,
                                 cudaStream_t st) {
   count_launch();
-  k_plane_maxabs<<<dim3(blocks, nplanes), kRedThreads, 0, st>>>(data, n, maxbits);
+  launch_pdl(k_plane_maxabs, dim3(blocks, nplanes), kRedThreads, 0, st, data, n, maxbits);
   return cudaGetLastError();
 }
 

@@ -6,6 +6,7 @@
 // (ccsym 'c'); real volumes float arrays, axis 2 contiguous.
 #include "fft_core.cuh"
 #include "internal.h"
+#include "launch.cuh"
 
 namespace nsst {
 
@@ -37,6 +38,7 @@ __device__ __forceinline__ int small_to_parent(int s, int K, int nr, int nsmall,
 
 __global__ void k_pyr_dec_lp(const float2* __restrict__ Xh, float2* __restrict__ Lp, size_t stride, int d1, int pitch,
                              int s0, int s1, int sh2, int spitch, PyrWin w, float invDN) {
+  pdl_sync();
   const float2* X = Xh + blockIdx.y * stride;
   float2* L = Lp + blockIdx.y * stride;
   const size_t total = (size_t)s0 * s1 * sh2;
@@ -63,6 +65,7 @@ __global__ void k_pyr_dec_lp(const float2* __restrict__ Xh, float2* __restrict__
 // (the last plane collects the padded ones).
 __global__ void k_fold_axis(const float* __restrict__ g, size_t g_stride, float* __restrict__ out, size_t o_stride,
                             int e0, int e1, int e2, int axis, int n) {
+  pdl_sync();
   const float* src = g + blockIdx.y * g_stride;
   float* dst = out + blockIdx.y * o_stride;
   const int f0 = axis == 0 ? n : e0, f1 = axis == 1 ? n : e1, f2 = axis == 2 ? n : e2;
@@ -90,7 +93,7 @@ cudaError_t launch_pyr_dec_lp(const float2* Xh, float2* Lp, size_t stride, int n
                               int s2, const PyrWin& w, float invDN, cudaStream_t st) {
   const int sh2 = s2 / 2 + 1;
   count_launch();
-  k_pyr_dec_lp<<<v3grid((size_t)s0 * s1 * sh2, n), 256, 0, st>>>(Xh, Lp, stride, d1, pitch, s0, s1, sh2,
+  launch_pdl(k_pyr_dec_lp, v3grid((size_t)s0 * s1 * sh2, n), 256, 0, st, Xh, Lp, stride, d1, pitch, s0, s1, sh2,
                                                                  v3_pitch(sh2), w, invDN);
   return cudaGetLastError();
 }
@@ -101,9 +104,9 @@ cudaError_t launch_fold_edge(const float* g, size_t g_stride, float* out, size_t
   float* t1 = scratch;                           // d0 x d1 x n2
   float* t2 = scratch + (size_t)d0 * d1 * n2;    // d0 x n1 x n2
   count_launch(3);
-  k_fold_axis<<<v3grid((size_t)d0 * d1 * n2, n), 256, 0, st>>>(g, g_stride, t1, s_stride, d0, d1, d2, 2, n2);
-  k_fold_axis<<<v3grid((size_t)d0 * n1 * n2, n), 256, 0, st>>>(t1, s_stride, t2, s_stride, d0, d1, n2, 1, n1);
-  k_fold_axis<<<v3grid((size_t)n0 * n1 * n2, n), 256, 0, st>>>(t2, s_stride, out, o_stride, d0, n1, n2, 0, n0);
+  launch_pdl(k_fold_axis, v3grid((size_t)d0 * d1 * n2, n), 256, 0, st, g, g_stride, t1, s_stride, d0, d1, d2, 2, n2);
+  launch_pdl(k_fold_axis, v3grid((size_t)d0 * n1 * n2, n), 256, 0, st, t1, s_stride, t2, s_stride, d0, d1, n2, 1, n1);
+  launch_pdl(k_fold_axis, v3grid((size_t)n0 * n1 * n2, n), 256, 0, st, t2, s_stride, out, o_stride, d0, n1, n2, 0, n0);
   return cudaGetLastError();
 }
 

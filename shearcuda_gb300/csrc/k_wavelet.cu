@@ -17,6 +17,7 @@
 // A level reads its input while other CTAs write its output, so the lowpass
 // alternates between two buffers.
 #include "internal.h"
+#include "launch.cuh"
 
 namespace nsst {
 
@@ -45,6 +46,7 @@ __global__ void __launch_bounds__(kWvThreads, 4)
     k_rdwt_fwd(const float* __restrict__ cur, size_t s_cur, float* __restrict__ yl, size_t s_yl,
                float* __restrict__ yh, size_t s_yh, int H, int W, int sf, const __grid_constant__ WvTaps t,
                const float* __restrict__ thr) {
+  pdl_sync();
   extern __shared__ float2 sm[];  // [row][column] (C_lo, C_hi)
   const int ph = blockIdx.x % sf, i0 = blockIdx.x / sf * TH, item = blockIdx.y, Hp = H / sf;
   const size_t HW = (size_t)H * W, rs = (size_t)sf * W;
@@ -118,6 +120,7 @@ template <int LH, int TH>
 __global__ void __launch_bounds__(kWvThreads, 4)
     k_rdwt_inv(const float* __restrict__ ll, size_t s_ll, const float* __restrict__ yh, size_t s_yh,
                float* __restrict__ out, size_t s_out, int H, int W, int sf, const __grid_constant__ WvTaps t) {
+  pdl_sync();
   extern __shared__ float2 sm[];
   float2 *s1 = sm, *sh = sm + TH / 2 * W;  // [row pair][column]: x1, xh of rows 2 q and 2 q + 1
   const int ph = blockIdx.x % sf, i0 = blockIdx.x / sf * TH, item = blockIdx.y, Hp = H / sf;
@@ -198,6 +201,7 @@ constexpr int kTvRows = 8, kTvWarps = 8, kTvCols = 31;
 __global__ void __launch_bounds__(32 * kTvWarps)
     k_tv_haar(const float* __restrict__ x, float* __restrict__ y, size_t stride, int H, int W, WvTaps ta, WvTaps ts,
               float gamma) {
+  pdl_sync();
   const int lane = threadIdx.x, c0 = blockIdx.x * kTvCols, item = blockIdx.z;
   const int r0 = (blockIdx.y * kTvWarps + threadIdx.y) * kTvRows;
   if (r0 >= H) return;  // whole warps
@@ -244,6 +248,7 @@ struct DTaps {
 };
 __global__ void __launch_bounds__(256) k_dwt_hh(const float* __restrict__ xb, size_t stride, int H, int W, DTaps t,
                                                 double* __restrict__ hhb) {
+  pdl_sync();
   const int l = blockIdx.x * 32 + threadIdx.x, k = blockIdx.y * 8 + threadIdx.y;
   if (l >= W / 2 || k >= H / 2) return;
   const float* x = xb + blockIdx.z * stride;
@@ -268,6 +273,7 @@ __global__ void __launch_bounds__(256) k_dwt_hh(const float* __restrict__ xb, si
 __global__ void k_sep_residual(const float* __restrict__ img, const float* __restrict__ p1,
                                const float* __restrict__ p2, float* __restrict__ ra1, float* __restrict__ ra2,
                                size_t n) {
+  pdl_sync();
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     const float a = p1[i], b = p2[i];
     const float r = (img[i] - a) - b;  // GPUminus twice (separate.m:146-148)
@@ -296,7 +302,7 @@ static cudaError_t launch_rdwt(K kernel, int th, int n, int H, int W, int sf, cu
     if (e != cudaSuccess) return e;
   }
   count_launch();
-  kernel<<<dim3((unsigned)(sf * ((H / sf + th - 1) / th)), (unsigned)n), kWvThreads, sm, st>>>(args...);
+  launch_pdl(kernel, dim3((unsigned)(sf * ((H / sf + th - 1) / th)), (unsigned)n), kWvThreads, sm, st, args...);
   return cudaGetLastError();
 }
 
@@ -351,7 +357,7 @@ cudaError_t launch_tv_haar(const float* x, float* y, size_t stride, int n, int H
   const WvTaps ta = analysis_taps(haar), ts = synthesis_taps(haar);
   count_launch();
   const int rows = kTvRows * kTvWarps;
-  k_tv_haar<<<dim3((W + kTvCols - 1) / kTvCols, (H + rows - 1) / rows, n), dim3(32, kTvWarps), 0, st>>>(
+  launch_pdl(k_tv_haar, dim3((W + kTvCols - 1) / kTvCols, (H + rows - 1) / rows, n), dim3(32, kTvWarps), 0, st, 
       x, y, stride, H, W, ta, ts, gamma);
   return cudaGetLastError();
 }
@@ -363,7 +369,7 @@ cudaError_t launch_dwt_hh(const float* x, size_t stride, int n, int H, int W, co
   t.lh = lh;
   for (int i = 0; i < lh; i++) t.b[i] = b[i];
   count_launch();
-  k_dwt_hh<<<dim3((W / 2 + 31) / 32, (H / 2 + 7) / 8, n), dim3(32, 8), 0, st>>>(x, stride, H, W, t, hh);
+  launch_pdl(k_dwt_hh, dim3((W / 2 + 31) / 32, (H / 2 + 7) / 8, n), dim3(32, 8), 0, st, x, stride, H, W, t, hh);
   return cudaGetLastError();
 }
 
@@ -371,7 +377,7 @@ cudaError_t launch_sep_residual(const float* img, const float* p1, const float* 
                                 size_t n, cudaStream_t st) {
   const int blocks = (int)std::min<size_t>((n + 255) / 256, 152 * 8);
   count_launch();
-  k_sep_residual<<<blocks, 256, 0, st>>>(img, p1, p2, ra1, ra2, n);
+  launch_pdl(k_sep_residual, blocks, 256, 0, st, img, p1, p2, ra1, ra2, n);
   return cudaGetLastError();
 }
 

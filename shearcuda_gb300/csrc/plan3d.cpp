@@ -635,6 +635,11 @@ nsst_status nsst3_plan_create(const nsst3_config* cfg, int n0, int n1, int n2, i
       if (!om || !om->pyr || (l < p->L && (!oc || !oc->conv)))
         return fail3(NSST_ERR_UNSUPPORTED_SIZE, "volume transform length not compiled");
     }
+  for (auto& kv : p->tw_off) {
+    cudaError_t e = v3_ops(kv.first)->prepare();
+    if (e != cudaSuccess) return cuda_fail3(e, "volume pass set-up");
+  }
+
   // one device arena
   const size_t B = (size_t)batch;
   size_t off = 0;

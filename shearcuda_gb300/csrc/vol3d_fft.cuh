@@ -27,10 +27,17 @@
 
 #include "fft_core.cuh"
 #include "internal.h"
+#include "launch.cuh"
 
 namespace nsst {
 
 constexpr int kLines = 8;  // lines per CTA: 64-byte rows along z on the strided axes
+// Shared memory share of the SM's L1 the passes run under: half, which holds
+// their resident CTAs' exchanges and leaves the rest to the twiddles and the
+// rows that several CTAs touch (4 x 128^3, us: 25 % 2225, 33 % 1657, 42 % 1645,
+// 50 % 1572, 60 % 1587, 75 % 1628, 100 % 1873; left to the driver, which picks
+// it per kernel, 1895).
+constexpr int kV3Carveout = 50;
 
 // Radices per length.  The larger second: every thread of a CTA then loads.
 template <int N>
@@ -125,6 +132,7 @@ __device__ __forceinline__ float v3_win(const float* __restrict__ v, int K, int 
 template <int N, int DIR, int LD, int ST, int G = 1>
 __global__ void __launch_bounds__(V3Cfg<N>::T * G, v3_loops(LD, ST) ? v3_min_ctas(V3Cfg<N>::T * G, 96) : 1)
     k_v3_cols(const V3Cols P, const float2* __restrict__ tw) {
+  pdl_sync();
   using C = V3Cfg<N>;
   constexpr int R1 = C::R1, R2 = C::R2;
   constexpr bool kLoop = v3_loops(LD, ST);
@@ -358,6 +366,7 @@ __global__ void __launch_bounds__(V3Cfg<N>::T * G, v3_loops(LD, ST) ? v3_min_cta
 // part of complex line s; X[k], X[N - k] separate into the two rows' spectra.
 template <int N>
 __global__ void __launch_bounds__(V3Cfg<N>::T) k_v3_real_fwd(const V3Real P, const float2* __restrict__ tw) {
+  pdl_sync();
   using C = V3Cfg<N>;
   constexpr int R1 = C::R1, R2 = C::R2, H = N / 2 + 1, NP = N + 1;
   __shared__ float2 ex[C::EXZ];
@@ -418,6 +427,7 @@ __global__ void __launch_bounds__(V3Cfg<N>::T) k_v3_real_fwd(const V3Real P, con
 // with A[N - k] = conj(A[k]) and the imaginary parts at 0 and N/2 dropped.
 template <int N>
 __global__ void __launch_bounds__(V3Cfg<N>::T) k_v3_real_inv(const V3Real P, const float2* __restrict__ tw) {
+  pdl_sync();
   using C = V3Cfg<N>;
   constexpr int R1 = C::R1, R2 = C::R2;
   __shared__ float2 ex[C::EXZ];
@@ -465,6 +475,7 @@ __global__ void __launch_bounds__(V3Cfg<N>::T) k_v3_real_inv(const V3Real P, con
 // fastest, so the items share each filter row through L2; y: share of the pairs.
 template <int N>
 __global__ void __launch_bounds__(V3Cfg<N>::T, v3_min_ctas(V3Cfg<N>::T, 112)) k_v3_pair_inv(const V3Pair P, const float2* __restrict__ tw) {
+  pdl_sync();
   using C = V3Cfg<N>;
   constexpr int R1 = C::R1, R2 = C::R2;
   __shared__ float2 ex[2][C::EXZ];
@@ -520,6 +531,7 @@ __global__ void __launch_bounds__(V3Cfg<N>::T, v3_min_ctas(V3Cfg<N>::T, 112)) k_
 // S (+)= conj(C) .* Z summed over the pairs in registers.
 template <int N>
 __global__ void __launch_bounds__(V3Cfg<N>::T, v3_min_ctas(V3Cfg<N>::T, 128)) k_v3_pair_fwd(const V3Pair P, const float2* __restrict__ tw) {
+  pdl_sync();
   using C = V3Cfg<N>;
   constexpr int R1 = C::R1, R2 = C::R2;
   __shared__ float2 ex[2][C::EXZ];
@@ -575,9 +587,9 @@ struct V3Launch {
     const dim3 grid((unsigned)((P.rows0 * P.rows1 + 2 * kLines - 1) / (2 * kLines)), (unsigned)items);
     count_launch();
     if (dir < 0)
-      k_v3_real_fwd<N><<<grid, T, 0, st>>>(P, tw);
+      launch_pdl(k_v3_real_fwd<N>, grid, T, 0, st, P, tw);
     else
-      k_v3_real_inv<N><<<grid, T, 0, st>>>(P, tw);
+      launch_pdl(k_v3_real_inv<N>, grid, T, 0, st, P, tw);
     return cudaGetLastError();
   }
   static cudaError_t cols(int dir, int ld, int st_mode, const V3Cols& P, const float2* tw, int npairs, cudaStream_t st) {
@@ -587,13 +599,13 @@ struct V3Launch {
     // groups of threads share it; with more CTAs the groups only wait for one another.
     if constexpr (CONV && N <= 108)
       if (st_mode == V3_ST_THRESH && P.pairs >= 4 && grid.x <= 2 * 152) {
-        k_v3_cols<N, 1, V3_LD_CPLX, V3_ST_THRESH, 4><<<grid, 4 * T, 0, st>>>(P, tw);
+        launch_pdl(k_v3_cols<N, 1, V3_LD_CPLX, V3_ST_THRESH, 4>, grid, 4 * T, 0, st, P, tw);
         return cudaGetLastError();
       }
 #define V3_COLS(cond, d, l, s)                          \
   if constexpr (cond)                                   \
     if (dir == d && ld == l && st_mode == s) {          \
-      k_v3_cols<N, d, l, s><<<grid, T, 0, st>>>(P, tw); \
+      launch_pdl(k_v3_cols<N, d, l, s>, grid, T, 0, st, P, tw); \
       return cudaGetLastError();                        \
     }
     V3_COLS(true, -1, V3_LD_CPLX, V3_ST_CPLX)
@@ -612,14 +624,42 @@ struct V3Launch {
       const dim3 grid((unsigned)((P.N0 * P.N1 + kLines - 1) / kLines * P.items), (unsigned)shares);
       count_launch();
       if (dir > 0)
-        k_v3_pair_inv<N><<<grid, T, 0, st>>>(P, tw);
+        launch_pdl(k_v3_pair_inv<N>, grid, T, 0, st, P, tw);
       else
-        k_v3_pair_fwd<N><<<grid, T, 0, st>>>(P, tw);
+        launch_pdl(k_v3_pair_fwd<N>, grid, T, 0, st, P, tw);
       return cudaGetLastError();
     }
     return cudaErrorInvalidValue;
   }
-  static V3Ops ops() { return {real, cols, pair, PYR, CONV}; }
+  // One shared-memory carve-out for every pass: with dependent launches the
+  // SMs do not drain between kernels, and a kernel placed under another's
+  // carve-out would keep the occupancy that it allows.
+  static cudaError_t prepare() {
+    cudaError_t e = cudaSuccess;
+    auto one = [&](auto kernel) {
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, kV3Carveout);
+    };
+    one(k_v3_real_fwd<N>);
+    one(k_v3_real_inv<N>);
+    one(k_v3_cols<N, -1, V3_LD_CPLX, V3_ST_CPLX>);
+    one(k_v3_cols<N, 1, V3_LD_CPLX, V3_ST_CPLX>);
+    if constexpr (PYR) {
+      one(k_v3_cols<N, 1, V3_LD_HP, V3_ST_CPLX>);
+      one(k_v3_cols<N, -1, V3_LD_CPLX, V3_ST_REC>);
+    }
+    if constexpr (CONV) {
+      one(k_v3_cols<N, 1, V3_LD_SYM, V3_ST_CPLX>);
+      one(k_v3_cols<N, -1, V3_LD_MASKED, V3_ST_CPLX>);
+      one(k_v3_cols<N, 1, V3_LD_CPLX, V3_ST_THRESH>);
+      one(k_v3_cols<N, 1, V3_LD_CPLX, V3_ST_PAIR>);
+      one(k_v3_pair_inv<N>);
+      one(k_v3_pair_fwd<N>);
+      if constexpr (N <= 108) one(k_v3_cols<N, 1, V3_LD_CPLX, V3_ST_THRESH, 4>);
+    }
+    return e;
+  }
+  static V3Ops ops() { return {real, cols, pair, prepare, PYR, CONV}; }
 };
 
 }  // namespace nsst
