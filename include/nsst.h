@@ -300,9 +300,9 @@ nsst_status nsst_denoise_batch(nsst_plan* plan, const float* const* x, float* co
 
 /* Uneven batches: images of several sizes denoised together.  A multi object
  * groups the items by plan (one plan per distinct size, each with enough
- * batch capacity), runs the groups on forked streams and captures the whole
- * batch (threshold uploads included) as one CUDA graph that is replayed while
- * the item pointers stay the same.  Each plan must hold its scalars
+ * batch capacity) and runs the groups on forked streams; a call with the item
+ * pointers of the call before it is captured (threshold uploads included) as
+ * one CUDA graph that is replayed while they stay the same.  Each plan must hold its scalars
  * (nsst_plan_set_scalars or nsst_compute_scalars). */
 typedef struct nsst_item {
   const float* x; /* device, H x W of the item's plan */

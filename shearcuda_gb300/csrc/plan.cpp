@@ -2694,8 +2694,10 @@ struct nsst_multi {
   cudaStream_t cap = nullptr;
   cudaEvent_t fork = nullptr, finished = nullptr;
   cudaGraphExec_t exec = nullptr;
-  std::vector<const void*> key;
+  std::vector<const void*> key;   // what exec was captured for
   int key_mode = -1;
+  std::vector<const void*> last;  // the previous call's
+  int last_mode = -1;
   std::mutex mu;
 };
 
@@ -2763,21 +2765,20 @@ nsst_status nsst_multi_denoise(nsst_multi* m, const nsst_item* items, int n, con
     if (!groups[g].empty() && !m->plans[g]->has_scalars)
       return fail(NSST_ERR_INVALID_ARG, "plan without stored scalars");
   }
-  for (nsst_plan* q : m->plans) q->saved_n = 0;  // the replay rewrites the plans' arenas
-  // thresholds into every plan's pinned staging; the previous replay must be done with them
-  NSST_CUDA(cudaEventSynchronize(m->finished));
+  // every group's thresholds, checked before anything is queued
+  std::vector<std::vector<float>> th(np);
   std::vector<char> lowth(np, 0);
   for (int g = 0; g < np; g++) {
     nsst_plan* p = m->plans[g];
-    for (size_t t = 0; t < groups[g].size(); t++) {
-      const double sg = items[groups[g][t]].sigma;
+    for (int i : groups[g]) {
+      const double sg = items[i].sigma;
       if (!std::isfinite(sg) || sg < 0) return fail(NSST_ERR_INVALID_ARG, "sigma must be finite and >= 0");
       for (int b = 0; b < p->nbands; b++) {
-        double th = K[p->band_level[b]] * sg * p->scalars[b];
-        if (!std::isfinite(th) || th < 0) return fail(NSST_ERR_INVALID_ARG, "thresholds must be finite and >= 0");
-        p->th_host[t * p->nbands + b] = (float)th;
+        const double t = K[p->band_level[b]] * sg * p->scalars[b];
+        if (!std::isfinite(t) || t < 0) return fail(NSST_ERR_INVALID_ARG, "thresholds must be finite and >= 0");
+        th[g].push_back((float)t);
+        if (b == 0 && (float)t > 0.f) lowth[g] = 1;
       }
-      if (p->th_host[t * p->nbands] > 0.f) lowth[g] = 1;
     }
   }
   std::vector<const void*> key;
@@ -2788,40 +2789,66 @@ nsst_status nsst_multi_denoise(nsst_multi* m, const nsst_item* items, int n, con
   }
   for (int g = 0; g < np; g++) key.push_back((const void*)(intptr_t)lowth[g]);
   cudaStream_t st = (cudaStream_t)stream;
-  if (!m->exec || key != m->key || mode != m->key_mode) {
-    if (m->exec) {
-      cudaGraphExecDestroy(m->exec);
-      m->exec = nullptr;
-    }
-    NSST_CUDA(cudaStreamBeginCapture(m->cap, cudaStreamCaptureModeThreadLocal));
-    nsst_status s = NSST_OK;
-    cudaError_t ce = cudaEventRecord(m->fork, m->cap);
-    for (int g = 0; g < np && s == NSST_OK && ce == cudaSuccess; g++) {
+  // thresholds into every plan's pinned staging, once its last copy has read it
+  for (int g = 0; g < np; g++) {
+    nsst_plan* p = m->plans[g];
+    p->saved_n = 0;  // the call rewrites the plans' arenas
+    if (groups[g].empty()) continue;
+    NSST_CUDA(cudaEventSynchronize(p->th_done));
+    std::memcpy(p->th_host, th[g].data(), th[g].size() * sizeof(float));
+  }
+  // Each group's pipeline on its own stream, forked from and joined to `from`;
+  // `direct`: outside a capture, the staging is free when its copy has run.
+  auto enqueue = [&](cudaStream_t from, bool direct) -> nsst_status {
+    NSST_CUDA(cudaEventRecord(m->fork, from));
+    for (int g = 0; g < np; g++) {
       if (groups[g].empty()) continue;
       nsst_plan* p = m->plans[g];
       std::lock_guard<std::mutex> plk(p->mu);
-      ce = cudaStreamWaitEvent(m->streams[g], m->fork, 0);
-      if (ce != cudaSuccess) break;
+      NSST_CUDA(cudaStreamWaitEvent(m->streams[g], m->fork, 0));
       const int cnt = (int)groups[g].size();
-      ce = cudaMemcpyAsync(p->th, p->th_host, sizeof(float) * p->nbands * cnt, cudaMemcpyHostToDevice,
-                           m->streams[g]);
-      if (ce != cudaSuccess) break;
+      NSST_CUDA(cudaMemcpyAsync(p->th, p->th_host, sizeof(float) * p->nbands * cnt, cudaMemcpyHostToDevice,
+                                m->streams[g]));
+      if (direct) NSST_CUDA(cudaEventRecord(p->th_done, m->streams[g]));
       std::vector<const float*> xs(cnt);
       std::vector<float*> os(cnt);
       for (int t = 0; t < cnt; t++) {
         xs[t] = items[groups[g][t]].x;
         os[t] = items[groups[g][t]].out;
       }
-      s = enqueue_denoise(p, cnt, xs.data(), os.data(), mode, lowth[g] != 0, m->streams[g]);
-      if (s == NSST_OK) ce = cudaEventRecord(m->done[g], m->streams[g]);
-      if (ce == cudaSuccess && s == NSST_OK) ce = cudaStreamWaitEvent(m->cap, m->done[g], 0);
+      const nsst_status s = enqueue_denoise(p, cnt, xs.data(), os.data(), mode, lowth[g] != 0, m->streams[g]);
+      // joined also after an error, so that nothing queued here is left beside the caller's stream
+      NSST_CUDA(cudaEventRecord(m->done[g], m->streams[g]));
+      NSST_CUDA(cudaStreamWaitEvent(from, m->done[g], 0));
+      NSST_TRY(s);
     }
+    return NSST_OK;
+  };
+  // A call with the pointers of the one before it is captured, and replayed
+  // while they stay; any other runs its launches directly: capturing and
+  // instantiating a graph costs more than they do, and the GPU would wait.
+  const bool again = key == m->last && mode == m->last_mode;
+  m->last = key;
+  m->last_mode = mode;
+  // calls on other streams share the plans' arenas with this one
+  NSST_CUDA(cudaStreamWaitEvent(st, m->finished, 0));
+  if (!m->exec || key != m->key || mode != m->key_mode) {
+    if (!again) {
+      const nsst_status s = enqueue(st, true);
+      NSST_CUDA(cudaEventRecord(m->finished, st));
+      return s;
+    }
+    if (m->exec) {
+      cudaGraphExecDestroy(m->exec);
+      m->exec = nullptr;
+    }
+    NSST_CUDA(cudaStreamBeginCapture(m->cap, cudaStreamCaptureModeThreadLocal));
+    const nsst_status s = enqueue(m->cap, false);
     cudaGraph_t graph = nullptr;
-    cudaError_t ce2 = cudaStreamEndCapture(m->cap, &graph);
-    if (s != NSST_OK || ce != cudaSuccess || ce2 != cudaSuccess) {
+    cudaError_t ce = cudaStreamEndCapture(m->cap, &graph);
+    if (s != NSST_OK || ce != cudaSuccess) {
       if (graph) cudaGraphDestroy(graph);
-      if (s != NSST_OK) return s;
-      return cuda_fail(ce != cudaSuccess ? ce : ce2, "multi capture");
+      return s != NSST_OK ? s : cuda_fail(ce, "multi capture");
     }
     ce = cudaGraphInstantiate(&m->exec, graph, 0);
     cudaGraphDestroy(graph);
@@ -2833,6 +2860,8 @@ nsst_status nsst_multi_denoise(nsst_multi* m, const nsst_item* items, int n, con
     m->key_mode = mode;
   }
   NSST_CUDA(cudaGraphLaunch(m->exec, st));
+  for (int g = 0; g < np; g++)
+    if (!groups[g].empty()) NSST_CUDA(cudaEventRecord(m->plans[g]->th_done, st));
   NSST_CUDA(cudaEventRecord(m->finished, st));
   return NSST_OK;
 }
