@@ -11,9 +11,10 @@
 // cp.async copies (H * CS / 2 of them per plane, with their address
 // arithmetic, then a wait and a block barrier), one thread issues
 // H / tma_box_rows(H) tensor-map copies per plane against an mbarrier, and
-// every thread waits on the mbarrier's phase.  The tensor map covers the
-// plan's whole arena as rows of W/2 float2, so a plane at arena offset o
-// (a multiple of W/2) starts at row o / (W/2).
+// every thread waits on the mbarrier's phase.  The tensor maps cover an
+// arena (the plan's or its gradient workspace) as rows of W/2 float2, so a
+// plane at offset o (a multiple of W/2) starts at row o / (W/2); the filter
+// spectra are in the plan's arena wherever the planes are.
 //
 // The filter spectrum of band k + 1 (analysis) or band plane k + 1
 // (synthesis) is requested as soon as the first FFT pass of band k has read
@@ -108,7 +109,8 @@ __device__ __forceinline__ ColBlock col_block(int per_level) {
 // DCT-III output order, forward FFT), into Y, before the band loop.
 template <int H, bool DCTANA>
 __global__ void __launch_bounds__(AnaCfg<H>::T, AnaCfg<H>::MINB)
-    k_band_analysis_ml_tma(const __grid_constant__ CUtensorMap amap, const ColJob* __restrict__ jobs, int n_active,
+    k_band_analysis_ml_tma(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap smap,
+                           const ColJob* __restrict__ jobs, int n_active,
                            int WH, float2* dst_base, const float2* __restrict__ spec_base, int spec_row0,
                            size_t band_stride, const float2* __restrict__ twH, const float2* __restrict__ wd,
                            int* err, int per_level) {
@@ -131,7 +133,7 @@ __global__ void __launch_bounds__(AnaCfg<H>::T, AnaCfg<H>::MINB)
     tma.init();
     tma.expect(2);
     tma.load(&amap, Y, yrow);
-    tma.load(&amap, Wb, srow);
+    tma.load(&smap, Wb, srow);
   }
   __syncthreads();  // the mbarrier is initialised before any thread waits on it
   if (job.nbands > 0) tma.wait(err);  // Y and band 0's filter group
@@ -165,7 +167,7 @@ __global__ void __launch_bounds__(AnaCfg<H>::T, AnaCfg<H>::MINB)
     };
     // the hook runs after the first pass's barrier: every thread has read Wb
     auto next = [&]() {
-      if (threadIdx.x == 0 && tma.ok && k + 1 < job.nbands) tma.refill(&amap, Wb, srow + (k + 1) * band_rows);
+      if (threadIdx.x == 0 && tma.ok && k + 1 < job.nbands) tma.refill(&smap, Wb, srow + (k + 1) * band_rows);
     };
     block_fft_hook_ip<H, CS, C::T, +1>(A, twH, ld, ColGlobalSt{dst_base + job.dst + (size_t)k * band_stride + col0, WH},
                                       next);
@@ -374,7 +376,8 @@ struct RaccCfg {
 // DCT-II post-processing (wd) follow in shared memory.
 template <int H, bool DCT2>
 __global__ void __launch_bounds__(RaccCfg<H>::T, RaccCfg<H>::MINB)
-    k_band_synthesis_racc(const __grid_constant__ CUtensorMap amap, const ColJob* __restrict__ jobs, int n_active,
+    k_band_synthesis_racc(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap smap,
+                          const ColJob* __restrict__ jobs, int n_active,
                           int WH, float2* dst_base, const float2* __restrict__ spec_base, int spec_row0,
                           size_t band_stride, const float2* __restrict__ twH, const float2* __restrict__ wd,
                           int* err, int per_level) {
@@ -401,7 +404,7 @@ __global__ void __launch_bounds__(RaccCfg<H>::T, RaccCfg<H>::MINB)
     tp.expect(1);
     tp.load(&amap, P, brow);
     tw.expect(1);
-    tw.load(&amap, Wc, srow);
+    tw.load(&smap, Wc, srow);
   }
   __syncthreads();  // the mbarriers are initialised before any thread waits on them
   float2 acc[IPT][RL];
@@ -422,7 +425,7 @@ __global__ void __launch_bounds__(RaccCfg<H>::T, RaccCfg<H>::MINB)
     };
     fft_ld_acc_passes<H, CS, T, -1, 1, 0>(A, twH, SmemLd<CS>{P}, next, spec_ready, accf, typename C::Plan{});
     // every thread has read Wc (the last pass ends with a barrier)
-    if (threadIdx.x == 0 && tw.ok && k + 1 < job.nbands) tw.refill(&amap, Wc, srow + (k + 1) * band_rows);
+    if (threadIdx.x == 0 && tw.ok && k + 1 < job.nbands) tw.refill(&smap, Wc, srow + (k + 1) * band_rows);
     if (dc && threadIdx.x % CS == 0) {  // + conj(M[u] X[-u]) on the packed DC/Nyquist column
       const float2* m0 = spec_base + job.m0 + (size_t)k * H;
 #pragma unroll
@@ -501,7 +504,7 @@ cudaError_t prepare_cols_tma(int H) {
   }
 }
 
-cudaError_t launch_cols_tma(ColOp op, const void* amap, const ColJob* jobs, int njobs, int n_active, int H, int W,
+cudaError_t launch_cols_tma(ColOp op, const void* amap, const void* smap, const ColJob* jobs, int njobs, int n_active, int H, int W,
                             float2* dst_base, const float2* spec_base, size_t spec_row0, size_t band_stride,
                             const float2* twH, int* err, cudaStream_t st, const float2* wd, int per_level) {
   const int WH = W / 2;
@@ -514,7 +517,7 @@ cudaError_t launch_cols_tma(ColOp op, const void* amap, const ColJob* jobs, int 
   if (band_stride % (size_t)WH != 0 || spec_row0 > (size_t)INT32_MAX) return cudaErrorInvalidValue;
   if (per_level < 0 || (per_level > 0 && njobs % per_level != 0)) return cudaErrorInvalidValue;
   count_launch();
-  const CUtensorMap& m = *reinterpret_cast<const CUtensorMap*>(amap);
+  const CUtensorMap &m = *reinterpret_cast<const CUtensorMap*>(amap), &sm = *reinterpret_cast<const CUtensorMap*>(smap);
   const int sr = (int)spec_row0;
   switch (H) {
 #define CASE(n)                                                                                                     \
@@ -522,10 +525,10 @@ cudaError_t launch_cols_tma(ColOp op, const void* amap, const ColJob* jobs, int 
     dim3 grid(WH / ColCfg<n>::CS, njobs);                                                                           \
     constexpr size_t sa = AnaCfg<n>::smem() + kBarBytes, ss = SynCfg<n>::smem() + kBarBytes;                        \
     if (op == ColOp::AnalysisLevel)                                                                                 \
-      launch_pdl(k_band_analysis_ml_tma<n, false>, grid, AnaCfg<n>::T, sa, st, m, jobs, n_active, WH, dst_base, spec_base,  \
+      launch_pdl(k_band_analysis_ml_tma<n, false>, grid, AnaCfg<n>::T, sa, st, m, sm, jobs, n_active, WH, dst_base, spec_base,  \
                                                                        sr, band_stride, twH, wd, err, per_level);   \
     else if (op == ColOp::AnalysisLevelDct)                                                                         \
-      launch_pdl(k_band_analysis_ml_tma<n, true>, grid, AnaCfg<n>::T, sa, st, m, jobs, n_active, WH, dst_base, spec_base,   \
+      launch_pdl(k_band_analysis_ml_tma<n, true>, grid, AnaCfg<n>::T, sa, st, m, sm, jobs, n_active, WH, dst_base, spec_base,   \
                                                                       sr, band_stride, twH, wd, err, per_level);    \
     else if (op == ColOp::AnalysisLevelPairs)                                                                       \
       launch_pdl(k_band_analysis_ml_p_tma<n>, grid, AnaCfg<n>::T, sa, st, m, jobs, n_active, WH, dst_base, spec_base, sr,   \
@@ -535,10 +538,10 @@ cudaError_t launch_cols_tma(ColOp op, const void* amap, const ColJob* jobs, int 
                                                               band_stride, twH, err, per_level);                    \
     else if (op == ColOp::SynthesisRegs)                                                                            \
       launch_pdl(k_band_synthesis_racc<n, false>, grid, RaccCfg<n>::T, RaccCfg<n>::smem(), st,                              \
-          m, jobs, n_active, WH, dst_base, spec_base, sr, band_stride, twH, wd, err, per_level);                    \
+          m, sm, jobs, n_active, WH, dst_base, spec_base, sr, band_stride, twH, wd, err, per_level);                    \
     else if (op == ColOp::SynthesisRegsDct2)                                                                        \
       launch_pdl(k_band_synthesis_racc<n, true>, grid, RaccCfg<n>::T, RaccCfg<n>::smem(), st,                               \
-          m, jobs, n_active, WH, dst_base, spec_base, sr, band_stride, twH, wd, err, per_level);                    \
+          m, sm, jobs, n_active, WH, dst_base, spec_base, sr, band_stride, twH, wd, err, per_level);                    \
     else                                                                                                            \
       launch_pdl(k_band_synthesis_p_tma<n>, grid, SynCfg<n>::T, ss, st, m, jobs, n_active, WH, dst_base, spec_base,         \
                                                                 band_stride, twH, err, per_level);                  \

@@ -145,6 +145,9 @@ struct nsst_plan {
   // start at row spec_row0
   alignas(64) unsigned char cols_tmap[128] = {};
   bool cols_tma_ok = false;
+  // the same over the gradient workspace (level spectra and bands of the backward, thresholded bands of the forward)
+  alignas(64) unsigned char gcols_tmap[128] = {};
+  bool gcols_tma_ok = false;
   size_t spec_row0 = 0;
   FusedJob* j_fused = nullptr;  // (B*nlev) levels with more bands first, then items
   int* dev_err = nullptr;       // error word of the bounded device waits
@@ -1092,19 +1095,21 @@ nsst_status enqueue_band_analysis(nsst_plan* p, int n, bool grad, cudaStream_t s
   const bool level = analysis_per_level(p, n, ana);
   const size_t bs = (size_t)p->H * p->WH;
   const float2* tw = pairs ? (const float2*)p->twH4 : p->twH;
+  const ColJob* jobs = grad ? p->gj_analysis_lev : p->j_analysis_lev;
+  const void* map = grad ? p->gcols_tmap : p->cols_tmap;
+  const bool tma_ok = p->cols_tma_ok && (!grad || (p->gcols_tma_ok && !pairs));
   if (dctana) {  // the level planes' columns are still to be transformed
-    if (!(level && tma && !pairs && !grad && p->cols_tma_ok && p->wdH))
+    if (!(level && tma && !pairs && tma_ok && p->wdH))
       return fail(NSST_ERR_INVALID_ARG, "internal: the level analysis cannot finish the level spectra");
-    NSST_CUDA(launch_cols_tma(ColOp::AnalysisLevelDct, p->cols_tmap, p->j_analysis_lev, p->B * p->nlev, n, p->H,
-                              p->W, base, p->spec, p->spec_row0, bs, p->twH, p->dev_err, st, p->wdH, p->B));
-  } else if (level && tma && !grad && p->cols_tma_ok) {
-    NSST_CUDA(launch_cols_tma(pairs ? ColOp::AnalysisLevelPairs : ColOp::AnalysisLevel, p->cols_tmap,
-                              p->j_analysis_lev, p->B * p->nlev, n, p->H, p->W, base, p->spec, p->spec_row0, bs, tw,
-                              p->dev_err, st, nullptr, p->B));
+    NSST_CUDA(launch_cols_tma(ColOp::AnalysisLevelDct, map, p->cols_tmap, jobs, p->B * p->nlev, n, p->H, p->W, base,
+                              p->spec, p->spec_row0, bs, p->twH, p->dev_err, st, p->wdH, p->B));
+  } else if (level && tma && tma_ok) {
+    NSST_CUDA(launch_cols_tma(pairs ? ColOp::AnalysisLevelPairs : ColOp::AnalysisLevel, map, p->cols_tmap, jobs,
+                              p->B * p->nlev, n, p->H, p->W, base, p->spec, p->spec_row0, bs, tw, p->dev_err, st,
+                              nullptr, p->B));
   } else if (level) {
-    NSST_CUDA(launch_cols(pairs ? ColOp::AnalysisLevelPairs : ColOp::AnalysisLevel,
-                          grad ? p->gj_analysis_lev : p->j_analysis_lev, p->B * p->nlev, n, p->H, p->W, base, base,
-                          p->spec, bs, tw, st));
+    NSST_CUDA(launch_cols(pairs ? ColOp::AnalysisLevelPairs : ColOp::AnalysisLevel, jobs, p->B * p->nlev, n, p->H,
+                          p->W, base, base, p->spec, bs, tw, st));
   } else {
     NSST_CUDA(launch_cols(ColOp::Analysis, grad ? p->gj_analysis : p->j_analysis, p->B * p->ndir_total, n, p->H,
                           p->W, base, base, p->spec, 0, p->twH, st));
@@ -1112,25 +1117,39 @@ nsst_status enqueue_band_analysis(nsst_plan* p, int n, bool grad, cudaStream_t s
   return NSST_OK;
 }
 
-// The band synthesis of n items (p->band -> p->sum) as choice c runs it.
-// sums_dct2: see enqueue_directional.
-nsst_status enqueue_band_synthesis(nsst_plan* p, int n, const DirChoice& c, cudaStream_t st, bool* sums_dct2) {
-  char* A = p->arena;
-  const bool tma = c.cols_tma && p->cols_tma_ok;
+// The band synthesis of n items as choice c runs it: jobs from planes of src
+// (tensor map tmap, used where tma_ok) to sums in dst.  sums_dct2: see
+// enqueue_directional.
+nsst_status enqueue_synthesis(nsst_plan* p, int n, const DirChoice& c, const void* tmap, bool tma_ok,
+                              const ColJob* jobs, void* src, void* dst, cudaStream_t st, bool* sums_dct2) {
+  const bool tma = c.cols_tma && tma_ok;
   const bool dct2 = sums_dct2 && tma && c.syn_regs && !c.cols_packed && p->wdH && dct_syn_fusion_pays(p);
   const ColOp syn = c.cols_packed          ? ColOp::SynthesisPairs
                     : (tma && c.syn_regs) ? (dct2 ? ColOp::SynthesisRegsDct2 : ColOp::SynthesisRegs)
                                           : ColOp::Synthesis;
   const float2* twc = c.cols_packed ? (const float2*)p->twH4 : p->twH;
   if (tma)
-    NSST_CUDA(launch_cols_tma(syn, p->cols_tmap, p->j_synthesis, p->B * p->nlev, n, p->H, p->W, (float2*)A, p->spec,
+    NSST_CUDA(launch_cols_tma(syn, tmap, p->cols_tmap, jobs, p->B * p->nlev, n, p->H, p->W, (float2*)dst, p->spec,
                               p->spec_row0, (size_t)p->H * p->WH, twc, p->dev_err, st, p->wdH, p->B));
   else
-    NSST_CUDA(launch_cols(syn, p->j_synthesis, p->B * p->nlev, n, p->H, p->W, (float2*)A, (float2*)A, p->spec,
+    NSST_CUDA(launch_cols(syn, jobs, p->B * p->nlev, n, p->H, p->W, (float2*)src, (float2*)dst, p->spec,
                           (size_t)p->H * p->WH, twc, st));
-  timer_mark(p, "band_synthesis_cols", st);
   if (dct2) *sums_dct2 = true;
   return NSST_OK;
+}
+// p->band -> p->sum
+nsst_status enqueue_band_synthesis(nsst_plan* p, int n, const DirChoice& c, cudaStream_t st, bool* sums_dct2) {
+  NSST_TRY(enqueue_synthesis(p, n, c, p->cols_tmap, p->cols_tma_ok, p->j_synthesis, p->arena, p->arena, st, sums_dct2));
+  timer_mark(p, "band_synthesis_cols", st);
+  return NSST_OK;
+}
+// The split choice of a call of n items in which band planes of the caller or
+// of the gradient workspace take part; there the columns do not run as pairs.
+DirChoice split_choice(const nsst_plan* p, int n, bool grad = false) {
+  DirChoice c = dir_choice(p, n);
+  c.fused = false;
+  if (grad) c.cols_packed = false;
+  return c;
 }
 
 // The directional stage of the fused denoise (level spectra in p->lev, band
@@ -1271,7 +1290,7 @@ nsst_status enqueue_denoise_dct(nsst_plan* p, int n, const float* const* x, floa
   char* A = p->arena;
   float2* A2 = (float2*)A;
   const int B = p->B, H = p->H, W = p->W;
-  const bool ana_dct = !keep && analysis_takes_dct(p, n);
+  const bool ana_dct = analysis_takes_dct(p, n);
   NSST_TRY(enqueue_dct_analysis(p, n, x, st, ana_dct));
   if (lowpass_th) {  // lowpass band -> threshold -> DCT2, in tmp plane 0
     NSST_TRY(enqueue_dct_lowpass_rows(p, n, st));
@@ -1282,17 +1301,17 @@ nsst_status enqueue_denoise_dct(nsst_plan* p, int n, const float* const* x, floa
     NSST_TRY(enqueue_dct_rows_io(p, n, t0c.data(), t0.data(), st));
     timer_mark(p, "dct_lowpass_threshold", st);
   }
+  bool sums_dct2 = false;
   if (keep) {  // the thresholded bands to bandT: band keeps the pre-threshold spectra for the backward
-    NSST_TRY(enqueue_band_analysis(p, n, false, st));
+    const DirChoice c = split_choice(p, n, true);
+    NSST_TRY(enqueue_band_analysis(p, n, false, st, c.ana, false, c.cols_tma, ana_dct));
     timer_mark(p, "band_analysis_cols", st);
-    NSST_CUDA(launch_rows(RowOp::Thresh, p->gj_rows_T, B * p->ndir_total, n, H, W, A, p->garena, p->twWh, p->twW, TH,
-                          mode, st));
+    NSST_CUDA(launch_rows_thresh(p->gj_rows_T, B * p->ndir_total, n, H, W, A, p->garena, p->twWh, p->twW, TH, mode,
+                                 c.row_tile, st, c.packed, p->twWh4, p->twW4));
     timer_mark(p, "band_rows_threshold", st);
-    NSST_CUDA(launch_cols(ColOp::Synthesis, p->gj_synth_T, B * p->nlev, n, H, W, (float2*)p->garena, A2, p->spec,
-                          (size_t)H * p->WH, p->twH, st));
+    NSST_TRY(enqueue_synthesis(p, n, c, p->gcols_tmap, p->gcols_tma_ok, p->gj_synth_T, p->garena, A, st, &sums_dct2));
     timer_mark(p, "band_synthesis_cols", st);
   }
-  bool sums_dct2 = false;
   if (!keep) NSST_TRY(enqueue_directional(p, n, mode, TH, st, &sums_dct2, ana_dct));
   return lowpass_th ? enqueue_dct_synthesis(p, n, p->tmp, p->s_tmp, p->dct_gl, out, st, sums_dct2)
                     : enqueue_dct_synthesis(p, n, p->pyr, p->s_pyr, p->dct_tl, out, st, sums_dct2);
@@ -1388,13 +1407,6 @@ nsst_status enqueue_band_maxima(nsst_plan* p, int n, const float* const* x, unsi
   return NSST_OK;
 }
 
-// The split choice of a one-image call whose band planes the caller keeps.
-DirChoice split_choice(const nsst_plan* p) {
-  DirChoice c = dir_choice(p, 1);
-  c.fused = false;
-  return c;
-}
-
 // shear_trans of one image into nbands caller planes; the plan must be locked.
 // adjoint: with the synthesis pyramid's responses, which is the adjoint of
 // inverse_shear (spectral pyramid only: tau_backward_dct has the reason).
@@ -1402,7 +1414,7 @@ nsst_status enqueue_shear_trans(nsst_plan* p, const float* x, float* coeffs, cud
   char* A = p->arena;
   float2* A2 = (float2*)A;
   float* yb = p->pyr;
-  const DirChoice c = split_choice(p);
+  const DirChoice c = split_choice(p, 1);
   const bool tma = c.cols_tma && p->cols_tma_ok;
   bool ana_dct = false;
   if (p->dct_on && aligned16(x)) {
@@ -1440,7 +1452,7 @@ nsst_status enqueue_inverse_shear(nsst_plan* p, const float* coeffs, float* x, c
   timer_mark(p, "band_rows_fwd", st);
   const bool spectral = p->dct_on && aligned16(x);
   bool sums_dct2 = false;
-  NSST_TRY(enqueue_band_synthesis(p, 1, split_choice(p), st, spectral ? &sums_dct2 : nullptr));
+  NSST_TRY(enqueue_band_synthesis(p, 1, split_choice(p, 1), st, spectral ? &sums_dct2 : nullptr));
   if (spectral) {
     // spectral pyramid: the lowpass coefficients DCT2'd into tmp plane 0,
     // then the band sums and that plane through the synthesis back end
@@ -2275,14 +2287,20 @@ nsst_status nsst_plan_enable_grad(nsst_plan* p) {
   };
   size_t o_gyp = take(sizeof(float) * NB * (p->nlev + 1) * HW), o_gy = take(sizeof(float) * NB * (p->nlev + 1) * HW);
   size_t o_gtmp = take(sizeof(float) * NB * 2 * HW), o_z = take(sizeof(float) * NB * p->s_zext);
-  size_t o_lev2 = take(sizeof(float2) * NB * p->nlev * HWh), o_band2 = take(sizeof(float2) * NB * p->ndir_total * HWh);
+  // planes that the TMA column kernels read start on a row of W/2 float2
+  auto take_rows = [&](size_t bytes) {
+    off = align_up(off, sizeof(float2) * p->WH);
+    return take(bytes);
+  };
+  size_t o_lev2 = take_rows(sizeof(float2) * NB * p->nlev * HWh);
+  size_t o_band2 = take_rows(sizeof(float2) * NB * p->ndir_total * HWh);
   size_t o_sum2 = take(sizeof(float2) * NB * p->nlev * HWh);
   size_t o_part = take(sizeof(float) * p->nbands * NB * p->ntiles);
   const size_t nL = NB * p->nlev, nD = NB * p->ndir_total;
   size_t o_j1 = take(sizeof(RowJob) * nL), o_j2 = take(sizeof(ColJob) * nL), o_j3 = take(sizeof(ColJob) * nD);
   size_t o_j4 = take(sizeof(RowJob) * nD), o_j5 = take(sizeof(ColJob) * nL), o_j6 = take(sizeof(RowJob) * nL);
   size_t o_j7 = take(sizeof(RowJob) * p->ndir_total), o_j8 = take(sizeof(RowJob) * p->ndir_total);
-  size_t o_bandT = take(sizeof(float2) * NB * p->ndir_total * HWh);
+  size_t o_bandT = take_rows(sizeof(float2) * NB * p->ndir_total * HWh);
   size_t o_jT = take(sizeof(RowJob) * nD), o_jS = take(sizeof(ColJob) * nL);
   size_t o_jA = take(sizeof(ColJob) * nL);
   size_t o_gd1 = 0, o_gd2 = 0, o_gd3 = 0, o_gd4 = 0, o_gd5 = 0, o_gd6 = 0;
@@ -2418,6 +2436,12 @@ nsst_status nsst_plan_enable_grad(nsst_plan* p) {
     if (ce == cudaSuccess) ce = up(p->gj_dct_syn, gy1.data(), gy1.size() * sizeof(RowJob));
     if (ce != cudaSuccess) return cuda_fail(ce, "upload spectral gradient job lists");
   }
+  if (p->cols_tma_ok) {
+    const size_t rows = p->garena_bytes / (sizeof(float2) * p->WH);
+    p->gcols_tma_ok = rows <= (size_t)INT32_MAX &&
+                      make_tmap_2d(p->gcols_tmap, G, p->WH, rows, col_tile(H), tma_box_rows(H)) == cudaSuccess;
+    if (!p->gcols_tma_ok) (void)cudaGetLastError();  // the cp.async column kernels stay
+  }
   for (int F : {p->pf.F[0], p->pf.F[1], p->pf.F[2], p->pf.F[3]}) {
     ce = prepare_atrous_kernels(F, 0, Mmax);
     if (ce != cudaSuccess) return cuda_fail(ce, "adjoint kernel set-up");
@@ -2537,9 +2561,11 @@ nsst_status tau_backward_dct(nsst_plan* p, const float* const* x, const float* c
   }
   // 1. the coefficient spectra of x (recomputed unless saved) and the
   //    pre-threshold lowpass band, spatial, in pyr plane 1
+  const DirChoice c = split_choice(p, n, true);
+  const bool ana_dct = analysis_takes_dct(p, n);
   if (x) {
-    NSST_TRY(enqueue_dct_analysis(p, n, x, st));
-    NSST_TRY(enqueue_band_analysis(p, n, false, st));
+    NSST_TRY(enqueue_dct_analysis(p, n, x, st, ana_dct));
+    NSST_TRY(enqueue_band_analysis(p, n, false, st, c.ana, false, c.cols_tma, ana_dct));
     timer_mark(p, "recompute_coefficients", st);
   }
   NSST_TRY(enqueue_dct_lowpass_rows(p, n, st));
@@ -2550,18 +2576,19 @@ nsst_status tau_backward_dct(nsst_plan* p, const float* const* x, const float* c
   NSST_CUDA(launch_dct_cols(kDct2, p->gj_dct_x, B, n, H, W, G, G, p->twH, p->wdH, st));
   NSST_CUDA(launch_dct_rows_ana(p->gj_dct_ana, B * L, n, H, W, G, G, p->dct_rs, HW, p->twWh, p->twW, p->twDW, false,
                                 st));
-  NSST_CUDA(launch_dct_cols(kDctAna, p->gj_cols_lev, B * L, n, H, W, G, G, p->twH, p->wdH, st));
+  const bool gana_dct = ana_dct && p->gcols_tma_ok;
+  if (!gana_dct) NSST_CUDA(launch_dct_cols(kDctAna, p->gj_cols_lev, B * L, n, H, W, G, G, p->twH, p->wdH, st));
   NSST_CUDA(launch_dct_rows_ana(p->gj_dct_low, B, n, H, W, G, G, p->dct_ra, HW, p->twWh, p->twW, p->twDW, true, st));
   NSST_TRY(enqueue_dct_cols_out(p, n, gt0c.data(), gyp0.data(), st));
-  NSST_TRY(enqueue_band_analysis(p, n, true, st));
+  NSST_TRY(enqueue_band_analysis(p, n, true, st, c.ana, false, c.cols_tma, gana_dct));
   timer_mark(p, "gradient_analysis", st);
   // 3. threshold subgradient per band (+ tau partials), then D^T
   const size_t pstride = (size_t)B * p->ntiles;
   NSST_CUDA(launch_rows_backward(p->gj_rows_backward, B * p->ndir_total, n, H, W, p->arena, G, p->twWh, p->twW, tau,
                                  mode, p->partials, pstride, st));
   timer_mark(p, "band_rows_backward", st);
-  NSST_CUDA(launch_cols(ColOp::Synthesis, p->gj_synthesis, B * L, n, H, W, (float2*)G, (float2*)G, p->spec,
-                        (size_t)H * p->WH, p->twH, st));
+  bool sums_dct2 = false;
+  NSST_TRY(enqueue_synthesis(p, n, c, p->gcols_tmap, p->gcols_tma_ok, p->gj_synthesis, G, G, st, &sums_dct2));
   timer_mark(p, "gradient_synthesis", st);
   for (int c0 = 0; c0 < n; c0 += kMaxAtrousJobs) {  // lowpass band mask -> gy plane 0
     const int cn = std::min(kMaxAtrousJobs, n - c0);
@@ -2572,7 +2599,7 @@ nsst_status tau_backward_dct(nsst_plan* p, const float* const* x, const float* c
   // 4. d loss / d x = IDCT2(sum_l R_l .* DCT2(g_l) + R_low .* DCT2(g_0))
   NSST_TRY(enqueue_dct_rows_io(p, n, gy0c.data(), gy0.data(), st));
   NSST_CUDA(launch_dct_cols(kDct2, p->gj_dct_gy0, B, n, H, W, G, G, p->twH, p->wdH, st));
-  NSST_CUDA(launch_dct_cols(kDct2, p->gj_dct_sum, B * L, n, H, W, G, G, p->twH, p->wdH, st));
+  if (!sums_dct2) NSST_CUDA(launch_dct_cols(kDct2, p->gj_dct_sum, B * L, n, H, W, G, G, p->twH, p->wdH, st));
   NSST_CUDA(launch_dct_rows_syn(p->gj_dct_syn, B, n, L, (size_t)H * p->WH, H, W, G, G, p->gy, (size_t)(L + 1) * HW,
                                 p->dct_ra, HW, p->dct_ra + (size_t)(2 * L + 1) * HW, p->twWh, p->twW, p->twDW, st));
   std::vector<const float*> gy1c(gy1.begin(), gy1.end());
