@@ -973,8 +973,8 @@ __device__ __forceinline__ void fft_ld_acc_passes(float2* buf, const float2* __r
 // values the forward transform's first pass needs (output r of butterfly j is
 // index j + r N/R, the first pass's input r of butterfly j), so the turn from
 // one transform to the other happens in registers, without a shared-memory
-// round trip or a barrier.  op(v, flag) maps each value and may set a
-// thread-local flag; the turn returns the block-wide OR of the flags (false:
+// round trip or a barrier.  op(v, flag, index, sequence) maps each value and
+// may set a thread-local flag; the turn returns the block-wide OR of the flags (false:
 // the forward transform has not run and buf holds the inverse transform's
 // next-to-last pass).
 // ---------------------------------------------------------------------------
@@ -1010,7 +1010,7 @@ __device__ __forceinline__ bool stockham_turn(float2* buf, const float2* __restr
       for (int r = 1; r < R; r++) v[it][r] = tw_mul<+1>(v[it][r], tw, r * j);  // NS = NB: k = j, STEP = 1
       Dft<R, +1>::run(v[it]);
 #pragma unroll
-      for (int r = 0; r < R; r++) v[it][r] = op(v[it][r], flag);
+      for (int r = 0; r < R; r++) v[it][r] = op(v[it][r], flag, j + r * NB, s);
       Dft<R, -1>::run(v[it]);  // the forward first pass: no twiddles
     }
   }
