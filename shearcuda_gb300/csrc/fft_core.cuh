@@ -1070,9 +1070,11 @@ __device__ __forceinline__ bool block_fft_inv_op_fwd(float2* buf, const float2* 
 // w / NSEQ, s = w % NSEQ), which is the first pass's input layout when the
 // plan's first radix is R: the first pass runs on the registers and writes
 // buf, the rest are the engine's, the last storing through st.
-template <int N, int NSEQ, int T, int DIR, int R, int IPT, class St>
+// hook runs after the first pass's barrier.
+template <int N, int NSEQ, int T, int DIR, int R, int IPT, class St, class Hook = NoHook>
 __device__ __forceinline__ void block_fft_from_regs(float2* buf, const float2* __restrict__ tw,
-                                                    const float2 (&v)[IPT][R], const St& st) {
+                                                    const float2 (&v)[IPT][R], const St& st,
+                                                    const Hook& hook = Hook{}) {
   using Plan = typename FftPlan<N>::type;
   static_assert(FirstRadix<Plan>::value == R, "the plan's first radix must be the registers' radix");
   constexpr int NB = N / R;
@@ -1090,6 +1092,7 @@ __device__ __forceinline__ void block_fft_from_regs(float2* buf, const float2* _
     for (int r = 0; r < R; r++) buf[swz_row<NSEQ, SWZ>(j * R + r) * NSEQ + s] = u[r];
   }
   __syncthreads();
+  hook();
   auto rd = [&](int row, int sq) -> float2 { return buf[row * NSEQ + sq]; };  // (the passes read buf)
   fft_hook_ip_passes<N, NSEQ, T, DIR, R, SWZ>(buf, tw, rd, st, NoHook{}, typename TailRadices<Plan>::type{});
 }

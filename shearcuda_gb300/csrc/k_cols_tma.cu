@@ -175,6 +175,111 @@ __global__ void __launch_bounds__(AnaCfg<H>::T, AnaCfg<H>::MINB)
   tma.drain(err);
 }
 
+// The same with the level spectrum's column group in registers: every thread
+// keeps its own first-pass inputs of Y, which are the same for every band.  A
+// CTA is bound by its shared-memory accesses between the barriers of the
+// passes, and the register copy takes one read of Y per band out of them (D
+// holds Y's column 0, of which the packed DC/Nyquist column needs the mirrored
+// element too).  Two planes of shared memory instead of three would let a
+// third CTA on the SM at 512 and 1024 rows, but at 64 registers less a thread
+// the sums spill: 64 x 512^2 took 4201 us with three CTAs, 4168 with two, 4305
+// before.  12 x 1024^2: 3984 us -> 3845; 2048^2: 1815 -> 1767.  At 256 rows
+// 128 threads x 5 CTAs (64 x 256^2: 1210 us -> 1088; x 4 1090, x 6 1097).
+// The lengths with a factor 3 lose by it (16 x 768 x 1024: 3959 us -> 4119,
+// 16 x 384 x 512: 932 -> 974), so they keep the plane.
+template <int H>
+struct AnaRegs {
+  using C = AnaCfg<H>;
+  static constexpr int R = FirstRadix<typename FftPlan<H>::type>::value;
+  static constexpr int T = H == 256 ? 128 : C::T;
+  static constexpr int MINB = H == 256 ? 5 : C::MINB;
+  static constexpr int IPT = H / R * C::CS / T;
+  static constexpr bool on = H == 256 || H == 512 || H == 1024 || H == 2048;
+  static constexpr size_t smem() { return (2 * (size_t)H * C::CS + H) * sizeof(float2); }
+};
+template <int H, bool DCTANA>
+__global__ void __launch_bounds__(AnaRegs<H>::T, AnaRegs<H>::MINB)
+    k_band_analysis_ml_regs(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap smap,
+                            const ColJob* __restrict__ jobs, int n_active, int WH, float2* dst_base,
+                            const float2* __restrict__ spec_base, int spec_row0, size_t band_stride,
+                            const float2* __restrict__ twH, const float2* __restrict__ wd, int* err, int per_level) {
+  pdl_sync();
+  using C = AnaCfg<H>;
+  constexpr int CS = C::CS, T = AnaRegs<H>::T, R = AnaRegs<H>::R, IPT = AnaRegs<H>::IPT, NB = H / R;
+  static_assert(NB * CS == IPT * T, "every thread owns IPT first-pass butterflies");
+  extern __shared__ __align__(1024) float2 tsm[];
+  float2* A = tsm;          // the level spectrum's column group, then the transform, in place
+  float2* Wb = A + H * CS;  // filter spectrum of the current band
+  float2* D = Wb + H * CS;  // Y's column 0
+  const ColBlock cb = col_block<CS>(per_level);
+  const ColJob job = jobs[cb.job];
+  if (job.item >= n_active || job.nbands <= 0) return;
+  const int col0 = cb.col0;
+  const bool dc = col0 == 0;
+  const int band_rows = (int)(band_stride / WH);
+  const int yrow = (int)(job.src / WH), srow = spec_row0 + (int)(job.spec / WH);
+  ColTma<H, CS> tma{smem_u32(D + H), col0};
+  if (threadIdx.x == 0) {
+    tma.init();
+    tma.expect(2);
+    tma.load(&amap, A, yrow);
+    tma.load(&smap, Wb, srow);
+  }
+  __syncthreads();  // the mbarrier is initialised before any thread waits on it
+  tma.wait(err);    // Y and band 0's filter group
+  if constexpr (DCTANA) {
+    // the level's column pass, as in k_band_analysis_ml_tma, in place
+    for (int e = threadIdx.x; e < (H / 2 + 1) * CS; e += T) {
+      const int s = e % CS, kk = e / CS;
+      if (kk == 0) continue;  // Z[0] = C[0]
+      const float2 w = __ldg(&wd[kk]);
+      const float2 a = A[kk * CS + s], b = A[(H - kk) * CS + s];
+      A[kk * CS + s] = cmulc(make_float2(a.x + b.y, a.y - b.x), w);
+      if (kk != H - kk) A[(H - kk) * CS + s] = cmul(make_float2(b.x + a.y, b.y - a.x), make_float2(-w.y, w.x));
+    }
+    __syncthreads();
+    auto row_of = [](int i) { return i < H / 2 ? 2 * i : 2 * H - 1 - 2 * i; };
+    block_fft_hook_ip<H, CS, T, +1>(A, twH, SmemLd<CS>{A},
+                                    [&](int i, int s, float2 v) { A[row_of(i) * CS + s] = v; });
+    block_fft_hook_ip<H, CS, T, -1>(A, twH, SmemLd<CS>{A}, SmemSt<CS>{A});
+  }
+  float2 y[IPT][R];
+#pragma unroll
+  for (int it = 0; it < IPT; it++) {
+    const int w = threadIdx.x + it * T;
+#pragma unroll
+    for (int r = 0; r < R; r++) y[it][r] = A[(w / CS + r * NB) * CS + w % CS];
+  }
+  if (dc)
+    for (int i = threadIdx.x; i < H; i += T) D[i] = A[i * CS];
+  __syncthreads();  // A may be overwritten
+  for (int k = 0; k < job.nbands; k++) {
+    if (k > 0) tma.wait(err);
+    // Wk .* Y, with the packed DC/Nyquist column's M term
+    // Z'[u] = P[u] Z[u] + M[u] conj(Z[-u])
+    float2 v[IPT][R];
+#pragma unroll
+    for (int it = 0; it < IPT; it++) {
+      const int w = threadIdx.x + it * T, s = w % CS, j = w / CS;
+#pragma unroll
+      for (int r = 0; r < R; r++) v[it][r] = cmul(Wb[(j + r * NB) * CS + s], y[it][r]);
+      if (dc && s == 0) {
+        const float2* m0 = spec_base + job.m0 + (size_t)k * H;
+#pragma unroll
+        for (int r = 0; r < R; r++)
+          v[it][r] = cadd(v[it][r], cmul(__ldg(&m0[j + r * NB]), cconj(D[(H - j - r * NB) % H])));
+      }
+    }
+    // after the first pass's barrier every thread has read Wb
+    auto next = [&]() {
+      if (threadIdx.x == 0 && tma.ok && k + 1 < job.nbands) tma.refill(&smap, Wb, srow + (k + 1) * band_rows);
+    };
+    block_fft_from_regs<H, CS, T, +1>(A, twH, v, ColGlobalSt{dst_base + job.dst + (size_t)k * band_stride + col0, WH},
+                                      next);
+  }
+  tma.drain(err);
+}
+
 // The same on split-complex column pairs (the math of k_band_analysis_ml_p):
 // twH4 is the broadcast twiddle table.
 template <int H>
@@ -482,14 +587,28 @@ static cudaError_t opt_in_tma(KernelT k, size_t bytes) {
   return e;
 }
 
+// The level analysis at H rows: the register form where AnaRegs takes it
+template <int H, bool DCTANA>
+struct LevelAnalysis {
+  static constexpr bool regs = AnaRegs<H>::on;
+  static constexpr int T = regs ? AnaRegs<H>::T : AnaCfg<H>::T;
+  static constexpr size_t smem = (regs ? AnaRegs<H>::smem() : AnaCfg<H>::smem()) + kBarBytes;
+  static constexpr auto kernel() {
+    if constexpr (regs)
+      return &k_band_analysis_ml_regs<H, DCTANA>;
+    else
+      return &k_band_analysis_ml_tma<H, DCTANA>;
+  }
+};
+
 bool cols_tma_supported(int H, int WH) { return col_len_supported(H) && WH % col_tile(H) == 0 && WH % 2 == 0; }
 
 cudaError_t prepare_cols_tma(int H) {
   switch (H) {
 #define CASE(n)                                                                           \
   case n: {                                                                               \
-    cudaError_t e = opt_in_tma(k_band_analysis_ml_tma<n, false>, AnaCfg<n>::smem() + kBarBytes); \
-    if (e == cudaSuccess) e = opt_in_tma(k_band_analysis_ml_tma<n, true>, AnaCfg<n>::smem() + kBarBytes); \
+    cudaError_t e = opt_in_tma(LevelAnalysis<n, false>::kernel(), LevelAnalysis<n, false>::smem);   \
+    if (e == cudaSuccess) e = opt_in_tma(LevelAnalysis<n, true>::kernel(), LevelAnalysis<n, true>::smem); \
     if (e == cudaSuccess) e = opt_in_tma(k_band_synthesis_tma<n>, SynCfg<n>::smem() + kBarBytes); \
     if (e == cudaSuccess) e = opt_in_tma(k_band_analysis_ml_p_tma<n>, AnaCfg<n>::smem() + kBarBytes); \
     if (e == cudaSuccess) e = opt_in_tma(k_band_synthesis_p_tma<n>, SynCfg<n>::smem() + kBarBytes); \
@@ -525,11 +644,11 @@ cudaError_t launch_cols_tma(ColOp op, const void* amap, const void* smap, const 
     dim3 grid(WH / ColCfg<n>::CS, njobs);                                                                           \
     constexpr size_t sa = AnaCfg<n>::smem() + kBarBytes, ss = SynCfg<n>::smem() + kBarBytes;                        \
     if (op == ColOp::AnalysisLevel)                                                                                 \
-      launch_pdl(k_band_analysis_ml_tma<n, false>, grid, AnaCfg<n>::T, sa, st, m, sm, jobs, n_active, WH, dst_base, spec_base,  \
-                                                                       sr, band_stride, twH, wd, err, per_level);   \
+      launch_pdl(LevelAnalysis<n, false>::kernel(), grid, LevelAnalysis<n, false>::T, LevelAnalysis<n, false>::smem, st, m, \
+                 sm, jobs, n_active, WH, dst_base, spec_base, sr, band_stride, twH, wd, err, per_level);            \
     else if (op == ColOp::AnalysisLevelDct)                                                                         \
-      launch_pdl(k_band_analysis_ml_tma<n, true>, grid, AnaCfg<n>::T, sa, st, m, sm, jobs, n_active, WH, dst_base, spec_base,   \
-                                                                      sr, band_stride, twH, wd, err, per_level);    \
+      launch_pdl(LevelAnalysis<n, true>::kernel(), grid, LevelAnalysis<n, true>::T, LevelAnalysis<n, true>::smem, st, m,    \
+                 sm, jobs, n_active, WH, dst_base, spec_base, sr, band_stride, twH, wd, err, per_level);            \
     else if (op == ColOp::AnalysisLevelPairs)                                                                       \
       launch_pdl(k_band_analysis_ml_p_tma<n>, grid, AnaCfg<n>::T, sa, st, m, jobs, n_active, WH, dst_base, spec_base, sr,   \
                                                                   band_stride, twH, err, per_level);                \
