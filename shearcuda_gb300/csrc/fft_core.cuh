@@ -437,7 +437,23 @@ template <int DIR> struct Dft<14, DIR> : DftCoprime<2, 7, DIR> {};
 template <int DIR> struct Dft<18, DIR> : DftCoprime<2, 9, DIR> {};
 
 // ---------------------------------------------------------------------------
-// Radix plans per length (product of radices == N).
+// Radix plans per length (product of radices == N): as few passes as the
+// registers allow, the wide radices first and last, the narrow one between.  The
+// first and the last pass carry the loads and stores and then run alike on all
+// threads; where they are equal, one transform goes to the next in registers
+// (the threshold's turn, the band sum's inverse).  Whole passes, us, against the
+// plans that ended on the narrow radix or began with 3:
+//   1024  16 4 16   12 x 1024^2 3849 -> 3701; 4 x 1024 x 2048 2922 -> 2715 (16 16 4;
+//                   8 16 8: 3966)
+//   2048  16 8 16   2048^2 1767 -> 1708 (16 16 8)
+//   768   16 3 16   16 x 768 x 1024 4377 -> 3960 (3 16 16; 8 12 8: 4294)
+//   384   16 3 8    32 x 384^2 1643 -> 1573, 16 x 384 x 512 966 -> 915, 16 x 384 x 768
+//                   1768 -> 1598 (3 16 8); 8 6 8: 1583, 933, 1581, and one image's
+//                   analysis at 384 x 512 101 against 98; 8 3 16: 1749 for 32 x 384^2
+//   192   16 12     32 x 192^2 468 -> 449, 32 x 192 x 384 888 -> 813 against 8 3 8, 518
+//                   and more with 3 8 8; 12 16: 491, 898; 4 12 4: 510
+//   96    8 12      16 x 256 x 192 320 -> 297 (3 4 8); 4 6 4: 305
+//   128   16 8      64 x 256^2 1084; 8 16: 1105
 // ---------------------------------------------------------------------------
 template <int... Rs>
 struct RadixList {};
@@ -445,15 +461,15 @@ struct RadixList {};
 template <int N>
 struct FftPlan;
 template <> struct FftPlan<64> { using type = RadixList<8, 8>; };
-template <> struct FftPlan<96> { using type = RadixList<3, 4, 8>; };
+template <> struct FftPlan<96> { using type = RadixList<8, 12>; };
 template <> struct FftPlan<128> { using type = RadixList<16, 8>; };
-template <> struct FftPlan<192> { using type = RadixList<3, 8, 8>; };
+template <> struct FftPlan<192> { using type = RadixList<16, 12>; };
 template <> struct FftPlan<256> { using type = RadixList<16, 16>; };
-template <> struct FftPlan<384> { using type = RadixList<3, 16, 8>; };
+template <> struct FftPlan<384> { using type = RadixList<16, 3, 8>; };
 template <> struct FftPlan<512> { using type = RadixList<8, 8, 8>; };
-template <> struct FftPlan<768> { using type = RadixList<3, 16, 16>; };
-template <> struct FftPlan<1024> { using type = RadixList<16, 16, 4>; };
-template <> struct FftPlan<2048> { using type = RadixList<16, 16, 8>; };
+template <> struct FftPlan<768> { using type = RadixList<16, 3, 16>; };
+template <> struct FftPlan<1024> { using type = RadixList<16, 4, 16>; };
+template <> struct FftPlan<2048> { using type = RadixList<16, 8, 16>; };
 
 // One Stockham pass of radix R over NSEQ sequences of length N, in place.
 // NS = product of the radices already applied.  All threads participate.

@@ -51,11 +51,11 @@ template <int N>
 struct AnaCfg : ColCfg<N> {
   static constexpr size_t smem() { return 3 * (size_t)N * ColCfg<N>::CS * sizeof(float2); }
   // the column kernels' thread count (every thread busy in the radix-16
-  // passes); shared memory allows two CTAs per SM below 2048 points.  The
-  // 3 x 16 x 16 and 3 x 16 x 8 plans (768 and 384 points) have 192
-  // radix-16 butterflies per column group: 192 threads, three CTAs per SM
-  // (their planes take 72 KB), where 256 threads left a quarter of the
-  // warps waiting at the barrier in those passes
+  // passes); shared memory allows two CTAs per SM below 2048 points.  At 768
+  // points (16 x 3 x 16) a column group has 192 radix-16 butterflies and at 384
+  // (16 x 3 x 8) 192 of them too: 192 threads, three CTAs per SM (their planes
+  // take 72 KB), where 256 threads left a quarter of the warps waiting at the
+  // barrier in those passes
   static constexpr bool ODD3 = N == 768 || N == 384;
   static constexpr int T = ODD3 ? 192 : ColCfg<N>::T;
   static constexpr int MINB = N >= 2048 ? 1 : ODD3 ? 3 : 2;
