@@ -363,7 +363,8 @@ def nsst_denoise_batch(xs, shear, sigmas, K, scalars=None, mode=THRESH_HARD, out
 
 
 class MultiBatch:
-    """Uneven batch over several plans (one per image size), replayed as one CUDA graph."""
+    """Uneven batch over several plans (one per image size), one stream per size;
+    replayed as one CUDA graph when the same buffers come again."""
 
     def __init__(self, plans):
         self.plans = list(plans)
