@@ -13,8 +13,13 @@ namespace nsst {
 template <int N>
 struct RowCfg {  // N = W/2 complex points per row
   static constexpr int RS = N >= 1024 ? 4 : 8;
-  // 256 = 16 x 16: a radix-16 pass has 16 butterflies per row, one per thread
-  static constexpr int T = N == 256 ? 128 : 256;
+  // Up to 256 points (16 x 16, 16 x 12, 16 x 8, ...) a pass has at most 16
+  // butterflies per row of the tile: with 256 threads half of them idled at 64 to
+  // 192 points (32 x 192^2: 452 -> 432 us, 32 x 256 x 384 923 -> 884, 64 x 256^2
+  // 1087 -> 1066; 64 threads up to 128 points: 1050 there, but one 256 x 192 image
+  // 81 -> 89).  Longer rows keep 256: 16 x 512 x 1024 2393, with 512 threads 2735,
+  // with 128 2993; 384 points with 192 threads 942 against 937 (16 x 256 x 768).
+  static constexpr int T = N <= 256 ? 128 : 256;
   static constexpr int MINB = 1024 / T;  // <= 64 registers: at least 32 warps per SM
   static constexpr int LD = RS;
   static constexpr size_t smem() { return 2 * (size_t)N * LD * sizeof(float2); }
