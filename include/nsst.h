@@ -59,11 +59,14 @@ typedef struct nsst_config {
                                    allow it.  nsst_shear_trans,
                                    nsst_inverse_shear, nsst_atrousdec,
                                    nsst_atrousrec, the differentiable denoise
-                                   (forward and backward), the separation,
-                                   nsst_re_weight_band and the operator
-                                   adjoints follow the same mode; calls that
-                                   pass images not 16-byte aligned use the
-                                   direct pyramid. */
+                                   (forward and backward), the separation and
+                                   the operator adjoints follow the same
+                                   mode; calls that pass images not 16-byte
+                                   aligned use the direct pyramid, and
+                                   nsst_re_weight_band always does: its result
+                                   may be much smaller than the image, and a
+                                   pixel that is not finite then stays within
+                                   the filters' support. */
 } nsst_config;
 
 typedef struct nsst_plan nsst_plan;
@@ -373,7 +376,7 @@ nsst_status nsst_thresh_max(nsst_plan* plan, float* coeffs, double sigma, const 
  * (x, out: H x W device; 2 <= nweights <= nlevels + 1).  Replaces
  * re_weight_band / re_weight_band_cuda (re_weight_band.m:23-29,
  * re_weight_band_cuda.cpp:59-183), which likewise take the level count from
- * the length of the weight vector. */
+ * the length of the weight vector.  out may overlap x. */
 nsst_status nsst_re_weight_band(nsst_plan* plan, const float* x, const double* weights, int nweights, float* out,
                                 void* stream);
 

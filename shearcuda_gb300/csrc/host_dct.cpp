@@ -7,7 +7,6 @@
 //     G_h,M[k1][k2] = sum_{a,b} h[a][b] cos(pi k1 M (a - c0) / H) cos(pi k2 M (b - c0) / W).
 // The tables chain those products the way atrousdec.m:33-48 and
 // atrousrec.m:27-40 chain the steps.
-#include <algorithm>
 #include <cmath>
 #include <thread>
 
@@ -65,25 +64,22 @@ void level_response(const std::vector<double>& h, int F, int M, int H, int W, st
 
 }  // namespace
 
-bool dct_pyramid_tables(const PyramidFilters& pf, int L, int H, int W, std::vector<float>* out) {
+void dct_pyramid_tables(const PyramidFilters& pf, int L, int H, int W, std::vector<float>* out) {
   const size_t HW = (size_t)H * W;
   out->assign((size_t)(2 * L + 3) * HW, 0.0f);
   const double s = 1.0 / ((double)H * W);
   std::vector<double> ch(HW, 1.0), cg(HW, 1.0);  // running products of the h0 / g0 responses
   std::vector<double> G[4];
-  double off = 0.0;  // largest |h0 g0 + h1 g1 - 1|, and |h1 g1| at 0
   for (int i = 0; i < L; i++) {  // dilation 2^i: directional level L-1-i
     std::vector<std::thread> th;
     for (int f = 0; f < 4; f++) th.emplace_back([&, f] { level_response(pf.h[f], pf.F[f], 1 << i, H, W, G[f]); });
     for (auto& t : th) t.join();
-    off = std::max(off, std::fabs(G[1][0] * G[3][0]));
     const int l = L - 1 - i;
     float* ra = out->data() + (size_t)l * HW;
     float* rs = out->data() + (size_t)(L + l) * HW;
     for (size_t e = 0; e < HW; e++) {
       ra[e] = (float)(s * ch[e] * G[1][e]);  // atrousdec.m: highpass after i lowpass steps
       rs[e] = (float)(s * G[3][e] * cg[e]);  // atrousrec.m: g1 step, then i g0 steps
-      off = std::max(off, std::fabs(G[0][e] * G[2][e] + G[1][e] * G[3][e] - 1.0));
       ch[e] *= G[0][e];
       cg[e] *= G[2][e];
     }
@@ -96,7 +92,6 @@ bool dct_pyramid_tables(const PyramidFilters& pf, int L, int H, int W, std::vect
     rl[e] = (float)(s * ch[e]);          // lowpass band (atrousdec.m's y{1})
     gl[e] = (float)(s * cg[e]);          // lowpass synthesis (atrousrec.m's L g0 steps)
   }
-  return off <= 1e-9;
 }
 
 std::vector<float4> dct_row_twiddles(int W) {

@@ -195,7 +195,7 @@ cudaError_t launch_atrous(const AtrousJobs& jobs, int njobs, int maxH, int maxW,
 // The DCT-domain pyramid of the fused pipeline (k_dct.cu).
 cudaError_t prepare_dct_kernels(int H, int WH);
 cudaError_t launch_dct_rows_fwd(const DctIo& io, int n, int H, int W, const float2* twWh, const float4* twD,
-                                cudaStream_t st, bool level = false);
+                                cudaStream_t st);
 cudaError_t launch_dct_rows_ana(const RowJob* jobs, int njobs, int n_active, int H, int W, const void* src_base,
                                 void* dst_base, const float* resp, size_t resp_stride, const float2* twWh,
                                 const float2* twW, const float4* twD, bool real_out, cudaStream_t st);
@@ -207,7 +207,7 @@ cudaError_t launch_dct_cols(int mode, const ColJob* jobs, int njobs, int n_activ
                             void* dst_base, const float2* twH, const float2* wdH, cudaStream_t st,
                             const float* thr = nullptr, int th_stride = 0, int th_mode = 0);
 cudaError_t launch_dct_cols_out(const DctIo& io, int n, int H, int W, const float2* twH, const float2* wdH,
-                                cudaStream_t st, const float* add = nullptr, float add_w = 0.f);
+                                cudaStream_t st);
 // Adjoint helper: out (Ho x Wo, extended domain) = zero-extended full
 // correlation of x with the *unflipped* filter h, Ho = H + M(F-1).
 cudaError_t launch_atrous_full(const AtrousJobs& jobs, int njobs, int maxHo, int maxWo, int M, int F, const float* h,
@@ -241,9 +241,6 @@ constexpr int kMaxPlaneWeights = NSST_MAX_LEVELS + 1;
 struct PlaneWeights {  // passed by value
   float w[kMaxPlaneWeights];
 };
-// V = w[0] T + sum_l w[1 + l] R_l Q_l n - base / n (the tables hold 1/n each), n = H W values
-cudaError_t launch_dct_weights(const float* ra, const float* rs, const float* tl, size_t n, int nlev,
-                               const PlaneWeights& w, float base, float* V, cudaStream_t st);
 cudaError_t launch_scale_planes(float* data, size_t n, int nplanes, const PlaneWeights& w, cudaStream_t st);
 
 // ------------------------------------------------------------------- 3-D path
@@ -377,9 +374,7 @@ std::vector<float2> half_twiddle_table(int n);       // exp(-2 pi i k / n), k < 
 // lowpass synthesis); row twiddles (exp(-i pi k / (2W)), exp(-2 pi i k / W)) for
 // k = 0..W/2; column twiddles exp(-i pi k / (2H)), k < H.
 bool filters_symmetric(const PyramidFilters& pf);
-// returns whether every step's filters reconstruct perfectly (h0 g0 + h1 g1 = 1) and
-// pass a constant by the lowpass alone (h1 g1 = 0 at 0), to 1e-9
-bool dct_pyramid_tables(const PyramidFilters& pf, int L, int H, int W, std::vector<float>* out);
+void dct_pyramid_tables(const PyramidFilters& pf, int L, int H, int W, std::vector<float>* out);
 std::vector<float4> dct_row_twiddles(int W);
 std::vector<float2> dct_col_twiddles(int H);
 

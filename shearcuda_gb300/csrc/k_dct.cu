@@ -58,16 +58,14 @@ __device__ __forceinline__ const float* rowf(const float2* P, int s) {
 // DCT-II input order of a real row in the padded row-major staging: element
 // m of the W/2-point complex view is (v[2m], v[2m+1]), v[j] = x[2j] for
 // j < W/2 and x[2W-1-2j] above.
-template <int WH, bool SUB = false>
+template <int WH>
 struct DctShufLd {
   const float2* P;
-  float sub = 0.f;  // SUB: taken off every sample
   __device__ __forceinline__ float2 operator()(int m, int s) const {
     constexpr int W = 2 * WH;
     const float* x = rowf<WH>(P, s);
     const int j0 = 2 * m, j1 = 2 * m + 1;
-    const float a = j0 < WH ? x[2 * j0] : x[2 * W - 1 - 2 * j0], b = j1 < WH ? x[2 * j1] : x[2 * W - 1 - 2 * j1];
-    return SUB ? make_float2(a - sub, b - sub) : make_float2(a, b);
+    return make_float2(j0 < WH ? x[2 * j0] : x[2 * W - 1 - 2 * j0], j1 < WH ? x[2 * j1] : x[2 * W - 1 - 2 * j1]);
   }
 };
 
@@ -168,10 +166,8 @@ struct DctMinB {
 // Row kernels, grid = (H / RS, jobs); RS rows per CTA staged row-major.
 // ---------------------------------------------------------------------------
 
-// real rows (the caller's images) -> DCT-II rows; LEVEL: of the images less a
-// constant near their mean (eight samples of the diagonal), which takes the
-// transform's rounding off the image's offset
-template <int WH, bool LEVEL>
+// real rows (the caller's images) -> DCT-II rows
+template <int WH>
 __global__ void __launch_bounds__(RowCfg<WH>::T, DctMinB<RowCfg<WH>::T>::value)
     k_dct_rows_fwd(const __grid_constant__ DctIo io, const float2* __restrict__ twWh, const float4* __restrict__ tw) {
   pdl_sync();
@@ -182,14 +178,7 @@ __global__ void __launch_bounds__(RowCfg<WH>::T, DctMinB<RowCfg<WH>::T>::value)
   fetch_rows_rm<WH, C::RS, C::T>(A, reinterpret_cast<const float2*>(io.src[blockIdx.y]) + off);
   cp_async_wait_all();
   __syncthreads();
-  float level = 0.f;
-  if constexpr (LEVEL) {
-    constexpr int W = 2 * WH;
-    const int H = gridDim.x * C::RS;
-#pragma unroll
-    for (int q = 1; q < 16; q += 2) level += 0.125f * __ldg(io.src[blockIdx.y] + (size_t)(q * H / 16) * W + q * W / 16);
-  }
-  block_fft_hook_ip<WH, C::RS, C::T, -1>(A, twWh, DctShufLd<WH, LEVEL>{A, level}, SmemStRM<WH>{A});
+  block_fft_hook_ip<WH, C::RS, C::T, -1>(A, twWh, DctShufLd<WH>{A}, SmemStRM<WH>{A});
   float* dst = io.dst[blockIdx.y] + 2 * off;
   for (int e = threadIdx.x; e < WH * C::RS; e += C::T) {
     const int k = e % WH, s = e / WH;
@@ -402,14 +391,13 @@ __global__ void __cluster_dims__(1, 1, kSynRanks) __launch_bounds__(RowCfg<WH>::
 // Column kernels, grid = (WH / CS, jobs): CS columns of a packed H x WH array.
 // ---------------------------------------------------------------------------
 // kDct2: DCT-II; kDct3: DCT-III; kDctAna: DCT-III then the forward FFT;
-// kDct3 with `add`: th times the add plane joins the result;
 // kDctThresh: DCT-III, the threshold (th, tmode) of both real columns of each
 // element, DCT-II (the DCT-II input order undoes the DCT-III output order, so
 // the threshold applies to the inverse FFT's output in place)
 template <int H, int MODE>
 __device__ __forceinline__ void dct_cols_body(const float2* src, float2* dst, int WH, float2* A,
                                               const float2* __restrict__ twH, const float2* __restrict__ wd,
-                                              float th = 0.0f, int tmode = 0, const float2* add = nullptr) {
+                                              float th = 0.0f, int tmode = 0) {
   using C = ColCfg<H>;
   auto row_of = [](int i) { return i < H / 2 ? 2 * i : 2 * H - 1 - 2 * i; };
   if (MODE == kDct2) {
@@ -447,14 +435,8 @@ __device__ __forceinline__ void dct_cols_body(const float2* src, float2* dst, in
   }
   __syncthreads();
   if (MODE == kDct3) {
-    block_fft_hook_ip<H, C::CS, C::T, +1>(A, twH, SmemLd<C::CS>{A}, [&](int i, int s, float2 v) {
-      const size_t o = (size_t)row_of(i) * WH + s;
-      if (add) {  // dst may be add
-        const float2 x = add[o];
-        v = make_float2(fmaf(th, x.x, v.x), fmaf(th, x.y, v.y));
-      }
-      dst[o] = v;
-    });
+    block_fft_hook_ip<H, C::CS, C::T, +1>(A, twH, SmemLd<C::CS>{A},
+                                          [&](int i, int s, float2 v) { dst[(size_t)row_of(i) * WH + s] = v; });
   } else if (MODE == kDctThresh) {
     block_fft_hook_ip<H, C::CS, C::T, +1>(A, twH, SmemLd<C::CS>{A}, [&](int i, int s, float2 v) {
       A[i * C::CS + s] = make_float2(apply_thresh(v.x, th, tmode), apply_thresh(v.y, th, tmode));
@@ -486,45 +468,17 @@ __global__ void __launch_bounds__(ColCfg<H>::T, DctMinB<ColCfg<H>::T>::value)
 template <int H>
 __global__ void __launch_bounds__(ColCfg<H>::T, DctMinB<ColCfg<H>::T>::value)
     k_dct_cols_out(const __grid_constant__ DctIo io, int WH, const float2* __restrict__ twH,
-                   const float2* __restrict__ wd, const float2* add, float add_w) {
+                   const float2* __restrict__ wd) {
   pdl_sync();
   extern __shared__ float2 smem[];
   const int col0 = blockIdx.x * ColCfg<H>::CS;
   dct_cols_body<H, kDct3>(reinterpret_cast<const float2*>(io.src[blockIdx.y]) + col0,
-                          reinterpret_cast<float2*>(io.dst[blockIdx.y]) + col0, WH, smem, twH, wd, add_w, 0,
-                          add ? add + col0 : nullptr);
-}
-
-// The response of a re-weighted pyramid (re_weight_band.m:23-29) less `base`:
-// 4 values per thread, bound by the 2 nlev + 1 table planes' reads.
-__global__ void __launch_bounds__(256)
-    k_dct_weights(const float4* __restrict__ ra, const float4* __restrict__ rs, const float4* __restrict__ tl, size_t n4,
-                  int nlev, const __grid_constant__ PlaneWeights w, float scale, float base, float4* __restrict__ V) {
-  pdl_sync();
-  const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
-  if (i >= n4) return;
-  const float4 t = __ldg(tl + i);
-  float4 v = make_float4(w.w[0] * t.x, w.w[0] * t.y, w.w[0] * t.z, w.w[0] * t.w);
-  for (int l = 0; l < nlev; l++) {
-    const float4 a = __ldg(ra + l * n4 + i), b = __ldg(rs + l * n4 + i);
-    const float c = w.w[1 + l] * scale;
-    v = make_float4(v.x + c * a.x * b.x, v.y + c * a.y * b.y, v.z + c * a.z * b.z, v.w + c * a.w * b.w);
-  }
-  V[i] = make_float4(v.x - base, v.y - base, v.z - base, v.w - base);
+                          reinterpret_cast<float2*>(io.dst[blockIdx.y]) + col0, WH, smem, twH, wd);
 }
 
 // ---------------------------------------------------------------------------
 // Launchers
 // ---------------------------------------------------------------------------
-cudaError_t launch_dct_weights(const float* ra, const float* rs, const float* tl, size_t n, int nlev,
-                               const PlaneWeights& w, float base, float* V, cudaStream_t st) {
-  if (nlev + 1 > kMaxPlaneWeights || n % 4) return cudaErrorInvalidValue;
-  count_launch();
-  launch_pdl(k_dct_weights, (unsigned)((n / 4 + 255) / 256), 256, 0, st, 
-      reinterpret_cast<const float4*>(ra), reinterpret_cast<const float4*>(rs), reinterpret_cast<const float4*>(tl),
-      n / 4, nlev, w, (float)n, (float)(base / (double)n), reinterpret_cast<float4*>(V));
-  return cudaGetLastError();
-}
 #define NSST_DCT_ROW_SIZES(X) X(64) X(96) X(128) X(192) X(256) X(384) X(512) X(1024)
 #define NSST_DCT_COL_SIZES(X) X(128) X(192) X(256) X(384) X(512) X(768) X(1024) X(2048)
 
@@ -538,8 +492,7 @@ cudaError_t prepare_dct_kernels(int H, int WH) {
   switch (WH) {
 #define CASE(n)                                                                  \
   case n:                                                                        \
-    e = dct_opt_in(k_dct_rows_fwd<n, false>, RowCfg<n>::smem_rm());              \
-    if (e == cudaSuccess) e = dct_opt_in(k_dct_rows_fwd<n, true>, RowCfg<n>::smem_rm()); \
+    e = dct_opt_in(k_dct_rows_fwd<n>, RowCfg<n>::smem_rm());                     \
     if (e == cudaSuccess) e = dct_opt_in(k_dct_rows_ana<n, false>, RowCfg<n>::smem_rm()); \
     if (e == cudaSuccess) e = dct_opt_in(k_dct_rows_ana<n, true>, RowCfg<n>::smem_rm()); \
     if (e == cudaSuccess) e = dct_opt_in(k_dct_rows_syn<n, false>, 2 * RowCfg<n>::smem_rm()); \
@@ -570,19 +523,14 @@ cudaError_t prepare_dct_kernels(int H, int WH) {
 }
 
 cudaError_t launch_dct_rows_fwd(const DctIo& io, int n, int H, int W, const float2* twWh, const float4* twD,
-                                cudaStream_t st, bool level) {
+                                cudaStream_t st) {
   if (n <= 0 || n > kMaxAtrousJobs) return n == 0 ? cudaSuccess : cudaErrorInvalidValue;
   count_launch();
   switch (W / 2) {
-#define CASE(n_)                                                                                    \
-  case n_: {                                                                                        \
-    const dim3 grid(H / RowCfg<n_>::RS, n);                                                         \
-    if (level)                                                                                      \
-      launch_pdl(k_dct_rows_fwd<n_, true>, grid, RowCfg<n_>::T, RowCfg<n_>::smem_rm(), st, io, twWh, twD);  \
-    else                                                                                            \
-      launch_pdl(k_dct_rows_fwd<n_, false>, grid, RowCfg<n_>::T, RowCfg<n_>::smem_rm(), st, io, twWh, twD); \
-    return cudaGetLastError();                                                                      \
-  }
+#define CASE(n_)                                                                                               \
+  case n_:                                                                                                     \
+    launch_pdl(k_dct_rows_fwd<n_>, dim3(H / RowCfg<n_>::RS, n), RowCfg<n_>::T, RowCfg<n_>::smem_rm(), st, io, twWh, twD); \
+    return cudaGetLastError();
     NSST_DCT_ROW_SIZES(CASE)
 #undef CASE
     default:
@@ -687,7 +635,7 @@ cudaError_t launch_dct_cols(int mode, const ColJob* jobs, int njobs, int n_activ
 }
 
 cudaError_t launch_dct_cols_out(const DctIo& io, int n, int H, int W, const float2* twH, const float2* wdH,
-                                cudaStream_t st, const float* add, float add_w) {
+                                cudaStream_t st) {
   if (n <= 0 || n > kMaxAtrousJobs) return n == 0 ? cudaSuccess : cudaErrorInvalidValue;
   count_launch();
   const int WH = W / 2;
@@ -695,7 +643,7 @@ cudaError_t launch_dct_cols_out(const DctIo& io, int n, int H, int W, const floa
 #define CASE(n_)                                                                                                   \
   case n_:                                                                                                         \
     launch_pdl(k_dct_cols_out<n_>, dim3(WH / ColCfg<n_>::CS, n), ColCfg<n_>::T, ColCfg<n_>::smem() / 2, st,           \
-        io, WH, twH, wdH, reinterpret_cast<const float2*>(add), add_w);                                            \
+        io, WH, twH, wdH);                                                                                         \
     return cudaGetLastError();
     NSST_DCT_COL_SIZES(CASE)
 #undef CASE

@@ -131,8 +131,6 @@ struct nsst_plan {
   RowJob* j_dct_low = nullptr; // pyr plane 0 -> tmp plane 0: the lowpass band (B)
   ColJob* j_dct_lowc = nullptr; // tmp plane 0 in place                 (B)
   RowJob* j_dct_rec = nullptr;  // lev (bands' DCT-II planes) -> pyr plane 1 (B)
-  RowJob* j_dct_weight = nullptr;  // item 0: pyr plane 0 -> tmp plane 0, response plane 0 (1)
-  bool dct_pr = false;             // the pyramid filters reconstruct perfectly and pass a constant by the lowpass alone
 
   // fused directional stage (k_dir_fused.cu): one thread-block cluster per
   // (item, level), the bands kept on chip
@@ -490,7 +488,7 @@ nsst_status create_plan(const nsst_config* cfg, int H, int W, int B, const Filte
   p->dct_ok = filters_symmetric(p->pf) && cfg->pyramid != NSST_PYRAMID_DIRECT;
   if (cfg->pyramid == NSST_PYRAMID_SPECTRAL && !p->dct_ok)
     return destroy(fail(NSST_ERR_INVALID_ARG, "the spectral pyramid needs pyramid filters symmetric in both axes"));
-  size_t o_dct = 0, o_twDW = 0, o_wdH = 0, o_jd1 = 0, o_jd2 = 0, o_jd3 = 0, o_jd4 = 0, o_jd5 = 0, o_jd6 = 0, o_jd7 = 0, o_jd8 = 0;
+  size_t o_dct = 0, o_twDW = 0, o_wdH = 0, o_jd1 = 0, o_jd2 = 0, o_jd3 = 0, o_jd4 = 0, o_jd5 = 0, o_jd6 = 0, o_jd7 = 0;
   if (p->dct_ok) {
     o_dct = take(sizeof(float) * HW * (2 * p->nlev + 3));
     o_twDW = take(sizeof(float4) * (p->WH + 1));
@@ -502,7 +500,6 @@ nsst_status create_plan(const nsst_config* cfg, int H, int W, int B, const Filte
     o_jd5 = take(sizeof(RowJob) * NB);
     o_jd6 = take(sizeof(ColJob) * NB);
     o_jd7 = take(sizeof(RowJob) * NB);
-    o_jd8 = take(sizeof(RowJob));
   }
   p->arena_bytes = off;
   ce = dev_alloc((void**)&p->arena, p->arena_bytes);
@@ -677,9 +674,8 @@ nsst_status create_plan(const nsst_config* cfg, int H, int W, int B, const Filte
     p->j_dct_low = (RowJob*)(A + o_jd5);
     p->j_dct_lowc = (ColJob*)(A + o_jd6);
     p->j_dct_rec = (RowJob*)(A + o_jd7);
-    p->j_dct_weight = (RowJob*)(A + o_jd8);
     std::vector<float> tab;
-    p->dct_pr = dct_pyramid_tables(p->pf, p->nlev, H, W, &tab);
+    dct_pyramid_tables(p->pf, p->nlev, H, W, &tab);
     auto tw = dct_row_twiddles(W);
     auto wh = dct_col_twiddles(H);
     auto f2 = [&](const void* ptr) { return (size_t)((const char*)ptr - A) / sizeof(float2); };
@@ -709,8 +705,6 @@ nsst_status create_plan(const nsst_config* cfg, int H, int W, int B, const Filte
     if (ce == cudaSuccess) ce = cudaMemcpy(p->j_dct_low, jl.data(), jl.size() * sizeof(RowJob), cudaMemcpyHostToDevice);
     if (ce == cudaSuccess) ce = cudaMemcpy(p->j_dct_lowc, jlc.data(), jlc.size() * sizeof(ColJob), cudaMemcpyHostToDevice);
     if (ce == cudaSuccess) ce = cudaMemcpy(p->j_dct_rec, jr.data(), jr.size() * sizeof(RowJob), cudaMemcpyHostToDevice);
-    const RowJob jw{f2(p->pyr), f2(p->tmp), 0, 0};
-    if (ce == cudaSuccess) ce = cudaMemcpy(p->j_dct_weight, &jw, sizeof(jw), cudaMemcpyHostToDevice);
     if (ce == cudaSuccess) ce = prepare_dct_kernels(H, p->WH);
     if (ce != cudaSuccess) return destroy(cuda_fail(ce, "DCT pyramid tables"));
     p->dct_on = true;
@@ -1587,7 +1581,11 @@ nsst_status nsst_thresh_max(nsst_plan* p, float* coeffs, double sigma, const dou
 }
 
 // re_weight_band.m:23-29 / re_weight_band_cuda.cpp:132-183: atrousdec with
-// nweights - 1 levels, weight per pyramid band, atrousrec
+// nweights - 1 levels, weight per pyramid band, atrousrec.  By the direct
+// pyramid whatever the plan's mode: one product in the DCT domain takes less
+// time (768 x 1024, three levels: 44 us, this 200) but rounds at the image's
+// scale, not the result's (white noise, lowpass alone: 5.3e-6 off against
+// 1.9e-7), and spreads a pixel that is not finite over the image.
 nsst_status nsst_re_weight_band(nsst_plan* p, const float* x, const double* weights, int nweights, float* out,
                                 void* stream) {
   if (!p || !x || !weights || !out) return fail(NSST_ERR_INVALID_ARG, "NULL argument");
@@ -1604,35 +1602,6 @@ nsst_status nsst_re_weight_band(nsst_plan* p, const float* x, const double* weig
   p->saved_n = 0;
   cudaStream_t st = (cudaStream_t)stream;
   timer_begin(p, st);
-  const int n = nweights - 1;
-  if (p->dct_on && aligned16(x) && aligned16(out) && p->dct_pr) {
-    // spectral pyramid: out = w0 x + IDCT2(DCT2(x - c) .* (V - w0)), V the
-    // weighted sum of the bands' round trips and w0 the lowpass weight.  V(0) =
-    // w0, so any constant c drops out: one near the image's mean keeps its
-    // offset out of the transform's rounding, which a larger weight of the
-    // detail would raise above the result's own scale.  The lowpass of fewer
-    // levels than the plan's is the plan's lowpass and coarser bands together
-    // (h0 g0 + h1 g1 = 1 per level).
-    const size_t HW = (size_t)p->H * p->W;
-    char* A = p->arena;
-    float *x1 = p->pyr + HW, *t0 = p->tmp, *V = p->tmp + HW;
-    PlaneWeights v{};
-    v.w[0] = w.w[0];
-    for (int l = 0; l < p->nlev; l++) v.w[1 + l] = l < p->nlev - n ? w.w[0] : w.w[1 + l - (p->nlev - n)];
-    const float base = v.w[0];
-    NSST_CUDA(launch_dct_weights(p->dct_ra, p->dct_rs, p->dct_tl, HW, p->nlev, v, base, V, st));
-    DctIo in{};
-    in.src[0] = x;
-    in.dst[0] = x1;
-    NSST_CUDA(launch_dct_rows_fwd(in, 1, p->H, p->W, p->twWh, p->twDW, st, true));
-    NSST_CUDA(launch_dct_cols(kDct2, p->j_dct_x, p->B, 1, p->H, p->W, A, A, p->twH, p->wdH, st));
-    NSST_CUDA(launch_dct_rows_ana(p->j_dct_weight, 1, 1, p->H, p->W, A, A, V, HW, p->twWh, p->twW, p->twDW, true, st));
-    DctIo io{};
-    io.src[0] = t0;
-    io.dst[0] = out;
-    NSST_CUDA(launch_dct_cols_out(io, 1, p->H, p->W, p->twH, p->wdH, st, x, base));
-    return NSST_OK;
-  }
   float* y = p->pyr;  // item 0's pyramid planes: lowpass, then band-pass coarse -> fine
   NSST_TRY(run_atrousdec(p, 1, &x, &y, nullptr, st, nweights - 1));
   NSST_CUDA(launch_scale_planes(y, (size_t)p->H * p->W, nweights, w, st));
