@@ -14,7 +14,11 @@ const V3Ops* v3_ops_large(int n) {
       return &ops;
     }
     case 216: {
-      static const V3Ops ops = V3Launch<216, false, true>::ops();
+      static const V3Ops ops = V3Launch<216, true, true>::ops();
+      return &ops;
+    }
+    case 256: {  // the convolution of the 216 grid
+      static const V3Ops ops = V3Launch<256, false, true>::ops();
       return &ops;
     }
     default:

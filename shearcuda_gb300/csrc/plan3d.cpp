@@ -38,7 +38,9 @@ constexpr int kSmCount = 152;
 constexpr int kCtasPerSm = 8;      // CTAs per SM that keep a pass's loads in flight
 // Band pairs in flight per level: the work buffer holds as many as fit here (at least one).
 constexpr size_t kPairBytes = (size_t)1 << 30;
+// The 2^a 3^b lengths: the grids of NSST3_GRID_FAST, and the convolution lengths that nsst3_level_dims reports.
 const int kFftLens[] = {16, 24, 32, 48, 64, 72, 96, 128, 144, 192, 216, 256};
+constexpr int kMaxLen = 256;
 
 bool is_fft_len(int n) {
   for (int v : kFftLens)
@@ -58,11 +60,15 @@ int conv_len(int m) {
 // and 7 beside 2 and 3 (and 11 and 17 where the padded grids have them anyway).
 // A level costs its convolution volume, so 156 -> 160 instead of 192, 108
 // instead of 128 and 76 -> 80 instead of 96 are 0.58, 0.60 and 0.58 of it.
-const int kConvLens[] = {32, 44, 48, 56, 64, 72, 80, 88, 100, 108, 140, 144, 160, 204, 216};
 int run_len(int m) {
-  for (int v : kConvLens)
-    if (v >= m + kSameOff) return v;
+  for (int v = m + kSameOff; v <= kMaxLen; v++)
+    if (const V3Ops* o = v3_ops(v); o && o->conv) return v;
   return -1;
+}
+// What a grid may have as a level size is what the pyramid is compiled for.
+bool is_pyr_len(int n) {
+  const V3Ops* o = v3_ops(n);
+  return o && o->pyr;
 }
 
 nsst_status fail3(nsst_status s, const std::string& msg) {
@@ -105,16 +111,16 @@ bool pyr_params(double mode, int L, double* w, double* tbw, double* D) {
 }
 
 // Level sizes of a grid g: g, g/D0, g/D0/D1, ...; false if one is not an
-// integer supported transform length or its convolution length is missing.
+// integer 2^a 3^b transform length or its convolution length is missing.
 bool level_sizes(int g, int L, const double* D, int* out) {
   double v = g;
   out[0] = g;
-  if (!is_fft_len(g) || conv_len(g) < 0) return false;
+  if (!is_fft_len(g) || !is_pyr_len(g) || run_len(g) < 0) return false;
   for (int l = 0; l < L; l++) {
     v /= D[l];
     const int iv = (int)std::lround(v);
-    if (std::fabs(v - iv) > 1e-9 || !is_fft_len(iv) || iv % 8) return false;
-    if (l + 1 < L && conv_len(iv) < 0) return false;
+    if (std::fabs(v - iv) > 1e-9 || !is_fft_len(iv) || !is_pyr_len(iv) || iv % 8) return false;
+    if (l + 1 < L && run_len(iv) < 0) return false;
     out[l + 1] = iv;
   }
   return true;
@@ -124,15 +130,8 @@ bool level_sizes(int g, int L, const double* D, int* out) {
 // mainAnySize.m:51): every dimension gains d - rem(n, d) planes, d = 3 2^(L-1)
 // (divFactor [3 6 12 24] of the level count), so that Pyr_mode 1.5's level
 // sizes g, g/1.5, g/3, ... are integers.  Its level sizes need transform
-// lengths with other prime factors (132 = 3 * 4 * 11, 204 = 3 * 4 * 17); the
-// pass kernels hold sequence groups that need not divide them.
-const int kOddLens[] = {22, 34, 44, 68, 88, 132, 136, 204};
-bool is_pyr_len(int n) {
-  if (is_fft_len(n)) return true;
-  for (int v : kOddLens)
-    if (v == n) return true;
-  return false;
-}
+// lengths with other prime factors (132 = 3 * 4 * 11, 204 = 3 * 4 * 17).  The
+// largest compiled one is 216, for sides up to 215 on one or two levels.
 int marshal_grid(int n, int L) {
   const int d = 3 << (L - 1);
   return n + d - n % d;
@@ -141,14 +140,14 @@ bool marshal_sizes(int g, int L, const double* D, int* out, int* missing) {
   double v = g;
   out[0] = g;
   *missing = 0;
-  if (!is_pyr_len(g) || conv_len(g) < 0) {
+  if (!is_pyr_len(g) || run_len(g) < 0) {
     *missing = g;
     return false;
   }
   for (int l = 0; l < L; l++) {
     v /= D[l];
     const int iv = (int)std::lround(v);
-    if (std::fabs(v - iv) > 1e-9 || !is_pyr_len(iv) || (l + 1 < L && conv_len(iv) < 0)) {
+    if (std::fabs(v - iv) > 1e-9 || !is_pyr_len(iv) || (l + 1 < L && run_len(iv) < 0)) {
       *missing = iv;
       return false;
     }
@@ -550,7 +549,7 @@ nsst_status nsst3_plan_create(const nsst3_config* cfg, int n0, int n1, int n2, i
         return fail3(NSST_ERR_UNSUPPORTED_SIZE,
                      "MarshalData grid " + std::to_string(p->g[k]) + " of dimension " + std::to_string(dims[k]) +
                          " needs transform length " + std::to_string(miss) +
-                         ", not compiled (level sizes of the 132 and 204 grids and the 2^a 3^b lengths are)");
+                         ", not compiled (level sizes of the 132 and 204 grids and the 2^a 3^b lengths up to 216 are)");
     } else {
       p->g[k] = grid_size(dims[k], p->L, p->D);
       if (p->g[k] < 0 || !level_sizes(p->g[k], p->L, p->D, sizes[k]))
@@ -571,9 +570,7 @@ nsst_status nsst3_plan_create(const nsst3_config* cfg, int n0, int n1, int n2, i
     a.xh_off = xh_off;
     xh_off += align_up3(a.half(), 32);
     if (l == p->L) break;
-    for (int k = 0; k < 3; k++)
-      if ((a.lc[k] = run_len(a.m[k])) < 0)
-        return fail3(NSST_ERR_UNSUPPORTED_SIZE, "volume level too large for the compiled convolution lengths");
+    for (int k = 0; k < 3; k++) a.lc[k] = run_len(a.m[k]);
     a.nd = cfg->num_dirs[l];
     a.nb = 3 * a.nd * a.nd;
     a.first_band = p->nbands;

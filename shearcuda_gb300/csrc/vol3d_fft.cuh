@@ -74,6 +74,7 @@ V3_RADIX(160, 10, 16)
 V3_RADIX(192, 12, 16)
 V3_RADIX(204, 12, 17)
 V3_RADIX(216, 12, 18)
+V3_RADIX(256, 16, 16)
 #undef V3_RADIX
 
 template <int N>
