@@ -422,14 +422,15 @@ nsst_status nsst_onfilter(const char* type, int par, double* out, int* len);
  * yl: n x H x W (the level-L lowpass); yh: n x 3L x H x W, per level the
  * planes LH, HL, HH (first letter: filtering along a row), level 1 first --
  * the reference's m x 3nL yh, block by block.  H and W must be multiples of
- * 2^L, W <= 8192.  x may equal yl.  Asynchronous on stream. */
+ * 2^L, W <= 8192.  x may equal yl.  Takes no scratch.  Asynchronous on
+ * stream. */
 nsst_status nsst_mrdwt(const float* x, int n, int H, int W, const double* h, int lh, int L, float* yl, float* yh,
                        void* stream);
 
 /* Inverse of nsst_mrdwt: mirdwt / mirdwt_cuda (src/mirdwt_r.h:115-219,
  * src_cuda/mirdwt_cuda.cpp).  yl, yh are left unchanged; x may equal yl.
- * Takes up to two planes of stream-ordered scratch per image, as does
- * nsst_mrdwt. */
+ * Takes stream-ordered scratch: one plane per image for L > 1, one more where
+ * x overlaps yl. */
 nsst_status nsst_mirdwt(const float* yl, const float* yh, int n, int H, int W, const double* h, int lh, int L,
                         float* x, void* stream);
 

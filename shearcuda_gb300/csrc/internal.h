@@ -404,6 +404,10 @@ struct WvPlanes {   // one level of n items (item strides in floats)
 // or NULL) hard-thresholds the three.  cur, yl and yh must not overlap.
 cudaError_t launch_rdwt_level(const WvPlanes& P, int n, int H, int W, int sf, const WvTaps& t, const float* thr,
                               cudaStream_t st);
+// The same with cur anywhere but in the level's own yh planes: it may be or
+// overlap yl.
+cudaError_t launch_rdwt_level_in_place(const WvPlanes& P, int n, int H, int W, int sf, const WvTaps& t,
+                                       const float* thr, cudaStream_t st);
 // mirdwt, one level: (ll, yh) -> x.  x must not overlap ll or yh.
 cudaError_t launch_irdwt_level(const float* ll, size_t s_ll, const float* yh, size_t s_yh, float* x, size_t s_x, int n,
                                int H, int W, int sf, const WvTaps& t, cudaStream_t st);

@@ -2879,38 +2879,54 @@ nsst_status check_rdwt(int n, int H, int W, int lh, int L) {
   return NSST_OK;
 }
 
-bool overlap(const float* a, const float* b, size_t n) { return a < b + n && b < a + n; }
+bool overlap(const float* a, size_t na, const float* b, size_t nb) { return a < b + nb && b < a + na; }
 
 // mrdwt_r.h:135-208 for n images (item strides: x, yl HW; yh 3 L HW); thr
 // (device, n floats) hard-thresholds every highpass plane as it is written
-// (thresh.m:44 with option 1), or NULL.  A level's lowpass goes to yl and to
-// s0 (n images) in turn, the last one to yl; where that makes the first level
-// write the images it reads (x overlaps yl), to s1 instead (n images; may be
-// NULL if x does not overlap yl).
+// (thresh.m:44 with option 1), or NULL.  A level's lowpass must not go where it
+// reads.  With s0 (n images) it goes to yl and to s0 in turn, the last one to
+// yl; x must not overlap yl then.  Without, it goes to the last level's own
+// planes, which nothing else uses before that level, in turn, and from the last
+// but one to yl, in which the last level then runs in place; so does a first
+// level that would write over the images it reads.  A buffer from the device's
+// pool in place of that level: 32 x 256^2 49 us, this 61; one 256^2 image 30, this
+// 24; and where a synchronisation follows each call, at which the pool gives the
+// memory back, 230 us, this 33.
 nsst_status enqueue_mrdwt(const float* x, int n, int H, int W, const WvTaps& t, int L, float* yl, float* yh,
-                          const float* thr, float* s0, float* s1, cudaStream_t st) {
-  const size_t HW = (size_t)H * W;
-  const float* cur = x;
+                          const float* thr, float* s0, cudaStream_t st) {
+  const size_t HW = (size_t)H * W, s_yh = (size_t)3 * L * HW;
+  float* park = yh + (size_t)3 * (L - 1) * HW;
+  const bool over_yl = overlap(x, n * HW, yl, n * HW), over_yh = overlap(x, n * HW, yh, n * s_yh);
+  WvPlanes P{x, HW, nullptr, HW, nullptr, s_yh};
   for (int l = 1; l <= L; l++) {
-    float* dst = (L - l) % 2 == 0 ? yl : s0;
-    if (l == 1 && dst == yl && overlap(x, yl, n * HW)) dst = s1;
-    const WvPlanes P{cur, HW, dst, HW, yh + (size_t)3 * (l - 1) * HW, (size_t)3 * L * HW};
-    NSST_CUDA(launch_rdwt_level(P, n, H, W, 1 << (l - 1), t, thr, st));
-    cur = dst;
+    P.yh = yh + (size_t)3 * (l - 1) * HW;
+    P.yl = yl;
+    P.s_yl = HW;
+    if (s0) {
+      if ((L - l) % 2) P.yl = s0;
+    } else if (l < L - 1) {
+      P.yl = park + (size_t)(l % 2) * HW;
+      P.s_yl = s_yh;
+    }
+    const bool in_place = !s0 && (l > 1 ? l == L : P.yl == yl ? over_yl : over_yh);
+    NSST_CUDA((in_place ? launch_rdwt_level_in_place : launch_rdwt_level)(P, n, H, W, 1 << (l - 1), t, thr, st));
+    P.cur = P.yl;
+    P.s_cur = P.s_yl;
   }
-  if (cur != yl) NSST_CUDA(cudaMemcpyAsync(yl, cur, n * HW * sizeof(float), cudaMemcpyDeviceToDevice, st));
   return NSST_OK;
 }
 
-// mirdwt_r.h:148-218 for n images; s0 and s1 as above, with x in yl's place and
-// the last level's yl in x's.
+// mirdwt_r.h:148-218 for n images.  A level's lowpass goes to x and to s0 (n
+// images) in turn, the last one to x; where that makes the first level write the
+// planes it reads (yl overlaps x), to s1 instead (n images; may be NULL if yl
+// does not overlap x).
 nsst_status enqueue_mirdwt(const float* yl, const float* yh, int n, int H, int W, const WvTaps& t, int L, float* x,
                            float* s0, float* s1, cudaStream_t st) {
   const size_t HW = (size_t)H * W, s_yh = (size_t)3 * L * HW;
   const float* cur = yl;
   for (int l = L; l >= 1; l--) {
     float* dst = (l - 1) % 2 == 0 ? x : s0;
-    if (l == L && dst == x && overlap(yl, x, n * HW)) dst = s1;
+    if (l == L && dst == x && overlap(yl, n * HW, x, n * HW)) dst = s1;
     NSST_CUDA(launch_irdwt_level(cur, HW, yh + (size_t)3 * (l - 1) * HW, s_yh, dst, HW, n, H, W, 1 << (l - 1), t, st));
     cur = dst;
   }
@@ -2974,14 +2990,7 @@ nsst_status nsst_mrdwt(const float* x, int n, int H, int W, const double* h, int
   if (!x || !h || !yl || !yh) return fail(NSST_ERR_INVALID_ARG, "NULL argument");
   NSST_TRY(check_rdwt(n, H, W, lh, L));
   const WvTaps t = analysis_taps(std::vector<double>(h, h + lh));
-  cudaStream_t st = (cudaStream_t)stream;
-  const size_t nHW = (size_t)n * H * W;
-  const bool over = overlap(x, yl, nHW);
-  AsyncScratch s;
-  s.st = st;
-  if (L > 1 || over) NSST_CUDA(cudaMallocAsync(&s.ptr, sizeof(float) * (over ? 2 : 1) * nHW, st));
-  float* s0 = (float*)s.ptr;
-  return enqueue_mrdwt(x, n, H, W, t, L, yl, yh, nullptr, s0, over ? s0 + nHW : nullptr, st);
+  return enqueue_mrdwt(x, n, H, W, t, L, yl, yh, nullptr, nullptr, (cudaStream_t)stream);
 }
 
 nsst_status nsst_mirdwt(const float* yl, const float* yh, int n, int H, int W, const double* h, int lh, int L,
@@ -2991,7 +3000,7 @@ nsst_status nsst_mirdwt(const float* yl, const float* yh, int n, int H, int W, c
   const WvTaps t = synthesis_taps(std::vector<double>(h, h + lh));
   cudaStream_t st = (cudaStream_t)stream;
   const size_t nHW = (size_t)n * H * W;
-  const bool over = overlap(yl, x, nHW);
+  const bool over = overlap(yl, nHW, x, nHW);
   AsyncScratch s;
   s.st = st;
   if (L > 1 || over) NSST_CUDA(cudaMallocAsync(&s.ptr, sizeof(float) * (over ? 2 : 1) * nHW, st));
@@ -3121,7 +3130,7 @@ nsst_status nsst_separate(nsst_plan* p, const float* img, int n, int level2, int
   NSST_TRY(enqueue_band_maxima(p, n, xw.data(), bits, st));
   // separate.m:119-126: buff(2) = max |yh| of the Symmlet-4 mrdwt, per image
   NSST_CUDA(cudaMemsetAsync(bits + (size_t)n * nb, 0, sizeof(unsigned) * n * 3 * L, st));
-  NSST_TRY(enqueue_mrdwt(imgw, n, H, W, ta, L, yl, yh, nullptr, wlow, nullptr, st));
+  NSST_TRY(enqueue_mrdwt(imgw, n, H, W, ta, L, yl, yh, nullptr, wlow, st));
   NSST_CUDA(launch_plane_maxabs(yh, HW, n * 3 * L, bits + (size_t)n * nb, kRedBlocks, st));
   NSST_CUDA(cudaMemcpyAsync(hb, bits, sizeof(unsigned) * nbits, cudaMemcpyDeviceToHost, st));
   // the noise estimates on the host cores while the maxima are computed
@@ -3185,7 +3194,7 @@ nsst_status nsst_separate(nsst_plan* p, const float* img, int n, int level2, int
     NSST_CUDA(cudaEventRecord(p->fork_ev, st));
     NSST_CUDA(cudaStreamWaitEvent(sd, p->fork_ev, 0));
     // points: wavelet hard threshold (second stream)
-    NSST_TRY(enqueue_mrdwt(ra2, n, H, W, ta, L, yl, yh, thW + (size_t)k * n, wlow, nullptr, sd));
+    NSST_TRY(enqueue_mrdwt(ra2, n, H, W, ta, L, yl, yh, thW + (size_t)k * n, wlow, sd));
     NSST_TRY(enqueue_mirdwt(yl, yh, n, H, W, ts, L, P, wlow, nullptr, sd));
     NSST_CUDA(cudaEventRecord(p->join_ev, sd));
     // curves: shearlet hard threshold, then TV correction
