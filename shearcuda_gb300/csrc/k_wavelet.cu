@@ -348,22 +348,27 @@ bool rdwt_width_supported(int W) { return W >= 2 && W <= kWvMaxW; }
 
 // Rows per CTA: as many as share the taps' rows (8, 4 or 2) while two CTAs fit
 // an SM and the grid fills the GPU; 2 where the width or the grid is small.
+constexpr size_t kWvTwoCtas = 110 * 1024;  // shared memory of a CTA of which two fit an SM
 static int rdwt_rows(int n, int H, int W, int sf) {
   for (int th : {8, 4})
-    if ((size_t)2 * th * W * sizeof(float) <= 110 * 1024 && (long)n * sf * ((H / sf + th - 1) / th) >= 2 * 152)
+    if ((size_t)2 * th * W * sizeof(float) <= kWvTwoCtas && (long)n * sf * ((H / sf + th - 1) / th) >= 2 * 152)
       return th;
   return 2;
 }
 
-template <class K, class... Args>
-static cudaError_t launch_rdwt(K kernel, int th, int n, int H, int W, int sf, cudaStream_t st, Args... args) {
+// The shared memory opted into is the most that the kernel is ever launched
+// with: the attribute is the function's, and a launch of another width in another
+// thread may come between a smaller one's setting and its launch.
+template <auto Kernel, class... Args>
+static cudaError_t launch_rdwt(int th, int n, int H, int W, int sf, cudaStream_t st, Args... args) {
   const size_t sm = (size_t)2 * th * W * sizeof(float);
   if (sm > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    const size_t most = th > 2 ? kWvTwoCtas : (size_t)2 * 2 * kWvMaxW * sizeof(float);
+    const cudaError_t e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
     if (e != cudaSuccess) return e;
   }
   count_launch();
-  launch_pdl(kernel, dim3((unsigned)(sf * ((H / sf + th - 1) / th)), (unsigned)n), kWvThreads, sm, st, args...);
+  launch_pdl(Kernel, dim3((unsigned)(sf * ((H / sf + th - 1) / th)), (unsigned)n), kWvThreads, sm, st, args...);
   return cudaGetLastError();
 }
 
@@ -374,7 +379,7 @@ cudaError_t launch_rdwt_level(const WvPlanes& P, int n, int H, int W, int sf, co
                               cudaStream_t st) {
   if (!rdwt_width_supported(W) || t.lh < 1 || t.lh > kMaxQmf || n < 1 || n > 65535) return cudaErrorInvalidValue;
 #define GO(l, h)                                                                                                   \
-  launch_rdwt(k_rdwt_fwd<l, h>, h, n, H, W, sf, st, P.cur, P.s_cur, P.yl, P.s_yl, P.yh, P.s_yh, H, W, sf, t, thr)
+  launch_rdwt<k_rdwt_fwd<l, h>>(h, n, H, W, sf, st, P.cur, P.s_cur, P.yl, P.s_yl, P.yh, P.s_yh, H, W, sf, t, thr)
 #define CASE(l)                                         \
   case l:                                               \
     switch (rdwt_rows(n, H, W, sf)) {             \
@@ -410,7 +415,7 @@ cudaError_t launch_rdwt_level_in_place(const WvPlanes& P, int n, int H, int W, i
 cudaError_t launch_irdwt_level(const float* ll, size_t s_ll, const float* yh, size_t s_yh, float* x, size_t s_x, int n,
                                int H, int W, int sf, const WvTaps& t, cudaStream_t st) {
   if (!rdwt_width_supported(W) || t.lh < 1 || t.lh > kMaxQmf || n < 1 || n > 65535) return cudaErrorInvalidValue;
-#define GO(l, h) launch_rdwt(k_rdwt_inv<l, h>, h, n, H, W, sf, st, ll, s_ll, yh, s_yh, x, s_x, H, W, sf, t)
+#define GO(l, h) launch_rdwt<k_rdwt_inv<l, h>>(h, n, H, W, sf, st, ll, s_ll, yh, s_yh, x, s_x, H, W, sf, t)
 #define CASE(l)                                         \
   case l:                                               \
     switch (rdwt_rows(n, H, W, sf)) {             \
