@@ -31,7 +31,7 @@ __device__ __forceinline__ float soft(float v, float t) {
   return r > 0.0f ? copysignf(r, v) : 0.0f;
 }
 
-// LH: the filter length (0: t.lh, taps re-read per output row); TH: rows per CTA.
+// LH: the filter length (0: t.lh); TH: rows per CTA.
 // Grid: x = row phase (fastest) and group of TH rows of the phase, y = item.
 // Taps are applied in ascending order whatever the form.  Two results that take
 // the same taps or the same sample share packed FP32 FMAs, which round as two
@@ -66,13 +66,23 @@ __global__ void __launch_bounds__(kWvThreads, 4)
         for (int k = 0; k < TH; k++)
           if (m - k >= 0 && m - k < LH) lh[k] = __ffma2_rn(make_float2(t.a[m - k], t.b[m - k]), v, lh[k]);
       }
-    } else {
-      for (int k = 0; k < TH; k++) {
-        int i = (i0 + k) % Hp;
-        for (int j = 0; j < t.lh; j++) {
-          lh[k] = __ffma2_rn(make_float2(t.a[j], t.b[j]), twice(__ldg(x + i * rs + c)), lh[k]);
-          if (++i == Hp) i = 0;
-        }
+    } else {  // the rows under tap j, rotated by one per tap
+      float v[TH];
+      int i = i0;
+#pragma unroll
+      for (int k = 0; k < TH - 1; k++) {
+        v[k] = __ldg(x + i * rs + c);
+        if (++i == Hp) i = 0;
+      }
+#pragma unroll TH
+      for (int j = 0; j < t.lh; j++) {
+        v[TH - 1] = __ldg(x + i * rs + c);
+        if (++i == Hp) i = 0;
+        const float2 ab = make_float2(t.a[j], t.b[j]);
+#pragma unroll
+        for (int k = 0; k < TH; k++) lh[k] = __ffma2_rn(ab, twice(v[k]), lh[k]);
+#pragma unroll
+        for (int k = 0; k < TH - 1; k++) v[k] = v[k + 1];
       }
     }
 #pragma unroll
@@ -206,16 +216,29 @@ __global__ void __launch_bounds__(kWvThreads, 4)
           if (tt >= 0 && tt < LH) x[k] = __ffma2_rn(twice(t.b[tt]), w, __ffma2_rn(twice(t.a[tt]), v, x[k]));
         }
       }
-    } else {
-      for (int k = 0; k < TH; k++) {
-        int i = (i0 + k) % Hp;
-        for (int tt = 0; tt < t.lh; tt++) {
-          const size_t o = i * rs + c;
-          const float2 v = make_float2(__ldg(p + o), __ldg(q + HW + o));
-          const float2 w = make_float2(__ldg(q + o), __ldg(q + 2 * HW + o));
-          x[k] = __ffma2_rn(twice(t.b[tt]), w, __ffma2_rn(twice(t.a[tt]), v, x[k]));
-          if (--i < 0) i = Hp - 1;
-        }
+    } else {  // the rows under tap tt, rotated by one per tap
+      float2 v[TH], w[TH];  // (LL, HL), (LH, HH)
+      auto row = [&](int k, int i) {
+        const size_t o = i * rs + c;
+        v[k] = make_float2(__ldg(p + o), __ldg(q + HW + o));
+        w[k] = make_float2(__ldg(q + o), __ldg(q + 2 * HW + o));
+      };
+      int i = i0;
+#pragma unroll
+      for (int k = 1; k < TH; k++) {
+        if (++i == Hp) i = 0;
+        row(k, i);
+      }
+      i = i0;
+#pragma unroll TH
+      for (int tt = 0; tt < t.lh; tt++) {
+        row(0, i);
+        if (--i < 0) i = Hp - 1;
+        const float2 a = twice(t.a[tt]), b = twice(t.b[tt]);
+#pragma unroll
+        for (int k = 0; k < TH; k++) x[k] = __ffma2_rn(b, w[k], __ffma2_rn(a, v[k], x[k]));
+#pragma unroll
+        for (int k = TH - 1; k > 0; k--) v[k] = v[k - 1], w[k] = w[k - 1];
       }
     }
 #pragma unroll
@@ -372,7 +395,11 @@ static cudaError_t launch_rdwt(int th, int n, int H, int W, int sf, cudaStream_t
   return cudaGetLastError();
 }
 
-// the lengths of the Haar, Daubechies, Symmlet, Coiflet-1..3 and Beylkin filters
+// The lengths of the Haar, Daubechies, Symmlet, Coiflet-1..3 and Beylkin filters
+// are compiled in.  The others (Coiflet-4 and -5, Vaidyanathan, Battle, a caller's
+// own) take the taps from a loop, with the rows under a tap rotating through
+// registers: 2048^2, four levels, 24 taps 331 and 384 us (analysis, synthesis);
+// with every output row's samples read anew 430 and 592.
 #define NSST_RDWT_LENS(X) X(2) X(4) X(6) X(8) X(10) X(12) X(14) X(16) X(18) X(20)
 
 cudaError_t launch_rdwt_level(const WvPlanes& P, int n, int H, int W, int sf, const WvTaps& t, const float* thr,
@@ -390,7 +417,11 @@ cudaError_t launch_rdwt_level(const WvPlanes& P, int n, int H, int W, int sf, co
   switch (t.lh) {
     NSST_RDWT_LENS(CASE)
     default:
-      return GO(0, 2);
+      switch (rdwt_rows(n, H, W, sf)) {
+        case 8: return GO(0, 8);
+        case 4: return GO(0, 4);
+        default: return GO(0, 2);
+      }
   }
 #undef CASE
 #undef GO
@@ -426,7 +457,11 @@ cudaError_t launch_irdwt_level(const float* ll, size_t s_ll, const float* yh, si
   switch (t.lh) {
     NSST_RDWT_LENS(CASE)
     default:
-      return GO(0, 2);
+      switch (rdwt_rows(n, H, W, sf)) {
+        case 8: return GO(0, 8);
+        case 4: return GO(0, 4);
+        default: return GO(0, 2);
+      }
   }
 #undef CASE
 #undef GO
