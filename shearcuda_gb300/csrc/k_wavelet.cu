@@ -31,8 +31,10 @@ __device__ __forceinline__ float soft(float v, float t) {
   return r > 0.0f ? copysignf(r, v) : 0.0f;
 }
 
-// LH: the filter length (0: t.lh); TH: rows per CTA.
-// Grid: x = row phase (fastest) and group of TH rows of the phase, y = item.
+// LH: the filter length (0: t.lh); TH: rows per CTA; T: its threads; PARTS: of
+// `tile`'s columns, not of the whole row.
+// Grid: x = row phase (fastest) and group of TH rows of the phase, y = item, z =
+// part of the row.
 // Taps are applied in ascending order whatever the form.  Two results that take
 // the same taps or the same sample share packed FP32 FMAs, which round as two
 // single ones.  Bound by latency and issue (40 % of it at 32 images of 256 x 256,
@@ -40,19 +42,27 @@ __device__ __forceinline__ float soft(float v, float t) {
 // an SM, took the four Symmlet-4 levels there from 93 to 66 us (analysis) and 105
 // to 78 us (synthesis); six CTAs (spills) 87 and 84.  Separate column and row
 // kernels measured 133 and 150 us.
+// Columns of a CTA: `out` of the results and `in` of what the row taps reach from
+// there, from their first column on (analysis) or up to their last (synthesis);
+// both the whole row, or in = out + (lh - 1) sf.
+struct WvTile {
+  int out, in;
+};
 __device__ __forceinline__ float2 twice(float v) { return make_float2(v, v); }
 
-template <int LH, int TH>
-__global__ void __launch_bounds__(kWvThreads, 4)
+template <int LH, int TH, int T, bool PARTS>
+__global__ void __launch_bounds__(T, 1024 / T)
     k_rdwt_fwd(const float* __restrict__ cur, size_t s_cur, float* __restrict__ yl, size_t s_yl,
-               float* __restrict__ yh, size_t s_yh, int H, int W, int sf, const __grid_constant__ WvTaps t,
-               const float* __restrict__ thr) {
+               float* __restrict__ yh, size_t s_yh, int H, int W, int sf, WvTile tile,
+               const __grid_constant__ WvTaps t, const float* __restrict__ thr) {
   pdl_sync();
-  extern __shared__ float2 sm[];  // [row][column] (C_lo, C_hi)
+  extern __shared__ float2 sm[];  // [row][column from c0 on] (C_lo, C_hi)
   const int ph = blockIdx.x % sf, i0 = blockIdx.x / sf * TH, item = blockIdx.y, Hp = H / sf;
+  const int c0 = PARTS ? blockIdx.z * tile.out : 0, SW = PARTS ? tile.in : W, n_out = PARTS ? min(tile.out, W - c0) : W;
   const size_t HW = (size_t)H * W, rs = (size_t)sf * W;
   const float* x = cur + item * s_cur + (size_t)ph * W;
-  for (int c = threadIdx.x; c < W; c += kWvThreads) {
+  for (int s = threadIdx.x; s < SW; s += T) {
+    const int c = PARTS && c0 + s >= W ? c0 + s - W : c0 + s;
     float2 lh[TH];  // (lo, hi)
 #pragma unroll
     for (int k = 0; k < TH; k++) lh[k] = twice(0.0f);
@@ -86,32 +96,32 @@ __global__ void __launch_bounds__(kWvThreads, 4)
       }
     }
 #pragma unroll
-    for (int k = 0; k < TH; k++) sm[k * W + c] = lh[k];
+    for (int k = 0; k < TH; k++) sm[k * SW + s] = lh[k];
   }
   __syncthreads();
   const float th = thr ? thr[item] : -1.0f;
   const int lh_n = LH > 0 ? LH : t.lh;
-  for (int c = threadIdx.x; c < W; c += kWvThreads) {
+  for (int s = threadIdx.x; s < n_out; s += T) {
     float2 lo[TH], hi[TH];  // (LL, LH), (HL, HH)
 #pragma unroll
     for (int k = 0; k < TH; k++) lo[k] = hi[k] = twice(0.0f);
-    int cc = c;
+    int ss = s;
 #pragma unroll
     for (int j = 0; j < lh_n; j++) {
       const float2 a = twice(t.a[j]), b = twice(t.b[j]);
 #pragma unroll
       for (int k = 0; k < TH; k++) {
-        const float2 v = sm[k * W + cc];
+        const float2 v = sm[k * SW + ss];
         lo[k] = __ffma2_rn(a, v, lo[k]);
         hi[k] = __ffma2_rn(b, v, hi[k]);
       }
-      cc += sf;
-      if (cc >= W) cc -= W;
+      ss += sf;
+      if (!PARTS && ss >= W) ss -= W;
     }
 #pragma unroll
     for (int k = 0; k < TH; k++) {
       if (i0 + k >= Hp) break;
-      const size_t o = (size_t)(ph + (i0 + k) * sf) * W + c;
+      const size_t o = (size_t)(ph + (i0 + k) * sf) * W + c0 + s;
       float lv = lo[k].y, hl = hi[k].x, hh = hi[k].y;
       if (th >= 0.0f) {
         hl = hard_keep(hl, th);
@@ -187,18 +197,24 @@ __global__ void __launch_bounds__(kWvThreads) k_rdwt_rows_fwd(float* yl, size_t 
   }
 }
 
-template <int LH, int TH>
-__global__ void __launch_bounds__(kWvThreads, 4)
+template <int LH, int TH, int T, bool PARTS>
+__global__ void __launch_bounds__(T, 1024 / T)
     k_rdwt_inv(const float* __restrict__ ll, size_t s_ll, const float* __restrict__ yh, size_t s_yh,
-               float* __restrict__ out, size_t s_out, int H, int W, int sf, const __grid_constant__ WvTaps t) {
+               float* __restrict__ out, size_t s_out, int H, int W, int sf, WvTile tile,
+               const __grid_constant__ WvTaps t) {
   pdl_sync();
   extern __shared__ float2 sm[];
-  float2 *s1 = sm, *sh = sm + TH / 2 * W;  // [row pair][column]: x1, xh of rows 2 q and 2 q + 1
   const int ph = blockIdx.x % sf, i0 = blockIdx.x / sf * TH, item = blockIdx.y, Hp = H / sf;
+  const int c0 = PARTS ? blockIdx.z * tile.out : 0, SW = PARTS ? tile.in : W, n_out = PARTS ? min(tile.out, W - c0) : W;
+  const int off = PARTS ? tile.in - tile.out : 0;
+  float2 *s1 = sm, *sh = sm + TH / 2 * SW;  // [row pair][column from c0 - off on]: x1, xh of rows 2 q and 2 q + 1
   const size_t HW = (size_t)H * W, rs = (size_t)sf * W;
   const float* p = ll + item * s_ll + (size_t)ph * W;
   const float* q = yh + item * s_yh + (size_t)ph * W;
-  for (int c = threadIdx.x; c < W; c += kWvThreads) {
+  for (int s = threadIdx.x; s < SW; s += T) {
+    int c = c0 - off + s;
+    if (PARTS && c < 0) c += W;
+    if (PARTS && c >= W) c -= W;
     float2 x[TH];  // (x1, xh)
 #pragma unroll
     for (int k = 0; k < TH; k++) x[k] = twice(0.0f);
@@ -243,29 +259,29 @@ __global__ void __launch_bounds__(kWvThreads, 4)
     }
 #pragma unroll
     for (int k = 0; k < TH; k += 2) {
-      s1[k / 2 * W + c] = make_float2(x[k].x, x[k + 1].x);
-      sh[k / 2 * W + c] = make_float2(x[k].y, x[k + 1].y);
+      s1[k / 2 * SW + s] = make_float2(x[k].x, x[k + 1].x);
+      sh[k / 2 * SW + s] = make_float2(x[k].y, x[k + 1].y);
     }
   }
   __syncthreads();
   const int lh_n = LH > 0 ? LH : t.lh;
-  for (int c = threadIdx.x; c < W; c += kWvThreads) {
+  for (int s = threadIdx.x; s < n_out; s += T) {
     float2 acc[TH / 2];
 #pragma unroll
     for (int k = 0; k < TH / 2; k++) acc[k] = twice(0.0f);
-    int cc = c;
+    int ss = s + off;
 #pragma unroll
     for (int j = 0; j < lh_n; j++) {
       const float2 a = twice(t.a[j]), b = twice(t.b[j]);
 #pragma unroll
-      for (int k = 0; k < TH / 2; k++) acc[k] = __ffma2_rn(b, sh[k * W + cc], __ffma2_rn(a, s1[k * W + cc], acc[k]));
-      cc -= sf;
-      if (cc < 0) cc += W;
+      for (int k = 0; k < TH / 2; k++) acc[k] = __ffma2_rn(b, sh[k * SW + ss], __ffma2_rn(a, s1[k * SW + ss], acc[k]));
+      ss -= sf;
+      if (!PARTS && ss < 0) ss += W;
     }
 #pragma unroll
     for (int k = 0; k < TH; k++)
       if (i0 + k < Hp)
-        out[item * s_out + (size_t)(ph + (i0 + k) * sf) * W + c] = k & 1 ? acc[k / 2].y : acc[k / 2].x;
+        out[item * s_out + (size_t)(ph + (i0 + k) * sf) * W + c0 + s] = k & 1 ? acc[k / 2].y : acc[k / 2].x;
   }
 }
 
@@ -369,12 +385,33 @@ __global__ void k_sep_residual(const float* __restrict__ img, const float* __res
 // ----------------------------------------------------------------- launchers
 bool rdwt_width_supported(int W) { return W >= 2 && W <= kWvMaxW; }
 
-// Rows per CTA: as many as share the taps' rows (8, 4 or 2) while two CTAs fit
-// an SM and the grid fills the GPU; 2 where the width or the grid is small.
 constexpr size_t kWvTwoCtas = 110 * 1024;  // shared memory of a CTA of which two fit an SM
-static int rdwt_rows(int n, int H, int W, int sf) {
+constexpr int kWvLong = kWvTwoCtas / (4 * sizeof(float2));  // longest row of which four fit there
+constexpr int kWvFill = 2 * 152;                            // CTAs that fill the GPU
+
+// Columns per CTA.  The whole row, whose columns are filtered once, as a rule.
+// Parts of it where it is longer than kWvLong, so that more than two rows share
+// the taps' rows (1024 x 8192, 8 taps: 60 and 104 us -> 56 and 83, 20 taps 145 and
+// 225 -> 94 and 149), and where the whole rows are too few CTAs (64 x 8192, 20
+// taps: 34 and 46 -> 16 and 16); up to a quarter of a part shared with the next.
+static WvTile rdwt_tile(int n, int H, int W, int sf, int lh) {
+  const int halo = (lh - 1) * sf;
+  const long groups = (long)n * sf * ((H / sf + 1) / 2);
+  WvTile t{W, W};
+  if (W <= kWvLong && groups >= kWvFill) return t;
+  for (int in : {1024, 512, 256}) {
+    if (in >= W || halo > in / 4) continue;
+    t = {in - halo, in};
+    if (groups * ((W + t.out - 1) / t.out) >= kWvFill) break;
+  }
+  return t;
+}
+// Rows per CTA: as many as share the taps' rows (8, 4 or 2) while two CTAs fit
+// an SM and the grid fills the GPU; 2 where the row or the grid is small.
+static int rdwt_rows(int n, int H, int W, int sf, WvTile t) {
   for (int th : {8, 4})
-    if ((size_t)2 * th * W * sizeof(float) <= kWvTwoCtas && (long)n * sf * ((H / sf + th - 1) / th) >= 2 * 152)
+    if (th * t.in * sizeof(float2) <= kWvTwoCtas &&
+        (long)n * sf * ((H / sf + th - 1) / th) * ((W + t.out - 1) / t.out) >= kWvFill)
       return th;
   return 2;
 }
@@ -383,15 +420,17 @@ static int rdwt_rows(int n, int H, int W, int sf) {
 // with: the attribute is the function's, and a launch of another width in another
 // thread may come between a smaller one's setting and its launch.
 template <auto Kernel, class... Args>
-static cudaError_t launch_rdwt(int th, int n, int H, int W, int sf, cudaStream_t st, Args... args) {
-  const size_t sm = (size_t)2 * th * W * sizeof(float);
+static cudaError_t launch_rdwt(int th, int threads, int n, int H, int W, int sf, WvTile t, cudaStream_t st,
+                               Args... args) {
+  const size_t sm = th * t.in * sizeof(float2);
   if (sm > 48 * 1024) {
-    const size_t most = th > 2 ? kWvTwoCtas : (size_t)2 * 2 * kWvMaxW * sizeof(float);
+    const size_t most = th > 2 ? kWvTwoCtas : 2 * kWvMaxW * sizeof(float2);
     const cudaError_t e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
     if (e != cudaSuccess) return e;
   }
   count_launch();
-  launch_pdl(Kernel, dim3((unsigned)(sf * ((H / sf + th - 1) / th)), (unsigned)n), kWvThreads, sm, st, args...);
+  launch_pdl(Kernel, dim3((unsigned)(sf * ((H / sf + th - 1) / th)), (unsigned)n, (unsigned)((W + t.out - 1) / t.out)),
+             threads, sm, st, args...);
   return cudaGetLastError();
 }
 
@@ -405,25 +444,26 @@ static cudaError_t launch_rdwt(int th, int n, int H, int W, int sf, cudaStream_t
 cudaError_t launch_rdwt_level(const WvPlanes& P, int n, int H, int W, int sf, const WvTaps& t, const float* thr,
                               cudaStream_t st) {
   if (!rdwt_width_supported(W) || t.lh < 1 || t.lh > kMaxQmf || n < 1 || n > 65535) return cudaErrorInvalidValue;
-#define GO(l, h)                                                                                                   \
-  launch_rdwt<k_rdwt_fwd<l, h>>(h, n, H, W, sf, st, P.cur, P.s_cur, P.yl, P.s_yl, P.yh, P.s_yh, H, W, sf, t, thr)
-#define CASE(l)                                         \
-  case l:                                               \
-    switch (rdwt_rows(n, H, W, sf)) {             \
-      case 8: return GO(l, 8);                          \
-      case 4: return GO(l, 4);                          \
-      default: return GO(l, 2);                         \
-    }
+  const WvTile tile = rdwt_tile(n, H, W, sf, t.lh);
+#define GO(l, h, T, parts)                                                                                                  \
+  launch_rdwt<k_rdwt_fwd<l, h, T, parts>>(h, T, n, H, W, sf, tile, st, P.cur, P.s_cur, P.yl, P.s_yl, P.yh, P.s_yh, H, W, sf, tile, t, thr)
+#define ROWS(l, parts)                                 \
+  switch (rdwt_rows(n, H, W, sf, tile)) {              \
+    case 8: return GO(l, 8, kWvThreads, parts);        \
+    case 4: return GO(l, 4, kWvThreads, parts);        \
+    default: return GO(l, 2, kWvThreads, parts);       \
+  }
+#define CASE(l) \
+  case l: ROWS(l, false)
+  if (tile.in < W) ROWS(0, true)
+  if (W > kWvLong) return GO(0, 2, 4 * kWvThreads, false);
   switch (t.lh) {
     NSST_RDWT_LENS(CASE)
     default:
-      switch (rdwt_rows(n, H, W, sf)) {
-        case 8: return GO(0, 8);
-        case 4: return GO(0, 4);
-        default: return GO(0, 2);
-      }
+      ROWS(0, false)
   }
 #undef CASE
+#undef ROWS
 #undef GO
 }
 
@@ -446,24 +486,25 @@ cudaError_t launch_rdwt_level_in_place(const WvPlanes& P, int n, int H, int W, i
 cudaError_t launch_irdwt_level(const float* ll, size_t s_ll, const float* yh, size_t s_yh, float* x, size_t s_x, int n,
                                int H, int W, int sf, const WvTaps& t, cudaStream_t st) {
   if (!rdwt_width_supported(W) || t.lh < 1 || t.lh > kMaxQmf || n < 1 || n > 65535) return cudaErrorInvalidValue;
-#define GO(l, h) launch_rdwt<k_rdwt_inv<l, h>>(h, n, H, W, sf, st, ll, s_ll, yh, s_yh, x, s_x, H, W, sf, t)
-#define CASE(l)                                         \
-  case l:                                               \
-    switch (rdwt_rows(n, H, W, sf)) {             \
-      case 8: return GO(l, 8);                          \
-      case 4: return GO(l, 4);                          \
-      default: return GO(l, 2);                         \
-    }
+  const WvTile tile = rdwt_tile(n, H, W, sf, t.lh);
+#define GO(l, h, T, parts) launch_rdwt<k_rdwt_inv<l, h, T, parts>>(h, T, n, H, W, sf, tile, st, ll, s_ll, yh, s_yh, x, s_x, H, W, sf, tile, t)
+#define ROWS(l, parts)                                 \
+  switch (rdwt_rows(n, H, W, sf, tile)) {              \
+    case 8: return GO(l, 8, kWvThreads, parts);        \
+    case 4: return GO(l, 4, kWvThreads, parts);        \
+    default: return GO(l, 2, kWvThreads, parts);       \
+  }
+#define CASE(l) \
+  case l: ROWS(l, false)
+  if (tile.in < W) ROWS(0, true)
+  if (W > kWvLong) return GO(0, 2, 4 * kWvThreads, false);
   switch (t.lh) {
     NSST_RDWT_LENS(CASE)
     default:
-      switch (rdwt_rows(n, H, W, sf)) {
-        case 8: return GO(0, 8);
-        case 4: return GO(0, 4);
-        default: return GO(0, 2);
-      }
+      ROWS(0, false)
   }
 #undef CASE
+#undef ROWS
 #undef GO
 }
 
