@@ -151,6 +151,7 @@ struct nsst_plan {
   int* dev_err = nullptr;       // error word of the bounded device waits
   // autotuner record (nsst_plan_autotune): per batch-size bucket the fastest
   // directional-stage candidate, and the candidate under test while tuning
+  uint64_t dir_version = 0;  // counts the changes of the directional choice: graphs of other objects hold its kernels
   bool tuned[kTuneBuckets] = {};
   DirChoice tuned_choice[kTuneBuckets];
   bool forcing = false;
@@ -918,6 +919,7 @@ nsst_status nsst_plan_set_directional(nsst_plan* p, int mode) {
                 "no fused directional configuration for this image size on this device (sizes 256x256, 384x512, "
                 "512x512)");
   if (mode != p->dir_mode) {  // captured graphs hold the other kernels
+    p->dir_version++;
     for (auto& g : p->graphs)
       if (g.exec) {
         cudaGraphExecDestroy(g.exec);
@@ -1877,6 +1879,7 @@ nsst_status nsst_plan_select_directional(nsst_plan* p, int n, int index) {
     p->tuned[b] = true;
     p->tuned_choice[b] = cands[index].first;
   }
+  p->dir_version++;
   for (auto& g : p->graphs)
     if (g.exec) {
       cudaGraphExecDestroy(g.exec);
@@ -2004,6 +2007,7 @@ nsst_status nsst_plan_autotune(nsst_plan* p, int n, nsst_tune_result* res) {
   const int b = tune_bucket(n);
   p->tuned[b] = true;
   p->tuned_choice[b] = cands[best].first;
+  p->dir_version++;
   for (auto& g : p->graphs)  // captured graphs hold the previous choice
     if (g.exec) {
       cudaGraphExecDestroy(g.exec);
@@ -2783,7 +2787,10 @@ nsst_status nsst_multi_denoise(nsst_multi* m, const nsst_item* items, int n, con
     key.push_back(items[i].out);
     key.push_back((const void*)(intptr_t)items[i].plan);
   }
-  for (int g = 0; g < np; g++) key.push_back((const void*)(intptr_t)lowth[g]);
+  for (int g = 0; g < np; g++) {
+    key.push_back((const void*)(intptr_t)lowth[g]);
+    if (!groups[g].empty()) key.push_back((const void*)(uintptr_t)m->plans[g]->dir_version);
+  }
   cudaStream_t st = (cudaStream_t)stream;
   // thresholds into every plan's pinned staging, once its last copy has read it
   for (int g = 0; g < np; g++) {
@@ -2820,8 +2827,8 @@ nsst_status nsst_multi_denoise(nsst_multi* m, const nsst_item* items, int n, con
     }
     return NSST_OK;
   };
-  // A call with the pointers of the one before it is captured, and replayed
-  // while they stay; any other runs its launches directly: capturing and
+  // A call with the pointers (and the plans' kernels) of the one before it is
+  // captured, and replayed while they stay; any other runs its launches directly: capturing and
   // instantiating a graph costs more than they do, and the GPU would wait.
   const bool again = key == m->last && mode == m->last_mode;
   m->last = key;
