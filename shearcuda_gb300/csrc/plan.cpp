@@ -8,6 +8,7 @@
 // reference it also owns static job lists for each kernel stage, so one call
 // is a fixed sequence of launches on the caller's stream.
 #include <algorithm>
+#include <functional>
 #include <initializer_list>
 #include <numeric>
 #include <atomic>
@@ -2760,11 +2761,21 @@ nsst_status nsst_multi_denoise(nsst_multi* m, const nsst_item* items, int n, con
       return fail(NSST_ERR_INVALID_ARG, "bad item");
     groups[items[i].plan].push_back(i);
   }
-  for (int g = 0; g < np; g++) {
+  for (int g = 0; g < np; g++)
     if ((int)groups[g].size() > m->plans[g]->B) return fail(NSST_ERR_INVALID_ARG, "group exceeds plan capacity");
-    if (!groups[g].empty() && !m->plans[g]->has_scalars)
-      return fail(NSST_ERR_INVALID_ARG, "plan without stored scalars");
-  }
+  // The plans stay locked, in an order that every call takes, until the batch has
+  // joined the caller's stream: another thread's call on one of them would write its
+  // staging, or, on the same stream, run between the fork and the join beside
+  // the group that uses its arena.
+  std::vector<nsst_plan*> used;
+  for (int g = 0; g < np; g++)
+    if (!groups[g].empty()) used.push_back(m->plans[g]);
+  std::sort(used.begin(), used.end(), std::less<nsst_plan*>());
+  used.erase(std::unique(used.begin(), used.end()), used.end());
+  std::vector<std::unique_lock<std::mutex>> plk;
+  for (nsst_plan* p : used) plk.emplace_back(p->mu);
+  for (nsst_plan* p : used)
+    if (!p->has_scalars) return fail(NSST_ERR_INVALID_ARG, "plan without stored scalars");
   // every group's thresholds, checked before anything is queued
   std::vector<std::vector<float>> th(np);
   std::vector<char> lowth(np, 0);
@@ -2807,7 +2818,6 @@ nsst_status nsst_multi_denoise(nsst_multi* m, const nsst_item* items, int n, con
     for (int g = 0; g < np; g++) {
       if (groups[g].empty()) continue;
       nsst_plan* p = m->plans[g];
-      std::lock_guard<std::mutex> plk(p->mu);
       NSST_CUDA(cudaStreamWaitEvent(m->streams[g], m->fork, 0));
       const int cnt = (int)groups[g].size();
       NSST_CUDA(cudaMemcpyAsync(p->th, p->th_host, sizeof(float) * p->nbands * cnt, cudaMemcpyHostToDevice,
