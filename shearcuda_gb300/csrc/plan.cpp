@@ -1060,7 +1060,7 @@ nsst_status upload_thresholds(nsst_plan* p, int n, const double* sigma, const do
 // (ana 0), or always (ana 1); otherwise (a single image, ana 2) one CTA per
 // (band, item) column group, which has ndir times more CTAs.  pairs: the
 // level form on split-complex column pairs; tma: the level form with its
-// column groups staged by TMA (forward arena only).
+// column groups staged by TMA (in either arena).
 bool analysis_per_level(const nsst_plan* p, int n, int ana) {
   const size_t ctas = (size_t)n * p->nlev * (p->WH / col_tile(p->H));
   return ana == 1 || (ana == 0 && ctas >= (size_t)2 * p->sm_count);
