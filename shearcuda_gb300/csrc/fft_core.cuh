@@ -1,15 +1,12 @@
 // Block-cooperative FP32 FFTs in shared memory, for the NSST directional stage.
 //
-// Layout convention used by every kernel: a CTA owns `NSEQ` sequences of
-// length N; element (sequence s, index i) lives at buf[i * LD + s] with
-// LD = NSEQ + 1 (one float2 of padding per index keeps the row-to-column
-// staging and the butterflies free of shared-memory bank conflicts).
+// A CTA owns NSEQ sequences of length N; element (index i, sequence s) lives at
+// buf[i * NSEQ + s] between the passes.
 //
 // The transform is a Stockham auto-sort FFT: every pass reads its R inputs
 // at stride N/R, twiddles them, runs an R-point DFT in registers and writes
 // the outputs to their sorted positions, so the result is in natural order
-// with no bit-reversal pass.  Radices 2, 3, 4 and 8 cover every length of
-// the form 2^a * 3^b (b <= 1) that the pyramid sizes need.
+// with no bit-reversal pass.  The radices per length are in FftPlan.
 //
 // Twiddles come from a table tw[t] = exp(-2 pi i t / N) computed in FP64 on
 // the host and rounded once to FP32 (no on-device trigonometry).
@@ -18,10 +15,6 @@
 #include <stdint.h>
 
 namespace nsst {
-
-struct cpx {
-  float x, y;
-};
 
 // Complex add / subtract as one packed FP32 instruction each (FADD2 / FFMA2
 // with -1, both rounded exactly like the two scalar operations).
@@ -471,69 +464,6 @@ template <> struct FftPlan<768> { using type = RadixList<16, 3, 16>; };
 template <> struct FftPlan<1024> { using type = RadixList<16, 4, 16>; };
 template <> struct FftPlan<2048> { using type = RadixList<16, 8, 16>; };
 
-// One Stockham pass of radix R over NSEQ sequences of length N, in place.
-// NS = product of the radices already applied.  All threads participate.
-template <int N, int NSEQ, int T, int R, int NS, int DIR>
-__device__ __forceinline__ void stockham_pass(float2* buf, const float2* __restrict__ tw) {
-  constexpr int LD = NSEQ + 1;
-  constexpr int NB = N / R;            // butterflies per sequence
-  constexpr int TOTAL = NB * NSEQ;     // butterflies in the CTA
-  constexpr int IPT = (TOTAL + T - 1) / T;
-  constexpr int STEP = N / (NS * R);   // twiddle index stride
-  float2 v[IPT][R];
-  const int tid = threadIdx.x;
-#pragma unroll
-  for (int it = 0; it < IPT; it++) {
-    int w = tid + it * T;
-    if (TOTAL % T == 0 || w < TOTAL) {
-      int s = w % NSEQ;
-      int j = w / NSEQ;
-#pragma unroll
-      for (int r = 0; r < R; r++) v[it][r] = buf[(j + r * NB) * LD + s];
-      if (NS > 1) {
-        int k = j % NS;
-#pragma unroll
-        for (int r = 1; r < R; r++) {
-          float2 t = __ldg(&tw[r * k * STEP]);
-          v[it][r] = DIR < 0 ? cmul(v[it][r], t) : cmulc(v[it][r], t);
-        }
-      }
-      Dft<R, DIR>::run(v[it]);
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int it = 0; it < IPT; it++) {
-    int w = tid + it * T;
-    if (TOTAL % T == 0 || w < TOTAL) {
-      int s = w % NSEQ;
-      int j = w / NSEQ;
-      int k = j % NS;
-      int base = (j / NS) * NS * R + k;
-#pragma unroll
-      for (int r = 0; r < R; r++) buf[(base + r * NS) * LD + s] = v[it][r];
-    }
-  }
-  __syncthreads();
-}
-
-template <int N, int NSEQ, int T, int DIR, int NS>
-__device__ __forceinline__ void fft_passes(float2*, const float2* __restrict__, RadixList<>) {}
-
-template <int N, int NSEQ, int T, int DIR, int NS, int R, int... Rest>
-__device__ __forceinline__ void fft_passes(float2* buf, const float2* __restrict__ tw, RadixList<R, Rest...>) {
-  stockham_pass<N, NSEQ, T, R, NS, DIR>(buf, tw);
-  fft_passes<N, NSEQ, T, DIR, NS * R>(buf, tw, RadixList<Rest...>{});
-}
-
-// In-place FFT of NSEQ sequences of length N held in shared memory
-// (layout buf[i * (NSEQ+1) + s]).  Unnormalised in both directions.
-// Caller must __syncthreads() before (data staged) — this routine ends synced.
-template <int N, int NSEQ, int T, int DIR>
-__device__ __forceinline__ void block_fft(float2* buf, const float2* __restrict__ tw) {
-  fft_passes<N, NSEQ, T, DIR, 1>(buf, tw, typename FftPlan<N>::type{});
-}
-
 // ---------------------------------------------------------------------------
 // Real <-> packed-complex row transforms.
 //
@@ -548,99 +478,13 @@ __device__ __forceinline__ void block_fft(float2* buf, const float2* __restrict_
 // so that inverse(forward(x)) = W x.
 // twW[k] = exp(-2 pi i k / W), k < W/2.
 // ---------------------------------------------------------------------------
-template <int WH, int NSEQ, int T>
-__device__ __forceinline__ void r2c_post(float2* buf, const float2* __restrict__ twW) {
-  constexpr int LD = NSEQ + 1;
-  constexpr int PAIRS = WH / 2 + 1;  // k = 0 .. WH/2
-  constexpr int TOTAL = PAIRS * NSEQ;
-  constexpr int IPT = (TOTAL + T - 1) / T;
-  float2 a[IPT], b[IPT];
-  const int tid = threadIdx.x;
-#pragma unroll
-  for (int it = 0; it < IPT; it++) {
-    int w = tid + it * T;
-    if (w < TOTAL) {
-      int s = w % NSEQ, k = w / NSEQ;
-      float2 zk = buf[k * LD + s];
-      if (k == 0) {
-        a[it] = make_float2(zk.x + zk.y, zk.x - zk.y);
-      } else {
-        float2 zm = buf[(WH - k) * LD + s];
-        float2 zmc = cconj(zm);
-        float2 E = cscale(cadd(zk, zmc), 0.5f);
-        float2 d = cscale(csub(zk, zmc), 0.5f);
-        float2 O = make_float2(d.y, -d.x);  // d / i
-        float2 To = cmul(__ldg(&twW[k]), O);
-        a[it] = cadd(E, To);
-        b[it] = cconj(csub(E, To));
-      }
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int it = 0; it < IPT; it++) {
-    int w = tid + it * T;
-    if (w < TOTAL) {
-      int s = w % NSEQ, k = w / NSEQ;
-      buf[k * LD + s] = a[it];
-      if (k != 0 && k != WH - k) buf[(WH - k) * LD + s] = b[it];
-    }
-  }
-  __syncthreads();
-}
 
-template <int WH, int NSEQ, int T>
-__device__ __forceinline__ void c2r_pre(float2* buf, const float2* __restrict__ twW) {
-  constexpr int LD = NSEQ + 1;
-  constexpr int PAIRS = WH / 2 + 1;
-  constexpr int TOTAL = PAIRS * NSEQ;
-  constexpr int IPT = (TOTAL + T - 1) / T;
-  float2 a[IPT], b[IPT];
-  const int tid = threadIdx.x;
-#pragma unroll
-  for (int it = 0; it < IPT; it++) {
-    int w = tid + it * T;
-    if (w < TOTAL) {
-      int s = w % NSEQ, k = w / NSEQ;
-      float2 xk = buf[k * LD + s];
-      if (k == 0) {
-        // X[0] = xk.x, X[W/2] = xk.y (both real)
-        a[it] = make_float2(xk.x + xk.y, xk.x - xk.y);
-      } else {
-        float2 xmc = cconj(buf[(WH - k) * LD + s]);
-        float2 E = cadd(xk, xmc);
-        float2 O = cmulc(csub(xk, xmc), __ldg(&twW[k]));  // * w^-k
-        float2 iO = make_float2(-O.y, O.x);
-        a[it] = cadd(E, iO);
-        b[it] = cconj(csub(E, iO));
-      }
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int it = 0; it < IPT; it++) {
-    int w = tid + it * T;
-    if (w < TOTAL) {
-      int s = w % NSEQ, k = w / NSEQ;
-      buf[k * LD + s] = a[it];
-      if (k != 0 && k != WH - k) buf[(WH - k) * LD + s] = b[it];
-    }
-  }
-  __syncthreads();
-}
-
-// ---------------------------------------------------------------------------
-// Ping-pong variant: each pass reads buffer `in` and writes buffer `out`, so a
-// thread only holds one butterfly's R values at a time (low register use) and
-// a pass needs a single barrier.  Returns the buffer that holds the result.
-//
-// Layout: element (index i, sequence s) at [phi(i) * NSEQ + s] with no padding.
-// A warp covers 32/NSEQ consecutive butterflies of NSEQ sequences each, so the
-// rows it touches in one access are consecutive (-> alternating bank groups,
-// conflict-free) in every pass except where the first pass (NS == 1) writes
-// rows R apart; that pass's output is row-swizzled, phi(i) = i ^ ((i / R) & m)
-// with m = 16/NSEQ - 1, and the second pass reads it back through the same phi.
-// ---------------------------------------------------------------------------
+// The row swizzle of the passes.  A warp covers 32/NSEQ consecutive butterflies of
+// NSEQ sequences each, so the rows it touches in one access are consecutive
+// (alternating bank groups, conflict-free) in every pass except where the first
+// pass (NS == 1) writes rows R apart; that pass's output is row-swizzled, phi(i) =
+// i ^ ((i / R) & m) with m = 16/NSEQ - 1, and the second pass reads it back through
+// the same phi.
 template <int NSEQ, int SWZ>
 __device__ __forceinline__ int swz_row(int i) {
   constexpr int M = 16 / NSEQ - 1;
@@ -648,169 +492,18 @@ __device__ __forceinline__ int swz_row(int i) {
   return i ^ ((i / SWZ) & M);
 }
 
-template <int N, int NSEQ, int T, int R, int NS, int DIR, int SWZ_IN, int SWZ_OUT>
-__device__ __forceinline__ void stockham_pp(const float2* __restrict__ in, float2* __restrict__ out,
-                                            const float2* __restrict__ tw) {
-  constexpr int NB = N / R;
-  constexpr int TOTAL = NB * NSEQ;
-  constexpr int STEP = N / (NS * R);
-#pragma unroll 2
-  for (int w = threadIdx.x; w < TOTAL; w += T) {
-    const int s = w % NSEQ;
-    const int j = w / NSEQ;
-    float2 v[R];
-#pragma unroll
-    for (int r = 0; r < R; r++) v[r] = in[swz_row<NSEQ, SWZ_IN>(j + r * NB) * NSEQ + s];
-    const int k = j % NS;
-    if (NS > 1) {
-#pragma unroll
-      for (int r = 1; r < R; r++) {
-        float2 t = __ldg(&tw[r * k * STEP]);
-        v[r] = DIR < 0 ? cmul(v[r], t) : cmulc(v[r], t);
-      }
-    }
-    Dft<R, DIR>::run(v);
-    const int base = (j / NS) * NS * R + k;
-#pragma unroll
-    for (int r = 0; r < R; r++) out[swz_row<NSEQ, SWZ_OUT>(base + r * NS) * NSEQ + s] = v[r];
-  }
-  __syncthreads();
-}
-
-template <int N, int NSEQ, int T, int DIR, int NS, int SWZ_IN>
-__device__ __forceinline__ float2* fft_pp_passes(float2* a, float2* b, const float2* __restrict__ tw, RadixList<>) {
-  return a;
-}
-
-template <int N, int NSEQ, int T, int DIR, int NS, int SWZ_IN, int R, int... Rest>
-__device__ __forceinline__ float2* fft_pp_passes(float2* a, float2* b, const float2* __restrict__ tw,
-                                                 RadixList<R, Rest...>) {
-  // only the first pass (NS == 1, even radix) writes rows R apart
-  constexpr int SWZ_OUT = (NS == 1 && R % 2 == 0 && sizeof...(Rest) > 0) ? R : 0;
-  stockham_pp<N, NSEQ, T, R, NS, DIR, SWZ_IN, SWZ_OUT>(a, b, tw);
-  return fft_pp_passes<N, NSEQ, T, DIR, NS * R, SWZ_OUT>(b, a, tw, RadixList<Rest...>{});
-}
-
-// FFT of the data in `a` (layout [i * NSEQ + s]) using `b` as the second
-// buffer; returns a or b, holding the result in the same unswizzled layout.
-template <int N, int NSEQ, int T, int DIR>
-__device__ __forceinline__ float2* block_fft_pp(float2* a, float2* b, const float2* __restrict__ tw) {
-  return fft_pp_passes<N, NSEQ, T, DIR, 1, 0>(a, b, tw, typename FftPlan<N>::type{});
-}
-// Same with an explicit radix plan (a RadixList whose product is N).
-template <int N, int NSEQ, int T, int DIR, class Plan>
-__device__ __forceinline__ float2* block_fft_pp_plan(float2* a, float2* b, const float2* __restrict__ tw) {
-  return fft_pp_passes<N, NSEQ, T, DIR, 1, 0>(a, b, tw, Plan{});
-}
-
 // ---------------------------------------------------------------------------
-// Ping-pong FFT with hooks: the first pass reads its inputs through `ld`
-// (natural index, sequence) and the last pass writes its outputs through
-// `st` (natural index, sequence, value) instead of the shared buffers, so a
-// prologue (a spectrum product, the packed-real pre-processing, a load from
-// global memory) or an epilogue (a threshold, a store to global memory) costs
-// no extra shared-memory round trip or barrier.  Intermediate passes use a
-// and b alternately (pass 1 writes b).  The first pass ends with a barrier
-// like every pass, so `ld` may read the buffer the second pass writes.
+// FFTs with hooks: the first pass reads its inputs through `ld` (natural index,
+// sequence) and the last pass writes its outputs through `st` (natural index,
+// sequence, value) instead of the shared buffer, so a prologue (a spectrum
+// product, the packed-real pre-processing, a load from global memory) or an
+// epilogue (a threshold, a store to global memory) costs no extra shared-memory
+// round trip or barrier.
 // ---------------------------------------------------------------------------
-template <typename RL>
-struct RadixCount;
-template <int... Rs>
-struct RadixCount<RadixList<Rs...>> {
-  static constexpr int value = sizeof...(Rs);
-};
-template <int N>
-__host__ __device__ constexpr int fft_npasses() {
-  return RadixCount<typename FftPlan<N>::type>::value;
-}
-
-template <int N, int NSEQ, int T, int R, int NS, int DIR, int SWZ_IN, int SWZ_OUT, class Rd, class Wr>
-__device__ __forceinline__ void stockham_hook(const Rd& rd, const Wr& wr, const float2* __restrict__ tw) {
-  constexpr int NB = N / R;
-  constexpr int TOTAL = NB * NSEQ;
-  constexpr int STEP = N / (NS * R);
-#pragma unroll 2
-  for (int w = threadIdx.x; w < TOTAL; w += T) {
-    const int s = w % NSEQ;
-    const int j = w / NSEQ;
-    float2 v[R];
-#pragma unroll
-    for (int r = 0; r < R; r++) v[r] = rd(swz_row<NSEQ, SWZ_IN>(j + r * NB), s);
-    const int k = j % NS;
-    if (NS > 1) {
-#pragma unroll
-      for (int r = 1; r < R; r++) {
-        float2 t = __ldg(&tw[r * k * STEP]);
-        v[r] = DIR < 0 ? cmul(v[r], t) : cmulc(v[r], t);
-      }
-    }
-    Dft<R, DIR>::run(v);
-    const int base = (j / NS) * NS * R + k;
-#pragma unroll
-    for (int r = 0; r < R; r++) wr(swz_row<NSEQ, SWZ_OUT>(base + r * NS), s, v[r]);
-  }
-  __syncthreads();
-}
-
-template <int N, int NSEQ, int T, int DIR, int NS, int SWZ_IN, class Ld, class St>
-__device__ __forceinline__ void fft_hook_passes(float2*, float2*, const float2* __restrict__, const Ld&, const St&,
-                                                RadixList<>) {}
-
-template <int N, int NSEQ, int T, int DIR, int NS, int SWZ_IN, class Ld, class St, int R, int... Rest>
-__device__ __forceinline__ void fft_hook_passes(float2* a, float2* b, const float2* __restrict__ tw, const Ld& ld,
-                                                const St& st, RadixList<R, Rest...>) {
-  constexpr bool first = NS == 1;
-  constexpr bool last = sizeof...(Rest) == 0;
-  constexpr int SWZ_OUT = (first && !last && R % 2 == 0) ? R : 0;
-  auto rd = [&](int row, int s) -> float2 {
-    if constexpr (first)
-      return ld(row, s);
-    else
-      return a[row * NSEQ + s];
-  };
-  auto wr = [&](int row, int s, float2 v) {
-    if constexpr (last)
-      st(row, s, v);
-    else
-      b[row * NSEQ + s] = v;
-  };
-  stockham_hook<N, NSEQ, T, R, NS, DIR, SWZ_IN, SWZ_OUT>(rd, wr, tw);
-  fft_hook_passes<N, NSEQ, T, DIR, NS * R, SWZ_OUT>(b, a, tw, ld, st, RadixList<Rest...>{});
-}
-
-// The buffer the last pass's default target would be (a for an even pass
-// count, b for an odd one); an `st` writing shared memory writes there.
-template <int N>
-__device__ __forceinline__ float2* fft_hook_target(float2* a, float2* b) {
-  return (fft_npasses<N>() & 1) ? b : a;
-}
-
-template <int N, int NSEQ, int T, int DIR, class Ld, class St>
-__device__ __forceinline__ void block_fft_hook(float2* a, float2* b, const float2* __restrict__ tw, const Ld& ld,
-                                               const St& st) {
-  fft_hook_passes<N, NSEQ, T, DIR, 1, 0>(a, b, tw, ld, st, typename FftPlan<N>::type{});
-}
-
-// block_fft_hook with an explicit radix plan; the last pass's default target
-// is plan_target<Plan>(a, b)
-template <int N, int NSEQ, int T, int DIR, class Plan, class Ld, class St>
-__device__ __forceinline__ void block_fft_hook_plan(float2* a, float2* b, const float2* __restrict__ tw,
-                                                    const Ld& ld, const St& st) {
-  fft_hook_passes<N, NSEQ, T, DIR, 1, 0>(a, b, tw, ld, st, Plan{});
-}
-template <int... Rs>
-__host__ __device__ constexpr int plan_passes(RadixList<Rs...>) {
-  return (int)sizeof...(Rs);
-}
-template <class Plan>
-__device__ __forceinline__ float2* plan_target(float2* a, float2* b) {
-  return (plan_passes(Plan{}) & 1) ? b : a;
-}
-
-// In-place variant of block_fft_hook on one buffer: every pass loads all of
-// the thread's butterflies into registers, synchronises, then writes them
-// back (two barriers per pass, half the shared memory of the ping-pong form,
-// so more CTAs fit on an SM).  `st` of the last pass may write `buf`.
+// On one buffer, in place: every pass loads all of the thread's butterflies into
+// registers, synchronises, then writes them back (two barriers per pass, half the
+// shared memory of two buffers, so more CTAs fit on an SM).  `st` of the last pass
+// may write `buf`.
 struct NoHook {
   __device__ __forceinline__ void operator()() const {}
 };
@@ -1134,63 +827,7 @@ __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src)
   const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gmem_src) : "memory");
 }
-// 8-byte asynchronous global -> shared copy (one float2)
-__device__ __forceinline__ void cp_async8(void* smem_dst, const void* gmem_src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(gmem_src) : "memory");
-}
-// 4-byte asynchronous global -> shared copy (one float)
-__device__ __forceinline__ void cp_async4(void* smem_dst, const void* gmem_src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(gmem_src) : "memory");
-}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
-
-// Out-of-place packed-real post-processing (after a forward FFT of the
-// W/2-point complex view); see r2c_post for the formulas.
-template <int WH, int NSEQ, int LD, int T>
-__device__ __forceinline__ void r2c_post_pp(const float2* __restrict__ in, float2* __restrict__ out,
-                                            const float2* __restrict__ twW) {
-  constexpr int TOTAL = (WH / 2 + 1) * NSEQ;
-  for (int w = threadIdx.x; w < TOTAL; w += T) {
-    const int s = w % NSEQ, k = w / NSEQ;
-    const float2 zk = in[k * LD + s];
-    if (k == 0) {
-      out[s] = make_float2(zk.x + zk.y, zk.x - zk.y);
-    } else {
-      const float2 zmc = cconj(in[(WH - k) * LD + s]);
-      const float2 E = cscale(cadd(zk, zmc), 0.5f);
-      const float2 d = cscale(csub(zk, zmc), 0.5f);
-      const float2 O = make_float2(d.y, -d.x);
-      const float2 To = cmul(__ldg(&twW[k]), O);
-      out[k * LD + s] = cadd(E, To);
-      if (k != WH - k) out[(WH - k) * LD + s] = cconj(csub(E, To));
-    }
-  }
-  __syncthreads();
-}
-
-// Out-of-place packed-real pre-processing (before an inverse FFT); see c2r_pre.
-template <int WH, int NSEQ, int LD, int T>
-__device__ __forceinline__ void c2r_pre_pp(const float2* __restrict__ in, float2* __restrict__ out,
-                                           const float2* __restrict__ twW) {
-  constexpr int TOTAL = (WH / 2 + 1) * NSEQ;
-  for (int w = threadIdx.x; w < TOTAL; w += T) {
-    const int s = w % NSEQ, k = w / NSEQ;
-    const float2 xk = in[k * LD + s];
-    if (k == 0) {
-      out[s] = make_float2(xk.x + xk.y, xk.x - xk.y);
-    } else {
-      const float2 xmc = cconj(in[(WH - k) * LD + s]);
-      const float2 E = cadd(xk, xmc);
-      const float2 O = cmulc(csub(xk, xmc), __ldg(&twW[k]));
-      const float2 iO = make_float2(-O.y, O.x);
-      out[k * LD + s] = cadd(E, iO);
-      if (k != WH - k) out[(WH - k) * LD + s] = cconj(csub(E, iO));
-    }
-  }
-  __syncthreads();
-}
 
 }  // namespace nsst

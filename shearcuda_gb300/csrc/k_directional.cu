@@ -28,7 +28,7 @@
 
 namespace nsst {
 
-// packed-real pre-processing of index k (see c2r_pre) is C2RPreLdRM (tiles.cuh):
+// packed-real pre-processing of index k is C2RPreLdRM (tiles.cuh):
 // Z[k] = E + iO with E = X[k] + conj(X[WH-k]), O = (X[k] - conj(X[WH-k])) w^-k;
 // k = 0 unpacks the two real bins.
 // ---------------------------------------------------------------------------
@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(RowTileP<WH, RS>::T, RowTileP<WH, RS>::MINB)
   fetch_rows_rm<WH, RS, T>(A, src_base + job.src + off);
   cp_async_wait_all();
   __syncthreads();
-  // C2R, pre-processing (see c2r_pre) in the first pass's loads:
+  // C2R, pre-processing in the first pass's loads:
   // Z[k] = E + iO, E = X[k] + conj(X[WH-k]), O = (X[k] - conj(X[WH-k])) w^-k
   auto ld = [&](int k, int p) -> cpx2 {
     const float2* r0 = A + 2 * p * RP;
@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(RowTileP<WH, RS>::T, RowTileP<WH, RS>::MINB)
     A[(2 * p + 1) * RP + i] = lane1(v);
   };
   block_fft_hook_ip_plan<WH, NP, T, -1, Plan>(D, twWh4, ldd, st_rm);
-  // post-processing (see r2c_post) fused with the store along the rows:
+  // post-processing fused with the store along the rows:
   // X[k] = E + w^k O, E = (Z[k] + conj(Z[WH-k]))/2, O = (Z[k] - conj(Z[WH-k]))/(2i)
   float2* dst = dst_base + job.dst + off;
 #pragma unroll 2

@@ -6,10 +6,11 @@
 
 namespace nsst {
 
-// Tile shapes: a row CTA owns RS rows, a column CTA owns CS columns, each as two
-// ping-pong shared buffers [index][sequence] (dense, see block_fft_pp).  They keep a thread's share of a tile at <= 16 complex values and the
-// shared memory low enough for 2-3 resident CTAs per SM: the kernels are bound
-// by global-memory latency, so resident CTAs are what hides it.
+// Tile shapes: a row CTA owns RS rows, a column CTA owns CS columns, transformed in
+// place in one shared buffer [index][sequence].  They keep a thread's share of a
+// tile at <= 16 complex values and the shared memory low enough for several
+// resident CTAs per SM: the kernels are bound by global-memory latency, so
+// resident CTAs are what hides it.
 template <int N>
 struct RowCfg {  // N = W/2 complex points per row
   static constexpr int RS = N >= 1024 ? 4 : 8;
@@ -140,7 +141,7 @@ struct ThreshStKept {
   }
 };
 
-// FFT hooks (see block_fft_hook).
+// FFT hooks (see block_fft_hook_ip).
 template <int NSEQ>
 struct SmemLd {
   const float2* p;
@@ -209,7 +210,7 @@ __device__ __forceinline__ void store_zero_rows(float2* __restrict__ dst) {
     *reinterpret_cast<float4*>(dst + (size_t)s * WH + 2 * c) = make_float4(0.f, 0.f, 0.f, 0.f);
   }
 }
-// packed-real post-processing of every index k (see r2c_post) fused with the
+// packed-real post-processing of every index k (formulas in fft_core.cuh) fused with the
 // store of the CTA's rows, from the padded row-major layout along the rows:
 // X[k] = E + w^k O, E = (Z[k] + conj(Z[WH-k]))/2, O = (Z[k] - conj(Z[WH-k]))/(2i);
 // k = 0 packs the two real bins.
