@@ -433,5 +433,6 @@ cudaError_t dev_alloc(void** p, size_t bytes);
 
 // launch accounting (every kernel launch site calls this once per launch)
 void count_launch(int n = 1);
+int sm_count();  // streaming multiprocessors of the device current at the first call
 
 }  // namespace nsst

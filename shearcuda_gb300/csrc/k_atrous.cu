@@ -206,7 +206,7 @@ static cudaError_t prepare_atrous_t(int Mmax) {
   return e;
 }
 
-static int sm_count() {
+int sm_count() {
   static const int n = [] {
     int dev = 0, c = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev) !=

@@ -568,7 +568,7 @@ cudaError_t launch_dct_rows_ana(const RowJob* jobs, int njobs, int n_active, int
 // Measured (one denoise, us, serial / cluster): 1024 tiles (16 x 512^2) 1203 /
 // 1182, 1536 (12 x 1024^2) 4010 / 3985, 2048 (64 x 256^2) 1226 / 1274, 4096
 // (64 x 512^2) 4329 / 4355.
-static bool syn_splits(long tiles) { return tiles <= 8 * 152; }
+static bool syn_splits(long tiles) { return tiles <= 8 * sm_count(); }
 
 cudaError_t launch_dct_rows_syn(const RowJob* jobs, int njobs, int n_active, int nlev, size_t lev_stride, int H,
                                 int W, const void* src_base, void* dst_base, const float* xbase, size_t xstride,

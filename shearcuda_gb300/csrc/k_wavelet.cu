@@ -387,7 +387,7 @@ bool rdwt_width_supported(int W) { return W >= 2 && W <= kWvMaxW; }
 
 constexpr size_t kWvTwoCtas = 110 * 1024;  // shared memory of a CTA of which two fit an SM
 constexpr int kWvLong = kWvTwoCtas / (4 * sizeof(float2));  // longest row of which four fit there
-constexpr int kWvFill = 2 * 152;                            // CTAs that fill the GPU
+static int fill() { return 2 * sm_count(); }                // CTAs that fill the GPU
 
 // Columns per CTA.  The whole row, whose columns are filtered once, as a rule.
 // Parts of it where it is longer than kWvLong, so that more than two rows share
@@ -398,11 +398,11 @@ static WvTile rdwt_tile(int n, int H, int W, int sf, int lh) {
   const int halo = (lh - 1) * sf;
   const long groups = (long)n * sf * ((H / sf + 1) / 2);
   WvTile t{W, W};
-  if (W <= kWvLong && groups >= kWvFill) return t;
+  if (W <= kWvLong && groups >= fill()) return t;
   for (int in : {1024, 512, 256}) {
     if (in >= W || halo > in / 4) continue;
     t = {in - halo, in};
-    if (groups * ((W + t.out - 1) / t.out) >= kWvFill) break;
+    if (groups * ((W + t.out - 1) / t.out) >= fill()) break;
   }
   return t;
 }
@@ -411,7 +411,7 @@ static WvTile rdwt_tile(int n, int H, int W, int sf, int lh) {
 static int rdwt_rows(int n, int H, int W, int sf, WvTile t) {
   for (int th : {8, 4})
     if (th * t.in * sizeof(float2) <= kWvTwoCtas &&
-        (long)n * sf * ((H / sf + th - 1) / th) * ((W + t.out - 1) / t.out) >= kWvFill)
+        (long)n * sf * ((H / sf + th - 1) / th) * ((W + t.out - 1) / t.out) >= fill())
       return th;
   return 2;
 }

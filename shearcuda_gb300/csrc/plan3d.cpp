@@ -34,7 +34,6 @@ namespace {
 constexpr int kCube = 24;          // Meyer filter support (GetMeyerBasedFilter.m:18)
 constexpr int kSameOff = 12;       // convnfft 'same' offset: ceil((24 - 1) / 2)
 constexpr int kMaxGrid = 192;      // largest padded grid per dimension
-constexpr int kSmCount = 152;
 constexpr int kCtasPerSm = 8;      // CTAs per SM that keep a pass's loads in flight
 // Band pairs in flight per level: the work buffer holds as many as fit here (at least one).
 constexpr size_t kPairBytes = (size_t)1 << 30;
@@ -381,7 +380,7 @@ int pair_chunk(const nsst3_plan* p, const nsst3_plan::Level& a, int n) {
 // The passes whose CTAs loop over the chunk's pairs (what the pairs share is
 // then read once) split them over the grid until it fills the GPU.
 int pair_shares(int ctas, int pairs) {
-  return std::min(pairs, std::max(1, (kSmCount * kCtasPerSm + ctas - 1) / ctas));
+  return std::min(pairs, std::max(1, (sm_count() * kCtasPerSm + ctas - 1) / ctas));
 }
 // Keep bits of the level's bands from band k on.
 void set_masks(const nsst3_plan* p, V3Cols& P, int l, int k) {

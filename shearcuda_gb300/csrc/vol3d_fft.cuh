@@ -599,7 +599,7 @@ struct V3Launch {
     // A band sum over few lines: its CTAs' chain of pairs is the time, so four
     // groups of threads share it; with more CTAs the groups only wait for one another.
     if constexpr (CONV && N <= 108)
-      if (st_mode == V3_ST_THRESH && P.pairs >= 4 && grid.x <= 2 * 152) {
+      if (st_mode == V3_ST_THRESH && P.pairs >= 4 && grid.x <= (unsigned)(2 * sm_count())) {
         launch_pdl(k_v3_cols<N, 1, V3_LD_CPLX, V3_ST_THRESH, 4>, grid, 4 * T, 0, st, P, tw);
         return cudaGetLastError();
       }
