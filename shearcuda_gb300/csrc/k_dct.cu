@@ -564,11 +564,13 @@ cudaError_t launch_dct_rows_ana(const RowJob* jobs, int njobs, int n_active, int
   }
 }
 
-// Row tiles up to which the synthesis rows run as clusters: eight per SM.
-// Measured (one denoise, us, serial / cluster): 1024 tiles (16 x 512^2) 1203 /
-// 1182, 1536 (12 x 1024^2) 4010 / 3985, 2048 (64 x 256^2) 1226 / 1274, 4096
-// (64 x 512^2) 4329 / 4355.
-static bool syn_splits(long tiles) { return tiles <= 8 * sm_count(); }
+// Row tiles up to which the synthesis rows run as clusters: ten and a half per SM
+// (1596 of 152).  Measured (one denoise, us, serial / cluster): 1024 tiles (16 x
+// 512^2) 1203 / 1182, 1280 (20 x 512^2) 1399 / 1385, (40 x 256^2) 703 / 680, 1536
+// (12 x 1024^2) 3710 / 3690, (16 x 768 x 1024) 3979 / 3952, 1792 (14 x 1024^2) 4258 /
+// 4269, (28 x 512^2) 1879 / 1890, 2048 (64 x 256^2) 1226 / 1274, 4096 (64 x 512^2)
+// 4329 / 4355.
+static bool syn_splits(long tiles) { return 2 * tiles <= 21 * sm_count(); }
 
 cudaError_t launch_dct_rows_syn(const RowJob* jobs, int njobs, int n_active, int nlev, size_t lev_stride, int H,
                                 int W, const void* src_base, void* dst_base, const float* xbase, size_t xstride,
