@@ -35,7 +35,8 @@ constexpr int kCube = 24;          // Meyer filter support (GetMeyerBasedFilter.
 constexpr int kSameOff = 12;       // convnfft 'same' offset: ceil((24 - 1) / 2)
 constexpr int kMaxGrid = 192;      // largest padded grid per dimension
 constexpr int kCtasPerSm = 8;      // CTAs per SM that keep a pass's loads in flight
-// Band pairs in flight per level: the work buffer holds as many as fit here (at least one).
+// Band pairs in flight per level: the work buffer holds as many as fit here (at least one; one,
+// if the device has no room for more).
 constexpr size_t kPairBytes = (size_t)1 << 30;
 // The 2^a 3^b lengths: the grids of NSST3_GRID_FAST, and the convolution lengths that nsst3_level_dims reports.
 const int kFftLens[] = {16, 24, 32, 48, 64, 72, 96, 128, 144, 192, 216, 256};
@@ -586,13 +587,14 @@ nsst_status nsst3_plan_create(const nsst3_config* cfg, int n0, int n1, int n2, i
     spec_off += (size_t)((a.nb + 1) / 2) * a.conv();  // one spectrum F_a + i F_b per band pair
     p->conv_elems = std::max(p->conv_elems, a.conv());
   }
+  size_t wk_least = 0;
   for (int l = 0; l < p->L; l++) {
     const nsst3_plan::Level& a = p->lev[l];
     const size_t one = a.pair() * batch;
     const size_t fit = std::max<size_t>(1, kPairBytes / (one * sizeof(float2)));
-    p->wk_elems = std::max(p->wk_elems, one * std::min<size_t>(a.npairs(), fit));
     // the backward's half spectra of S and its fold scratch live there too
-    p->wk_elems = std::max(p->wk_elems, (size_t)a.m[0] * a.lc[1] * v3_pitch(a.lc[2] / 2 + 1) * batch);
+    wk_least = std::max({wk_least, one, (size_t)a.m[0] * a.lc[1] * v3_pitch(a.lc[2] / 2 + 1) * batch});
+    p->wk_elems = std::max({p->wk_elems, wk_least, one * std::min<size_t>(a.npairs(), fit)});
   }
   p->bp_floats = bp_off;
   p->xh_elems = xh_off;
@@ -649,12 +651,20 @@ nsst_status nsst3_plan_create(const nsst3_config* cfg, int n0, int n1, int n2, i
   const size_t o_tw = take(tw_host.size() * sizeof(float2));
   const size_t o_xh = take(B * p->xh_elems * sizeof(float2));
   const size_t o_y = take(B * p->conv_elems * sizeof(float2));
-  const size_t o_w = take(p->wk_elems * sizeof(float2));
   const size_t o_bp = take(B * p->bp_floats * sizeof(float));
   const size_t o_rbp = take(B * p->bp_floats * sizeof(float));
   const size_t o_th = take(B * p->nbands * sizeof(float));
+  const size_t o_w = off;  // last: its size depends on the room there is
   void* arena = nullptr;
+  take(p->wk_elems * sizeof(float2));
   cudaError_t e = dev_alloc(&arena, off);
+  if (e == cudaErrorMemoryAllocation && wk_least < p->wk_elems) {
+    (void)cudaGetLastError();
+    p->wk_elems = wk_least;
+    off = o_w;
+    take(p->wk_elems * sizeof(float2));
+    e = dev_alloc(&arena, off);
+  }
   if (e != cudaSuccess) return cuda_fail3(e, "plan arena");
   p->arena = (char*)arena;
   p->arena_bytes = off;
