@@ -59,14 +59,15 @@ typedef struct nsst_config {
                                    allow it.  nsst_shear_trans,
                                    nsst_inverse_shear, nsst_atrousdec,
                                    nsst_atrousrec, the differentiable denoise
-                                   (forward and backward), the separation and
-                                   the operator adjoints follow the same
-                                   mode; calls that pass images not 16-byte
-                                   aligned use the direct pyramid, and
-                                   nsst_re_weight_band always does: its result
-                                   may be much smaller than the image, and a
-                                   pixel that is not finite then stays within
-                                   the filters' support. */
+                                   (forward and backward) and the separation
+                                   follow the same mode; calls that pass images
+                                   not 16-byte aligned (an error under
+                                   _SPECTRAL), nsst_re_weight_band and the
+                                   operator adjoints use the direct pyramid:
+                                   the results of the last two may be smaller
+                                   than the rounding of a transform of the
+                                   image, and a value that is not finite stays
+                                   within the filters' support. */
 } nsst_config;
 
 typedef struct nsst_plan nsst_plan;
@@ -319,16 +320,18 @@ nsst_status nsst_multi_denoise(nsst_multi* m, const nsst_item* items, int n, con
 nsst_status nsst_multi_destroy(nsst_multi* m);
 
 /* ---- Differentiation (no counterpart in the reference).  The adjoint of
- * every stage is hand-written: transposed pyramid steps (zero-extended
- * correlation with the unflipped filter, then the mirrored margins folded
- * back), conjugate-spectrum directional synthesis/analysis, and the threshold
+ * every stage is hand-written: transposed pyramid steps (with filters symmetric
+ * in both axes the steps themselves; else zero-extended correlation with the
+ * unflipped filter, then the mirrored margins folded back), conjugate-spectrum
+ * directional synthesis/analysis, and the threshold
  * subgradient 1[|c| > t] (soft rule: d/dt = -sign(c) 1[|c| > t]). */
 
 /* Allocate the gradient workspace of a plan (once; about twice the plan's
  * own work buffers).  Required by the calls below. */
 nsst_status nsst_plan_enable_grad(nsst_plan* plan);
 
-/* x = A^T c, the adjoint of nsst_shear_trans (coeffs: nbands x H x W). */
+/* x = A^T c, the adjoint of nsst_shear_trans (coeffs: nbands x H x W, 16-byte
+ * aligned). */
 nsst_status nsst_shear_trans_adjoint(nsst_plan* plan, const float* coeffs, float* x, void* stream);
 
 /* c = R^T x, the adjoint of nsst_inverse_shear. */

@@ -133,7 +133,7 @@ int col_tile(int h);
 
 cudaError_t prepare_row_kernels(int wh);
 cudaError_t prepare_col_kernels(int h);
-cudaError_t prepare_atrous_kernels(int FA, int FB, int Mmax);
+cudaError_t prepare_atrous_kernels(int FA, int FB, int Mmax, bool apart = false);
 cudaError_t launch_rows(RowOp op, const RowJob* jobs, int njobs, int n_active, int H, int W, const void* src_base,
                         void* dst_base, const float2* twWh, const float2* twW, const float* thr, int mode,
                         cudaStream_t st);
@@ -190,8 +190,9 @@ cudaError_t launch_dir_fused(const void* ymap, const FusedJob* jobs, int njobs, 
                              int W, float2* dst_base, const float2* spec_base, size_t band_stride, const float2* twH,
                              const float2* twWh, const float2* twW, const float* thr, int mode, int* err,
                              cudaStream_t st);
+// apart: the two convolutions of an output summed each for itself (the analysis filters' pairs)
 cudaError_t launch_atrous(const AtrousJobs& jobs, int njobs, int maxH, int maxW, int M, int FA, const float* ha,
-                          int FB, const float* hb, cudaStream_t st);
+                          int FB, const float* hb, cudaStream_t st, bool apart = false);
 // The DCT-domain pyramid of the fused pipeline (k_dct.cu).
 cudaError_t prepare_dct_kernels(int H, int WH);
 cudaError_t launch_dct_rows_fwd(const DctIo& io, int n, int H, int W, const float2* twWh, const float4* twD,

@@ -117,7 +117,9 @@ __device__ __forceinline__ void atrous_accumulate(const float* __restrict__ x, i
 }
 
 // out = conv(xa, filter A) [+ conv(xb, filter B)].  grid = (W/64, M * ceil(ceil(H/M)/(8 P)), njobs)
-template <int FA, int FB, bool ZERO = false, int P = kAtP, bool ZR = false>
+// APART: the two convolutions are summed each for itself and then added.  One chain
+// over both rounds more (the adjoint of the '9-7' analysis: 3.4e-7, apart 2.6e-7).
+template <int FA, int FB, bool ZERO = false, int P = kAtP, bool ZR = false, bool APART = false>
 __global__ void __launch_bounds__(kAtThreads, (FA <= 13 && FB == 0) ? 4 : 3) k_atrous(const __grid_constant__ AtrousJobs jobs, int M,
                                                         const __grid_constant__ AtrousTaps<FA> ta,
                                                         const __grid_constant__ AtrousTaps<FB> tb) {
@@ -145,8 +147,17 @@ __global__ void __launch_bounds__(kAtThreads, (FA <= 13 && FB == 0) ? 4 : 3) k_a
     for (int e = threadIdx.x; e < FB * FB; e += kAtThreads) s_taps[e] = tb.w[e];
     for (int e = threadIdx.x; e < tb.ncols; e += kAtThreads) s_cols[e] = tb.cols[e];
     __syncthreads();
+    float2 first[APART ? P : 1];
+    if constexpr (APART) {
+#pragma unroll
+      for (int p = 0; p < P; p++) first[p] = acc[p], acc[p] = make_float2(0.f, 0.f);
+    }
     atrous_accumulate<(FB > 0 ? FB : 1), ZERO, P, ZR>(job.xb, H, W, M, phase, prow0, col0, s_taps, s_cols,
                                                        tb.ncols, at_smem, acc);
+    if constexpr (APART) {
+#pragma unroll
+      for (int p = 0; p < P; p++) acc[p] = __fadd2_rn(first[p], acc[p]);
+    }
   }
   const int tx = threadIdx.x % kAtHX, ty = threadIdx.x / kAtHX;
   const int c = col0 + tx;
@@ -175,7 +186,7 @@ static size_t atrous_smem_pair(int M) {
 
 // The shared-memory opt-in only ever grows: plans (and the no-allocation
 // entry point) with different pyramid depths share these kernels.
-template <int FA, int FB>
+template <int FA, int FB, bool APART = false>
 static cudaError_t prepare_atrous_t(int Mmax) {
   constexpr int kDevs = 64;
   static std::mutex mu;
@@ -187,16 +198,17 @@ static cudaError_t prepare_atrous_t(int Mmax) {
   if (want > 227 * 1024) return cudaErrorInvalidValue;
   std::lock_guard<std::mutex> lk(mu);
   if (dev >= 0 && dev < kDevs && configured[dev] >= want) return cudaSuccess;
-  e = cudaFuncSetAttribute(k_atrous<FA, FB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want);
+  e = cudaFuncSetAttribute(k_atrous<FA, FB, false, kAtP, false, APART>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)want);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_atrous<FA, FB, false, kAtPSmall>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    e = cudaFuncSetAttribute(k_atrous<FA, FB, false, kAtPSmall, false, APART>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_atrous<FA, FB, false, kAtP, true, APART>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)want);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_atrous<FA, FB, false, kAtP, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)want);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_atrous<FA, FB, false, kAtPSmall, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)want);
+    e = cudaFuncSetAttribute(k_atrous<FA, FB, false, kAtPSmall, true, APART>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want);
   if (e == cudaSuccess && FB == 0)
     e = cudaFuncSetAttribute(k_atrous<FA, FB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want);
   if (e == cudaSuccess && FB == 0)
@@ -229,7 +241,7 @@ static bool zero_rows_1(const float* h, int F) {
   return true;
 }
 
-template <int FA, int FB>
+template <int FA, int FB, bool APART = false>
 static cudaError_t launch_atrous_t(const AtrousJobs& jobs, int njobs, int maxH, int maxW, int M, const float* ha,
                                    const float* hb, cudaStream_t st) {
   AtrousTaps<FA> ta;
@@ -244,14 +256,14 @@ static cudaError_t launch_atrous_t(const AtrousJobs& jobs, int njobs, int maxH, 
   if ((size_t)grid.x * grid.y * grid.z < (size_t)2 * sm_count()) {  // half-height tiles: twice the CTAs
     grid.y = M * ((nprow_max + kAtPSmall * kAtTY - 1) / (kAtPSmall * kAtTY));
     if (zr)
-      launch_pdl(k_atrous<FA, FB, false, kAtPSmall, true>, grid, kAtThreads, sm, st, jobs, M, ta, tb);
+      launch_pdl(k_atrous<FA, FB, false, kAtPSmall, true, APART>, grid, kAtThreads, sm, st, jobs, M, ta, tb);
     else
-      launch_pdl(k_atrous<FA, FB, false, kAtPSmall>, grid, kAtThreads, sm, st, jobs, M, ta, tb);
+      launch_pdl(k_atrous<FA, FB, false, kAtPSmall, false, APART>, grid, kAtThreads, sm, st, jobs, M, ta, tb);
   } else {
     if (zr)
-      launch_pdl(k_atrous<FA, FB, false, kAtP, true>, grid, kAtThreads, sm, st, jobs, M, ta, tb);
+      launch_pdl(k_atrous<FA, FB, false, kAtP, true, APART>, grid, kAtThreads, sm, st, jobs, M, ta, tb);
     else
-      launch_pdl(k_atrous<FA, FB, false>, grid, kAtThreads, sm, st, jobs, M, ta, tb);
+      launch_pdl(k_atrous<FA, FB, false, kAtP, false, APART>, grid, kAtThreads, sm, st, jobs, M, ta, tb);
   }
   return cudaGetLastError();
 }
@@ -275,8 +287,17 @@ static cudaError_t launch_atrous_full_t(const AtrousJobs& jobs, int njobs, int m
 }
 
 #define NSST_AT_PAIRS(X) X(13, 0) X(19, 0) X(19, 13) X(9, 0) X(7, 0) X(5, 0) X(7, 9) X(7, 5) X(7, 7)
+// the analysis filters' pairs, highpass first (APART)
+#define NSST_AT_ANALYSIS(X) X(19, 13) X(7, 9) X(7, 5) X(5, 5)
 
-cudaError_t prepare_atrous_kernels(int FA, int FB, int Mmax) {
+cudaError_t prepare_atrous_kernels(int FA, int FB, int Mmax, bool apart) {
+  if (apart) {
+#define NSST_AT(a, b) \
+  if (FA == a && FB == b) return prepare_atrous_t<a, b, true>(Mmax);
+    NSST_AT_ANALYSIS(NSST_AT)
+#undef NSST_AT
+    return cudaErrorInvalidValue;
+  }
 #define NSST_AT(a, b) \
   if (FA == a && FB == b) return prepare_atrous_t<a, b>(Mmax);
   NSST_AT_PAIRS(NSST_AT)
@@ -285,9 +306,16 @@ cudaError_t prepare_atrous_kernels(int FA, int FB, int Mmax) {
 }
 
 cudaError_t launch_atrous(const AtrousJobs& jobs, int njobs, int maxH, int maxW, int M, int FA, const float* ha,
-                          int FB, const float* hb, cudaStream_t st) {
+                          int FB, const float* hb, cudaStream_t st, bool apart) {
   if (njobs == 0) return cudaSuccess;
   if (njobs > kMaxAtrousJobs) return cudaErrorInvalidValue;
+  if (apart) {
+#define NSST_AT(a, b) \
+  if (FA == a && FB == b) return launch_atrous_t<a, b, true>(jobs, njobs, maxH, maxW, M, ha, hb, st);
+    NSST_AT_ANALYSIS(NSST_AT)
+#undef NSST_AT
+    return cudaErrorInvalidValue;
+  }
 #define NSST_AT(a, b) \
   if (FA == a && FB == b) return launch_atrous_t<a, b>(jobs, njobs, maxH, maxW, M, ha, hb, st);
   NSST_AT_PAIRS(NSST_AT)

@@ -960,9 +960,12 @@ namespace {
 
 // atrousdec.m:19-51 on the device for n items: x[i] -> y(i, 0) lowpass,
 // y(i, 1..nlev) bandpass coarse -> fine; y(i, k) = ybase[i] + k * HW.
+// adjoint: with the synthesis filters.  With the half-sample symmetric extension
+// a step whose filter is symmetric in both axes is a symmetric matrix, so that is
+// the transpose of run_atrousrec (symmetric filters only).
 nsst_status run_atrousdec(nsst_plan* p, int n, const float* const* x, float* const* ybase, float* lowpass0,
-                          cudaStream_t st, int levels = 0) {
-  const int H = p->H, W = p->W, L = levels > 0 ? levels : p->nlev;
+                          cudaStream_t st, int levels = 0, bool adjoint = false) {
+  const int H = p->H, W = p->W, L = levels > 0 ? levels : p->nlev, lo_f = adjoint ? 2 : 0, hi_f = adjoint ? 3 : 1;
   const size_t HW = (size_t)H * W;
   static const char* kHi[] = {"atrous_dec_h1_M1",  "atrous_dec_h1_M2",  "atrous_dec_h1_M4",  "atrous_dec_h1_M8",
                               "atrous_dec_h1_M16", "atrous_dec_h1_M32", "atrous_dec_h1_M64", "atrous_dec_h1_M128"};
@@ -978,7 +981,7 @@ nsst_status run_atrousdec(nsst_plan* p, int n, const float* const* x, float* con
         const float* cur = (i == 0) ? x[it] : p->tmp + it * p->s_tmp + (size_t)((i - 1) & 1) * HW;
         jh.j[t] = AtrousJob{cur, nullptr, ybase[it] + (size_t)(L - i) * HW, H, W};
       }
-      cudaError_t e = launch_atrous(jh, cn, H, W, M, p->pf.F[1], p->hflip[1].data(), 0, nullptr, st);
+      cudaError_t e = launch_atrous(jh, cn, H, W, M, p->pf.F[hi_f], p->hflip[hi_f].data(), 0, nullptr, st);
       if (e != cudaSuccess) return cuda_fail(e, "atrous analysis launch");
     }
     timer_mark(p, kHi[i], st);
@@ -992,7 +995,7 @@ nsst_status run_atrousdec(nsst_plan* p, int n, const float* const* x, float* con
                                  : p->tmp + it * p->s_tmp + (size_t)(i & 1) * HW;
         jl.j[t] = AtrousJob{cur, nullptr, lo, H, W};
       }
-      cudaError_t e = launch_atrous(jl, cn, H, W, M, p->pf.F[0], p->hflip[0].data(), 0, nullptr, st);
+      cudaError_t e = launch_atrous(jl, cn, H, W, M, p->pf.F[lo_f], p->hflip[lo_f].data(), 0, nullptr, st);
       if (e != cudaSuccess) return cuda_fail(e, "atrous analysis launch");
     }
     timer_mark(p, kLo[i], st);
@@ -1001,9 +1004,10 @@ nsst_status run_atrousdec(nsst_plan* p, int n, const float* const* x, float* con
 }
 
 // atrousrec.m:18-41 on the device for n items: y(i, k) = ybase[i] + k*HW,
-// except that low[i] (if given) replaces y(i, 0).
+// except that low[i] (if given) replaces y(i, 0).  adjoint: with the analysis
+// filters, the transpose of run_atrousdec (symmetric filters only).
 nsst_status run_atrousrec(nsst_plan* p, int n, const float* const* ybase, const float* const* low, float* const* out,
-                          cudaStream_t st, int levels = 0) {
+                          cudaStream_t st, int levels = 0, bool adjoint = false) {
   const int H = p->H, W = p->W, L = levels > 0 ? levels : p->nlev;
   const size_t HW = (size_t)H * W;
   static const char* kRec[] = {"atrous_rec_M1",  "atrous_rec_M2",  "atrous_rec_M4",  "atrous_rec_M8",
@@ -1018,10 +1022,13 @@ nsst_status run_atrousrec(nsst_plan* p, int n, const float* const* ybase, const 
         const float* cur = (i == L - 1) ? (low && low[it] ? low[it] : ybase[it])
                                         : p->tmp + it * p->s_tmp + (size_t)((i + 1) & 1) * HW;
         float* dst = (i == 0) ? out[it] : p->tmp + it * p->s_tmp + (size_t)(i & 1) * HW;
-        j.j[t] = AtrousJob{cur, ybase[it] + (size_t)(L - i) * HW, dst, H, W};
+        const float* band = ybase[it] + (size_t)(L - i) * HW;
+        // the analysis pair's compiled order is highpass first
+        j.j[t] = adjoint ? AtrousJob{band, cur, dst, H, W} : AtrousJob{cur, band, dst, H, W};
       }
+      const int a = adjoint ? 1 : 2, b = adjoint ? 0 : 3;
       cudaError_t e =
-          launch_atrous(j, cn, H, W, M, p->pf.F[2], p->hflip[2].data(), p->pf.F[3], p->hflip[3].data(), st);
+          launch_atrous(j, cn, H, W, M, p->pf.F[a], p->hflip[a].data(), p->pf.F[b], p->hflip[b].data(), st, adjoint);
       if (e != cudaSuccess) return cuda_fail(e, "atrous synthesis launch");
     }
     timer_mark(p, kRec[i], st);
@@ -1217,10 +1224,9 @@ nsst_status enqueue_dct_cols_out(nsst_plan* p, int n, const float* const* src, f
 // Spectral analysis front of n items: X = DCT2(x) in pyr plane 0 (through
 // plane 1), then every level's spectrum (p->lev) from X .* R_l.
 // skip_cols_levels: the directional stage's level analysis finishes the
-// level spectra's columns (analysis_takes_dct).  resp: the level responses,
-// R_l, or, for the adjoint of the synthesis, Q_l.
+// level spectra's columns (analysis_takes_dct).
 nsst_status enqueue_dct_analysis(nsst_plan* p, int n, const float* const* x, cudaStream_t st,
-                                 bool skip_cols_levels = false, const float* resp = nullptr) {
+                                 bool skip_cols_levels = false) {
   char* A = p->arena;
   const int B = p->B, H = p->H, W = p->W;
   const size_t HW = (size_t)H * W;
@@ -1230,8 +1236,8 @@ nsst_status enqueue_dct_analysis(nsst_plan* p, int n, const float* const* x, cud
   timer_mark(p, "dct_rows_image", st);
   NSST_CUDA(launch_dct_cols(kDct2, p->j_dct_x, B, n, H, W, A, A, p->twH, p->wdH, st));
   timer_mark(p, "dct_cols_image", st);
-  NSST_CUDA(launch_dct_rows_ana(p->j_dct_ana, B * p->nlev, n, H, W, A, A, resp ? resp : p->dct_ra, HW, p->twWh,
-                                p->twW, p->twDW, false, st));
+  NSST_CUDA(launch_dct_rows_ana(p->j_dct_ana, B * p->nlev, n, H, W, A, A, p->dct_ra, HW, p->twWh, p->twW, p->twDW,
+                                false, st));
   timer_mark(p, "dct_rows_levels", st);
   if (!skip_cols_levels) {
     NSST_CUDA(launch_dct_cols(kDctAna, p->j_cols_lev, B * p->nlev, n, H, W, A, A, p->twH, p->wdH, st));
@@ -1241,13 +1247,11 @@ nsst_status enqueue_dct_analysis(nsst_plan* p, int n, const float* const* x, cud
 }
 
 // The lowpass band y0 = IDCT2(X .* R_low) of n items as rows DCT-III'd into
-// tmp plane 0 (its columns still in the DCT domain).  synthesis: G_low in
-// R_low's place, the plane after it.
-nsst_status enqueue_dct_lowpass_rows(nsst_plan* p, int n, cudaStream_t st, bool synthesis = false) {
+// tmp plane 0 (its columns still in the DCT domain).
+nsst_status enqueue_dct_lowpass_rows(nsst_plan* p, int n, cudaStream_t st) {
   char* A = p->arena;
-  const size_t HW = (size_t)p->H * p->W;
-  NSST_CUDA(launch_dct_rows_ana(p->j_dct_low, p->B, n, p->H, p->W, A, A, p->dct_ra + (synthesis ? HW : 0), HW,
-                                p->twWh, p->twW, p->twDW, true, st));
+  NSST_CUDA(launch_dct_rows_ana(p->j_dct_low, p->B, n, p->H, p->W, A, A, p->dct_ra, (size_t)p->H * p->W, p->twWh,
+                                p->twW, p->twDW, true, st));
   return NSST_OK;
 }
 
@@ -1256,10 +1260,8 @@ nsst_status enqueue_dct_lowpass_rows(nsst_plan* p, int n, cudaStream_t st, bool 
 // .* Q_l summed over the levels with low .* lowtab (low: a DCT-domain plane
 // per item at lowbase + i * lowstride), DCT-III (pyr plane 1), and DCT-III down
 // the columns into out[i].
-// resp: the level responses, Q_l, or, for the adjoint of the analysis, R_l.
 nsst_status enqueue_dct_synthesis(nsst_plan* p, int n, const float* lowbase, size_t lowstride, const float* lowtab,
-                                  float* const* out, cudaStream_t st, bool sums_dct2 = false,
-                                  const float* resp = nullptr) {
+                                  float* const* out, cudaStream_t st, bool sums_dct2 = false) {
   char* A = p->arena;
   const int B = p->B, H = p->H, W = p->W;
   const size_t HW = (size_t)H * W;
@@ -1268,7 +1270,7 @@ nsst_status enqueue_dct_synthesis(nsst_plan* p, int n, const float* lowbase, siz
     timer_mark(p, "dct_cols_sums", st);
   }
   NSST_CUDA(launch_dct_rows_syn(p->j_dct_syn, B, n, p->nlev, (size_t)H * p->WH, H, W, A, A, lowbase, lowstride,
-                                resp ? resp : p->dct_rs, HW, lowtab, p->twWh, p->twW, p->twDW, st));
+                                p->dct_rs, HW, lowtab, p->twWh, p->twW, p->twDW, st));
   timer_mark(p, "dct_rows_synthesis", st);
   std::vector<const float*> p1(n);
   for (int i = 0; i < n; i++) p1[i] = p->pyr + (size_t)i * p->s_pyr + HW;
@@ -1405,8 +1407,12 @@ nsst_status enqueue_band_maxima(nsst_plan* p, int n, const float* const* x, unsi
 }
 
 // shear_trans of one image into nbands caller planes; the plan must be locked.
-// adjoint: with the synthesis pyramid's responses, which is the adjoint of
-// inverse_shear (spectral pyramid only: tau_backward_dct has the reason).
+// adjoint: with the synthesis filters, which is the adjoint of inverse_shear
+// (symmetric filters only), by the direct pyramid: its error is that of the
+// convolutions alone (at most 3.1e-7 over sizes and filter sets; in the DCT domain
+// 4.3e-7), and a pixel that is not finite leaves the rest of the lowpass coefficients
+// alone.  Both adjoints at 512^2: 287 us, in the DCT domain 192, by transposed
+// convolutions and folds 528.
 nsst_status enqueue_shear_trans(nsst_plan* p, const float* x, float* coeffs, cudaStream_t st, bool adjoint = false) {
   char* A = p->arena;
   float2* A2 = (float2*)A;
@@ -1414,18 +1420,22 @@ nsst_status enqueue_shear_trans(nsst_plan* p, const float* x, float* coeffs, cud
   const DirChoice c = split_choice(p, 1);
   const bool tma = c.cols_tma && p->cols_tma_ok;
   bool ana_dct = false;
-  if (p->dct_on && aligned16(x)) {
+  if (p->dct_on && aligned16(x) && !adjoint) {
     // spectral pyramid: the level spectra from X = DCT2(x); the lowpass
     // IDCT2(X .* R_low) straight to coefficient plane 0
     ana_dct = analysis_takes_dct(p, 1);
-    NSST_TRY(enqueue_dct_analysis(p, 1, &x, st, ana_dct, adjoint ? p->dct_rs : p->dct_ra));
-    NSST_TRY(enqueue_dct_lowpass_rows(p, 1, st, adjoint));
+    NSST_TRY(enqueue_dct_analysis(p, 1, &x, st, ana_dct));
+    NSST_TRY(enqueue_dct_lowpass_rows(p, 1, st));
     const float* t0 = p->tmp;
     NSST_TRY(enqueue_dct_cols_out(p, 1, &t0, &coeffs, st));
     timer_mark(p, "dct_lowpass", st);
   } else {
-    // the lowpass goes straight to coefficient plane 0
-    NSST_TRY(run_atrousdec(p, 1, &x, &yb, coeffs, st));
+    // the lowpass goes straight to coefficient plane 0, but for the adjoint's single
+    // level: that launch reads x, which may overlap the plane
+    const bool through = adjoint && p->nlev == 1;
+    NSST_TRY(run_atrousdec(p, 1, &x, &yb, through ? nullptr : coeffs, st, 0, adjoint));
+    if (through)
+      NSST_CUDA(cudaMemcpyAsync(coeffs, yb, (size_t)p->H * p->W * sizeof(float), cudaMemcpyDeviceToDevice, st));
     NSST_CUDA(launch_rows(RowOp::Fwd, p->j_rows_lev_fwd, p->nlev, 1, p->H, p->W, A, A, p->twWh, p->twW, nullptr, 0,
                           st));
     NSST_CUDA(launch_cols(ColOp::Fwd, p->j_cols_lev, p->nlev, 1, p->H, p->W, A2, A2, nullptr, 0, p->twH, st));
@@ -1439,15 +1449,14 @@ nsst_status enqueue_shear_trans(nsst_plan* p, const float* x, float* coeffs, cud
   return NSST_OK;
 }
 
-// inverse_shear of nbands caller planes; the plan must be locked.  adjoint:
-// with the analysis pyramid's responses, the adjoint of shear_trans (spectral
-// pyramid only).
+// inverse_shear of nbands caller planes; the plan must be locked.  adjoint: with
+// the analysis filters, the adjoint of shear_trans, as in enqueue_shear_trans.
 nsst_status enqueue_inverse_shear(nsst_plan* p, const float* coeffs, float* x, cudaStream_t st, bool adjoint = false) {
   char* A = p->arena;
   NSST_CUDA(launch_rows(RowOp::Fwd, p->j_coeff_fwd, p->ndir_total, 1, p->H, p->W, coeffs, A, p->twWh, p->twW,
                         nullptr, 0, st));
   timer_mark(p, "band_rows_fwd", st);
-  const bool spectral = p->dct_on && aligned16(x);
+  const bool spectral = p->dct_on && aligned16(x) && !adjoint;
   bool sums_dct2 = false;
   NSST_TRY(enqueue_band_synthesis(p, 1, split_choice(p, 1), st, spectral ? &sums_dct2 : nullptr));
   if (spectral) {
@@ -1457,14 +1466,17 @@ nsst_status enqueue_inverse_shear(nsst_plan* p, const float* coeffs, float* x, c
     NSST_TRY(enqueue_dct_rows_io(p, 1, &coeffs, &t0, st));
     NSST_CUDA(launch_dct_cols(kDct2, p->j_dct_lowc, p->B, 1, p->H, p->W, A, A, p->twH, p->wdH, st));
     timer_mark(p, "dct_lowpass", st);
-    const float* low = adjoint ? p->dct_ra + (size_t)p->dct_rl_plane * p->H * p->W : p->dct_gl;
-    return enqueue_dct_synthesis(p, 1, p->tmp, p->s_tmp, low, &x, st, sums_dct2, adjoint ? p->dct_ra : p->dct_rs);
+    return enqueue_dct_synthesis(p, 1, p->tmp, p->s_tmp, p->dct_gl, &x, st, sums_dct2);
   }
   NSST_CUDA(launch_rows(RowOp::Inv, p->j_rows_lev_inv, p->nlev, 1, p->H, p->W, A, A, p->twWh, p->twW, nullptr, 0,
                         st));
   timer_mark(p, "fft_rows_inv", st);
-  const float* yr = p->rec;
-  return run_atrousrec(p, 1, &yr, &coeffs, &x, st);
+  const float *yr = p->rec, *low = coeffs;
+  if (adjoint && p->nlev == 1) {  // the one launch reads the lowpass, which x may overlap
+    NSST_CUDA(cudaMemcpyAsync(p->tmp, low, (size_t)p->H * p->W * sizeof(float), cudaMemcpyDeviceToDevice, st));
+    low = p->tmp;
+  }
+  return run_atrousrec(p, 1, &yr, &low, &x, st, 0, adjoint);
 }
 
 }  // namespace
@@ -2416,6 +2428,10 @@ nsst_status nsst_plan_enable_grad(nsst_plan* p) {
                       make_tmap_2d(p->gcols_tmap, G, p->WH, rows, col_tile(H), tma_box_rows(H)) == cudaSuccess;
     if (!p->gcols_tma_ok) (void)cudaGetLastError();  // the cp.async column kernels stay
   }
+  if (p->dct_on) {  // the adjoint of the analysis: the synthesis kernel with the analysis filters
+    ce = prepare_atrous_kernels(p->pf.F[1], p->pf.F[0], Mmax, true);
+    if (ce != cudaSuccess) return cuda_fail(ce, "adjoint kernel set-up");
+  }
   for (int F : {p->pf.F[0], p->pf.F[1], p->pf.F[2], p->pf.F[3]}) {
     ce = prepare_atrous_kernels(F, 0, Mmax);
     if (ce != cudaSuccess) return cuda_fail(ce, "adjoint kernel set-up");
@@ -2433,8 +2449,8 @@ nsst_status nsst_shear_trans_adjoint(nsst_plan* p, const float* coeffs, float* x
   p->saved_n = 0;  // the arena no longer holds the last differentiable forward
   cudaStream_t st = (cudaStream_t)stream;
   timer_begin(p, st);
-  // spectral pyramid: every pyramid operator is symmetric, so the adjoint of
-  // the analysis is the synthesis with the analysis responses
+  // symmetric filters: every step of the pyramid is a symmetric matrix, so the
+  // adjoint of the analysis is the synthesis with the analysis filters
   if (p->dct_on && aligned16(x)) return enqueue_inverse_shear(p, coeffs, x, st, true);
   char* G = p->garena;
   float2* G2 = (float2*)G;
