@@ -373,7 +373,7 @@ def volume_bench(sc, torch, dev, stream, flush, rank, reps=3, sizes=(128, 192), 
             fwd()
             sc.denoise3_backward(gy, p, out=gx)
 
-        res = {'grid': p.grid[0], 'conv_lengths': [c[0] for c in p.conv_dims[:3]],
+        res = {'grid': p.grid[0], 'conv_lengths_2a3b': [c[0] for c in p.conv_dims[:3]],  # the transforms run at a shorter one
                'device_bytes': p.device_bytes()}
         c0 = sc.launch_count()
         fwd()
@@ -702,7 +702,7 @@ def run_gpu(args):
         line['plain_images_per_s'] = plain
         line['batched_vs_plain'] = value / world / plain
 
-        # ---- uneven batch of 64 (sizes from the batched config), one captured graph
+        # ---- uneven batch of 64 (sizes from the batched config), replayed as one graph
         items = uneven_batch(BATCH, seed=3, sizes=BATCH_SIZES)
         counts = {}
         for _, nz, _ in items:

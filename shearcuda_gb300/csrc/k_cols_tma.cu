@@ -185,8 +185,8 @@ __global__ void __launch_bounds__(AnaCfg<H>::T, AnaCfg<H>::MINB)
 // the sums spill: 64 x 512^2 took 4201 us with three CTAs, 4168 with two, 4305
 // before.  12 x 1024^2: 3984 us -> 3845; 2048^2: 1815 -> 1767.  At 256 rows
 // 128 threads x 5 CTAs (64 x 256^2: 1210 us -> 1088; x 4 1090, x 6 1097).
-// The lengths with a factor 3 lose by it (16 x 768 x 1024: 3959 us -> 4119,
-// 16 x 384 x 512: 932 -> 974), so they keep the plane.
+// The lengths with a factor 3 lose by it (16 x 768 x 1024: 3955 us -> 4127,
+// 16 x 384 x 512: 915 -> 954, 32 x 384^2: 1531 -> 1574), so they keep the plane.
 template <int H>
 struct AnaRegs {
   using C = AnaCfg<H>;

@@ -37,11 +37,12 @@ __device__ __forceinline__ float soft(float v, float t) {
 // part of the row.
 // Taps are applied in ascending order whatever the form.  Two results that take
 // the same taps or the same sample share packed FP32 FMAs, which round as two
-// single ones.  Bound by latency and issue (40 % of it at 32 images of 256 x 256,
-// 6 to 15 % of HBM: the planes stay in L2): 64 registers, so that four CTAs share
-// an SM, took the four Symmlet-4 levels there from 93 to 66 us (analysis) and 105
-// to 78 us (synthesis); six CTAs (spills) 87 and 84.  Separate column and row
-// kernels measured 133 and 150 us.
+// single ones.  Bound by issue (71 % of it in the analysis and 50 % in the synthesis
+// at 32 images of 256 x 256; HBM 8 and 23 %, the planes stay in L2): 64 registers, so
+// that four CTAs share an SM, took the four Symmlet-4 levels there from 93 to 66 us
+// (analysis) and 105 to 78 us (synthesis); six CTAs (spills) 87 and 84.  Separate
+// column and row kernels measured 133 and 150 us.  With dependent launches a level
+// takes 12 and 16 us.
 // Columns of a CTA: `out` of the results and `in` of what the row taps reach from
 // there, from their first column on (analysis) or up to their last (synthesis);
 // both the whole row, or in = out + (lh - 1) sf.
